@@ -221,6 +221,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   // twiddles of the L0 transform; host tables used by every prove
   tw0_ = twiddles(S.k_code);
   (void)moore_inverse();
+  if (S.slots.size() != 1 || !S.identity) jagged_ = std::make_unique<JaggedAssist>(S, device_);
   CUDA_OK(cudaDeviceSynchronize());
 }
 
@@ -796,18 +797,7 @@ uint32_t GpuBackend::launch_build_w(const std::vector<WeightClaim>& cl, uint32_t
   const F128d* dt = upload(tabs);
   if (S.slots.size() == 1 && S.identity)
     return launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_);
-  JaggedSegs g;
-  uint64_t base = 0;
-  for (const SlotInfo& T : S.slots) {
-    if (!T.count || !T.used_cols) continue;
-    if (g.n == 4) throw std::runtime_error("the merged weight supports at most four non-empty slots");
-    g.base[g.n] = base;
-    g.rows[g.n] = T.count;
-    g.cols[g.n] = T.used_cols;
-    g.col_off[g.n] = T.col_offset(S.nu);
-    base += T.count * T.used_cols;
-    g.n++;
-  }
+  const JaggedSegs g = jagged_segs(S);
   return launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_, &g);
 }
 

@@ -1,6 +1,7 @@
 // Device backend of prove_fast (one setup = one statement shape, one stream, buffers
 // allocated once and reused by every prove of that shape).
 #pragma once
+#include "assist.h"
 #include "kernels.h"
 #include "../host/prover.h"
 #include <map>
@@ -53,6 +54,11 @@ class GpuBackend : public ProverBackend {
   // Proof-of-work searches of 6 or more bits run on the device (own stream, thread-safe:
   // the forked multipoint transcript grinds concurrently with the main one).
   PowSearchFn pow_search() override;
+  // A statement that is not one full-height slot takes the general jagged assist.
+  JaggedAssistOps* jagged_assist() override { return jagged_.get(); }
+  // Spin until the mapped flag holds seq (bounded: an error after 20 s, stream errors
+  // reported as they occur).
+  static void wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream);
   // Device-time breakdown of a prove (CUDA events on the backend's stream).
   enum Stage {
     ST_WITNESS, ST_L0_FILL, ST_L0_NTT, ST_L0_MERKLE, ST_ZC_ROUND1, ST_ZC_FOLD_SKIP, ST_ZC_FOLDS, ST_LINCHECK,
@@ -209,6 +215,7 @@ class GpuBackend : public ProverBackend {
   bool pend_induced_ = false;
   uint64_t pend_n_ = 0;
   std::vector<Level> levels_;
+  std::unique_ptr<JaggedAssist> jagged_;
 
   // mapped pinned memory the message reductions publish into
   F128d* h_pub_ = nullptr;
@@ -217,9 +224,6 @@ class GpuBackend : public ProverBackend {
   uint32_t* d_flag_ = nullptr;
   uint32_t seq_ = 0;
   void wait_published(uint32_t seq);
-  // Spin until the mapped flag holds seq (bounded: an error after 20 s, stream errors
-  // reported as they occur).
-  void wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream);
   std::vector<F128> read_published(uint32_t seq, uint32_t width);
   uint32_t* pub_counter_ = nullptr;  // ticket counter of in-kernel publication (device)
   FusedPublish fused_publish() { FusedPublish p; p.out = d_pub_; p.flag = d_flag_; p.counter = pub_counter_; p.seq = ++seq_; return p; }

@@ -135,6 +135,16 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
                            const F128d* tables, uint32_t nu, uint64_t area, uint64_t n, F128d* w, F128d* part,
                            cudaStream_t s, const JaggedSegs* segs = nullptr);                          // width 2
 
+// assist.cu: the multipoint assist over a general jagged layout (union proofs). Dual values
+// out[i * n_points + j] of claim i (row points z_row[i * n ..), run weights w[i * n_runs ..)) at
+// points[j * m ..); runs: (t_c, t_next) pairs of 64-bit words.
+void launch_as_dual(const F128d* z_row, uint32_t n, const F128d* points, uint32_t m, uint32_t n_claims,
+                    uint32_t n_points, const void* runs, const F128d* w, uint32_t n_runs, F128d* out, cudaStream_t s);
+// The sumcheck's vectors abar and g (n entries, abar zero from `area` on) and its first message.
+void launch_as_build(const F128d* er0, const F128d* ec0, const F128d* er1, const F128d* ec1, const F128d* eq_lo,
+                     uint32_t lo_bits, const F128d* eq_hi, const F128d* table, uint64_t area, uint64_t n,
+                     const JaggedSegs& segs, F128d* abar, F128d* g, F128d* part, cudaStream_t s, FusedPublish pub);
+
 void launch_lg_eq_fill(const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n, F128d* out, bool add,
                        cudaStream_t s);
 // b = eq_a + eq_b for two eq splits (lo tables unscaled, hi tables carrying the scales) with

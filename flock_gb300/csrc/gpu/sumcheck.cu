@@ -9,6 +9,7 @@
 // * hi[i >> lo_bits], and kernels that sum eq-weighted terms walk chunks of 2^lo_bits
 // consecutive indices, summing lo-weighted terms and multiplying by hi once per chunk.
 #include "kernels.h"
+#include "reduce.cuh"
 #include <atomic>
 #include <mutex>
 #include <set>
@@ -16,25 +17,6 @@
 
 namespace flock {
 namespace gpu {
-
-__device__ __forceinline__ F128d block_xor(F128d v, F128d* sh) {
-  v = warp_xor(v);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  F128d r = f128_zero();
-  if (w == 0) {
-    r = l < nw ? sh[l] : f128_zero();
-    r = warp_xor(r);
-  }
-  return r;  // valid in thread 0
-}
-
-__device__ __forceinline__ F128d eq_at(const F128d* lo, uint32_t lo_bits, const F128d* hi, uint64_t i) {
-  F128d l = lo[i & ((1ull << lo_bits) - 1)];
-  return hi ? l * hi[i >> lo_bits] : l;
-}
 
 // ------------------------------------------------------------------ generic pieces
 __global__ void eq_table_kernel(const F128d* __restrict__ p, uint32_t n, F128d scale, F128d* __restrict__ out) {
@@ -595,40 +577,6 @@ uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d
   return blocks;
 }
 
-// ------------------------------------------------------------------ fused publication
-// Called by every block after thread 0 stored its `width` partials at part[block * width]:
-// the block takes a ticket; the block that takes the last one reduces all partials (the
-// other blocks' stores are visible to it after their fences and the atomic), writes the
-// message to mapped memory, then the sequence number, and resets the counter.
-__device__ void publish_if_last(const F128d* part, uint32_t width, const FusedPublish& pub, F128d* sh) {
-  __shared__ uint32_t ticket;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    ticket = atomicAdd(pub.counter, 1u);
-  }
-  __syncthreads();
-  if (ticket != gridDim.x - 1) return;
-  __threadfence();
-  for (uint32_t j = 0; j < width; ++j) {
-    F128d acc = f128_zero();
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-      const F128d* p = part + (uint64_t)b * width + j;
-      acc += f128(__ldcg(&p->lo), __ldcg(&p->hi));
-    }
-    acc = block_xor(acc, sh);
-    if (threadIdx.x == 0) {
-      volatile F128d* o = pub.out;
-      o[j].lo = acc.lo;
-      o[j].hi = acc.hi;
-    }
-  }
-  if (threadIdx.x == 0) {
-    *pub.counter = 0;
-    __threadfence_system();
-    *(volatile uint32_t*)pub.flag = pub.seq;
-  }
-}
-
 // ------------------------------------------------------------------ pair fold + message
 // Folds of at least this many pairs take their products by r from byte tables. A block's
 // table build costs about as much shared-memory traffic as 300 table products, so the
@@ -1051,29 +999,6 @@ void launch_lc_s_hat_v(const F128d* zv, const F128d* et, uint32_t n_tail, F128d*
 // W[d] = sum_c fold_one_slot(er_c[row] * ec_c[col], table_c) for d < area (row = d mod 2^nu,
 // col = d >> nu), else 0; round-0 prime over (q, W): u0 = sum q[2i] W[2i],
 // u2 = sum (q[2i] + q[2i+1]) (W[2i] + W[2i+1]).
-__device__ __forceinline__ F128d fold_slot(F128d x, const F128d* tab) {
-  F128d acc = f128_zero();
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc += tab[k * 256 + ((x.lo >> (8 * k)) & 255)];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc += tab[(8 + k) * 256 + ((x.hi >> (8 * k)) & 255)];
-  return acc;
-}
-// Jagged unrank of a union's committed stack: slot s holds dense [base, base + rows * cols),
-// column-major with `rows` (the declared count) words per column, its first column at
-// union chunk-column col_off.
-__device__ __forceinline__ bool jagged_unrank(const JaggedSegs& g, uint64_t d, uint64_t& row, uint64_t& col) {
-  for (uint32_t s = 0; s < g.n; ++s) {
-    const uint64_t end = g.base[s] + g.rows[s] * g.cols[s];
-    if (d >= g.base[s] && d < end) {
-      const uint64_t local = d - g.base[s];
-      col = g.col_off[s] + local / g.rows[s];
-      row = local % g.rows[s];
-      return true;
-    }
-  }
-  return false;
-}
 template <bool JAGGED>
 __global__ void __launch_bounds__(512, 1)
 mo_build_w_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er0, const F128d* __restrict__ ec0,

@@ -652,16 +652,33 @@ inline F128 jagged_weight_eval(const AssistStatement& a, const std::vector<F128>
   return acc;
 }
 
+// The bulk steps of prove_multipoint_jagged, for a backend that runs them elsewhere: the
+// dual values, the materialised vectors abar and g with the first message, and each fold at
+// r with the next message. Called from the assist's thread.
+class JaggedAssistOps {
+ public:
+  virtual ~JaggedAssistOps() = default;
+  // values[i][j] = jagged_weight_eval(unit[i], points[j], m); every unit has the same runs.
+  virtual void dual_values(const std::vector<AssistStatement>& unit, const std::vector<std::vector<F128>>& points,
+                           uint32_t m, std::vector<std::vector<F128>>& values) = 0;
+  // abar(d) = sum_i scale_i eq(z_row_i, row(d)) eq(z_col_i, col(d)) and g(d) = T(eq(rho, d)), T
+  // given by its 16 x 256 byte tables.
+  virtual void build(const std::vector<RsClaimPoint>& claims, const std::vector<F128>& scale,
+                     const std::vector<F128>& rho, const std::vector<F128>& table, F128& g1, F128& gi) = 0;
+  virtual void fold(F128 r, F128& g1, F128& gi) = 0;
+};
+
 // The multipoint twisted evaluation over a general jagged layout (jagged.rs:2884-3380,
 // the materialised path): dual values A_ij = sum_d a_i(d) eq(rho^(2^-j), d) from the
 // branching-program DP, then the m-round two-product sumcheck of sum_d abar(d) g(d) with
 // abar = sum_i gamma^(128 i) a_i and g = sum_j gamma^j eq(rho^(2^-j), .) both
 // materialised (g(d) is the F2-linear map x -> sum_j gamma^j x^(2^-j) of eq(rho, d)),
 // then the untwisted anchor. The same field values as prove_multipoint on an aligned layout.
+// With `ops` the bulk steps run there, otherwise on the host thread pool.
 inline MultipointTwistedProof prove_multipoint_jagged(Transcript& T, const JaggedLayout& L,
                                                       const std::vector<RsClaimPoint>& claims,
                                                       const std::vector<F128>& rho, uint32_t round_bits,
-                                                      uint32_t anchor_round_bits) {
+                                                      uint32_t anchor_round_bits, JaggedAssistOps* ops = nullptr) {
   const uint32_t n = L.n, m = L.m;
   const size_t R = claims.size();
   auto rp = rho_inverse_powers(rho);
@@ -669,7 +686,8 @@ inline MultipointTwistedProof prove_multipoint_jagged(Transcript& T, const Jagge
   std::vector<AssistStatement> unit(R);
   for (size_t i = 0; i < R; ++i) unit[i] = jagged_statement(L, claims[i].z_row, claims[i].z_col, F128::one());
   pf.values.assign(R, std::vector<F128>(128));
-  parallel_for(R * 128, [&](size_t ij) {
+  if (ops) ops->dual_values(unit, rp, m, pf.values);
+  else parallel_for(R * 128, [&](size_t ij) {
     const size_t i = ij / 128, j = ij % 128;
     pf.values[i][j] = jagged_weight_eval(unit[i], rp[j], m);
   });
@@ -682,10 +700,24 @@ inline MultipointTwistedProof prove_multipoint_jagged(Transcript& T, const Jagge
   std::vector<F128> gpow(128 * R);
   F128 p = F128::one();
   for (auto& g : gpow) { g = p; p = p * gamma; }
-  // ---- materialised abar (zero past the area) and g
-  const size_t N = size_t(1) << m;
-  std::vector<F128> abar(N), g(N);
+  // ---- materialised abar (zero past the area) and g; g's map as byte tables
+  std::vector<F128> tab;
   {
+    // images of the basis under x -> sum_j gamma^j x^(2^(128-j))
+    std::vector<F128> img(128);
+    parallel_for(128, [&](size_t b) {
+      std::vector<F128> sq(128);
+      F128 x = bit_basis((int)b);
+      for (int e = 0; e < 128; ++e) { sq[e] = x; x = x * x; }
+      F128 acc;
+      for (int j = 0; j < 128; ++j) acc += gpow[j] * sq[(128 - j) % 128];
+      img[b] = acc;
+    });
+    tab = fold_byte_table(img);
+  }
+  const size_t N = ops ? 0 : size_t(1) << m;
+  std::vector<F128> abar(N), g(N);
+  if (!ops) {
     std::vector<std::vector<F128>> er(R), ec(R);
     for (size_t i = 0; i < R; ++i) { er[i] = build_eq(claims[i].z_row); ec[i] = build_eq(claims[i].z_col); }
     const size_t ncol = L.pfx.size() - 1;
@@ -696,23 +728,6 @@ inline MultipointTwistedProof prove_multipoint_jagged(Transcript& T, const Jagge
         abar[d] = acc;
       }
     });
-    // images of the basis under x -> sum_j gamma^j x^(2^(128-j)), byte tables
-    std::vector<F128> img(128);
-    parallel_for(128, [&](size_t b) {
-      std::vector<F128> sq(128);
-      F128 x = bit_basis((int)b);
-      for (int e = 0; e < 128; ++e) { sq[e] = x; x = x * x; }
-      F128 acc;
-      for (int j = 0; j < 128; ++j) acc += gpow[j] * sq[(128 - j) % 128];
-      img[b] = acc;
-    });
-    std::vector<F128> tab(16 * 256);
-    for (int kb = 0; kb < 16; ++kb)
-      for (int v = 0; v < 256; ++v) {
-        F128 acc;
-        for (int i = 0; i < 8; ++i) if ((v >> i) & 1) acc += img[8 * kb + i];
-        tab[kb * 256 + v] = acc;
-      }
     auto e = build_eq(rho);
     parallel_for((N + 4095) / 4096, [&](size_t c) {
       for (size_t d = c * 4096; d < std::min(N, (c + 1) * 4096); ++d) g[d] = fold_one_slot(e[d], tab.data());
@@ -748,7 +763,13 @@ inline MultipointTwistedProof prove_multipoint_jagged(Transcript& T, const Jagge
   std::vector<F128> s;
   F128 g1, gi;
   size_t len = N;
-  message(len, g1, gi);
+  if (ops) {
+    std::vector<F128> scale(R);
+    for (size_t i = 0; i < R; ++i) scale[i] = gpow[128 * i];
+    ops->build(claims, scale, rho, tab, g1, gi);
+  } else {
+    message(len, g1, gi);
+  }
   for (uint32_t t = 0; t < m; ++t) {
     T.observe_f128(g1); T.observe_f128(gi);
     F128 r;
@@ -757,9 +778,13 @@ inline MultipointTwistedProof prove_multipoint_jagged(Transcript& T, const Jagge
     pf.rounds.push_back({g1, gi});
     s.push_back(r);
     if (t + 1 == m) break;
-    fold(len, r);
-    len /= 2;
-    message(len, g1, gi);
+    if (ops) {
+      ops->fold(r, g1, gi);
+    } else {
+      fold(len, r);
+      len /= 2;
+      message(len, g1, gi);
+    }
   }
   (void)n;
   // ---- anchor at the endpoint rho'' = s

@@ -112,6 +112,8 @@ class ProverBackend {
 
   // Device proof-of-work search (optional): smallest nonce with the PoW property.
   virtual PowSearchFn pow_search() { return {}; }
+  // Bulk steps of the jagged multipoint assist (optional), used from the assist's thread.
+  virtual JaggedAssistOps* jagged_assist() { return nullptr; }
 
 };
 
@@ -388,9 +390,10 @@ inline ProveResult prove_fast(const Statement& S, ProverBackend& B, const std::v
   fcl[1].z_row = wc[1].z_row; fcl[1].z_col = wc[1].z_col;
   Transcript ch_a = T.fork("flock-par-assist-v1");
   double assist_ms = 0;
-  std::thread assist([&] {
+  auto assist = std::async(std::launch::async, [&] {
     double a0 = now_ms();
-    mo.frobenius = aligned ? prove_multipoint(ch_a, J, fcl, rho, 2, 2) : prove_multipoint_jagged(ch_a, JL, fcl, rho, 2, 2);
+    mo.frobenius = aligned ? prove_multipoint(ch_a, J, fcl, rho, 2, 2)
+                           : prove_multipoint_jagged(ch_a, JL, fcl, rho, 2, 2, B.jagged_assist());
     assist_ms = now_ms() - a0;
   });
 
@@ -548,7 +551,7 @@ inline ProveResult prove_fast(const Statement& S, ProverBackend& B, const std::v
     B.lg_glue(pb3.second);
   }
   double w0 = now_ms();
-  assist.join();
+  assist.get();
   R.t.assist_wait = now_ms() - w0;
   R.t.assist = assist_ms;
   T.merge_child(ch_a);
