@@ -103,7 +103,9 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
     if (t.csc_a) b += 4 * (t.csc_a->col_ptr.size() + t.csc_a->rows_flat.size() + t.csc_b->col_ptr.size() + t.csc_b->rows_flat.size());
   }
   b += (W + W + W / 2) * 16;                // merged weight and fold buffers
-  b += W * 16 + 4 * (W / 2) * 32 + (W / 2) * 16;  // Ligerito basis, f/b ping-pong, pending
+  const uint64_t D = uint64_t(1) << S.log_dim;
+  b += lane_fold_groups(S.lanes, D) * D * 32;  // Ligerito: lane fold partials,
+  b += 4 * 2 * D * 32 + 2 * D * 16;            // f/b ping-pong, pending
   b += (uint64_t(1) << 20) * 16 + 4096 * 16 + (size_t(96) << 20) + (size_t(8) << 20);  // partials, scratch, staging
   b += n_pos * 16;                          // L0 twiddles
   // recursive levels: codeword 2^(log_cols + rate) x 2^k, tree, twiddles
@@ -184,12 +186,14 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   moAw_ = dmalloc<F128d>(W / 2, owned_, device_bytes_);
   moBq_ = dmalloc<F128d>(W / 4, owned_, device_bytes_);
   moBw_ = dmalloc<F128d>(W / 4, owned_, device_bytes_);
-  lb128_ = dmalloc<F128d>(W, owned_, device_bytes_);
+  lane_part_ = dmalloc<F256d>(lane_fold_groups(S.lanes, rows()) * rows(), owned_, device_bytes_);
   for (int k = 0; k < 2; ++k) {
-    lf_[k] = dmalloc<F256d>(W / 2, owned_, device_bytes_);
-    lb_[k] = dmalloc<F256d>(W / 2, owned_, device_bytes_);
+    lf_[k] = dmalloc<F256d>(2 * rows(), owned_, device_bytes_);
+    lb_[k] = dmalloc<F256d>(2 * rows(), owned_, device_bytes_);
   }
-  pend_ = dmalloc<F128d>(W / 2, owned_, device_bytes_);
+  pend_ = dmalloc<F128d>(2 * rows(), owned_, device_bytes_);
+  CUDA_OK(cudaHostAlloc(&h_tail_, 2 * lanes_pow2() * sizeof(F128d), cudaHostAllocMapped));
+  CUDA_OK(cudaHostGetDevicePointer(&d_tail_, h_tail_, 0));
   part_cap_ = 1u << 20;
   part_ = dmalloc<F128d>(part_cap_, owned_, device_bytes_);
   red_ = dmalloc<F128d>(4096, owned_, device_bytes_);
@@ -238,6 +242,7 @@ GpuBackend::~GpuBackend() {
   cudaFreeHost(h_pow_flag_);
   cudaFreeHost(h_pub_);
   cudaFreeHost(h_flag_);
+  cudaFreeHost(h_tail_);
   cudaStreamDestroy(pow_st_);
   cudaStreamDestroy(st_);
 }
@@ -291,7 +296,8 @@ GpuBackend::Mark::~Mark() {
 void GpuBackend::begin_prove(const void* d_inputs) {
   lg_pend_fold_.active = false;
   lg_pend_switch_ = false;
-  lg_pend_basis_ = false;
+  lane_ = LaneStage();
+  mo_lane_q_.clear();
   d_user_inputs_ = d_inputs;
   h2d_ = d2h_ = 0;
   spans_.clear();
@@ -815,98 +821,196 @@ void GpuBackend::mo_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uin
   mo_w_ = mw_;
   mo_len_ = Q_;
   mo_live_ = std::min<uint64_t>(Q_, area);
+  mo_chal_.clear();
+  mo_tail_q_.clear();
+  mo_tail_w_.clear();
+  mo_lane_q_.clear();
 }
 
 void GpuBackend::mo_round(F128 r, bool last, F128& g1, F128& gi) {
-  if (mo_len_ == 2) {
-    auto q = fetch(mo_q_, 2);
-    mo_final_ = q[0] + r * (q[1] + q[0]);
-    mo_len_ = 1;
+  mo_chal_.push_back(r);
+  if (!mo_tail_q_.empty()) {  // the lane bits, on the host
+    std::vector<F128>&q = mo_tail_q_, &w = mo_tail_w_;
+    const size_t half = q.size() / 2;
+    for (size_t i = 0; i < half; ++i) {
+      q[i] = q[2 * i] + r * (q[2 * i + 1] + q[2 * i]);
+      w[i] = w[2 * i] + r * (w[2 * i + 1] + w[2 * i]);
+    }
+    q.resize(half);
+    w.resize(half);
+    g1 = gi = F128();
+    for (size_t i = 0; i + 1 < half && !last; i += 2) {
+      g1 += q[i + 1] * w[i + 1];
+      gi += (q[i] + q[i + 1]) * (w[i] + w[i + 1]);
+    }
     return;
   }
   F128d* oq = (mo_q_ == moAq_) ? moBq_ : moAq_;
   F128d* ow = (mo_q_ == moAq_) ? moBw_ : moAw_;
   uint64_t n_pairs = mo_len_ / 4;
   const uint64_t live_pairs = std::min<uint64_t>(n_pairs, (mo_live_ + 3) / 4);
+  // one entry per lane left: written to mapped memory (one block, published with the message)
+  const bool tail = 2 * n_pairs == lanes_pow2();
+  if (tail) {
+    oq = d_tail_;
+    ow = d_tail_ + lanes_pow2();
+  }
   // chunking only sets the work split: 2^10 pairs per chunk for the table form's rounds,
   // 2^8 (one pair per thread) for the small, latency-bound ones
   uint32_t chunk_bits = std::min<uint32_t>(n_pairs >= (uint64_t(1) << 17) ? 10 : 8, ceil_log2(n_pairs));
-  FusedPublish fp;
-  if (!last) fp = fused_publish();
+  FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_MO_ROUNDS);
     launch_pair_fold(mo_q_, mo_w_, n_pairs, live_pairs, dev(r), nullptr, nullptr, chunk_bits, nullptr, oq, ow, part_,
-                     !last, st_, fp);
+                     true, st_, fp);
   }
   mo_q_ = oq;
   mo_w_ = ow;
   mo_len_ /= 2;
   mo_live_ = std::min(mo_len_, 2 * live_pairs);
-  if (!last) {
-    auto v = read_published(fp.seq, 2);
-    g1 = v[0];
-    gi = v[1];
+  auto v = read_published(fp.seq, 2);
+  g1 = v[0];
+  gi = v[1];
+  if (tail) {
+    const volatile F128d* t = h_tail_;
+    for (uint64_t i = 0; i < mo_len_; ++i) {
+      mo_tail_q_.push_back(F128(t[i].lo, t[i].hi));
+      mo_tail_w_.push_back(F128(t[mo_len_ + i].lo, t[mo_len_ + i].hi));
+    }
+    d2h_ += 2 * mo_len_ * sizeof(F128d);
+    mo_lane_q_ = mo_tail_q_;
   }
 }
 
 F128 GpuBackend::mo_q_eval() {
-  if (mo_len_ == 1) return mo_final_;
-  return fetch(mo_q_, 1)[0];
+  if (mo_tail_q_.size() != 1) throw std::runtime_error("merged open: the claim is evaluated after its last round");
+  return mo_tail_q_[0];
 }
 
 // ------------------------------------------------------------------ Ligerito
-void GpuBackend::lg_basis_eq(F128 gamma, const std::vector<F128>& rho) {
-  lg_flush_fold();
+// Lane dots h[l] = sum_p q[l D + p] eq(point[.. log_dim), p). The merged open folded q at its
+// round challenges: the lane dots at that point are its last row fold.
+std::vector<F128> GpuBackend::lane_dots(const std::vector<F128>& point) {
+  if (!mo_lane_q_.empty() && mo_chal_.size() >= S.log_dim && point.size() >= S.log_dim &&
+      std::equal(point.begin(), point.begin() + S.log_dim, mo_chal_.begin()))
+    return mo_lane_q_;
   scr_off_ = 0;
+  EqSplit e = eq_split(std::vector<F128>(point.begin(), point.begin() + S.log_dim), F128::one(),
+                       lane_dots_lo_bits(S.log_dim));
+  uint32_t nb;
+  { Mark mk(this, ST_LIGERITO); nb = launch_lg_lane_dots(q_, S.lanes, S.log_dim, e.lo, e.hi, part_, st_); }
+  std::vector<F128> h = reduce(nb, S.lanes);
+  h.resize(lanes_pow2());  // the lanes past the committed ones are zero
+  return h;
+}
+
+void GpuBackend::add_lane_term(F128 coef, const std::vector<F128>& point) {
+  LaneTerm t;
+  t.coef = coef;
+  t.row_point.assign(point.begin(), point.begin() + S.log_dim);
+  for (F128 v : build_eq(std::vector<F128>(point.begin() + S.log_dim, point.end()))) t.e.push_back(F256(v));
+  for (F128 v : (point == lane_.dot_point ? lane_.dots : lane_dots(point))) t.h.push_back(F256(v));
+  if (lane_.terms.size() == LaneTerms::MAX) throw std::runtime_error("too many basis terms");
+  lane_.terms.push_back(std::move(t));
+}
+
+void GpuBackend::lg_basis_eq(F128 gamma, const std::vector<F128>& rho) {
   if ((uint64_t(1) << rho.size()) != Q_) throw std::runtime_error("Ligerito basis size mismatch");
-  lg_pend_basis_ = true;  // filled with the first OOD eq (lg_add_eq) or alone (lg_flush_basis)
-  lg_basis_gamma_ = gamma;
-  lg_basis_rho_ = rho;
-  lg_base_ = true;
+  lg_pend_fold_.active = lg_pend_switch_ = false;
+  lane_ = LaneStage();
+  lane_.active = true;
+  lane_.w.assign(1, F256::one());
+  add_lane_term(gamma, rho);
   lg_n_ = Q_;
-  lg_live_ = std::min<uint64_t>(Q_, S.dense_words);  // q is zero from the dense words on
-  lg_cur_ = 0;
 }
 
 F128 GpuBackend::lg_eval_eq(const std::vector<F128>& zp) {
-  lg_flush_pending();  // reads q only: a held-back basis fill stays held back
-  scr_off_ = 0;
-  if (!lg_base_) throw std::runtime_error("OOD evaluation expects the committed base vector");
-  // chunks of 2^13 words (one eq_hi table each) where there are enough of them for every SM
-  EqSplit e = eq_split(zp, F128::one(), (Q_ >> 13) >= (uint64_t)sm_count() ? 13 : 10);
-  uint32_t nb;
-  // q is zero from the dense words on (the zero tail of the committed vector)
-  { Mark mk(this, ST_LIGERITO); nb = launch_lg_dot_eq(q_, 1, e.lo, e.lo_bits, e.hi, Q_, S.dense_words, part_, st_); }
-  return reduce(nb, 1)[0];
+  if (!lane_.active || lane_.bound || (uint64_t(1) << zp.size()) != Q_)
+    throw std::runtime_error("OOD evaluation expects the committed base vector");
+  lane_.dots = lane_dots(zp);
+  lane_.dot_point = zp;
+  const std::vector<F128> e = build_eq(std::vector<F128>(zp.begin() + S.log_dim, zp.end()));
+  F128 y;
+  for (size_t l = 0; l < e.size(); ++l) y += e[l] * lane_.dots[l];
+  return y;
 }
 
 void GpuBackend::lg_add_eq(F128 beta, const std::vector<F128>& zp) {
-  lg_flush_pending();
-  scr_off_ = 0;
-  if (!lg_base_) throw std::runtime_error("basis update expects the base stage");
-  EqSplit e = eq_split(zp, beta, 13);
-  if (lg_pend_basis_) {
-    // b = gamma eq(rho) + beta eq(z) in one pass
-    lg_pend_basis_ = false;
-    EqSplit eb = eq_split(lg_basis_rho_, lg_basis_gamma_, 13);
-    if (eb.lo_bits != e.lo_bits) throw std::runtime_error("basis and OOD eq splits differ");
-    Mark mk(this, ST_LIGERITO);
-    launch_lg_eq_fill2(eb.lo, eb.hi, e.lo, e.hi, e.lo_bits, Q_, lb128_, st_);
-    return;
-  }
-  { Mark mk(this, ST_LIGERITO); launch_lg_eq_fill(e.lo, e.lo_bits, e.hi, Q_, lb128_, true, st_); }
+  if (!lane_.active || lane_.bound) throw std::runtime_error("basis update expects the base stage");
+  add_lane_term(beta, zp);
 }
 
-void GpuBackend::lg_flush_basis() {
-  if (!lg_pend_basis_) return;
-  lg_pend_basis_ = false;
-  EqSplit e = eq_split(lg_basis_rho_, lg_basis_gamma_, 13);  // chunks of 2^13 entries: one eq_hi table each
-  Mark mk(this, ST_LIGERITO);
-  launch_lg_eq_fill(e.lo, e.lo_bits, e.hi, Q_, lb128_, false, st_);
+// u0 = sum_t c_t sum_j e_t[2j] h_t[2j], u2 = sum_t c_t sum_j (e_t[2j] + e_t[2j+1]) (h_t[2j] + h_t[2j+1]):
+// the message over the row pairs of lanes 2j and 2j + 1, summed over the rows.
+Msg256 GpuBackend::lane_message() const {
+  Msg256 m;
+  for (const LaneTerm& t : lane_.terms) {
+    F256 u0, u2;
+    for (size_t j = 0; j + 1 < t.e.size(); j += 2) {
+      u0 += t.e[j] * t.h[j];
+      u2 += (t.e[j] + t.e[j + 1]) * (t.h[j] + t.h[j + 1]);
+    }
+    m.u0 += u0 * t.coef;
+    m.u2 += u2 * t.coef;
+  }
+  return m;
+}
+
+void GpuBackend::lane_fold(F256 r) {
+  for (LaneTerm& t : lane_.terms)
+    for (std::vector<F256>* v : {&t.e, &t.h}) {
+      for (size_t j = 0; j < v->size() / 2; ++j) (*v)[j] = (*v)[2 * j] + r * ((*v)[2 * j + 1] + (*v)[2 * j]);
+      v->resize(v->size() / 2);
+    }
+  const size_t n = lane_.w.size();
+  lane_.w.resize(2 * n);
+  for (size_t l = 0; l < n; ++l) {
+    lane_.w[n + l] = lane_.w[l] * r;
+    lane_.w[l] = lane_.w[l] + lane_.w[n + l];
+  }
+  lane_.bound++;
+}
+
+// All lanes folded and the code switched, in two launches; the message over the switched pairs.
+Msg256 GpuBackend::lane_switch() {
+  scr_off_ = 0;
+  LaneTerms lt;
+  lt.n = (uint32_t)lane_.terms.size();
+  for (uint32_t t = 0; t < lt.n; ++t) {
+    EqSplit e = eq_split(lane_.terms[t].row_point, F128::one(), 10);
+    lt.lo[t] = e.lo;
+    lt.hi[t] = e.hi;
+    lt.lo_bits = e.lo_bits;
+    lt.coef[t] = dev(lane_.terms[t].e[0] * lane_.terms[t].coef);
+  }
+  const F256d* dw = static_cast<const F256d*>(upload(lane_.w.data(), lane_.w.size() * sizeof(F256)));
+  FusedPublish fp = fused_publish();
+  {
+    Mark mk(this, ST_LIGERITO);
+    launch_lg_lane_fold(q_, dw, S.lanes, rows(), lane_part_, st_);
+    launch_lg_lane_switch(lane_part_, lane_fold_groups(S.lanes, rows()), lt, rows(), lf_[0], lb_[0], part_, st_, fp);
+  }
+  lane_ = LaneStage();
+  lg_cur_ = 0;
+  lg_n_ = 2 * rows();
+  return message256(fp);
+}
+
+Msg256 GpuBackend::message256(const FusedPublish& fp) {
+  auto v = read_published(fp.seq, 4);
+  Msg256 m;
+  m.u0 = F256(v[0], v[1]);
+  m.u2 = F256(v[2], v[3]);
+  return m;
 }
 
 Msg256 GpuBackend::lg_message(size_t d) {
-  lg_flush_basis();  // the base message reads b
+  if (lane_.active) {
+    if (lane_.folded && d == 1) return lane_switch();
+    if (lane_.folded || lane_.bound == S.log_batch || d != rows())
+      throw std::runtime_error("the lane stage's messages pair lanes, then the switched entries");
+    return lane_message();
+  }
   if (lg_pend_switch_ && (d == 1 || 2 * lg_n_ == d)) {
     // code switch and the message over its pairs (2i, 2i + 1) in one pass
     lg_pend_switch_ = false;
@@ -914,70 +1018,37 @@ Msg256 GpuBackend::lg_message(size_t d) {
     FusedPublish fp = fused_publish();
     {
       Mark mk(this, ST_LIGERITO);
-      launch_lg_switch_msg(lf_[lg_cur_], lb_[lg_cur_], lg_n_, lg_live_, lf_[nx], lb_[nx], part_, st_, fp);
+      launch_lg_switch_msg(lf_[lg_cur_], lb_[lg_cur_], lg_n_, lf_[nx], lb_[nx], part_, st_, fp);
     }
     lg_cur_ = nx;
     lg_n_ *= 2;
-    lg_live_ = std::min(lg_n_, 2 * lg_live_);
-    auto v = read_published(fp.seq, 4);
-    Msg256 m;
-    m.u0 = F256(v[0], v[1]);
-    m.u2 = F256(v[2], v[3]);
-    return m;
+    return message256(fp);
   }
   if (lg_pend_switch_) lg_flush_fold();  // a code switch followed by a message with other pairs
   if (lg_pend_fold_.active) {
-    // fold and message in one pass (over the base vectors for the first fold)
+    // fold and message in one pass
     const uint64_t n_out = lg_n_ / 2;
     const size_t dm = (d == 1 || n_out == d) ? 1 : d;
-    const int nx = lg_pend_fold_.base ? 0 : lg_cur_ ^ 1;
+    const int nx = lg_cur_ ^ 1;
     FusedPublish fp = fused_publish();
     {
       Mark mk(this, ST_LIGERITO);
-      if (lg_pend_fold_.base)
-        launch_lg_fold_msg128(q_, lb128_, n_out, lg_live_, dev(lg_pend_fold_.r), lg_pend_fold_.d, dm, lf_[0], lb_[0],
-                              part_, st_, fp);
-      else
-        launch_lg_fold_msg256(lf_[lg_cur_], lb_[lg_cur_], n_out, lg_live_, dev(lg_pend_fold_.r), lg_pend_fold_.d, dm,
-                              lf_[nx], lb_[nx], part_, st_, fp);
+      launch_lg_fold_msg256(lf_[lg_cur_], lb_[lg_cur_], n_out, dev(lg_pend_fold_.r), lg_pend_fold_.d, dm, lf_[nx],
+                            lb_[nx], part_, st_, fp);
     }
-    if (lg_pend_fold_.base) lg_base_ = false;
     lg_pend_fold_.active = false;
     lg_cur_ = nx;
     lg_n_ = n_out;
-    lg_live_ = fold_live(lg_live_, lg_pend_fold_.d);
-    auto v = read_published(fp.seq, 4);
-    Msg256 m;
-    m.u0 = F256(v[0], v[1]);
-    m.u2 = F256(v[2], v[3]);
-    return m;
+    return message256(fp);
   }
-  uint64_t n = lg_n_;
-  if (d == 1 || n == d) d = 1;
-  Msg256 m;
-  if (lg_base_) {
-    FusedPublish fp = fused_publish();
-    { Mark mk(this, ST_LIGERITO); launch_lg_message128(q_, lb128_, n, lg_live_, d, part_, st_, fp); }
-    auto v = read_published(fp.seq, 2);
-    m.u0 = F256(v[0]);
-    m.u2 = F256(v[1]);
-  } else {
-    FusedPublish fp = fused_publish();
-    { Mark mk(this, ST_LIGERITO); launch_lg_message256(lf_[lg_cur_], lb_[lg_cur_], n, lg_live_, d, part_, st_, fp); }
-    auto v = read_published(fp.seq, 4);
-    m.u0 = F256(v[0], v[1]);
-    m.u2 = F256(v[2], v[3]);
-  }
-  return m;
+  if (d == 1 || lg_n_ == d) d = 1;
+  FusedPublish fp = fused_publish();
+  { Mark mk(this, ST_LIGERITO); launch_lg_message256(lf_[lg_cur_], lb_[lg_cur_], lg_n_, d, part_, st_, fp); }
+  return message256(fp);
 }
 
 void GpuBackend::lg_flush_fold() {
-  lg_flush_basis();
-  lg_flush_pending();
-}
-
-void GpuBackend::lg_flush_pending() {
-  if (lg_pend_fold_.active && lg_pend_fold_.base) lg_flush_basis();  // the base fold reads b
+  if (lane_.active) throw std::runtime_error("the lane stage ends with its code switch and message");
   if (lg_pend_switch_) {
     lg_pend_switch_ = false;
     const int nx = lg_cur_ ^ 1;
@@ -987,22 +1058,10 @@ void GpuBackend::lg_flush_pending() {
     }
     lg_cur_ = nx;
     lg_n_ *= 2;
-    lg_live_ = std::min(lg_n_, 2 * lg_live_);
   }
   if (!lg_pend_fold_.active) return;
   lg_pend_fold_.active = false;
   const uint64_t n_out = lg_n_ / 2;
-  if (lg_pend_fold_.base) {
-    {
-      Mark mk(this, ST_LIGERITO);
-      launch_lg_fold128(q_, lb128_, n_out, dev(lg_pend_fold_.r), nullptr, lg_pend_fold_.d, lf_[0], lb_[0], st_);
-    }
-    lg_cur_ = 0;
-    lg_base_ = false;
-    lg_n_ = n_out;
-    lg_live_ = fold_live(lg_live_, lg_pend_fold_.d);
-    return;
-  }
   const int nx = lg_cur_ ^ 1;
   {
     Mark mk(this, ST_LIGERITO);
@@ -1011,22 +1070,29 @@ void GpuBackend::lg_flush_pending() {
   }
   lg_cur_ = nx;
   lg_n_ = n_out;
-  lg_live_ = fold_live(lg_live_, lg_pend_fold_.d);
 }
 
 void GpuBackend::lg_fold(F256 r, size_t d) {
+  if (lane_.active) {
+    if (lane_.bound == S.log_batch || d != rows()) throw std::runtime_error("the lane stage folds lane pairs");
+    lane_fold(r);
+    return;
+  }
   lg_flush_fold();
   // held back: the next message runs fused with it, any other call performs it first
   lg_pend_fold_.active = true;
-  lg_pend_fold_.base = lg_base_;
   lg_pend_fold_.r = r;
   lg_pend_fold_.d = d;
 }
 
 void GpuBackend::lg_code_switch() {
+  if (lane_.active) {
+    if (lane_.bound != S.log_batch) throw std::runtime_error("code switch before the last lane fold");
+    lane_.folded = true;
+    return;
+  }
   lg_flush_fold();
-  if (lg_base_) throw std::runtime_error("code switch before the first fold");
-  if (2 * lg_n_ > W_ / 2) throw std::runtime_error("code switch exceeds the Ligerito buffers");
+  if (2 * lg_n_ > 2 * rows()) throw std::runtime_error("code switch exceeds the Ligerito buffers");
   lg_pend_switch_ = true;  // performed by the next message, or by lg_flush_fold
 }
 

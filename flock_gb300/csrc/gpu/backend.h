@@ -177,18 +177,46 @@ class GpuBackend : public ProverBackend {
   const F128d* mo_w_ = nullptr;
   uint64_t mo_len_ = 0;
   uint64_t mo_live_ = 0;  // entries of q and W that can be nonzero (both are zero from the area on)
-  F128 mo_final_;
 
-  F128d* lb128_ = nullptr;
+  // The tail of the merged open: the fold that leaves one entry per lane writes q and W to
+  // mapped memory, and the last rounds (over the lane bits) run on the host.
+  F128d *h_tail_ = nullptr, *d_tail_ = nullptr;
+  std::vector<F128> mo_tail_q_, mo_tail_w_;  // current tail vectors (empty before the tail)
+  std::vector<F128> mo_chal_;                // the round challenges so far
+  std::vector<F128> mo_lane_q_;              // q folded at the row challenges: the lane dots at that point
+  uint64_t lanes_pow2() const { return uint64_t(1) << S.log_batch; }
+  uint64_t rows() const { return uint64_t(1) << S.log_dim; }
+
+  // Ligerito's lane stage (the first log_batch folds): the basis as terms coef eq(point), each
+  // with its lane eq table e and its lane dots h, both folded at the challenges so far; w the
+  // lane weights of f in the challenges so far.
+  struct LaneTerm {
+    F128 coef;
+    std::vector<F128> row_point;
+    std::vector<F256> e, h;
+  };
+  struct LaneStage {
+    bool active = false, folded = false;  // folded: the code switch after the last lane fold was asked for
+    uint32_t bound = 0;
+    std::vector<LaneTerm> terms;
+    std::vector<F256> w;
+    std::vector<F128> dot_point, dots;    // the last evaluation point and its lane dots
+  };
+  LaneStage lane_;
+  std::vector<F128> lane_dots(const std::vector<F128>& point);
+  void add_lane_term(F128 coef, const std::vector<F128>& point);
+  Msg256 lane_message() const;
+  void lane_fold(F256 r);
+  Msg256 lane_switch();
+  Msg256 message256(const FusedPublish& fp);  // the published message (u0, u2)
+  F256d* lane_part_ = nullptr;
   F256d* lf_[2] = {nullptr, nullptr};
   F256d* lb_[2] = {nullptr, nullptr};
   int lg_cur_ = 0;
-  bool lg_base_ = true;
   // An F256 fold is held back until the next call: a message over the folded vectors then
   // runs fused with it (one pass); any other call first performs it on its own.
   struct PendingFold {
     bool active = false;
-    bool base = false;  // the first fold: of the base vectors q_ and lb128_ into lf_[0], lb_[0]
     F256 r;
     size_t d = 0;
   };
@@ -196,21 +224,8 @@ class GpuBackend : public ProverBackend {
   // A code switch is held back the same way: the next message (pairs one apart) runs fused
   // with it; any other call first performs it on its own (lg_flush_fold does both).
   bool lg_pend_switch_ = false;
-  // The basis eq fill is held back too: the first OOD sample's eq is added in the same pass
-  // over b (launch_lg_eq_fill2); any other use of b performs it alone first.
-  bool lg_pend_basis_ = false;
-  F128 lg_basis_gamma_;
-  std::vector<F128> lg_basis_rho_;
-  void lg_flush_basis();
-  void lg_flush_pending();  // the held-back code switch and fold
-  void lg_flush_fold();     // lg_flush_basis, then lg_flush_pending
+  void lg_flush_fold();
   uint64_t lg_n_ = 0;
-  // f (the folded committed vector) is zero from entry lg_live_ on: the committed vector's
-  // zero tail, halved through the folds, doubled by the code switch
-  uint64_t lg_live_ = 0;
-  static uint64_t fold_live(uint64_t live, uint64_t d) {  // output i is live when f[pair_lo(i, d)] may be nonzero
-    return (live / (2 * d)) * d + std::min<uint64_t>(d, live % (2 * d));
-  }
   F128d* pend_ = nullptr;
   bool pend_induced_ = false;
   uint64_t pend_n_ = 0;

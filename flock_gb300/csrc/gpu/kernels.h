@@ -135,7 +135,7 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
                            const F128d* tables, uint32_t nu, uint64_t area, uint64_t n, F128d* w, F128d* part,
                            cudaStream_t s, const JaggedSegs* segs = nullptr);                          // width 2
 
-// assist.cu: the multipoint assist over a general jagged layout (union proofs). Dual values
+// rounds.cu: the multipoint assist over a general jagged layout (union proofs). Dual values
 // out[i * n_points + j] of claim i (row points z_row[i * n ..), run weights w[i * n_runs ..)) at
 // points[j * m ..); runs: (t_c, t_next) pairs of 64-bit words.
 void launch_as_dual(const F128d* z_row, uint32_t n, const F128d* points, uint32_t m, uint32_t n_claims,
@@ -145,37 +145,36 @@ void launch_as_build(const F128d* er0, const F128d* ec0, const F128d* er1, const
                      uint32_t lo_bits, const F128d* eq_hi, const F128d* table, uint64_t area, uint64_t n,
                      const JaggedSegs& segs, F128d* abar, F128d* g, F128d* part, cudaStream_t s, FusedPublish pub);
 
-void launch_lg_eq_fill(const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n, F128d* out, bool add,
-                       cudaStream_t s);
-// b = eq_a + eq_b for two eq splits (lo tables unscaled, hi tables carrying the scales) with
-// the same lo_bits, in one pass.
-void launch_lg_eq_fill2(const F128d* lo_a, const F128d* hi_a, const F128d* lo_b, const F128d* hi_b, uint32_t lo_bits,
-                        uint64_t n, F128d* out, cudaStream_t s);
-uint32_t launch_lg_dot_eq(const F128d* f, uint32_t stride, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi,
-                          uint64_t n, uint64_t live, F128d* part, cudaStream_t s);  // f zero from `live` on                                    // width 1
-// f_live: f is zero from that entry on (pairs wholly past it add nothing and are skipped).
-uint32_t launch_lg_message128(const F128d* f, const F128d* b, uint64_t n, uint64_t f_live, uint64_t d, F128d* part,
-                              cudaStream_t s, FusedPublish pub = FusedPublish());
-uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64_t f_live, uint64_t d, F128d* part,
-                              cudaStream_t s, FusedPublish pub = FusedPublish());
-void launch_lg_fold128(const F128d* f, const F128d* b, uint64_t n_out, F256d r, const F256d* r_dev, uint64_t d,
-                       F256d* fo, F256d* bo, cudaStream_t s);
-// The first fold (of the base vectors into F256 vectors) fused with the next message,
-// like launch_lg_fold_msg256.
-// f_live: the input f is zero from that entry on; message pairs whose inputs all lie past
-// it fold only b (their f outputs are written as zero) and add nothing to the message.
-uint32_t launch_lg_fold_msg128(const F128d* f, const F128d* b, uint64_t n_out, uint64_t f_live, F256d r, uint64_t d_fold,
-                               uint64_t d_msg, F256d* fo, F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub);
-uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, uint64_t f_live, F256d r, uint64_t d_fold,
-                               uint64_t d_msg, F256d* fo, F256d* bo, F128d* part, cudaStream_t s,
+// The lane stage (see the kernels): lane dots h[l] = sum_p q[l 2^log_d + p] eq(p) as `splits`
+// partial rows of width `lanes` (returned; eq split with lane_dots_lo_bits(log_d) low bits),
+// the fold of every lane by lambda into lane_fold_groups(lanes, D) partial rows of D entries,
+// and the switched vectors with their message.
+uint32_t lane_dots_lo_bits(uint32_t log_d);
+uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, const F128d* eq_hi,
+                             F128d* part, cudaStream_t s);
+uint32_t lane_fold_groups(uint32_t lanes, uint64_t D);
+void launch_lg_lane_fold(const F128d* q, const F256d* lambda, uint32_t lanes, uint64_t D, F256d* part, cudaStream_t s);
+// b = sum of n terms coef eq(point), each point's eq as lo (lo_bits) x hi tables.
+struct LaneTerms {
+  static constexpr uint32_t MAX = 4;
+  uint32_t n = 0, lo_bits = 0;
+  const F128d *lo[MAX] = {}, *hi[MAX] = {};
+  F256d coef[MAX] = {};
+};
+uint32_t launch_lg_lane_switch(const F256d* fpart, uint32_t groups, const LaneTerms& terms, uint64_t D, F256d* fo,
+                               F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub);  // width 4
+uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64_t d, F128d* part, cudaStream_t s,
+                              FusedPublish pub = FusedPublish());
+uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, uint64_t d_fold, uint64_t d_msg,
+                               F256d* fo, F256d* bo, F128d* part, cudaStream_t s,
                                FusedPublish pub = FusedPublish());                                  // width 4
 void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, const F256d* r_dev, uint64_t d,
                        F256d* fo, F256d* bo, cudaStream_t s);
 void launch_lg_code_switch(const F256d* f, const F256d* b, uint64_t n, F256d* fo, F256d* bo, cudaStream_t s);
 // The code switch and the round message over the switched vectors with pairs one apart,
 // in one pass; published like launch_lg_message256 (four words).
-uint32_t launch_lg_switch_msg(const F256d* f, const F256d* b, uint64_t n, uint64_t f_live, F256d* fo, F256d* bo,
-                              F128d* part, cudaStream_t s, FusedPublish pub);
+uint32_t launch_lg_switch_msg(const F256d* f, const F256d* b, uint64_t n, F256d* fo, F256d* bo, F128d* part, cudaStream_t s,
+                              FusedPublish pub);
 void launch_lg_replicate(const F256d* f, uint64_t msg, uint64_t total, F128d* mat, cudaStream_t s);
 uint32_t launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n,
                             F128d* pend, F128d* part, cudaStream_t s,

@@ -10,6 +10,7 @@
 // consecutive indices, summing lo-weighted terms and multiplying by hi once per chunk.
 #include "kernels.h"
 #include "reduce.cuh"
+#include "wintable.cuh"
 #include <atomic>
 #include <mutex>
 #include <set>
@@ -1117,174 +1118,148 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
 }
 
 // ------------------------------------------------------------------ Ligerito
-// b[i] = eq(i) (the hi table carries the scale).
-__global__ void lg_eq_fill_kernel(const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi,
-                                  uint64_t n, F128d* __restrict__ out, int add) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  F128d e = eq_at(eq_lo, lo_bits, eq_hi, i);
-  if (add) out[i] += e;
-  else out[i] = e;
-}
-// The same fill one chunk (2^lo_bits entries sharing eq_hi[chunk]) per block iteration:
-// the first half of a chunk takes its products by eq_hi[chunk] from the chunk's byte
-// tables, the second half from its split form; each thread forms one of each per
-// iteration, so the load/store and multiply pipes share the products.
-__global__ void __launch_bounds__(256, 2)
-lg_eq_fill_tbl_kernel(const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi, uint64_t n,
-                      F128d* __restrict__ out, int add) {
-  extern __shared__ __align__(16) F128d htab[];  // build_byte_table's BYTE_TABLE_SMEM_ENTRIES
-  __shared__ F128split hs;
-  const uint64_t chunk = 1ull << lo_bits, n_chunks = n >> lo_bits;
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    __syncthreads();  // the previous chunk's table and split are no longer read
-    const F128d h = eq_hi[ch];
-    if (threadIdx.x == 0) hs = split_factor(h);
-    build_byte_table(h, htab);
-    F128d* o = out + ch * chunk;
-    const uint64_t half = chunk / 2;
-    for (uint64_t i = threadIdx.x; i < half; i += blockDim.x) {
-      const F128d e0 = mul_table(eq_lo[i], htab);
-      const F128d e1 = mul_split(eq_lo[half + i], hs);
-      if (add) {
-        o[i] += e0;
-        o[half + i] += e1;
-      } else {
-        o[i] = e0;
-        o[half + i] = e1;
-      }
-    }
-  }
-}
-// b[i] = eq_a(i) + eq_b(i) for two eq splits with the same lo_bits (the basis eq and the
-// first OOD eq in one pass over b): per chunk, the products by eq_hi_a[chunk] from its byte
-// tables and those by eq_hi_b[chunk] from its split form, one of each per entry.
-__global__ void __launch_bounds__(256, 2)
-lg_eq_fill2_tbl_kernel(const F128d* __restrict__ lo_a, const F128d* __restrict__ hi_a, const F128d* __restrict__ lo_b,
-                       const F128d* __restrict__ hi_b, uint32_t lo_bits, uint64_t n, F128d* __restrict__ out) {
-  extern __shared__ __align__(16) F128d htab[];  // build_byte_table's BYTE_TABLE_SMEM_ENTRIES
-  __shared__ F128split hs;
-  const uint64_t chunk = 1ull << lo_bits, n_chunks = n >> lo_bits;
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    __syncthreads();  // the previous chunk's table and split are no longer read
-    if (threadIdx.x == 0) hs = split_factor(hi_b[ch]);
-    build_byte_table(hi_a[ch], htab);
-    F128d* o = out + ch * chunk;
-    for (uint64_t i = threadIdx.x; i < chunk; i += blockDim.x) o[i] = mul_table(lo_a[i], htab) + mul_split(lo_b[i], hs);
-  }
-}
-__global__ void lg_eq_fill2_kernel(const F128d* __restrict__ lo_a, const F128d* __restrict__ hi_a,
-                                   const F128d* __restrict__ lo_b, const F128d* __restrict__ hi_b, uint32_t lo_bits,
-                                   uint64_t n, F128d* __restrict__ out) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  out[i] = eq_at(lo_a, lo_bits, hi_a, i) + eq_at(lo_b, lo_bits, hi_b, i);
-}
-void launch_lg_eq_fill2(const F128d* lo_a, const F128d* hi_a, const F128d* lo_b, const F128d* hi_b, uint32_t lo_bits,
-                        uint64_t n, F128d* out, cudaStream_t s) {
-  if (lo_bits >= 12 && (n >> lo_bits) >= (uint64_t)sm_count() * 2 && (n & ((1ull << lo_bits) - 1)) == 0) {
-    const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-    set_dynamic_smem((const void*)lg_eq_fill2_tbl_kernel, smem);
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(n >> lo_bits, (uint64_t)sm_count() * 2);
-    lg_eq_fill2_tbl_kernel<<<blocks, 256, smem, s>>>(lo_a, hi_a, lo_b, hi_b, lo_bits, n, out);
-    LAUNCH_OK();
-    return;
-  }
-  lg_eq_fill2_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(lo_a, hi_a, lo_b, hi_b, lo_bits, n, out);
-  LAUNCH_OK();
-}
-// Chunks of at least 2^12 entries (one table build per chunk), and enough of them to give
-// every SM two blocks, use the table form.
-constexpr uint32_t LG_EQ_FILL_TABLE_MIN_LO_BITS = 12;
-void launch_lg_eq_fill(const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n, F128d* out, bool add,
-                       cudaStream_t s) {
-  if (eq_hi && lo_bits >= LG_EQ_FILL_TABLE_MIN_LO_BITS && (n >> lo_bits) >= (uint64_t)sm_count() * 2 &&
-      (n & ((1ull << lo_bits) - 1)) == 0) {
-    const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-    set_dynamic_smem((const void*)lg_eq_fill_tbl_kernel, smem);
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(n >> lo_bits, (uint64_t)sm_count() * 2);
-    lg_eq_fill_tbl_kernel<<<blocks, 256, smem, s>>>(eq_lo, lo_bits, eq_hi, n, out, add ? 1 : 0);
-    LAUNCH_OK();
-    return;
-  }
-  lg_eq_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(eq_lo, lo_bits, eq_hi, n, out, add ? 1 : 0);
-  LAUNCH_OK();
-}
-// sum_i f[i * stride] (F128 words) * eq(i), chunked.
-__global__ void lg_dot_eq_kernel(const F128d* __restrict__ f, uint32_t stride, const F128d* __restrict__ eq_lo,
-                                 uint32_t lo_bits, const F128d* __restrict__ eq_hi, uint64_t n,
-                                 F128d* __restrict__ part) {
-  __shared__ F128d sh[32];
-  const uint64_t chunk = 1ull << lo_bits;
-  const uint64_t n_chunks = (n + chunk - 1) / chunk;
-  F128d G = f128_zero();
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    F128d g = f128_zero();
-    uint64_t end = min(n, (ch + 1) * chunk);
-    for (uint64_t i = ch * chunk + threadIdx.x; i < end; i += blockDim.x) g += f[i * stride] * eq_lo[i & (chunk - 1)];
-    g = block_xor(g, sh);
-    if (threadIdx.x == 0) G += (eq_hi ? eq_hi[ch] : f128_one()) * g;
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = G;
-}
-// The same sum with chunks of 2^13 words and unit stride, reordered so that every
-// per-word product is by a block constant:
-//   sum_i f[i] eq(i) = sum_a eq_lo[a] h[a],  h[a] = sum_chunks eq_hi[chunk] f[chunk 2^13 + a].
-// Thread t of the 512 owns the 16 low indices a = t + 512 k and accumulates its block's
-// share of h[a] chunk by chunk; the products by the chunk's eq_hi come half from its byte
-// tables, half from its split form. Then 16 products by eq_lo[a] and the block reduction.
-constexpr uint32_t DOT_EQ_TBL_LO_BITS = 13;
+// ---- the lane stage: the first initial_k folds, over the lanes of the committed stack
+// q[l * D + p] (lane l, row p < D). The basis there is a sum of terms c_t eq(x_t) over all
+// variables, so it is never formed: with the lane dots
+//   h_t[l] = sum_p q[l D + p] eq_t(p)
+// every message of these folds is a sum over lane pairs (on the host, at most 64 lanes), and
+// once all the challenges are known f is folded by all of them in one pass,
+//   f[p] = sum_l lambda_l q[l D + p],  lambda = eq(challenges) in F256,
+// and the basis is sum_t e_t eq_t(p). This reads q once for the dots and once for the fold.
+// Forming the basis and folding both vectors challenge by challenge read and wrote them six
+// times: the whole Ligerito stage took 26.4 ms of a Keccak-f 2^18 proof (now 9.3), 4.8 ms of
+// SHA-256 2^16 (2.6), 0.94 ms of BLAKE3 2^12 (0.69; six kernels and round trips fewer).
+
+// Lane dots: part[split * lanes + l] = the split's share of h[l]. Chunk (2^13 rows) c of a
+// lane: h[l] = sum_a eq_lo[a] G[a], G[a] = sum_c eq_hi[c] q[l D + c 2^13 + a], thread t of the
+// 512 owning a = t + 512 k, so the products per word are by the chunk's constant eq_hi[c]:
+// three in four from its window table, one in four split (both pipes; 1.12e11 products/s in
+// isolation). One block per (lane, split), one block per SM beside the 169 KB table.
+constexpr uint32_t LANE_DOT_LO_BITS = 13;
 __global__ void __launch_bounds__(512, 1)
-lg_dot_eq_tbl_kernel(const F128d* __restrict__ f, const F128d* __restrict__ eq_lo, const F128d* __restrict__ eq_hi,
-                     uint64_t n_chunks, F128d* __restrict__ part) {
-  extern __shared__ __align__(16) F128d htab[];  // build_byte_table's BYTE_TABLE_SMEM_ENTRIES
+lg_lane_dots_tbl_kernel(const F128d* __restrict__ q, uint32_t lanes, uint32_t log_d, uint32_t splits,
+                        const F128d* __restrict__ eq_lo, const F128d* __restrict__ eq_hi, F128d* __restrict__ part) {
+  extern __shared__ __align__(16) char wt[];  // WinTable<6>
   __shared__ F128split hs;
   __shared__ F128d sh[32];
+  const uint32_t l = blockIdx.x % lanes, sp = blockIdx.x / lanes, lane16 = win_lane();
+  const uint32_t n_ch = 1u << (log_d - LANE_DOT_LO_BITS), per = n_ch / splits;
   F128d h[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) h[k] = f128_zero();
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
+  for (uint32_t ch = sp * per; ch < (sp + 1) * per; ++ch) {
     __syncthreads();  // the previous chunk's table and split are no longer read
     const F128d e = eq_hi[ch];
     if (threadIdx.x == 0) hs = split_factor(e);
-    build_byte_table(e, htab);
-    const F128d* fc = f + (ch << DOT_EQ_TBL_LO_BITS) + threadIdx.x;
+    build_win_table<6>(e, wt);
+    __syncthreads();
+    const F128d* fc = q + ((uint64_t)l << log_d) + ((uint64_t)ch << LANE_DOT_LO_BITS) + threadIdx.x;
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
       const F128d x = fc[512 * k];
-      h[k] += (k & 1) ? mul_split(x, hs) : mul_table(x, htab);
+      h[k] += (k & 3) == 3 ? mul_split(x, hs) : mul_win<6>(x, wt, lane16);
     }
   }
   F128d g = f128_zero();
 #pragma unroll
   for (int k = 0; k < 16; ++k) g += mul_call(h[k], eq_lo[threadIdx.x + 512 * k]);
   g = block_xor(g, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = g;
+  if (threadIdx.x == 0) part[(uint64_t)sp * lanes + l] = g;
 }
-uint32_t launch_lg_dot_eq(const F128d* f, uint32_t stride, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi,
-                          uint64_t n, uint64_t live, F128d* part, cudaStream_t s) {
-  live = std::min(live, n);  // f is zero from `live` on
-  if (stride == 1 && eq_hi && lo_bits == DOT_EQ_TBL_LO_BITS && (n & ((1ull << lo_bits) - 1)) == 0 &&
-      (n >> lo_bits) >= (uint64_t)sm_count()) {
-    const uint64_t n_chunks = std::max<uint64_t>(1, (live + (1ull << lo_bits) - 1) >> lo_bits);
-    const uint32_t blocks = (uint32_t)sm_count();
-    const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-    set_dynamic_smem((const void*)lg_dot_eq_tbl_kernel, smem);
-    lg_dot_eq_tbl_kernel<<<blocks, 512, smem, s>>>(f, eq_lo, eq_hi, n_chunks, part);
+// The same for few rows: block (lane, chunk of 2^lo_bits rows), one product a word.
+__global__ void __launch_bounds__(256)
+lg_lane_dots_kernel(const F128d* __restrict__ q, uint32_t lanes, uint32_t log_d, const F128d* __restrict__ eq_lo,
+                    uint32_t lo_bits, const F128d* __restrict__ eq_hi, F128d* __restrict__ part) {
+  __shared__ F128d sh[32];
+  const uint32_t l = blockIdx.x % lanes, ch = blockIdx.x / lanes;
+  const F128d* fc = q + ((uint64_t)l << log_d) + ((uint64_t)ch << lo_bits);
+  F128d g = f128_zero();
+  for (uint32_t a = threadIdx.x; a < (1u << lo_bits); a += blockDim.x) g += mul_call(fc[a], eq_lo[a]);
+  g = block_xor(g, sh);
+  if (threadIdx.x == 0) part[(uint64_t)ch * lanes + l] = mul_call(eq_hi[ch], g);
+}
+// From 2^16 rows (eight chunks a lane) the table form: below, its blocks would hold a chunk or
+// two each and a 169 KB table build apiece.
+constexpr uint32_t LANE_DOT_TABLE_MIN_LOG = 16;
+uint32_t lane_dots_lo_bits(uint32_t log_d) { return log_d >= LANE_DOT_TABLE_MIN_LOG ? LANE_DOT_LO_BITS : std::min(log_d, 10u); }
+uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, const F128d* eq_hi,
+                             F128d* part, cudaStream_t s) {
+  const uint32_t lo = lane_dots_lo_bits(log_d);
+  if (lo == LANE_DOT_LO_BITS) {
+    uint32_t splits = 1;  // eight blocks per SM in all: the last wave then costs a few percent
+    while (splits < (1u << (log_d - lo)) && splits * lanes < (uint32_t)sm_count() * 8) splits <<= 1;
+    set_dynamic_smem((const void*)lg_lane_dots_tbl_kernel, WinTable<6>::BYTES);
+    lg_lane_dots_tbl_kernel<<<lanes * splits, 512, WinTable<6>::BYTES, s>>>(q, lanes, log_d, splits, eq_lo, eq_hi, part);
     LAUNCH_OK();
-    return blocks;
+    return splits;
   }
-  n = std::max<uint64_t>(live, 1);
-  uint64_t n_chunks = (n + (1ull << lo_bits) - 1) >> lo_bits;
-  uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
-  lg_dot_eq_kernel<<<blocks, 256, 0, s>>>(f, stride, eq_lo, lo_bits, eq_hi, n, part);
+  lg_lane_dots_kernel<<<lanes << (log_d - lo), 256, 0, s>>>(q, lanes, log_d, eq_lo, lo, eq_hi, part);
   LAUNCH_OK();
-  return blocks;
+  return 1u << (log_d - lo);
 }
 
+// The fold of all lanes: part[g D + p] = sum over the lanes of group g of lambda_l q[l D + p].
+// A block holds LANE_FOLD_ROWS rows' F256 sums in registers and walks its lanes: per lane the
+// window tables of lambda's two halves (W = 5, 202 KB, one block per SM), the next lane's words
+// loaded before the tables are built; two products a word, one in four split. Groups split the
+// lanes where the rows alone do not fill the SMs; lg_lane_switch sums them.
+constexpr uint32_t LANE_FOLD_THREADS = 512, LANE_FOLD_PER = 6;
+constexpr uint32_t LANE_FOLD_ROWS = LANE_FOLD_THREADS * LANE_FOLD_PER;
+__global__ void __launch_bounds__(LANE_FOLD_THREADS, 1)
+lg_lane_fold_kernel(const F128d* __restrict__ q, const F256d* __restrict__ lambda, uint32_t lanes, uint64_t D,
+                    F256d* __restrict__ part) {
+  extern __shared__ __align__(16) char wt[];  // the WinTable<5> of lambda.c0, then lambda.c1's
+  __shared__ F128split s1;
+  const uint32_t l0 = lanes * blockIdx.y / gridDim.y, l1 = lanes * (blockIdx.y + 1) / gridDim.y, lane16 = win_lane();
+  const uint64_t p0 = (uint64_t)blockIdx.x * LANE_FOLD_ROWS + threadIdx.x;
+  F128d c0[LANE_FOLD_PER], c1[LANE_FOLD_PER], x[LANE_FOLD_PER];
+#pragma unroll
+  for (uint32_t k = 0; k < LANE_FOLD_PER; ++k) {
+    const uint64_t p = p0 + k * LANE_FOLD_THREADS;
+    c0[k] = c1[k] = f128_zero();
+    x[k] = p < D ? q[l0 * D + p] : f128_zero();
+  }
+  for (uint32_t l = l0; l < l1; ++l) {
+    __syncthreads();  // the previous lane's tables are no longer read
+    const F256d lam = lambda[l];
+    if (threadIdx.x == 0) s1 = split_factor(lam.c1);
+    build_win_table<5>(lam.c0, wt);
+    build_win_table<5>(lam.c1, wt + WinTable<5>::BYTES);
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < LANE_FOLD_PER; ++k) {
+      c0[k] += mul_win<5>(x[k], wt, lane16);
+      c1[k] += (k & 1) ? mul_split(x[k], s1) : mul_win<5>(x[k], wt + WinTable<5>::BYTES, lane16);
+    }
+    if (l + 1 < l1) {
+#pragma unroll
+      for (uint32_t k = 0; k < LANE_FOLD_PER; ++k) {
+        const uint64_t p = p0 + k * LANE_FOLD_THREADS;
+        if (p < D) x[k] = q[(l + 1) * D + p];
+      }
+    }
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < LANE_FOLD_PER; ++k) {
+    const uint64_t p = p0 + k * LANE_FOLD_THREADS;
+    if (p < D) part[blockIdx.y * D + p] = f256(c0[k], c1[k]);
+  }
+}
+// Lane groups: enough that the grid holds about eight blocks per SM (or a lane a group).
+uint32_t lane_fold_groups(uint32_t lanes, uint64_t D) {
+  const uint64_t rows = (D + LANE_FOLD_ROWS - 1) / LANE_FOLD_ROWS, want = (uint64_t)sm_count() * 8;
+  return (uint32_t)std::min<uint64_t>(lanes, (want + rows - 1) / rows);
+}
+void launch_lg_lane_fold(const F128d* q, const F256d* lambda, uint32_t lanes, uint64_t D, F256d* part, cudaStream_t s) {
+  const int smem = 2 * WinTable<5>::BYTES;
+  set_dynamic_smem((const void*)lg_lane_fold_kernel, smem);
+  const dim3 grid((unsigned)((D + LANE_FOLD_ROWS - 1) / LANE_FOLD_ROWS), lane_fold_groups(lanes, D));
+  lg_lane_fold_kernel<<<grid, LANE_FOLD_THREADS, smem, s>>>(q, lambda, lanes, D, part);
+  LAUNCH_OK();
+}
 // Round message with block pairing d: pairs (lo, lo + d), lo = 2 d blk + k.
-//   u0 = sum f[lo] b[lo], u2 = sum (f[lo] + f[hi]) (b[lo] + b[hi]).
-// F128 (base) variant: outputs 2 words per block; F256 variant: 4 words (u0.c0, u0.c1, u2.c0, u2.c1).
+//   u0 = sum f[lo] b[lo], u2 = sum (f[lo] + f[hi]) (b[lo] + b[hi]),
+// four words per block (u0.c0, u0.c1, u2.c0, u2.c1).
 // The pairing distances are powers of two (the kernels take log2 d).
 static uint32_t log2_distance(uint64_t d) {
   if (d == 0 || (d & (d - 1))) throw std::runtime_error("Ligerito pair distance must be a power of two");
@@ -1295,36 +1270,12 @@ static uint32_t log2_distance(uint64_t d) {
 __device__ __forceinline__ uint64_t pair_lo(uint64_t i, uint32_t d_log) {
   return ((i >> d_log) << (d_log + 1)) | (i & ((1ull << d_log) - 1));
 }
-__global__ void lg_message128_kernel(const F128d* __restrict__ f, const F128d* __restrict__ b, uint64_t n, uint64_t f_live,
-                                     uint32_t d_log, F128d* __restrict__ part, FusedPublish pub) {
-  __shared__ F128d sh[32];
-  F128d u0 = f128_zero(), u2 = f128_zero();
-  for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n / 2; p += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t lo = pair_lo(p, d_log), hi = lo + (1ull << d_log);
-    if (lo >= f_live) continue;  // f[lo] = f[hi] = 0: the pair adds nothing
-    F128d f0 = f[lo], f1 = f[hi], b0 = b[lo], b1 = b[hi];
-    u0 += f0 * b0;
-    u2 += (f0 + f1) * (b0 + b1);
-  }
-  u0 = block_xor(u0, sh);
-  u2 = block_xor(u2, sh);
-  if (threadIdx.x == 0) { part[blockIdx.x * 2] = u0; part[blockIdx.x * 2 + 1] = u2; }
-  if (pub.out) publish_if_last(part, 2, pub, sh);
-}
-uint32_t launch_lg_message128(const F128d* f, const F128d* b, uint64_t n, uint64_t f_live, uint64_t d, F128d* part,
-                              cudaStream_t s, FusedPublish pub) {
-  uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n / 2 + 255) / 256, (uint64_t)sm_count() * 8));
-  lg_message128_kernel<<<blocks, 256, 0, s>>>(f, b, n, f_live, log2_distance(d), part, pub);
-  LAUNCH_OK();
-  return blocks;
-}
-__global__ void lg_message256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n, uint64_t f_live,
+__global__ void lg_message256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n,
                                      uint32_t d_log, F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d sh[32];
   F256d u0 = f256(f128_zero(), f128_zero()), u2 = u0;
   for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n / 2; p += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t lo = pair_lo(p, d_log), hi = lo + (1ull << d_log);
-    if (lo >= f_live) continue;  // f[lo] = f[hi] = 0: the pair adds nothing
     F256d f0 = f[lo], f1 = f[hi], b0 = b[lo], b1 = b[hi];
     u0 += f256_mul_call(f0, b0);
     u2 += f256_mul_call(f0 + f1, b0 + b1);
@@ -1336,39 +1287,12 @@ __global__ void lg_message256_kernel(const F256d* __restrict__ f, const F256d* _
   }
   if (pub.out) publish_if_last(part, 4, pub, sh);
 }
-uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64_t f_live, uint64_t d, F128d* part,
+uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64_t d, F128d* part,
                               cudaStream_t s, FusedPublish pub) {
   uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n / 2 + 255) / 256, (uint64_t)sm_count() * 8));
-  lg_message256_kernel<<<blocks, 256, 0, s>>>(f, b, n, f_live, log2_distance(d), part, pub);
+  lg_message256_kernel<<<blocks, 256, 0, s>>>(f, b, n, log2_distance(d), part, pub);
   LAUNCH_OK();
   return blocks;
-}
-// o[i] = v[lo] + r (v[hi] + v[lo]), i = blk d + k, lo = 2 d blk + k. The products by r.c0
-// come from byte tables of r.c0 (load/store pipe), those by r.c1 from its split form
-// (multiply pipe); grid-stride, so each block's table serves many elements.
-__global__ void __launch_bounds__(256, 2)
-lg_fold128_kernel(const F128d* __restrict__ f, const F128d* __restrict__ b, uint64_t n_out, F256d r,
-                  const F256d* __restrict__ r_dev, uint32_t d_log, F256d* __restrict__ fo, F256d* __restrict__ bo) {
-  extern __shared__ __align__(16) F128d rtab[];  // build_byte_table's BYTE_TABLE_SMEM_ENTRIES
-  __shared__ F128split r1s;
-  const F256d rv = r_dev ? *r_dev : r;
-  if (threadIdx.x == 0) r1s = split_factor(rv.c1);
-  build_byte_table(rv.c0, rtab);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_out; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t lo = pair_lo(i, d_log), hi = lo + (1ull << d_log);
-    F128d f0 = f[lo], df = f[hi] + f0, b0 = b[lo], db = b[hi] + b0;
-    fo[i] = f256(f0 + mul_table(df, rtab), mul_split(df, r1s));
-    bo[i] = f256(b0 + mul_table(db, rtab), mul_split(db, r1s));
-  }
-}
-void launch_lg_fold128(const F128d* f, const F128d* b, uint64_t n_out, F256d r, const F256d* r_dev, uint64_t d,
-                       F256d* fo, F256d* bo, cudaStream_t s) {
-  const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-  set_dynamic_smem((const void*)lg_fold128_kernel, smem);
-  // at least 2048 elements per block (two table products each) for one table build
-  const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count() * 2, n_out / 2048));
-  lg_fold128_kernel<<<(unsigned)blocks, 256, smem, s>>>(f, b, n_out, r, r_dev, log2_distance(d), fo, bo);
-  LAUNCH_OK();
 }
 __global__ void lg_fold256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, F256d r,
                                   const F256d* __restrict__ r_dev, uint32_t d_log, F256d* __restrict__ fo,
@@ -1403,7 +1327,7 @@ __device__ __forceinline__ void lg_fold_at(const F256d* __restrict__ f, const F2
 // 512-thread block per SM holds the two tables (141 KB).
 template <bool TBL>
 __global__ void __launch_bounds__(TBL ? 512 : 256, TBL ? 1 : 2)
-lg_fold_msg256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, uint64_t f_live, F256d r,
+lg_fold_msg256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, F256d r,
                       uint32_t dlog_fold, uint32_t dlog_msg, F256d* __restrict__ fo, F256d* __restrict__ bo,
                       F128d* __restrict__ part, FusedPublish pub) {
   extern __shared__ __align__(16) F128d rtab[];  // TBL: tables of r.c0 and r.c1
@@ -1431,26 +1355,9 @@ lg_fold_msg256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, 
       lg_fold_at(f, b, r, dlog_fold, i, fi, bi);
     }
   };
-  auto fold_b_at = [&](uint64_t i) {  // f is zero at both inputs of i: only b folds
-    const uint64_t lo = pair_lo(i, dlog_fold), hi = lo + (1ull << dlog_fold);
-    const F256d b0 = b[lo], db = b[hi] + b0;
-    fo[i] = f256(f128_zero(), f128_zero());
-    if (TBL) {
-      const F128d p0 = mul_table(db.c0, rtab), p1 = mul_table(db.c1, rtab + BYTE_TABLE_ENTRIES),
-                  p2 = mul_split_call(db.c0 + db.c1, &rsum);
-      bo[i] = b0 + f256(p0 + mul_by_x_inv(p1), p2 + p0);
-    } else {
-      bo[i] = b0 + f256_mul_call(r, db);
-    }
-  };
   F256d u0 = f256(f128_zero(), f128_zero()), u2 = u0;
   for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_out / 2; p += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t olo = pair_lo(p, dlog_msg), ohi = olo + (1ull << dlog_msg);
-    if (pair_lo(olo, dlog_fold) >= f_live) {  // f is zero at every input of both entries
-      fold_b_at(olo);
-      fold_b_at(ohi);
-      continue;
-    }
     F256d fl, bl, fh, bh;
     fold_at(olo, fl, bl);
     fo[olo] = fl;
@@ -1467,89 +1374,25 @@ lg_fold_msg256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, 
     part[blockIdx.x * 4 + 2] = r2; part[blockIdx.x * 4 + 3] = r3;
   }
   if (pub.out) publish_if_last(part, 4, pub, sh);
-}
-// The first fold, of the base (F128) vectors at r, fused with the next message: the
-// products r.c0 (f[hi] + f[lo]) and r.c1 (f[hi] + f[lo]) come from byte tables of r.c0 and
-// r.c1 (8 table products per message pair on the load/store pipe) and the message's two
-// F256 products of variables (6 F128 products) from integer multiplies. One 512-thread
-// block per SM holds the two tables.
-__global__ void __launch_bounds__(512, 1)
-lg_fold_msg128_kernel(const F128d* __restrict__ f, const F128d* __restrict__ b, uint64_t n_out, uint64_t f_live, F256d r,
-                      uint32_t dlog_fold, uint32_t dlog_msg, F256d* __restrict__ fo, F256d* __restrict__ bo,
-                      F128d* __restrict__ part, FusedPublish pub) {
-  extern __shared__ __align__(16) F128d rtab[];  // tables of r.c0 and r.c1
-  __shared__ F128d sh[32];
-  const F128d* T0 = rtab;
-  const F128d* T1 = rtab + BYTE_TABLE_ENTRIES;
-  build_byte_table(r.c0, rtab);
-  build_byte_table(r.c1, rtab + BYTE_TABLE_ENTRIES);  // its scratch follows the second table
-  auto fold_at = [&](uint64_t i, F256d& fi, F256d& bi) {
-    const uint64_t lo = pair_lo(i, dlog_fold), hi = lo + (1ull << dlog_fold);
-    const F128d f0 = f[lo], df = f[hi] + f0, b0 = b[lo], db = b[hi] + b0;
-    fi = f256(f0 + mul_table(df, T0), mul_table(df, T1));
-    bi = f256(b0 + mul_table(db, T0), mul_table(db, T1));
-  };
-  auto fold_b_at = [&](uint64_t i) {  // f is zero at both inputs of i: only b folds
-    const uint64_t lo = pair_lo(i, dlog_fold), hi = lo + (1ull << dlog_fold);
-    const F128d b0 = b[lo], db = b[hi] + b0;
-    fo[i] = f256(f128_zero(), f128_zero());
-    bo[i] = f256(b0 + mul_table(db, T0), mul_table(db, T1));
-  };
-  F256d u0 = f256(f128_zero(), f128_zero()), u2 = u0;
-  for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_out / 2; p += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t olo = pair_lo(p, dlog_msg), ohi = olo + (1ull << dlog_msg);
-    if (pair_lo(olo, dlog_fold) >= f_live) {  // f is zero at every input of both entries
-      fold_b_at(olo);
-      fold_b_at(ohi);
-      continue;
-    }
-    F256d fl, bl, fh, bh;
-    fold_at(olo, fl, bl);
-    fo[olo] = fl;
-    bo[olo] = bl;
-    u0 += f256_mul_call(fl, bl);
-    fold_at(ohi, fh, bh);
-    fo[ohi] = fh;
-    bo[ohi] = bh;
-    u2 += f256_mul_call(fl + fh, bl + bh);
-  }
-  F128d r0 = block_xor(u0.c0, sh), r1 = block_xor(u0.c1, sh), r2 = block_xor(u2.c0, sh), r3 = block_xor(u2.c1, sh);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x * 4] = r0; part[blockIdx.x * 4 + 1] = r1;
-    part[blockIdx.x * 4 + 2] = r2; part[blockIdx.x * 4 + 3] = r3;
-  }
-  if (pub.out) publish_if_last(part, 4, pub, sh);
-}
-uint32_t launch_lg_fold_msg128(const F128d* f, const F128d* b, uint64_t n_out, uint64_t f_live, F256d r, uint64_t d_fold,
-                               uint64_t d_msg, F256d* fo, F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub) {
-  const int smem = (int)((BYTE_TABLE_ENTRIES + BYTE_TABLE_SMEM_ENTRIES) * sizeof(F128d));
-  set_dynamic_smem((const void*)lg_fold_msg128_kernel, smem);
-  // at least 512 message pairs per block for its two table builds
-  const uint32_t blocks =
-      (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sm_count(), n_out / 2 / 512));
-  lg_fold_msg128_kernel<<<blocks, 512, smem, s>>>(f, b, n_out, f_live, r, log2_distance(d_fold), log2_distance(d_msg),
-                                                   fo, bo, part, pub);
-  LAUNCH_OK();
-  return blocks;
 }
 // Folds of at least this many output entries use the table form, with at least
 // LG_FOLD_TABLE_MIN_BLOCK_PAIRS message pairs per block for its two table builds.
 constexpr uint64_t LG_FOLD_TABLE_MIN_OUT = uint64_t(1) << 17;
 constexpr uint64_t LG_FOLD_TABLE_MIN_BLOCK_PAIRS = 512;
-uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, uint64_t f_live, F256d r, uint64_t d_fold,
+uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, uint64_t d_fold,
                                uint64_t d_msg, F256d* fo, F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub) {
   if (n_out >= LG_FOLD_TABLE_MIN_OUT) {
     const int smem = (int)((BYTE_TABLE_ENTRIES + BYTE_TABLE_SMEM_ENTRIES) * sizeof(F128d));
     set_dynamic_smem((const void*)lg_fold_msg256_kernel<true>, smem);
     const uint32_t blocks = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>((uint64_t)sm_count(), n_out / 2 / LG_FOLD_TABLE_MIN_BLOCK_PAIRS));
-    lg_fold_msg256_kernel<true><<<blocks, 512, smem, s>>>(f, b, n_out, f_live, r, log2_distance(d_fold),
+    lg_fold_msg256_kernel<true><<<blocks, 512, smem, s>>>(f, b, n_out, r, log2_distance(d_fold),
                                                           log2_distance(d_msg), fo, bo, part, pub);
     LAUNCH_OK();
     return blocks;
   }
   uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n_out / 2 + 255) / 256, (uint64_t)sm_count() * 8));
-  lg_fold_msg256_kernel<false><<<blocks, 256, 0, s>>>(f, b, n_out, f_live, r, log2_distance(d_fold),
+  lg_fold_msg256_kernel<false><<<blocks, 256, 0, s>>>(f, b, n_out, r, log2_distance(d_fold),
                                                       log2_distance(d_msg), fo, bo, part, pub);
   LAUNCH_OK();
   return blocks;
@@ -1575,36 +1418,66 @@ void launch_lg_code_switch(const F256d* f, const F256d* b, uint64_t n, F256d* fo
 //   u0 += f.c0 b = (f.c0 b.c0, f.c0 b.c1),
 //   u2 += (f.c0 + f.c1)(b + u b) = s (b.c0 + x^-1 b.c1, b.c0),  s = f.c0 + f.c1,
 // with u b = (x^-1 b.c1, b.c0 + b.c1) as the switch writes it.
-__global__ void lg_switch_msg_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n, uint64_t f_live,
-                                     F256d* __restrict__ fo, F256d* __restrict__ bo, F128d* __restrict__ part,
-                                     FusedPublish pub) {
-  __shared__ F128d sh[32];
-  F128d u00 = f128_zero(), u01 = f128_zero(), u20 = f128_zero(), u21 = f128_zero();
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const F256d fv = f[i], bv = b[i];
-    const F128d ub0 = mul_by_x_inv(bv.c1);
-    fo[2 * i] = f256_base(fv.c0);
-    fo[2 * i + 1] = f256_base(fv.c1);
-    bo[2 * i] = bv;
-    bo[2 * i + 1] = f256(ub0, bv.c0 + bv.c1);
-    if (i >= f_live) continue;  // f[i] = 0: both products vanish
-    const F128d sv = fv.c0 + fv.c1;
-    u00 += mul_call(fv.c0, bv.c0);
-    u01 += mul_call(fv.c0, bv.c1);
-    u20 += mul_call(sv, bv.c0 + ub0);
-    u21 += mul_call(sv, bv.c0);
-  }
-  F128d r0 = block_xor(u00, sh), r1 = block_xor(u01, sh), r2 = block_xor(u20, sh), r3 = block_xor(u21, sh);
+__device__ __forceinline__ void switch_pair(F256d fv, F256d bv, uint64_t i, F256d* __restrict__ fo,
+                                            F256d* __restrict__ bo, F128d& u00, F128d& u01, F128d& u20, F128d& u21) {
+  const F128d ub0 = mul_by_x_inv(bv.c1);
+  fo[2 * i] = f256_base(fv.c0);
+  fo[2 * i + 1] = f256_base(fv.c1);
+  bo[2 * i] = bv;
+  bo[2 * i + 1] = f256(ub0, bv.c0 + bv.c1);
+  const F128d sv = fv.c0 + fv.c1;
+  u00 += mul_call(fv.c0, bv.c0);
+  u01 += mul_call(fv.c0, bv.c1);
+  u20 += mul_call(sv, bv.c0 + ub0);
+  u21 += mul_call(sv, bv.c0);
+}
+__device__ __forceinline__ void switch_publish(F128d u00, F128d u01, F128d u20, F128d u21, F128d* __restrict__ part,
+                                               const FusedPublish& pub, F128d* sh) {
+  const F128d r0 = block_xor(u00, sh), r1 = block_xor(u01, sh), r2 = block_xor(u20, sh), r3 = block_xor(u21, sh);
   if (threadIdx.x == 0) {
     part[blockIdx.x * 4] = r0; part[blockIdx.x * 4 + 1] = r1;
     part[blockIdx.x * 4 + 2] = r2; part[blockIdx.x * 4 + 3] = r3;
   }
   if (pub.out) publish_if_last(part, 4, pub, sh);
 }
-uint32_t launch_lg_switch_msg(const F256d* f, const F256d* b, uint64_t n, uint64_t f_live, F256d* fo, F256d* bo,
-                              F128d* part, cudaStream_t s, FusedPublish pub) {
+__global__ void lg_switch_msg_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n,
+                                     F256d* __restrict__ fo, F256d* __restrict__ bo, F128d* __restrict__ part,
+                                     FusedPublish pub) {
+  __shared__ F128d sh[32];
+  F128d u00 = f128_zero(), u01 = f128_zero(), u20 = f128_zero(), u21 = f128_zero();
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    switch_pair(f[i], b[i], i, fo, bo, u00, u01, u20, u21);
+  switch_publish(u00, u01, u20, u21, part, pub, sh);
+}
+uint32_t launch_lg_switch_msg(const F256d* f, const F256d* b, uint64_t n, F256d* fo, F256d* bo, F128d* part,
+                              cudaStream_t s, FusedPublish pub) {
   uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 8));
-  lg_switch_msg_kernel<<<blocks, 256, 0, s>>>(f, b, n, f_live, fo, bo, part, pub);
+  lg_switch_msg_kernel<<<blocks, 256, 0, s>>>(f, b, n, fo, bo, part, pub);
+  LAUNCH_OK();
+  return blocks;
+}
+// The end of the lane stage: f[p] summed over the fold's lane groups, b[p] = sum_t e_t eq_t(p),
+// then the code switch and its message as lg_switch_msg. The live entries are the rows.
+__global__ void lg_lane_switch_kernel(const F256d* __restrict__ fpart, uint32_t groups, LaneTerms terms, uint64_t D,
+                                      F256d* __restrict__ fo, F256d* __restrict__ bo, F128d* __restrict__ part,
+                                      FusedPublish pub) {
+  __shared__ F128d sh[32];
+  F128d u00 = f128_zero(), u01 = f128_zero(), u20 = f128_zero(), u21 = f128_zero();
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (uint64_t)gridDim.x * blockDim.x) {
+    F256d fv = fpart[i], bv = f256(f128_zero(), f128_zero());
+    for (uint32_t g = 1; g < groups; ++g) fv += fpart[g * D + i];
+    for (uint32_t t = 0; t < terms.n; ++t) {
+      const F128d e = mul_call(terms.lo[t][i & ((1ull << terms.lo_bits) - 1)], terms.hi[t][i >> terms.lo_bits]);
+      bv += f256(mul_call(terms.coef[t].c0, e), mul_call(terms.coef[t].c1, e));
+    }
+    switch_pair(fv, bv, i, fo, bo, u00, u01, u20, u21);
+  }
+  switch_publish(u00, u01, u20, u21, part, pub, sh);
+}
+uint32_t launch_lg_lane_switch(const F256d* fpart, uint32_t groups, const LaneTerms& terms, uint64_t D, F256d* fo,
+                               F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub) {
+  const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((D + 255) / 256, (uint64_t)sm_count() * 8));
+  lg_lane_switch_kernel<<<blocks, 256, 0, s>>>(fpart, groups, terms, D, fo, bo, part, pub);
   LAUNCH_OK();
   return blocks;
 }
