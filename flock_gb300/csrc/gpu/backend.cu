@@ -69,21 +69,44 @@ static T* dmalloc(size_t n, std::vector<void*>& owned, uint64_t& counter) {
   return static_cast<T*>(p);
 }
 
-// Entries of the split eq tables of the skip fold (over L coordinates) and of every
-// later zerocheck fold round (over the suffixes of L - 1, L - 2, ..., 0 coordinates).
-// Round i splits its n = L - 1 - i coordinates as lo + hi with lo = zc_round_lo_bits(n).
-static uint32_t zc_round_lo_bits(uint32_t n) {
-  // chunks of 2^10 pairs where the round has enough of them for the table form, else of
-  // 2^8 (one pair per thread: four times the blocks of a small, latency-bound round)
-  return std::min(n, n >= 17 ? 10u : 8u);
-}
-static uint64_t zc_tables_entries(uint32_t L) {
-  uint64_t total = (uint64_t(1) << 10) + (uint64_t(1) << (L - 10));
+// The eq tables of the zerocheck, over coordinates [off, off + n) of the skip fold's point of
+// length L: table 0 and 1 are the skip fold's low and high ones, tables 2 + 2i and 3 + 2i those
+// of fold round i, whose message runs over the L - 1 - i coordinates from 1 + i on. Plain form
+// (weighted = 0): each split as lo + hi, chunks of 2^8 pairs (one pair per thread). Weighted form
+// with chunks of 2^w words: table 1 is the chunk weight h over [w, L), and the rounds i < w only
+// have the low part [1 + i, w) of their coordinates.
+struct ZcTable {
+  uint32_t off, n;
+};
+static std::vector<ZcTable> zc_table_list(uint32_t L, uint32_t w) {
+  std::vector<ZcTable> t;
+  const uint32_t lo0 = w ? w : 10;
+  t.push_back({0, lo0});
+  t.push_back({lo0, L - lo0});
   for (uint32_t i = 0; i < L; ++i) {
-    uint32_t n = L - 1 - i, lo = zc_round_lo_bits(n);
-    total += (uint64_t(1) << lo) + (uint64_t(1) << (n - lo));
+    const uint32_t n = L - 1 - i;
+    const uint32_t lo = i < w ? w - 1 - i : std::min(n, 8u);
+    t.push_back({1 + i, lo});
+    t.push_back({1 + i + lo, i < w ? 0 : n - lo});
   }
+  return t;
+}
+static uint64_t zc_tables_entries(uint32_t L, uint32_t w) {
+  uint64_t total = 0;
+  for (const ZcTable& t : zc_table_list(L, w)) total += uint64_t(1) << t.n;
   return total;
+}
+// Words of z, a and b that can be nonzero: a single slot's witness fills chunk-columns
+// c < used_cols of word (c << nu) + instance.
+static uint64_t live_words_of(const Statement& S) {
+  const uint64_t W = uint64_t(1) << (S.m - 7);
+  return S.slots.size() == 1 && S.slots[0].offset == 0 ? std::min<uint64_t>(W, S.slots[0].used_cols << S.nu) : W;
+}
+// Room for either form (a degenerate challenge takes the plain one), and for the reciprocal
+// weights beside the tables.
+static uint64_t zc_tables_room(const Statement& S) {
+  const uint32_t L = S.m - 7, w = zc_weighted_lo_bits(live_words_of(S));
+  return std::max(zc_tables_entries(L, 0), w ? zc_tables_entries(L, w) + (uint64_t(1) << (L - w)) : 0);
 }
 
 // Device bytes a backend for this statement holds after its first prove (the buffers of
@@ -96,7 +119,7 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   if (!S.identity) b += S.committed_words * 16;  // the compacted stack
   b += n_pos * S.lanes * 16 + 2 * n_pos * 32;  // L0 codeword and tree
   b += (W / 2 * 2 + W * 2 + 64) * 16;       // zerocheck folds
-  b += zc_tables_entries(S.m - 7) * 16;
+  b += zc_tables_room(S) * 16;
   b += 6 * K * 16;                          // lincheck vectors
   for (const SlotInfo& t : S.slots) {
     b += 2 * (uint64_t(16) << t.k_log);
@@ -127,9 +150,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   upload_constants_once();
   W_ = uint64_t(1) << (S.m - 7);
   K_ = 1u << S.k_log;
-  zc_live_words_ = (S.slots.size() == 1 && S.slots[0].offset == 0)
-                       ? std::min<uint64_t>(W_, S.slots[0].used_cols << S.nu)
-                       : W_;
+  zc_live_words_ = live_words_of(S);
   const uint64_t W = W_;
   in_bytes_ = 0;
   for (const SlotInfo& t : S.slots) in_bytes_ += (size_t)t.count * input_record_bytes(t.hash);
@@ -210,7 +231,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   *(volatile uint32_t*)h_flag_ = 0;
   pub_counter_ = dmalloc<uint32_t>(1, owned_, device_bytes_);
   CUDA_OK(cudaMemsetAsync(pub_counter_, 0, sizeof(uint32_t), st_));
-  zc_tabs_cap_ = zc_tables_entries(S.m - 7);
+  zc_tabs_cap_ = zc_tables_room(S);
   zc_tabs_ = dmalloc<F128d>(zc_tabs_cap_, owned_, device_bytes_);
   CUDA_OK(cudaStreamCreateWithFlags(&pow_st_, cudaStreamNonBlocking));
   d_pow_ = dmalloc<unsigned long long>(1, owned_, device_bytes_);
@@ -589,35 +610,54 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   if (L < 10) throw std::runtime_error("zerocheck skip fold needs m >= 17");
   const F128d* dw = upload(w);
   const F128d* dp = upload(eq_point);
+  // the weighted form divides by the high coordinates' eq once: none may be 0 or 1
+  zc_w_ = zc_weighted_lo_bits(zc_live_words_);
+  for (uint32_t j = zc_w_; zc_w_ && j < L; ++j)
+    if (eq_point[j].is_zero() || eq_point[j] == F128::one()) zc_w_ = 0;
   // Every later fold round i uses eq over the suffix eq_point[1 + i ..]: build all the
-  // split tables now, in one launch.
+  // tables now, in one launch.
   zc_desc_.clear();
   uint64_t total = 0;
-  auto add = [&](uint32_t off, uint32_t n) {
+  for (const ZcTable& t : zc_table_list(L, zc_w_)) {
     EqDesc d;
-    d.p_off = off;
-    d.n = n;
+    d.p_off = t.off;
+    d.n = t.n;
     d.out_off = total;
     d.scale = dev(F128::one());
     zc_desc_.push_back(d);
-    total += uint64_t(1) << n;
-  };
-  add(0, 10);
-  add(10, L - 10);
-  for (uint32_t i = 0; i < L; ++i) {  // round i: eq over eq_point[1 + i ..), L - 1 - i coordinates
-    uint32_t n = L - 1 - i, lo = zc_round_lo_bits(n);
-    add(1 + i, lo);
-    add(1 + i + lo, n - lo);
+    total += uint64_t(1) << t.n;
   }
-  if (total != zc_tables_entries(L)) throw std::runtime_error("zerocheck eq tables: size mismatch");
+  zc_inv_ = zc_tabs_ + total;
+  if (total + (zc_w_ ? uint64_t(1) << (L - zc_w_) : 0) > zc_tabs_cap_) throw std::runtime_error("zerocheck eq tables: size mismatch");
   const EqDesc* ddesc = static_cast<const EqDesc*>(upload(zc_desc_.data(), zc_desc_.size() * sizeof(EqDesc)));
   uint32_t nb;
   {
     Mark mk(this, ST_ZC_FOLD_SKIP);
     launch_eq_tables(dp, ddesc, (uint32_t)zc_desc_.size(), total, zc_tabs_, st_);
     // words from zc_live_words_ on are zero and add nothing to the message
-    nb = launch_zc_fold_skip(a_, b_, dw, zc_live_words_, zc_tabs_, 10, zc_tabs_ + zc_desc_[1].out_off, part_, st_);
+    const F128d* hi = zc_tabs_ + zc_desc_[1].out_off;
+    nb = zc_w_ ? launch_zc_fold_skip_weighted(a_, b_, dw, zc_live_words_, zc_w_, zc_tabs_, hi, part_, st_)
+               : launch_zc_fold_skip(a_, b_, dw, zc_live_words_, zc_tabs_, 10, hi, part_, st_);
     CUDA_OK(cudaMemcpyAsync(zc_w64_, dw, 64 * sizeof(F128d), cudaMemcpyDeviceToDevice, st_));
+  }
+  if (zc_w_) {
+    // reciprocals of 1 + r_j and r_j (one inversion of their product), then of the weights h;
+    // queued behind the skip fold
+    std::vector<F128> f, pre;
+    F128 p = F128::one();
+    for (uint32_t j = zc_w_; j < L; ++j)
+      for (F128 v : {F128::one() + eq_point[j], eq_point[j]}) {
+        f.push_back(v);
+        pre.push_back(p);
+        p = p * v;
+      }
+    F128 q = inv(p);
+    for (size_t i = f.size(); i-- > 0;) {
+      const F128 v = f[i];
+      f[i] = q * pre[i];
+      q = q * v;
+    }
+    launch_factor_table(upload(f), L - zc_w_, zc_inv_, st_);
   }
   auto v = reduce(nb, 2);
   g1 = v[0];
@@ -633,7 +673,8 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
   uint64_t n_pairs = zc_len_ / 4;
   if ((uint64_t(1) << eq_point.size()) != n_pairs) throw std::runtime_error("zerocheck fold: eq size mismatch");
   size_t k = 2 + 2 * zc_round_;
-  if (k + 1 >= zc_desc_.size() || zc_desc_[k].n + zc_desc_[k + 1].n != eq_point.size())
+  if (k + 1 >= zc_desc_.size() ||
+      zc_desc_[k].n + (zc_round_ < zc_w_ ? zc_desc_[1].n : zc_desc_[k + 1].n) != eq_point.size())
     throw std::runtime_error("zerocheck fold: round tables out of step");
   const EqDesc& lo = zc_desc_[k];
   const EqDesc& hi = zc_desc_[k + 1];
@@ -645,14 +686,20 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
   uint32_t nb, pub_seq = 0;
   {
     Mark mk(this, ST_ZC_FOLDS);
-    if (zc_round_ == 0) {
+    const F128d* elo = zc_tabs_ + lo.out_off;
+    const bool weighted = zc_round_ < zc_w_;  // the low coordinates of the weighted form
+    const F128d* ehi = weighted ? nullptr : zc_tabs_ + hi.out_off;
+    if (zc_round_ == 0 && weighted) {
+      nb = launch_zc_fold2_weighted(a_, b_, zc_w64_, dev(rho), n_pairs, live_pairs, zc_w_, elo,
+                                    zc_tabs_ + zc_desc_[1].out_off, oa, ob, part_, st_);
+    } else if (zc_round_ == 0) {
       F128d* tabs = static_cast<F128d*>(scratch(4096 * sizeof(F128d)));
-      nb = launch_zc_fold2(a_, b_, zc_w64_, dev(rho), tabs, n_pairs, live_pairs, zc_tabs_ + lo.out_off, lo.n,
-                           zc_tabs_ + hi.out_off, oa, ob, part_, st_);
+      nb = launch_zc_fold2(a_, b_, zc_w64_, dev(rho), tabs, n_pairs, live_pairs, elo, lo.n, ehi, oa, ob, part_, st_);
     } else {
       FusedPublish fp = fused_publish();
-      launch_pair_fold(zc_cur_a_, zc_cur_b_, n_pairs, live_pairs, dev(rho), nullptr, zc_tabs_ + lo.out_off, lo.n,
-                       zc_tabs_ + hi.out_off, oa, ob, part_, true, st_, fp);
+      // the first fold past the weighted rounds divides by h
+      launch_pair_fold(zc_cur_a_, zc_cur_b_, n_pairs, live_pairs, dev(rho), elo, lo.n, ehi,
+                       zc_w_ && zc_round_ == zc_w_ ? zc_inv_ : nullptr, oa, ob, part_, st_, fp);
       nb = 0;
       pub_seq = fp.seq;
     }
@@ -855,14 +902,10 @@ void GpuBackend::mo_round(F128 r, bool last, F128& g1, F128& gi) {
     oq = d_tail_;
     ow = d_tail_ + lanes_pow2();
   }
-  // chunking only sets the work split: 2^10 pairs per chunk for the table form's rounds,
-  // 2^8 (one pair per thread) for the small, latency-bound ones
-  uint32_t chunk_bits = std::min<uint32_t>(n_pairs >= (uint64_t(1) << 17) ? 10 : 8, ceil_log2(n_pairs));
   FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_MO_ROUNDS);
-    launch_pair_fold(mo_q_, mo_w_, n_pairs, live_pairs, dev(r), nullptr, nullptr, chunk_bits, nullptr, oq, ow, part_,
-                     true, st_, fp);
+    launch_pair_fold(mo_q_, mo_w_, n_pairs, live_pairs, dev(r), nullptr, 0, nullptr, nullptr, oq, ow, part_, st_, fp);
   }
   mo_q_ = oq;
   mo_w_ = ow;

@@ -246,6 +246,10 @@ class GpuBackend : public ProverBackend {
   F128d* zc_tabs_ = nullptr;
   uint64_t zc_tabs_cap_ = 0;
   std::vector<EqDesc> zc_desc_;
+  // low bits of the weighted form's chunks in this prove (0: the plain form), and the
+  // reciprocals of its chunk weights
+  uint32_t zc_w_ = 0;
+  F128d* zc_inv_ = nullptr;
 
   std::mutex pow_mu_;
   cudaStream_t pow_st_ = nullptr;

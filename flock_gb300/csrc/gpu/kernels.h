@@ -80,6 +80,18 @@ uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, u
 uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d rho, F128d* tabs, uint64_t n_pairs,
                          uint64_t live_pairs, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* aout,
                          F128d* bout, F128d* part, cudaStream_t s);                                     // width 2
+// The weighted form (see the kernels): low bits of its chunks for this many live words, 0 where
+// the plain form runs; the skip fold's message and the first fold with its message. eq_lo: eq
+// over the chunk's low coordinates (of words, then of pairs), h: eq over the high ones.
+uint32_t zc_weighted_lo_bits(uint64_t live_words);
+uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
+                                      uint32_t lo_bits, const F128d* eq_lo, const F128d* h, F128d* part,
+                                      cudaStream_t s);                                                   // width 2
+uint32_t launch_zc_fold2_weighted(const F128d* a, const F128d* b, const F128d* w64, F128d rho, uint64_t n_pairs,
+                                  uint64_t live_pairs, uint32_t lo_bits, const F128d* eq_lo, const F128d* h,
+                                  F128d* aout, F128d* bout, F128d* part, cudaStream_t s);                // width 2
+// out[c] = prod_j f[2j + bit j of c] over n factor pairs.
+void launch_factor_table(const F128d* f, uint32_t n, F128d* out, cudaStream_t s);
 // In-kernel publication of a round message: the last block to finish (a device-wide
 // ticket counter) XOR-reduces every block's partials, writes the message to mapped host
 // memory and then the sequence number, as launch_reduce_publish does in a launch of its
@@ -90,12 +102,12 @@ struct FusedPublish {
   uint32_t* counter = nullptr; // device memory
   uint32_t seq = 0;
 };
-// r_dev (when not null) is the device address of the challenge, read by the kernel. Pairs
-// from live_pairs on have zero inputs (zeros written, nothing added to the message).
+// eq_lo == nullptr: eq = 1; eq_hi == nullptr: eq(j) = eq_lo[j mod 2^lo_bits]; else the split eq.
+// unweight (or null): factors of the folded a entries. Pairs from live_pairs on have zero
+// inputs (zeros written, nothing added to the message).
 uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, uint64_t live_pairs, F128d r,
-                          const F128d* r_dev, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* aout,
-                          F128d* bout, F128d* part, bool msg, cudaStream_t s,
-                          FusedPublish pub = FusedPublish());  // width 2
+                          const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, const F128d* unweight, F128d* aout,
+                          F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub);  // width 2
 
 void launch_lc_eq_inner(const F128d* w64, const F128d* er, uint32_t K, F128d* eqi, cudaStream_t s);
 void launch_csc_fold(const uint32_t* col_ptr, const uint32_t* rows, uint32_t K, const F128d* eqi, F128d* out,

@@ -331,11 +331,9 @@ void JaggedAssist::fold(F128 r, F128& g1, F128& gi) {
   if (len_ < 4) throw std::runtime_error("assist: no fold left");
   const int nx = cur_ == 1 ? 2 : 1;
   const uint64_t n_pairs = len_ / 4;
-  uint32_t chunk = n_pairs >= (uint64_t(1) << 17) ? 10 : 8;  // as the merged open's rounds: only the work split
-  while ((uint64_t(1) << chunk) > n_pairs) --chunk;
   FusedPublish fp = publish();
-  launch_pair_fold(a_[cur_], g_[cur_], n_pairs, n_pairs, dev(r), nullptr, nullptr, chunk, nullptr, a_[nx], g_[nx],
-                   part_, true, st_, fp);
+  launch_pair_fold(a_[cur_], g_[cur_], n_pairs, n_pairs, dev(r), nullptr, 0, nullptr, nullptr, a_[nx], g_[nx], part_, st_,
+                   fp);
   cur_ = nx;
   len_ /= 2;
   read(fp, g1, gi);

@@ -415,55 +415,65 @@ zc_fold_skip_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, co
   }
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
 }
-// The same message with the eq factors applied in the other order, for chunks of 1024
-// words (lo_bits = 10) and 256 threads: thread t sees the four low indices l = t + 256 k of
-// every chunk, so
-//   g1 = sum_k eq_lo[l_k] S1_k,  S1_k = sum_chunks eq_hi[chunk] (a1 b1)[chunk 1024 + l_k]
-// (ginf alike), and each per-word product by eq_lo becomes a product by the chunk's eq_hi,
-// taken from the chunk's byte tables on the load/store pipe; eq_lo enters in eight
-// products per thread at the end. Per word two products of variables stay on the multiply
-// pipe instead of four.
-constexpr uint32_t ZC_SKIP_DEFER_LO_BITS = 10;
-__global__ void __launch_bounds__(256, 2)
-zc_fold_skip_defer_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ w64,
-                          uint64_t n_chunks, const F128d* __restrict__ eq_lo, const F128d* __restrict__ eq_hi,
-                          F128d* __restrict__ part) {
-  __shared__ F128d T[8][256];
+// ---- the weighted form of the zerocheck rounds
+// The eq factor of a message over words is eq_lo(low coordinates) * h(chunk), a chunk being
+// the 2^LO words that share the high coordinates. a enters every message linearly
+// and comes out of tables of the weights, so h is multiplied into a's tables once per chunk:
+// the vector kept is a~ = h a, which folds over the low coordinates like a does. eq_lo is left
+// to the end: a thread's words (later its pairs) have low indices that do not change from
+// chunk to chunk, so it sums a~ b per low index and multiplies each sum by eq_lo once. What is
+// left of a message are its two products of variables; the plain form has four (and the
+// table form before took two of them from byte tables rebuilt for every 1024 words). When the
+// low coordinates are used up, the fold divides by h once (pair_fold's `unweight`), which needs
+// every high coordinate to differ from 0 and 1; otherwise the plain form runs.
+// All lookups are from window tables (wintable.cuh). Keccak-f 2^18 (87 M live words): skip fold
+// 8.05 -> 5.59 ms, folds 12.4 -> 8.4; SHA-256 2^16: 1.25 -> 0.88, 2.25 -> 1.64; BLAKE3 2^12: 83 ->
+// 61 us, 0.39 -> 0.37 ms.
+//
+// Skip fold: tables of h w64 (for a) and w64 (for b), six-bit windows, 2 x 82 KB, one block per
+// SM; 44 lookups (5.5 cycles of the shared-memory pipe) and two products (13 of the multiply
+// pipe) a word.
+constexpr uint32_t ZC_W_THREADS = 512;
+template <int LO>
+__global__ void __launch_bounds__(ZC_W_THREADS, 1)
+zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ w64,
+                             uint64_t n_chunks, uint64_t n_words, const F128d* __restrict__ eq_lo,
+                             const F128d* __restrict__ h, F128d* __restrict__ part) {
+  constexpr uint32_t PER = (1u << LO) / ZC_W_THREADS;
+  extern __shared__ __align__(16) char wt[];  // a's table, then b's
+  __shared__ F128d img[64];
   __shared__ F128d sh[32];
-  extern __shared__ __align__(16) F128d htab[];  // build_byte_table's BYTE_TABLE_SMEM_ENTRIES
-  for (uint32_t e = threadIdx.x; e < 2048; e += blockDim.x) {
-    uint32_t c = e >> 8, v = e & 255;
-    F128d acc = f128_zero();
-    for (int k = 0; k < 8; ++k)
-      if ((v >> k) & 1) acc += w64[8 * c + k];
-    T[c][v] = acc;
-  }
-  F128d S1[4], SI[4];
+  const uint32_t lane = win_lane(), team = threadIdx.x >> 3, teams = ZC_W_THREADS / 8;
+  char* TB = wt + WinMap<6, 64>::BYTES;
+  build_win_map<6, 64>(w64, TB, team, teams);
+  F128d S1[PER], SI[PER];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) S1[k] = SI[k] = f128_zero();
+  for (uint32_t k = 0; k < PER; ++k) S1[k] = SI[k] = f128_zero();
   for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    __syncthreads();  // T is complete; the previous chunk's table is no longer read
-    build_byte_table(eq_hi[ch], htab);
+    __syncthreads();  // the previous chunk's table is no longer read
+    if (threadIdx.x < 64) img[threadIdx.x] = mul_call(h[ch], w64[threadIdx.x]);
+    __syncthreads();
+    build_win_map<6, 64>(img, wt, team, teams);
+    __syncthreads();
+    const uint64_t w0 = (ch << LO) + threadIdx.x;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t wi = (ch << ZC_SKIP_DEFER_LO_BITS) + threadIdx.x + 256 * k;
+    for (uint32_t k = 0; k < PER; ++k) {
+      const uint64_t wi = w0 + k * ZC_W_THREADS;
+      if (wi >= n_words) continue;  // a zero tail
       const F128d av = a[wi], bv = b[wi];
       F128d a0 = f128_zero(), a1 = f128_zero(), b0 = f128_zero(), b1 = f128_zero();
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        a0 += T[c][(av.lo >> (8 * c)) & 255];
-        a1 += T[c][(av.hi >> (8 * c)) & 255];
-        b0 += T[c][(bv.lo >> (8 * c)) & 255];
-        b1 += T[c][(bv.hi >> (8 * c)) & 255];
-      }
-      S1[k] += mul_table(mul_call(a1, b1), htab);
-      SI[k] += mul_table(mul_call(a0 + a1, b0 + b1), htab);
+      add_win_map64<6>(a1, av.hi, wt, lane);
+      add_win_map64<6>(b1, bv.hi, TB, lane);
+      S1[k] += mul_call(a1, b1);
+      add_win_map64<6>(a0, av.lo, wt, lane);
+      add_win_map64<6>(b0, bv.lo, TB, lane);
+      SI[k] += mul_call(a0 + a1, b0 + b1);
     }
   }
   F128d G1 = f128_zero(), GI = f128_zero();
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const F128d e = eq_lo[threadIdx.x + 256 * k];
+  for (uint32_t k = 0; k < PER; ++k) {
+    const F128d e = eq_lo[threadIdx.x + k * ZC_W_THREADS];
     G1 += mul_call(e, S1[k]);
     GI += mul_call(e, SI[k]);
   }
@@ -471,19 +481,35 @@ zc_fold_skip_defer_kernel(const F128d* __restrict__ a, const F128d* __restrict__
   GI = block_xor(GI, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
 }
+// A chunk's tables are rebuilt for it (about 2000 cycles beside 13 a word), so chunks are as
+// long as leaves every SM four, down to 2^10 words with one an SM; smaller vectors take the
+// plain form, whose launches are bound by latency.
+uint32_t zc_weighted_lo_bits(uint64_t live_words) {
+  const uint64_t sms = (uint64_t)sm_count();
+  if ((live_words >> 12) >= 4 * sms) return 12;
+  if ((live_words >> 11) >= 4 * sms) return 11;
+  return (live_words >> 10) >= sms ? 10 : 0;
+}
+template <int LO>
+static uint32_t fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
+                                   const F128d* eq_lo, const F128d* h, F128d* part, cudaStream_t s) {
+  const uint64_t n_chunks = (n_words + (1ull << LO) - 1) >> LO;
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count());
+  const int smem = 2 * WinMap<6, 64>::BYTES;
+  set_dynamic_smem((const void*)zc_fold_skip_weighted_kernel<LO>, smem);
+  zc_fold_skip_weighted_kernel<LO><<<blocks, ZC_W_THREADS, smem, s>>>(a, b, w64, n_chunks, n_words, eq_lo, h, part);
+  LAUNCH_OK();
+  return blocks;
+}
+uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
+                                      uint32_t lo_bits, const F128d* eq_lo, const F128d* h, F128d* part,
+                                      cudaStream_t s) {
+  if (lo_bits == 12) return fold_skip_weighted<12>(a, b, w64, n_words, eq_lo, h, part, s);
+  if (lo_bits == 11) return fold_skip_weighted<11>(a, b, w64, n_words, eq_lo, h, part, s);
+  return fold_skip_weighted<10>(a, b, w64, n_words, eq_lo, h, part, s);
+}
 uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words, const F128d* eq_lo,
                              uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s) {
-  if (eq_hi && lo_bits == ZC_SKIP_DEFER_LO_BITS && (n_words & ((1ull << lo_bits) - 1)) == 0 &&
-      (n_words >> lo_bits) >= (uint64_t)sm_count() * 8) {
-    // two resident blocks per SM, each looping over its share of the chunks
-    const uint64_t n_chunks = n_words >> lo_bits;
-    const uint32_t blocks = (uint32_t)sm_count() * 2;
-    const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-    set_dynamic_smem((const void*)zc_fold_skip_defer_kernel, smem);
-    zc_fold_skip_defer_kernel<<<blocks, 256, smem, s>>>(a, b, w64, n_chunks, eq_lo, eq_hi, part);
-    LAUNCH_OK();
-    return blocks;
-  }
   uint64_t n_chunks = (n_words + (1ull << lo_bits) - 1) >> lo_bits;
   uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
   zc_fold_skip_kernel<<<blocks, 256, 0, s>>>(a, b, w64, n_words, eq_lo, lo_bits, eq_hi, part);
@@ -578,98 +604,272 @@ uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d
   return blocks;
 }
 
+// The weighted form of the first fold (see above): per chunk the tables of h (1 + rho) w and
+// h rho w for a, once per block those of (1 + rho) w and rho w for b, five-bit windows, 4 x 50
+// KB, one block per SM; 104 lookups (13 cycles) and two products (13) a pair.
+template <int LO>
+__global__ void __launch_bounds__(ZC_W_THREADS, 1)
+zc_fold2_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ w64,
+                         F128d rho, uint64_t n_pairs, uint64_t live_pairs, const F128d* __restrict__ eq_lo,
+                         const F128d* __restrict__ h, F128d* __restrict__ aout, F128d* __restrict__ bout,
+                         F128d* __restrict__ part) {
+  constexpr uint32_t PAIRS = 1u << (LO - 1), PER = PAIRS / ZC_W_THREADS, TAB = WinMap<5, 64>::BYTES;
+  extern __shared__ __align__(16) char wt[];  // a's tables for the low and high halves, then b's
+  __shared__ F128d wr[2][64], img[2][64];
+  __shared__ F128d sh[32];
+  const uint32_t lane = win_lane();
+  // two halves of the block build the two tables of a vector
+  const uint32_t half = threadIdx.x >= ZC_W_THREADS / 2, team = (threadIdx.x & (ZC_W_THREADS / 2 - 1)) >> 3,
+                 teams = ZC_W_THREADS / 16;
+  if (threadIdx.x < 64) {
+    const F128d v = mul_call(rho, w64[threadIdx.x]);
+    wr[1][threadIdx.x] = v;                    // rho w
+    wr[0][threadIdx.x] = v + w64[threadIdx.x];  // (1 + rho) w
+  }
+  __syncthreads();
+  build_win_map<5, 64>(wr[half], wt + (2 + half) * TAB, team, teams);
+  F128d S1[PER], SI[PER];
+#pragma unroll
+  for (uint32_t k = 0; k < PER; ++k) S1[k] = SI[k] = f128_zero();
+  const uint64_t n_chunks = (n_pairs + PAIRS - 1) / PAIRS;
+  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
+    const bool live = ch * PAIRS < live_pairs;  // block-uniform
+    if (live) {
+      __syncthreads();  // the previous chunk's tables are no longer read
+      if (threadIdx.x < 128) img[threadIdx.x >> 6][threadIdx.x & 63] = mul_call(h[ch], wr[threadIdx.x >> 6][threadIdx.x & 63]);
+      __syncthreads();
+      build_win_map<5, 64>(img[half], wt + half * TAB, team, teams);
+      __syncthreads();
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < PER; ++k) {
+      const uint64_t j = ch * PAIRS + threadIdx.x + k * ZC_W_THREADS;
+      if (j >= n_pairs) continue;
+      if (j >= live_pairs) {  // zero words: zero outputs, nothing added to the message
+        aout[2 * j] = aout[2 * j + 1] = bout[2 * j] = bout[2 * j + 1] = f128_zero();
+        continue;
+      }
+      F128d A[2], B[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const F128d av = a[2 * j + q], bv = b[2 * j + q];
+        A[q] = B[q] = f128_zero();
+        add_win_map64<5>(A[q], av.lo, wt, lane);
+        add_win_map64<5>(A[q], av.hi, wt + TAB, lane);
+        add_win_map64<5>(B[q], bv.lo, wt + 2 * TAB, lane);
+        add_win_map64<5>(B[q], bv.hi, wt + 3 * TAB, lane);
+        aout[2 * j + q] = A[q];
+        bout[2 * j + q] = B[q];
+      }
+      S1[k] += mul_call(A[1], B[1]);
+      SI[k] += mul_call(A[0] + A[1], B[0] + B[1]);
+    }
+  }
+  F128d G1 = f128_zero(), GI = f128_zero();
+#pragma unroll
+  for (uint32_t k = 0; k < PER; ++k) {
+    const F128d e = eq_lo[threadIdx.x + k * ZC_W_THREADS];
+    G1 += mul_call(e, S1[k]);
+    GI += mul_call(e, SI[k]);
+  }
+  G1 = block_xor(G1, sh);
+  GI = block_xor(GI, sh);
+  if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+}
+template <int LO>
+static uint32_t fold2_weighted(const F128d* a, const F128d* b, const F128d* w64, F128d rho, uint64_t n_pairs,
+                               uint64_t live_pairs, const F128d* eq_lo, const F128d* h, F128d* aout, F128d* bout,
+                               F128d* part, cudaStream_t s) {
+  const int smem = 4 * WinMap<5, 64>::BYTES;
+  set_dynamic_smem((const void*)zc_fold2_weighted_kernel<LO>, smem);
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>((n_pairs + (1ull << (LO - 1)) - 1) >> (LO - 1), (uint64_t)sm_count());
+  zc_fold2_weighted_kernel<LO><<<blocks, ZC_W_THREADS, smem, s>>>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout,
+                                                                  bout, part);
+  LAUNCH_OK();
+  return blocks;
+}
+uint32_t launch_zc_fold2_weighted(const F128d* a, const F128d* b, const F128d* w64, F128d rho, uint64_t n_pairs,
+                                  uint64_t live_pairs, uint32_t lo_bits, const F128d* eq_lo, const F128d* h,
+                                  F128d* aout, F128d* bout, F128d* part, cudaStream_t s) {
+  live_pairs = std::min(live_pairs, n_pairs);
+  if (lo_bits == 12) return fold2_weighted<12>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s);
+  if (lo_bits == 11) return fold2_weighted<11>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s);
+  return fold2_weighted<10>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s);
+}
+// out[c] = prod_j (bit j of c ? f[2j + 1] : f[2j]), j < n: the reciprocals of an eq table from
+// those of its factors.
+__global__ void factor_table_kernel(const F128d* __restrict__ f, uint32_t n, F128d* __restrict__ out) {
+  const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= (1ull << n)) return;
+  F128d v = f128_one();
+  for (uint32_t j = 0; j < n; ++j) v = mul_call(v, f[2 * j + ((c >> j) & 1)]);
+  out[c] = v;
+}
+void launch_factor_table(const F128d* f, uint32_t n, F128d* out, cudaStream_t s) {
+  factor_table_kernel<<<(unsigned)(((1ull << n) + 255) / 256), 256, 0, s>>>(f, n, out);
+  LAUNCH_OK();
+}
+
 // ------------------------------------------------------------------ pair fold + message
-// Folds of at least this many pairs take their products by r from byte tables. A block's
-// table build costs about as much shared-memory traffic as 300 table products, so the
-// table form also keeps at least PAIR_FOLD_TABLE_MIN_BLOCK_PAIRS pairs (4 table products
-// each) per block.
-constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;
-constexpr uint64_t PAIR_FOLD_TABLE_MIN_BLOCK_PAIRS = 512;
-// Fold the low variable of two vectors at r (out[i] = in[2i] + r (in[2i+1] + in[2i]))
-// and, unless `msg` is false, emit the pair message over the folded vectors:
+// Fold the low variable of two vectors at r (out[i] = in[2i] + r (in[2i+1] + in[2i])) and emit
+// the pair message over the folded vectors:
 //   g1 = sum_j eq(j) A1 B1, ginf = sum_j eq(j) (A0 + A1)(B0 + B1), (A0, A1) = out[2j..2j+2).
-// eq_lo == nullptr means eq = 1. n_pairs = output length / 2 (>= 1).
-// TBL: the four products by r come from byte tables of r in shared memory (load/store
-// pipe) while the message's products of two variables stay integer multiplies; the
-// block builds its table first, so this form is used where each block folds enough pairs
-// to pay for that. Otherwise r is split once per block for mul_split.
-template <bool TBL>
-__global__ void __launch_bounds__(256, TBL ? 3 : 2)
+// n_pairs = output length / 2 (>= 1). eq by mode:
+enum PairEq : int {
+  EQ_NONE,   // eq = 1
+  EQ_FIXED,  // eq(j) = eq_lo[j mod 2^lo_bits] (the zerocheck's weighted form): the grid's thread
+             // count is a multiple of 2^lo_bits, so a thread multiplies its sum by eq_lo once
+  EQ_SPLIT,  // eq(j) = eq_lo[j mod 2^lo_bits] eq_hi[j >> lo_bits], one eq_hi per chunk
+};
+// Folds of at least this many pairs take their products by r from the window table of r (six
+// bits, 169 KB, one block per SM): four table products (11 cycles of the shared-memory pipe)
+// beside the message's two products of variables (13 of the multiply pipe). The byte tables it
+// replaced (three 256-thread blocks per SM) took 4.8 ms for the merged open's rounds of Keccak-f
+// 2^18, this form 3.5. Below the threshold a block would fold less than two rounds of its threads.
+constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;
+constexpr uint32_t PAIR_FOLD_TABLE_THREADS = 512;
+template <int EQ>
+__global__ void __launch_bounds__(PAIR_FOLD_TABLE_THREADS, 1)
+pair_fold_tbl_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bin, uint64_t n_pairs, uint64_t live_pairs,
+                     F128d r, const F128d* __restrict__ eq_lo, uint32_t lo_bits, F128d* __restrict__ aout,
+                     F128d* __restrict__ bout, F128d* __restrict__ part, FusedPublish pub) {
+  extern __shared__ __align__(16) char wt[];  // WinTable<6>
+  __shared__ F128d sh[32];
+  build_win_table<6>(r, wt);
+  __syncthreads();
+  const uint32_t lane = win_lane();
+  const uint64_t j0 = (uint64_t)blockIdx.x * PAIR_FOLD_TABLE_THREADS + threadIdx.x;
+  MulAcc m1, mi;
+  for (uint64_t j = j0; j < n_pairs; j += (uint64_t)gridDim.x * PAIR_FOLD_TABLE_THREADS) {
+    if (j >= live_pairs) {  // zero inputs: zero outputs, nothing added to the message
+      aout[2 * j] = aout[2 * j + 1] = bout[2 * j] = bout[2 * j + 1] = f128_zero();
+      continue;
+    }
+    const F128d x0 = ain[4 * j], x1 = ain[4 * j + 1], x2 = ain[4 * j + 2], x3 = ain[4 * j + 3];
+    const F128d y0 = bin[4 * j], y1 = bin[4 * j + 1], y2 = bin[4 * j + 2], y3 = bin[4 * j + 3];
+    const F128d A0 = x0 + mul_win<6>(x1 + x0, wt, lane), A1 = x2 + mul_win<6>(x3 + x2, wt, lane);
+    const F128d B0 = y0 + mul_win<6>(y1 + y0, wt, lane), B1 = y2 + mul_win<6>(y3 + y2, wt, lane);
+    aout[2 * j] = A0; aout[2 * j + 1] = A1;
+    bout[2 * j] = B0; bout[2 * j + 1] = B1;
+    m1.add(A1, B1);
+    mi.add(A0 + A1, B0 + B1);
+  }
+  F128d g1 = m1.value(), gi = mi.value();
+  if (EQ == EQ_FIXED) {
+    const F128d e = eq_lo[j0 & ((1ull << lo_bits) - 1)];
+    g1 = mul_call(e, g1);
+    gi = mul_call(e, gi);
+  }
+  g1 = block_xor(g1, sh);
+  gi = block_xor(gi, sh);
+  if (threadIdx.x == 0) { part[blockIdx.x * 2] = g1; part[blockIdx.x * 2 + 1] = gi; }
+  publish_if_last(part, 2, pub, sh);
+}
+// The same with r split once per block for mul_split (small, latency-bound rounds). unweight
+// (when not null): the folded a entry i is multiplied by unweight[i] before it is stored.
+template <int EQ>
+__global__ void __launch_bounds__(256, 2)
 pair_fold_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bin, uint64_t n_pairs, uint64_t live_pairs,
-                 F128d r, const F128d* __restrict__ r_dev, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
-                 const F128d* __restrict__ eq_hi, F128d* __restrict__ aout, F128d* __restrict__ bout,
-                 F128d* __restrict__ part, int msg, FusedPublish pub) {
-  extern __shared__ __align__(16) F128d rtab[];  // TBL: build_byte_table's BYTE_TABLE_SMEM_ENTRIES
+                 F128d r, const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi,
+                 const F128d* __restrict__ unweight, F128d* __restrict__ aout, F128d* __restrict__ bout,
+                 F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d sh[32];
   __shared__ F128split rs;  // the fold challenge, split once
-  if (TBL) {
-    build_byte_table(r_dev ? *r_dev : r, rtab);
-  } else {
-    if (threadIdx.x == 0) rs = split_factor(r_dev ? *r_dev : r);
-    __syncthreads();
-  }
-  auto by_r = [&](F128d v) { return TBL ? mul_table(v, rtab) : mul_split_call(v, &rs); };
-  const uint64_t chunk = 1ull << lo_bits;
-  const uint64_t n_chunks = (n_pairs + chunk - 1) / chunk;
+  if (threadIdx.x == 0) rs = split_factor(r);
+  __syncthreads();
+  // pairs are walked in chunks of 2^lo_bits under EQ_SPLIT, with the grid's stride otherwise
+  const uint64_t chunk = EQ == EQ_SPLIT ? 1ull << lo_bits : n_pairs;
+  const uint64_t n_chunks = EQ == EQ_SPLIT ? (n_pairs + chunk - 1) / chunk : 1;
+  const uint64_t j0 = EQ == EQ_SPLIT ? threadIdx.x : (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t step = EQ == EQ_SPLIT ? blockDim.x : (uint64_t)gridDim.x * blockDim.x;
   F128d G1 = f128_zero(), GI = f128_zero();
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
+  for (uint64_t ch = EQ == EQ_SPLIT ? blockIdx.x : 0; ch < n_chunks; ch += EQ == EQ_SPLIT ? gridDim.x : 1) {
     F128d g1 = f128_zero(), gi = f128_zero();
-    uint64_t end = min(n_pairs, (ch + 1) * chunk);
-    for (uint64_t j = ch * chunk + threadIdx.x; j < end; j += blockDim.x) {
+    const uint64_t end = min(n_pairs, (ch + 1) * chunk);
+    for (uint64_t j = ch * chunk + j0; j < end; j += step) {
       if (j >= live_pairs) {  // zero inputs: zero outputs, nothing added to the message
         aout[2 * j] = aout[2 * j + 1] = bout[2 * j] = bout[2 * j + 1] = f128_zero();
         continue;
       }
       F128d x0 = ain[4 * j], x1 = ain[4 * j + 1], x2 = ain[4 * j + 2], x3 = ain[4 * j + 3];
       F128d y0 = bin[4 * j], y1 = bin[4 * j + 1], y2 = bin[4 * j + 2], y3 = bin[4 * j + 3];
-      F128d A0 = x0 + by_r(x1 + x0), A1 = x2 + by_r(x3 + x2);
-      F128d B0 = y0 + by_r(y1 + y0), B1 = y2 + by_r(y3 + y2);
+      F128d A0 = x0 + mul_split_call(x1 + x0, &rs), A1 = x2 + mul_split_call(x3 + x2, &rs);
+      F128d B0 = y0 + mul_split_call(y1 + y0, &rs), B1 = y2 + mul_split_call(y3 + y2, &rs);
+      if (unweight) {
+        A0 = mul_call(A0, unweight[2 * j]);
+        A1 = mul_call(A1, unweight[2 * j + 1]);
+      }
       aout[2 * j] = A0; aout[2 * j + 1] = A1;
       bout[2 * j] = B0; bout[2 * j + 1] = B1;
-      if (msg) {
-        F128d t1 = mul_call(A1, B1), ti = mul_call(A0 + A1, B0 + B1);
-        if (eq_lo) {
-          F128d e = eq_lo[j & (chunk - 1)];
-          t1 = mul_call(e, t1);
-          ti = mul_call(e, ti);
-        }
-        g1 += t1;
-        gi += ti;
+      F128d t1 = mul_call(A1, B1), ti = mul_call(A0 + A1, B0 + B1);
+      if (EQ == EQ_SPLIT) {
+        F128d e = eq_lo[j & (chunk - 1)];
+        t1 = mul_call(e, t1);
+        ti = mul_call(e, ti);
       }
+      g1 += t1;
+      gi += ti;
     }
-    if (msg) {
-      g1 = block_xor(g1, sh);
-      gi = block_xor(gi, sh);
-      if (threadIdx.x == 0) {
-        F128d h = (eq_lo && eq_hi) ? eq_hi[ch] : f128_one();
-        G1 += h * g1;
-        GI += h * gi;
-      }
+    if (EQ == EQ_FIXED) {
+      const F128d e = eq_lo[j0 & ((1ull << lo_bits) - 1)];
+      g1 = mul_call(e, g1);
+      gi = mul_call(e, gi);
+    }
+    g1 = block_xor(g1, sh);
+    gi = block_xor(gi, sh);
+    if (threadIdx.x == 0) {
+      const F128d h = EQ == EQ_SPLIT && eq_hi ? eq_hi[ch] : f128_one();
+      G1 += h * g1;
+      GI += h * gi;
     }
   }
-  if (msg && threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
-  if (msg && pub.out) publish_if_last(part, 2, pub, sh);
+  if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+  publish_if_last(part, 2, pub, sh);
 }
 uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, uint64_t live_pairs, F128d r,
-                          const F128d* r_dev, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* aout,
-                          F128d* bout, F128d* part, bool msg, cudaStream_t s, FusedPublish pub) {
+                          const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, const F128d* unweight, F128d* aout,
+                          F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub) {
   live_pairs = std::min(live_pairs, n_pairs);
-  uint64_t n_chunks = (n_pairs + (1ull << lo_bits) - 1) >> lo_bits;
-  if (n_pairs >= PAIR_FOLD_TABLE_MIN_PAIRS) {
-    // three resident blocks per SM (74 KB of shared memory each), each building its table
-    // once for its share of the chunks
-    const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-    set_dynamic_smem((const void*)pair_fold_kernel<true>, smem);
-    uint32_t blocks = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 6),
-                                                   n_pairs / PAIR_FOLD_TABLE_MIN_BLOCK_PAIRS);
-    pair_fold_kernel<true><<<blocks, 256, smem, s>>>(ain, bin, n_pairs, live_pairs, r, r_dev, eq_lo, lo_bits, eq_hi,
-                                                     aout, bout, part, msg ? 1 : 0, pub);
+  const bool fixed = eq_lo && !eq_hi;
+  if (n_pairs >= PAIR_FOLD_TABLE_MIN_PAIRS && !eq_hi && !unweight) {
+    // one block per SM; under EQ_FIXED a multiple of 2^lo_bits threads in all
+    const int smem = WinTable<6>::BYTES;
+    uint32_t blocks = (uint32_t)sm_count();
+    if (fixed && (1u << lo_bits) > PAIR_FOLD_TABLE_THREADS) {
+      const uint32_t q = (1u << lo_bits) / PAIR_FOLD_TABLE_THREADS;
+      blocks = std::max(q, blocks / q * q);
+    }
+    if (fixed) {
+      set_dynamic_smem((const void*)pair_fold_tbl_kernel<EQ_FIXED>, smem);
+      pair_fold_tbl_kernel<EQ_FIXED><<<blocks, PAIR_FOLD_TABLE_THREADS, smem, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo,
+                                                                                   lo_bits, aout, bout, part, pub);
+    } else {
+      set_dynamic_smem((const void*)pair_fold_tbl_kernel<EQ_NONE>, smem);
+      pair_fold_tbl_kernel<EQ_NONE><<<blocks, PAIR_FOLD_TABLE_THREADS, smem, s>>>(ain, bin, n_pairs, live_pairs, r, nullptr,
+                                                                                  0, aout, bout, part, pub);
+    }
     LAUNCH_OK();
     return blocks;
   }
-  uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
-  pair_fold_kernel<false><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, r_dev, eq_lo, lo_bits, eq_hi, aout,
-                                                 bout, part, msg ? 1 : 0, pub);
+  if (eq_hi) {
+    const uint64_t n_chunks = (n_pairs + (1ull << lo_bits) - 1) >> lo_bits;
+    const uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
+    pair_fold_kernel<EQ_SPLIT><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo, lo_bits, eq_hi, unweight,
+                                                      aout, bout, part, pub);
+    LAUNCH_OK();
+    return blocks;
+  }
+  uint32_t blocks = (uint32_t)std::min<uint64_t>((n_pairs + 255) / 256, (uint64_t)sm_count() * 8);
+  if (fixed && (uint64_t)blocks * 256 < n_pairs && (1u << lo_bits) > 256) {
+    const uint32_t q = (1u << lo_bits) / 256;
+    blocks = std::max(q, blocks / q * q);
+  }
+  if (fixed)
+    pair_fold_kernel<EQ_FIXED><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo, lo_bits, nullptr, unweight,
+                                                      aout, bout, part, pub);
+  else
+    pair_fold_kernel<EQ_NONE><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, nullptr, 0, nullptr, unweight, aout,
+                                                     bout, part, pub);
   LAUNCH_OK();
   return blocks;
 }

@@ -75,6 +75,66 @@ __device__ __forceinline__ void build_win_table(F128d c, char* T) {
   }
 }
 
+// The table of any GF(2)-linear map of the low `BITS` bits of a word from the map's images
+// E[i] of x^i (readable by every thread: shared or global memory), the same walk.
+template <int W, int BITS>
+struct WinMap {
+  static constexpr int WINDOWS = (BITS + W - 1) / W;
+  static constexpr int TOP_BITS = BITS - W * (WINDOWS - 1);
+  static constexpr int ENTRIES = (WINDOWS - 1) * (1 << W) + (1 << TOP_BITS);
+  static constexpr int BYTES = ENTRIES * 128;
+};
+// `teams` groups of eight threads share the work; this thread's is `team` (whole warps call).
+template <int W, int BITS>
+__device__ __forceinline__ void build_win_map(const F128d* E, char* T, uint32_t team, uint32_t teams) {
+  using WM = WinMap<W, BITS>;
+  constexpr int LOW = W - 1;
+  constexpr int ITEMS = WM::WINDOWS * 2;
+  const uint32_t r = threadIdx.x & 7;
+  for (uint32_t it = team; it < ITEMS; it += teams) {
+    const uint32_t k = it >> 1, part = it & 1;
+    F128d e[W];
+#pragma unroll
+    for (int b = 0; b < W; ++b) e[b] = W * k + b < BITS ? E[W * k + b] : f128_zero();
+    const uint32_t limit = k == WM::WINDOWS - 1 ? 1u << WM::TOP_BITS : 1u << W;
+    if ((part << LOW) < limit) {
+      char* o = T + ((k << W) + (part << LOW)) * 128 + r * 16;
+      F128d acc = part ? e[LOW] : f128_zero();
+      *reinterpret_cast<F128d*>(o) = acc;
+#pragma unroll
+      for (int g = 1; g < (1 << LOW); ++g) {
+        int b = 0;
+        while (!((g >> b) & 1)) ++b;
+        acc += e[b];
+        const int v = g ^ (g >> 1);
+        if ((uint32_t)v < limit) *reinterpret_cast<F128d*>(o + v * 128) = acc;
+      }
+    }
+  }
+}
+// acc += the map's value at the 64-bit x.
+template <int W>
+__device__ __forceinline__ void add_win_map64(F128d& acc, uint64_t x64, const char* T, uint32_t lane) {
+  using WM = WinMap<W, 64>;
+  const uint32_t x0 = (uint32_t)x64, x1 = (uint32_t)(x64 >> 32);
+  uint32_t r0 = (uint32_t)acc.lo, r1 = (uint32_t)(acc.lo >> 32), r2 = (uint32_t)acc.hi, r3 = (uint32_t)(acc.hi >> 32);
+#pragma unroll
+  for (int k = 0; k < WM::WINDOWS; ++k) {
+    const int o = W * k, s = o & 31;
+    const int bits = k == WM::WINDOWS - 1 ? WM::TOP_BITS : W;
+    uint32_t v;
+    if (s + bits <= 32) v = s >= 7 ? (o < 32 ? x0 : x1) >> (s - 7) : (o < 32 ? x0 : x1) << (7 - s);
+    else v = __funnelshift_r(x0, x1, s - 7);
+    v = (v & (((1u << bits) - 1) << 7)) | lane;
+    const uint4 t = *reinterpret_cast<const uint4*>(T + k * ((1 << W) * 128) + v);
+    r0 ^= t.x;
+    r1 ^= t.y;
+    r2 ^= t.z;
+    r3 ^= t.w;
+  }
+  acc = f128(r0 | ((uint64_t)r1 << 32), r2 | ((uint64_t)r3 << 32));
+}
+
 // This thread's bank group: the offset its lookups add.
 __device__ __forceinline__ uint32_t win_lane() { return (threadIdx.x & 7) << 4; }
 
