@@ -9,6 +9,7 @@
 // one position's `lanes` words. Trees are flat: leaves [0, N), then each level, root last.
 #include "kernels.h"
 #include "sha256.cuh"
+#include "wintable.cuh"
 #include <atomic>
 
 namespace flock {
@@ -46,24 +47,6 @@ void launch_fill_lane_major(const F128d* q, F128d* cw, uint32_t lanes, uint32_t 
   LAUNCH_OK();
 }
 
-// One butterfly layer: thread per (pair, lane). tw[(1 << layer) - 1 + block].
-__global__ void ntt_layer_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, uint32_t layer,
-                                 const F128d* __restrict__ tw) {
-  uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  uint64_t n_pairs = 1ull << (log_d - 1);
-  if (gid >= n_pairs * lanes) return;
-  uint64_t pair = gid / lanes;
-  uint32_t l = (uint32_t)(gid - pair * lanes);
-  uint32_t sh = log_d - layer - 1;
-  uint64_t block = pair >> sh, within = pair & ((1ull << sh) - 1);
-  uint64_t i0 = (block << (sh + 1)) + within, i1 = i0 + (1ull << sh);
-  F128d t = tw[(1ull << layer) - 1 + block];
-  F128d u = data[i0 * lanes + l], v = data[i1 * lanes + l];
-  F128d nu = block == 0 ? u : u + v * t;  // the first block's twiddle is zero in every layer
-  data[i0 * lanes + l] = nu;
-  data[i1 * lanes + l] = v + nu;
-}
-
 // Table layers: butterfly layers whose twiddle blocks are large. Each block of a launch
 // handles a contiguous share of one twiddle block's butterflies (2^cpb_log launch blocks
 // per twiddle block), builds that twiddle's byte tables once and takes half of its
@@ -72,7 +55,7 @@ __global__ void ntt_layer_kernel(F128d* __restrict__ data, uint32_t lanes, uint3
 // u = [b 2^(sh+1) lanes, + 2^sh lanes) and v = u + 2^sh lanes, sh = log_d - layer - 1
 // (lane-minor layout); the first twiddle block's twiddle is zero in every layer.
 //
-// Two layers per pass: twiddle block b of `layer` spans the quarters x0..x3 of
+// Two layers per pass, byte tables: twiddle block b of `layer` spans the quarters x0..x3 of
 // Q = lanes 2^(sh-1) elements each; `layer` pairs (x0, x2) and (x1, x3) by t_b (table),
 // layer + 1 pairs (x0, x1) by t_2b and (x2, x3) by t_2b+1 (split). One read and one write
 // of the data per two layers.
@@ -111,61 +94,67 @@ ntt_layer2_tbl_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, 
     x[3 * Q + k] = a3;
   }
 }
-// One layer per pass (for an odd table layer): per thread and iteration one butterfly by
-// table and one by the split twiddle, the next iteration's operands loaded before this
-// one's products.
-__global__ void __launch_bounds__(256, 2)
-ntt_layer_tbl_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, uint32_t layer,
-                     const F128d* __restrict__ tw, uint32_t cpb_log) {
-  extern __shared__ __align__(16) F128d ttab[];  // build_byte_table's BYTE_TABLE_SMEM_ENTRIES
-  __shared__ F128split ts;
+// The same from two window tables (wintable.cuh, five bits, 2 x 101 KB, one 512-thread block per
+// SM): t_b and t_2b by table, t_2b+1 split, the next unit's elements loaded before this one's
+// products. Per unit 9.75 cycles of the shared-memory pipe and one product of the multiply
+// pipe. Keccak-f 2^18 (42 lanes, 2^22 positions): 1.86 ms a pass against 2.35 for the byte
+// table, SHA-256 2^16 0.34 against 0.37. Its build is not hidden by other blocks, so the
+// byte-table form (three blocks per SM) stays the better one where a twiddle serves few units:
+// 5376 units 2.26 (byte) against 2.27 ms, 3200 units 0.373 against 0.399.
+constexpr int NTT_WIN = 5;
+constexpr uint32_t NTT_WIN_THREADS = 512;
+__global__ void __launch_bounds__(NTT_WIN_THREADS, 1)
+ntt_layer2_win_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, uint32_t layer,
+                      const F128d* __restrict__ tw, uint32_t cpb_log) {
+  extern __shared__ __align__(16) char wt[];  // t_b's table, then t_2b's
+  __shared__ F128split s1;
   const uint64_t b = blockIdx.x >> cpb_log, part = blockIdx.x & ((1ull << cpb_log) - 1);
-  const uint32_t sh = log_d - layer - 1;
-  const uint64_t M = ((uint64_t)lanes) << sh;  // butterflies of twiddle block b
-  const uint64_t per = M >> cpb_log;           // this block's share (even: cpb_log < sh)
-  F128d* u = data + ((b << (sh + 1)) * lanes) + part * per;
-  F128d* v = u + M;
-  const bool zero = (b == 0);  // block-uniform
-  if (!zero) {
-    const F128d t = tw[(1ull << layer) - 1 + b];
-    if (threadIdx.x == 0) ts = split_factor(t);
-    build_byte_table(t, ttab);
-  }
-  const uint64_t half = per / 2;
+  const uint32_t sh = log_d - layer - 1, lane = win_lane();
+  const uint64_t Q = ((uint64_t)lanes) << (sh - 1);
+  const uint64_t per = Q >> cpb_log;
+  F128d* x = data + ((b << (sh + 1)) * lanes) + part * per;
+  const bool zero = (b == 0);  // block-uniform: t_b and t_2b are zero
   uint64_t k = threadIdx.x;
-  F128d u0, v0, u1, v1;
-  if (k < half) {
-    u0 = u[k];
-    v0 = v[k];
-    u1 = u[half + k];
-    v1 = v[half + k];
+  F128d a0, a1, a2, a3;
+  if (k < per) { a0 = x[k]; a1 = x[Q + k]; a2 = x[2 * Q + k]; a3 = x[3 * Q + k]; }
+  if (threadIdx.x == 0) s1 = split_factor(tw[(2ull << layer) - 1 + 2 * b + 1]);
+  if (!zero) {
+    build_win_table<NTT_WIN>(tw[(1ull << layer) - 1 + b], wt);
+    build_win_table<NTT_WIN>(tw[(2ull << layer) - 1 + 2 * b], wt + WinTable<NTT_WIN>::BYTES);
   }
-  for (; k < half; k += blockDim.x) {
-    const uint64_t kn = k + blockDim.x;
-    F128d p0, q0, p1, q1;
-    if (kn < half) {
-      p0 = u[kn];
-      q0 = v[kn];
-      p1 = u[half + kn];
-      q1 = v[half + kn];
+  __syncthreads();
+  for (; k < per; k += NTT_WIN_THREADS) {
+    const uint64_t kn = k + NTT_WIN_THREADS;
+    F128d n0, n1, n2, n3;
+    if (kn < per) { n0 = x[kn]; n1 = x[Q + kn]; n2 = x[2 * Q + kn]; n3 = x[3 * Q + kn]; }
+    if (!zero) {
+      a0 += mul_win<NTT_WIN>(a2, wt, lane);
+      a1 += mul_win<NTT_WIN>(a3, wt, lane);
     }
-    const F128d n0 = zero ? u0 : u0 + mul_table(v0, ttab);
-    const F128d n1 = zero ? u1 : u1 + mul_split_call(v1, &ts);
-    u[k] = n0;
-    v[k] = v0 + n0;
-    u[half + k] = n1;
-    v[half + k] = v1 + n1;
-    u0 = p0;
-    v0 = q0;
-    u1 = p1;
-    v1 = q1;
+    a2 += a0;
+    a3 += a1;
+    if (!zero) a0 += mul_win<NTT_WIN>(a1, wt + WinTable<NTT_WIN>::BYTES, lane);
+    a1 += a0;
+    a2 += mul_split(a3, s1);
+    a3 += a2;
+    x[k] = a0;
+    x[Q + k] = a1;
+    x[2 * Q + k] = a2;
+    x[3 * Q + k] = a3;
+    a0 = n0; a1 = n1; a2 = n2; a3 = n3;
   }
 }
-// A layer is a table layer while its twiddle blocks hold at least this many butterflies
-// (a table build costs about as much shared-memory traffic as 300 table products), each
-// launch block getting at least NTT_TBL_MIN_BLOCK_BUTTERFLIES of them, and while the
-// transform is large enough to give every SM two such launch blocks.
-constexpr uint64_t NTT_TBL_MIN_TWIDDLE_BUTTERFLIES = uint64_t(1) << 11;
+// Two layers run as a table pass while the first one's twiddle blocks hold at least this many
+// units (lanes 2^(sh-1)): from WIN units on with window tables, from TBL on with a byte table.
+// Against the fused pass (two of its layers): 42 lanes, 1344 units 2.59 against 4.24 ms; 50
+// lanes, 800 units 0.436 against 0.61, but then four layers are left for it instead of six,
+// which cost more each (1.38 for four, 1.84 for six): below TBL a pass is only taken while more
+// than six layers are left, down to MORE units (13 lanes, 416 units: 0.074 ms against about
+// 0.09). Each launch block gets at least NTT_TBL_MIN_BLOCK_BUTTERFLIES of a twiddle block's
+// butterflies, and the transform has to give every SM two such blocks.
+constexpr uint64_t NTT_WIN_MIN_UNITS = 8192;
+constexpr uint64_t NTT_TBL_MIN_UNITS = 1024;
+constexpr uint64_t NTT_TBL_MORE_UNITS = 256;
 constexpr uint64_t NTT_TBL_MIN_BLOCK_BUTTERFLIES = uint64_t(1) << 12;
 
 // Several consecutive layers [layer, layer + nl) fused through shared memory. A block
@@ -267,18 +256,24 @@ static uint32_t ntt_block_threads(uint32_t lane_tile, size_t smem) {
   return best;
 }
 
-void launch_ntt(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t start_layer, const F128d* tw, cudaStream_t s) {
-  const int NL = 6;  // layers fused per pass
-  uint32_t layer = start_layer;
-  uint32_t lane_tile = lanes < 64 ? lanes : 64;
+template <int NL>
+static void launch_ntt_fused(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t layer, const F128d* tw,
+                             cudaStream_t s) {
+  const uint32_t lane_tile = lanes < 64 ? lanes : 64;
   const size_t tw_bytes = ((1u << NL) - 1) * sizeof(F128split);
-  // the top layers, whose twiddles are each shared by many butterflies: table layers, two
-  // per launch
+  const uint64_t n_groups = 1ull << (log_d - NL), lane_tiles = (lanes + lane_tile - 1) / lane_tile;
+  const size_t smem = (size_t)(1u << NL) * lane_tile * sizeof(F128d) + tw_bytes;
+  set_dynamic_smem((const void*)ntt_fused_kernel<NL>, (int)((1u << NL) * 64 * sizeof(F128d) + tw_bytes));
+  const uint32_t threads = ntt_block_threads<NL>(lane_tile, smem);
+  ntt_fused_kernel<NL><<<(unsigned)(n_groups * lane_tiles), threads, smem, s>>>(data, lanes, log_d, layer, tw, lane_tile);
+  LAUNCH_OK();
+}
+
+void launch_ntt(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t start_layer, const F128d* tw, cudaStream_t s) {
+  uint32_t layer = start_layer;
+  // the top layers, whose twiddles are each shared by many butterflies: table passes
   const uint64_t butterflies = (uint64_t)lanes << (log_d - 1);
   const bool tables = butterflies >= (uint64_t)sm_count() * 2 * NTT_TBL_MIN_BLOCK_BUTTERFLIES;
-  auto table_layer = [&](uint32_t l) {
-    return tables && l + 1 < log_d && ((uint64_t)lanes << (log_d - l - 1)) >= NTT_TBL_MIN_TWIDDLE_BUTTERFLIES;
-  };
   // launch blocks per twiddle block: about eight per SM in all, and each with at least
   // NTT_TBL_MIN_BLOCK_BUTTERFLIES of the `share` butterflies of its twiddle block
   auto blocks_log = [&](uint32_t l, uint64_t share, uint32_t max_log) {
@@ -288,42 +283,38 @@ void launch_ntt(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t start_laye
       ++c;
     return c;
   };
-  const int tbl_smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
-  while (table_layer(layer)) {
+  constexpr uint32_t MAX_NL = 6;  // layers fused per pass
+  while (tables && log_d - layer >= 3) {
     const uint32_t sh = log_d - layer - 1;
-    if (table_layer(layer + 1) && sh >= 2) {
-      // radix-4 units of 4 elements; a block's share counted in butterflies (2 per unit)
-      const uint32_t c = blocks_log(layer, (uint64_t)lanes << sh, sh - 1);
-      set_dynamic_smem((const void*)ntt_layer2_tbl_kernel, tbl_smem);
-      ntt_layer2_tbl_kernel<<<(unsigned)(1ull << (layer + c)), 256, tbl_smem, s>>>(data, lanes, log_d, layer, tw, c);
-      LAUNCH_OK();
-      layer += 2;
+    const uint64_t units = (uint64_t)lanes << (sh - 1);
+    if (units < (log_d - layer > MAX_NL ? NTT_TBL_MORE_UNITS : NTT_TBL_MIN_UNITS)) break;
+    // a block's share counted in butterflies (two per unit and layer)
+    const uint32_t c = blocks_log(layer, (uint64_t)lanes << sh, sh - 1);
+    const unsigned blocks = (unsigned)(1ull << (layer + c));
+    if (units >= NTT_WIN_MIN_UNITS) {
+      const int smem = 2 * WinTable<NTT_WIN>::BYTES;
+      set_dynamic_smem((const void*)ntt_layer2_win_kernel, smem);
+      ntt_layer2_win_kernel<<<blocks, NTT_WIN_THREADS, smem, s>>>(data, lanes, log_d, layer, tw, c);
     } else {
-      const uint32_t c = blocks_log(layer, (uint64_t)lanes << sh, sh - 1);
-      set_dynamic_smem((const void*)ntt_layer_tbl_kernel, tbl_smem);
-      ntt_layer_tbl_kernel<<<(unsigned)(1ull << (layer + c)), 256, tbl_smem, s>>>(data, lanes, log_d, layer, tw, c);
-      LAUNCH_OK();
-      layer += 1;
+      const int smem = (int)(BYTE_TABLE_SMEM_ENTRIES * sizeof(F128d));
+      set_dynamic_smem((const void*)ntt_layer2_tbl_kernel, smem);
+      ntt_layer2_tbl_kernel<<<blocks, 256, smem, s>>>(data, lanes, log_d, layer, tw, c);
     }
+    LAUNCH_OK();
+    layer += 2;
   }
+  // the rest in as few fused passes as there can be, of even depth (nine layers: five and four)
   while (layer < log_d) {
-    uint32_t remaining = log_d - layer;
-    if (remaining >= (uint32_t)NL) {
-      uint64_t n_groups = 1ull << (log_d - NL);
-      uint64_t lane_tiles = (lanes + lane_tile - 1) / lane_tile;
-      size_t smem = (size_t)(1u << NL) * lane_tile * sizeof(F128d) + tw_bytes;
-      set_dynamic_smem((const void*)ntt_fused_kernel<NL>, (int)((1u << NL) * 64 * sizeof(F128d) + tw_bytes));
-      const uint32_t threads = ntt_block_threads<NL>(lane_tile, smem);
-      ntt_fused_kernel<NL><<<(unsigned)(n_groups * lane_tiles), threads, smem, s>>>(data, lanes, log_d, layer, tw,
-                                                                                     lane_tile);
-      LAUNCH_OK();
-      layer += NL;
-    } else {
-      uint64_t work = (1ull << (log_d - 1)) * lanes;
-      ntt_layer_kernel<<<(unsigned)((work + 255) / 256), 256, 0, s>>>(data, lanes, log_d, layer, tw);
-      LAUNCH_OK();
-      layer += 1;
+    const uint32_t left = log_d - layer, passes = (left + MAX_NL - 1) / MAX_NL, nl = (left + passes - 1) / passes;
+    switch (nl) {
+      case 1: launch_ntt_fused<1>(data, lanes, log_d, layer, tw, s); break;
+      case 2: launch_ntt_fused<2>(data, lanes, log_d, layer, tw, s); break;
+      case 3: launch_ntt_fused<3>(data, lanes, log_d, layer, tw, s); break;
+      case 4: launch_ntt_fused<4>(data, lanes, log_d, layer, tw, s); break;
+      case 5: launch_ntt_fused<5>(data, lanes, log_d, layer, tw, s); break;
+      default: launch_ntt_fused<6>(data, lanes, log_d, layer, tw, s); break;
     }
+    layer += nl;
   }
 }
 
