@@ -759,15 +759,13 @@ void GpuBackend::lc_fold_slot(HashKind hash, const SlotDev& sd) {
 void GpuBackend::lc_zvec(const std::vector<F128>& x_outer) {
   scr_off_ = 0;
   const uint32_t nu = S.nu;
-  const F128d* dp = upload(x_outer);
-  F128d* eq = static_cast<F128d*>(scratch(size_t(16) << nu));
   Mark mk(this, ST_LINCHECK);
-  launch_eq_table(dp, nu, dev(F128::one()), eq, st_);
+  const EqSplit e = eq_split(x_outer, F128::one(), 10);
   // a single slot folds its used columns only; a union folds every union column (the
   // gaps and unused columns of z are zero)
   uint32_t used = S.slots.size() == 1 ? (uint32_t)S.slots[0].used_cols : K_ / 128;
   if ((uint64_t)used * 128 < K_) CUDA_OK(cudaMemsetAsync(zv_ + used * 128, 0, (K_ - used * 128) * 16, st_));
-  launch_lc_zvec(z_, nu, used, eq, part_, zv_, st_);
+  launch_lc_zvec(z_, nu, used, e.lo, e.lo_bits, e.hi, part_, part_cap_, zv_, st_);
   CUDA_OK(cudaMemcpyAsync(zvcap_, zv_, K_ * 16, cudaMemcpyDeviceToDevice, st_));
   lc_len_ = K_;
 }
@@ -938,10 +936,9 @@ std::vector<F128> GpuBackend::lane_dots(const std::vector<F128>& point) {
       std::equal(point.begin(), point.begin() + S.log_dim, mo_chal_.begin()))
     return mo_lane_q_;
   scr_off_ = 0;
-  EqSplit e = eq_split(std::vector<F128>(point.begin(), point.begin() + S.log_dim), F128::one(),
-                       lane_dots_lo_bits(S.log_dim));
+  EqSplit e = eq_split(std::vector<F128>(point.begin(), point.begin() + S.log_dim), F128::one(), 10);
   uint32_t nb;
-  { Mark mk(this, ST_LIGERITO); nb = launch_lg_lane_dots(q_, S.lanes, S.log_dim, e.lo, e.hi, part_, st_); }
+  { Mark mk(this, ST_LIGERITO); nb = launch_lg_lane_dots(q_, S.lanes, S.log_dim, e.lo, e.lo_bits, e.hi, part_, st_); }
   std::vector<F128> h = reduce(nb, S.lanes);
   h.resize(lanes_pow2());  // the lanes past the committed ones are zero
   return h;

@@ -58,7 +58,6 @@ void launch_gather_paths(const uint8_t* tree, uint64_t n_leaves, const uint64_t*
 
 // sumcheck.cu. Kernels returning a block count wrote per-block partials of the stated
 // width into `part`; launch_reduce_parts XORs them.
-void launch_eq_table(const F128d* d_point, uint32_t n, F128d scale, F128d* out, cudaStream_t s);
 // The lo and hi tables of an eq split (lo unscaled, hi times scale) in one launch.
 void launch_eq_split(const F128d* d_point, uint32_t lo_bits, uint32_t hi_bits, F128d scale, F128d* lo, F128d* hi,
                      cudaStream_t s);
@@ -121,8 +120,9 @@ struct KeccakColumnConsts {
 };
 void launch_keccak_lincheck_columns(const F128d* eqi, F128d* ca, F128d* cb, const KeccakColumnConsts& kc,
                                     cudaStream_t s);
-void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F128d* eq, F128d* part, F128d* zv,
-                    cudaStream_t s);
+// Row fold of the used chunk columns; part holds part_cap entries (at least 128 a column).
+void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F128d* eq_lo, uint32_t lo_bits,
+                    const F128d* eq_hi, F128d* part, uint64_t part_cap, F128d* zv, cudaStream_t s);
 uint32_t launch_lc_start(const F128d* ca, const F128d* cb, F128d alpha, F128d beta, uint32_t pin, uint32_t K,
                          F128d* comb, const F128d* zv, F128d* part, cudaStream_t s);                   // width 2
 uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, bool msg, F128d* part, cudaStream_t s,
@@ -158,12 +158,10 @@ void launch_as_build(const F128d* er0, const F128d* ec0, const F128d* er1, const
                      const JaggedSegs& segs, F128d* abar, F128d* g, F128d* part, cudaStream_t s, FusedPublish pub);
 
 // The lane stage (see the kernels): lane dots h[l] = sum_p q[l 2^log_d + p] eq(p) as `splits`
-// partial rows of width `lanes` (returned; eq split with lane_dots_lo_bits(log_d) low bits),
-// the fold of every lane by lambda into lane_fold_groups(lanes, D) partial rows of D entries,
+// partial rows of width `lanes` (returned), the fold of every lane by lambda into lane_fold_groups(lanes, D) partial rows of D entries,
 // and the switched vectors with their message.
-uint32_t lane_dots_lo_bits(uint32_t log_d);
-uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, const F128d* eq_hi,
-                             F128d* part, cudaStream_t s);
+uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, uint32_t lo_bits,
+                             const F128d* eq_hi, F128d* part, cudaStream_t s);
 uint32_t lane_fold_groups(uint32_t lanes, uint64_t D);
 void launch_lg_lane_fold(const F128d* q, const F256d* lambda, uint32_t lanes, uint64_t D, F256d* part, cudaStream_t s);
 // b = sum of n terms coef eq(point), each point's eq as lo (lo_bits) x hi tables.

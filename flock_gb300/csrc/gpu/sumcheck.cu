@@ -20,22 +20,6 @@ namespace flock {
 namespace gpu {
 
 // ------------------------------------------------------------------ generic pieces
-__global__ void eq_table_kernel(const F128d* __restrict__ p, uint32_t n, F128d scale, F128d* __restrict__ out) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (1ull << n)) return;
-  F128d v = scale;
-  for (uint32_t j = 0; j < n; ++j) {
-    F128d r = p[j];
-    if (!((i >> j) & 1)) r.lo ^= 1;
-    v = v * r;
-  }
-  out[i] = v;
-}
-void launch_eq_table(const F128d* d_point, uint32_t n, F128d scale, F128d* out, cudaStream_t s) {
-  uint64_t len = 1ull << n;
-  eq_table_kernel<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(d_point, n, scale, out);
-  LAUNCH_OK();
-}
 // Both tables of an eq split in one launch: lo = eq(p[0 .. lo_bits)) and
 // hi = scale * eq(p[lo_bits .. lo_bits + hi_bits)); entry e < 2^lo_bits is a lo entry.
 __global__ void eq_split_kernel(const F128d* __restrict__ p, uint32_t lo_bits, uint32_t hi_bits, F128d scale,
@@ -104,6 +88,229 @@ void set_dynamic_smem(const void* kernel, int bytes) {
   if (done.count(key)) return;
   CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   done.insert(key);
+}
+
+// ------------------------------------------------------------------ bit sums
+// U[col][t] = sum_row eq(row) * bit_t(z[col * col_stride + row * row_stride]) over the 128 bits of
+// each word: the s_hat_v_c sums of the zerocheck (rows = xo, columns = the 64 words of an xo),
+// the lincheck's row fold (rows = instances, columns = chunk columns) and Ligerito's lane dots
+// (rows of a lane; sum_t x^t U[lane][t] is the field dot product, so it needs no product a word).
+// No multiply: 32 rows at a time, a warp transposes a column's 32 words (lane c then holds, per
+// 32-bit limb, bit c of all 32 rows) and looks up the subset sums of the rows' eq weights, in
+// windows of 7, 7, 6, 6 and 6 rows. The tables depend on the rows alone and serve every column of
+// the block, so they are stored eight times, once per bank group (wintable.cuh): no lookup
+// conflicts. Per word 20 lookups and 20 shuffles of a warp over 32 words: 3.1 cycles of the
+// shared-memory pipe, plus the build (448 stores a tile) shared by up to 64 columns. Two table
+// buffers, one barrier a tile. eq(row) = eq_lo[row mod 2^lo_bits] eq_hi[row >> lo_bits], 512 rows'
+// products at a time. The forms it replaced read four- and eight-row tables with
+// conflicts or took field products: Keccak-f 2^18 (87 M words) s_hat_v_c 4.7 -> 1.7 ms, lincheck
+// row fold 3.9 -> 1.4, lane dots 1.6 -> 1.5; SHA-256 2^16 0.69 -> 0.34, 0.55 -> 0.19, 0.51 -> 0.27.
+enum BitSumOut : int {
+  BITS_RAW,      // part[(col * splits + split) * 128 + t] = U
+  BITS_COLUMNS,  // part[(split * groups + group) * 128 + t] = sum over the group's columns of weight[col] U
+  BITS_DOT,      // part[split * n_cols + col] = sum_t x^t U
+};
+constexpr uint32_t BITS_THREADS = 512, BITS_WARPS = BITS_THREADS / 32, BITS_EQ_ROWS = 512;
+constexpr uint32_t BITS_TABLE_BYTES = (2 * 128 + 3 * 64) * 128;
+// Warp-wide 32 x 32 bit transpose: lane r holds word x_r; afterwards lane c holds the word
+// whose bit r is bit c of x_r (five exchange stages of halving block size).
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t masks[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+    const uint32_t j = 16u >> s, m = masks[s];
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
+  }
+  return x;
+}
+
+__device__ __forceinline__ void build_bit_tables(const F128d* e, char* T) {
+  // a team of eight threads (one per copy) walks eight entries: 16 teams for each seven-row
+  // window, 8 for each six-row one
+  const uint32_t team = threadIdx.x >> 3, r = threadIdx.x & 7;
+  if (team >= 56) return;
+  const uint32_t win = team < 32 ? team >> 4 : 2 + ((team - 32) >> 3);
+  const uint32_t hi = team < 32 ? team & 15 : team & 7;                    // the entry's bits from 3 on
+  const uint32_t row0 = win < 2 ? 7 * win : 14 + 6 * (win - 2);
+  const uint32_t ent0 = (win < 2 ? 128 * win : 256 + 64 * (win - 2)) + 8 * hi;
+  F128d acc = f128_zero();
+#pragma unroll
+  for (uint32_t b = 0; b < 4; ++b) {
+    const uint64_t m = 0ull - (uint64_t)((hi >> b) & 1);
+    const F128d w = e[min(row0 + 3 + b, 31u)];  // b = 3 is never set in a six-row window
+    acc.lo ^= w.lo & m;
+    acc.hi ^= w.hi & m;
+  }
+  const F128d e0 = e[row0], e1 = e[row0 + 1], e2 = e[row0 + 2];
+  char* o = T + ent0 * 128 + r * 16;
+  auto put = [&](uint32_t v) { *reinterpret_cast<F128d*>(o + v * 128) = acc; };
+  put(0);
+  acc += e0; put(1);
+  acc += e1; put(3);
+  acc += e0; put(2);
+  acc += e2; put(6);
+  acc += e0; put(7);
+  acc += e1; put(5);
+  acc += e0; put(4);
+}
+template <int CPW, int OUT>
+__global__ void __launch_bounds__(BITS_THREADS, 1)
+bit_sums_kernel(const F128d* __restrict__ z, uint64_t col_stride, uint64_t row_stride, uint32_t n_cols, uint64_t n_rows,
+                uint64_t rows_per_split, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
+                const F128d* __restrict__ eq_hi, const F128d* __restrict__ weight, F128d* __restrict__ part) {
+  extern __shared__ __align__(16) char bt[];  // two tables
+  __shared__ F128d eq[2][BITS_EQ_ROWS];       // this stage's row weights and the next one's
+  const uint32_t warp = threadIdx.x >> 5, t = threadIdx.x & 31, lane16 = win_lane();
+  const uint32_t col0 = (blockIdx.x * BITS_WARPS + warp) * CPW;
+  const uint64_t row_begin = (uint64_t)blockIdx.y * rows_per_split;
+  const uint64_t row_end = min(n_rows, row_begin + rows_per_split);
+  auto stage_eq = [&](uint64_t row, uint32_t buf) {
+    F128d v = f128_zero();  // rows past the end weigh nothing
+    if (row + threadIdx.x < row_end) {
+      const uint64_t x = row + threadIdx.x;
+      v = mul_call(eq_lo[x & ((1ull << lo_bits) - 1)], eq_hi[x >> lo_bits]);
+    }
+    eq[buf][threadIdx.x] = v;
+  };
+  F128d U[CPW][4];
+#pragma unroll
+  for (int c = 0; c < CPW; ++c)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) U[c][q] = f128_zero();
+  if (row_begin < row_end) {
+    const uint32_t tiles = (uint32_t)((row_end - row_begin + 31) / 32);
+    constexpr uint32_t STAGE = BITS_EQ_ROWS / 32;  // tiles per eq stage
+    stage_eq(row_begin, 0);
+    __syncthreads();
+    build_bit_tables(eq[0], bt);
+    for (uint32_t i = 0; i < tiles; ++i) {
+      const uint64_t row = row_begin + (uint64_t)i * 32 + t;
+      uint4 x[CPW];
+#pragma unroll
+      for (int c = 0; c < CPW; ++c)
+        x[c] = col0 + c < n_cols && row < row_end
+                   ? *reinterpret_cast<const uint4*>(z + (col0 + c) * col_stride + row * row_stride)
+                   : make_uint4(0, 0, 0, 0);
+      // the next stage's weights, written a tile before the first table that reads them is built
+      if (i % STAGE == STAGE - 2) stage_eq(row_begin + (uint64_t)(i / STAGE + 1) * BITS_EQ_ROWS, (i / STAGE + 1) & 1);
+      __syncthreads();  // this tile's table is complete, the other buffer no longer read
+      if (i + 1 < tiles)
+        build_bit_tables(eq[((i + 1) / STAGE) & 1] + 32 * ((i + 1) % STAGE), bt + ((i + 1) & 1) * BITS_TABLE_BYTES);
+      const char* T = bt + (i & 1) * BITS_TABLE_BYTES;
+      if (col0 < n_cols) {  // warp-uniform
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) {
+          const uint32_t w[4] = {x[c].x, x[c].y, x[c].z, x[c].w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t y = warp_transpose32(w[q]);
+            const uint32_t o[5] = {((y << 7) & (127u << 7)) | lane16, (y & (127u << 7)) | lane16,
+                                   ((y >> 7) & (63u << 7)) | lane16, ((y >> 13) & (63u << 7)) | lane16,
+                                   ((y >> 19) & (63u << 7)) | lane16};
+            U[c][q] += *reinterpret_cast<const F128d*>(T + o[0]);
+            U[c][q] += *reinterpret_cast<const F128d*>(T + 128 * 128 + o[1]);
+            U[c][q] += *reinterpret_cast<const F128d*>(T + 256 * 128 + o[2]);
+            U[c][q] += *reinterpret_cast<const F128d*>(T + 320 * 128 + o[3]);
+            U[c][q] += *reinterpret_cast<const F128d*>(T + 384 * 128 + o[4]);
+          }
+        }
+      }
+    }
+  }
+  if (OUT == BITS_RAW) {
+#pragma unroll
+    for (int c = 0; c < CPW; ++c)
+      if (col0 + c < n_cols)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) part[((uint64_t)(col0 + c) * gridDim.y + blockIdx.y) * 128 + 32 * q + t] = U[c][q];
+  } else if (OUT == BITS_DOT) {
+#pragma unroll
+    for (int c = 0; c < CPW; ++c) {
+      F128d v = f128_zero();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v += mul_by_power(U[c][q], 32 * q + t);
+      v = warp_xor(v);
+      if (t == 0 && col0 + c < n_cols) part[(uint64_t)blockIdx.y * n_cols + col0 + c] = v;
+    }
+  } else {
+    F128d v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = f128_zero();
+#pragma unroll
+    for (int c = 0; c < CPW; ++c)
+      if (col0 + c < n_cols)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] += mul_call(weight[col0 + c], U[c][q]);
+    F128d* red = reinterpret_cast<F128d*>(bt);  // [warp][128]
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) red[warp * 128 + 32 * q + t] = v[q];
+    __syncthreads();
+    if (threadIdx.x < 128) {
+      F128d a = f128_zero();
+      for (uint32_t w = 0; w < BITS_WARPS; ++w) a += red[w * 128 + threadIdx.x];
+      part[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * 128 + threadIdx.x] = a;
+    }
+  }
+}
+// Columns per warp and row splits. A block costs about 105 cycles a tile and column slot (used or
+// not) and 700 for the tile's tables; one block runs per SM, so the splits are the ones that fill
+// up to four whole waves best, within max_splits partial rows and at least a tile each.
+struct BitSumPlan {
+  uint32_t cpw, groups, splits;
+  uint64_t rows_per_split;
+};
+static BitSumPlan bit_sum_plan(uint32_t n_cols, uint64_t n_rows, uint64_t max_splits) {
+  BitSumPlan p{};
+  uint64_t best = ~0ull;
+  for (uint32_t cpw = 1; cpw <= 4; ++cpw) {
+    const uint32_t groups = (n_cols + BITS_WARPS * cpw - 1) / (BITS_WARPS * cpw);
+    const uint64_t cost = (uint64_t)groups * (105 * BITS_WARPS * cpw + 700);
+    if (cost < best) {
+      best = cost;
+      p.cpw = cpw;
+      p.groups = groups;
+    }
+  }
+  const uint64_t tiles = (n_rows + 31) / 32, sms = (uint64_t)sm_count();
+  max_splits = std::max<uint64_t>(1, std::min(max_splits, tiles));
+  p.splits = 1;
+  double fill = 0;
+  for (uint64_t waves = 1; waves <= 4; ++waves) {
+    const uint64_t s = std::min(max_splits, std::max<uint64_t>(1, waves * sms / p.groups));
+    const uint64_t used = (s * p.groups + sms - 1) / sms;
+    const double f = (double)(s * p.groups) / (double)(used * sms);
+    if (f > fill + 0.02) {
+      fill = f;
+      p.splits = (uint32_t)s;
+    }
+  }
+  p.rows_per_split = (tiles + p.splits - 1) / p.splits * 32;
+  p.splits = (uint32_t)((n_rows + p.rows_per_split - 1) / p.rows_per_split);
+  return p;
+}
+template <int CPW, int OUT>
+static void bit_sums_cpw(const BitSumPlan& p, const F128d* z, uint64_t col_stride, uint64_t row_stride, uint32_t n_cols,
+                         uint64_t n_rows, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, const F128d* weight,
+                         F128d* part, cudaStream_t s) {
+  const int smem = 2 * (int)BITS_TABLE_BYTES;
+  set_dynamic_smem((const void*)bit_sums_kernel<CPW, OUT>, smem);
+  bit_sums_kernel<CPW, OUT><<<dim3(p.groups, p.splits), BITS_THREADS, smem, s>>>(
+      z, col_stride, row_stride, n_cols, n_rows, p.rows_per_split, eq_lo, lo_bits, eq_hi, weight, part);
+  LAUNCH_OK();
+}
+template <int OUT>
+static void bit_sums(const BitSumPlan& p, const F128d* z, uint64_t col_stride, uint64_t row_stride, uint32_t n_cols,
+                     uint64_t n_rows, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, const F128d* weight,
+                     F128d* part, cudaStream_t s) {
+  switch (p.cpw) {
+    case 1: return bit_sums_cpw<1, OUT>(p, z, col_stride, row_stride, n_cols, n_rows, eq_lo, lo_bits, eq_hi, weight, part, s);
+    case 2: return bit_sums_cpw<2, OUT>(p, z, col_stride, row_stride, n_cols, n_rows, eq_lo, lo_bits, eq_hi, weight, part, s);
+    case 3: return bit_sums_cpw<3, OUT>(p, z, col_stride, row_stride, n_cols, n_rows, eq_lo, lo_bits, eq_hi, weight, part, s);
+    default: return bit_sums_cpw<4, OUT>(p, z, col_stride, row_stride, n_cols, n_rows, eq_lo, lo_bits, eq_hi, weight, part, s);
+  }
 }
 
 // ------------------------------------------------------------------ zerocheck round 1
@@ -224,96 +431,6 @@ zc_round1_ab_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, ui
   for (int k = 0; k < 4; ++k) part[row * 64 + 4 * lane + k] = acc[k];
 }
 
-// Warp-wide 32 x 32 bit transpose: lane r holds word x_r; afterwards lane c holds the word
-// whose bit r is bit c of x_r (five exchange stages of halving block size).
-__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t masks[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const uint32_t j = 16u >> s, m = masks[s];
-    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
-    x = (lane & j) ? ((x & ~m) | ((y & ~m) >> j)) : ((x & m) | ((y & m) << j));
-  }
-  return x;
-}
-
-// s_hat_v_c[t] = sum_xo eq_o(xo) sum_w wconst[w] bit_t(z[64 xo + w]). The word constants
-// and the eq_hi factor are applied once per eq_hi chunk, not per xo:
-//   part[t] = sum_chunks eq_hi(chunk) * sum_{w in group} wconst[w] * U[w][t],
-//   U[w][t] = sum_{xo in chunk} eq_lo(xo) bit_t(z[64 xo + w]),
-// so the inner loop has no multiply. Block = 128 threads (one per bit t; warp = 32-bit
-// limb) x one group of 8 words (blockIdx.y) x a run of xo_per_block consecutive xo
-// (blockIdx.x); runs and chunks are powers of two. Per tile of 32 xo and word w, the warp
-// transposes the 32 xo's limb words (lane r loads xo r), so thread t holds bit t of all 32
-// xo in one register; each byte of it indexes the 256 subset sums of eight xo's eq weights.
-constexpr uint32_t SVC_WORDS = 8;
-constexpr uint32_t SVC_TILE = 32;  // xo staged in shared memory per step (one warp's lanes)
-constexpr uint32_t SVC_ZS_STRIDE = SVC_WORDS * 4 + 1;  // 32-bit words per staged xo, padded
-__global__ void __launch_bounds__(128)
-zc_svc_kernel(const F128d* __restrict__ z, uint64_t xo_per_block, uint64_t xo_live, const ZcConsts* __restrict__ gconst,
-              const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi,
-              F128d* __restrict__ part) {
-  __shared__ uint32_t zs[SVC_TILE * SVC_ZS_STRIDE];  // zs[xo * stride + 4 w + limb]
-  __shared__ F128d et[SVC_TILE];
-  __shared__ F128d et4[SVC_TILE / 4][16];   // et4[q][v] = sum of et[4 q + k] over the bits k of v
-  __shared__ F128d et8[SVC_TILE / 8][256];  // et8[q][v] = sum of et[8 q + k] over the bits k of v
-  const uint32_t t = threadIdx.x, limb = t >> 5, lane = t & 31;
-  const uint32_t g = blockIdx.y;
-  const uint64_t xo0 = (uint64_t)blockIdx.x * xo_per_block;
-  const uint64_t chunk = 1ull << lo_bits;
-  const uint64_t seg = xo_per_block < chunk ? xo_per_block : chunk;
-  const uint32_t tile = seg < SVC_TILE ? (uint32_t)seg : SVC_TILE;
-  const F128d* wc = gconst->wconst + g * SVC_WORDS;
-  const uint32_t* z32 = reinterpret_cast<const uint32_t*>(z);
-  // xo from xo_live on hold zero words: the block stops there (a block wholly past it
-  // writes a zero partial)
-  const uint64_t xo_end = xo0 + xo_per_block < xo_live ? xo0 + xo_per_block : xo_live;
-  F128d acc = f128_zero();
-  for (uint64_t s0 = xo0; s0 < xo_end; s0 += seg) {
-    F128d U[SVC_WORDS];
-#pragma unroll
-    for (uint32_t w = 0; w < SVC_WORDS; ++w) U[w] = f128_zero();
-    const uint64_t s_end = s0 + seg < xo_end ? s0 + seg : xo_end;
-    for (uint64_t xt = s0; xt < s_end; xt += tile) {
-      const uint32_t cur = xt + tile <= s_end ? tile : (uint32_t)(s_end - xt);
-      __syncthreads();
-      // xo past a short tile are staged as zero words with zero weight: they add nothing
-      for (uint32_t i = t; i < SVC_TILE * SVC_WORDS * 4; i += blockDim.x) {
-        const uint32_t xl = i / (SVC_WORDS * 4), rem = i % (SVC_WORDS * 4);
-        zs[xl * SVC_ZS_STRIDE + rem] = xl < cur ? z32[((xt + xl) * 64 + g * SVC_WORDS) * 4 + rem] : 0u;
-      }
-      if (t < SVC_TILE) et[t] = t < cur ? eq_lo[(xt + t) & (chunk - 1)] : f128_zero();
-      __syncthreads();
-      {
-        const uint32_t q = t >> 4, v = t & 15;  // 128 threads: one nibble-table entry each
-        F128d a = f128_zero();
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k)
-          if ((v >> k) & 1) a += et[4 * q + k];
-        et4[q][v] = a;
-      }
-      __syncthreads();
-      for (uint32_t i = t; i < (SVC_TILE / 8) * 256; i += blockDim.x) {
-        const uint32_t q = i >> 8, v = i & 255;
-        et8[q][v] = et4[2 * q][v & 15] + et4[2 * q + 1][v >> 4];
-      }
-      __syncthreads();
-#pragma unroll
-      for (uint32_t w = 0; w < SVC_WORDS; ++w) {
-        const uint32_t bits = warp_transpose32(zs[lane * SVC_ZS_STRIDE + 4 * w + limb]);  // bit r: xo r
-#pragma unroll
-        for (uint32_t q = 0; q < SVC_TILE / 8; ++q) U[w] += et8[q][(bits >> (8 * q)) & 255];
-      }
-    }
-    F128d v = f128_zero();
-#pragma unroll
-    for (uint32_t w = 0; w < SVC_WORDS; ++w) v += mul_call(wc[w], U[w]);
-    acc += eq_hi ? mul_call(eq_hi[s0 >> lo_bits], v) : v;
-  }
-  part[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * 128 + t] = acc;
-}
-
 static ZcConsts* g_zc_consts_dev[MAX_DEVICES] = {};  // written under the caller's lock, before any prover launches
 static ZcConsts* zc_consts() { return g_zc_consts_dev[current_device()]; }
 void upload_zc_consts(const uint8_t* ext, const F128d* phi8, const uint8_t mulk[8][256], const F128d* wconst) {
@@ -357,13 +474,10 @@ void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m
   zc_round1_ab_kernel<<<blocks, 16 * ZC_TEAMS, smem, s>>>(a, b, xo_live, g_zc_consts, eq_lo, lo_bits, eq_hi, part_ab);
   LAUNCH_OK();
   *nrows_ab = blocks * ZC_TEAMS;
-  // at most 256 runs of xo per word group (n_xo and the chunks are powers of two)
-  const uint64_t runs = std::min<uint64_t>(n_xo, 256);
-  const uint64_t run = n_xo / runs;
-  zc_svc_kernel<<<dim3((uint32_t)runs, 64 / SVC_WORDS), 128, 0, s>>>(z, run, xo_live, g_zc_consts, eq_lo, lo_bits,
-                                                                   eq_hi, part_svc);
-  LAUNCH_OK();
-  *nrows_svc = (uint32_t)(runs * (64 / SVC_WORDS));
+  // s_hat_v_c[t] = sum_xo eq_o(xo) sum_w wconst[w] bit_t(z[64 xo + w])
+  const BitSumPlan p = bit_sum_plan(64, xo_live, 1024);
+  bit_sums<BITS_COLUMNS>(p, z, 1, 64, 64, xo_live, eq_lo, lo_bits, eq_hi, g_zc_consts->wconst, part_svc, s);
+  *nrows_svc = p.groups * p.splits;
 }
 
 // ------------------------------------------------------------------ zerocheck skip fold
@@ -989,49 +1103,6 @@ void launch_keccak_lincheck_columns(const F128d* eqi, F128d* ca, F128d* cb, cons
   LAUNCH_OK();
 }
 
-// z_vec[128 cc + t] = sum_row eq(row) * bit_t(z[(cc << nu) + row]). Block = (cc, row split),
-// thread = bit t; rows staged through shared memory.
-constexpr uint32_t ZV_TILE = 256;
-__global__ void __launch_bounds__(128)
-lc_zvec_kernel(const F128d* __restrict__ z, uint32_t nu, uint32_t n_split, const F128d* __restrict__ eq,
-               F128d* __restrict__ part) {
-  __shared__ F128d wz[ZV_TILE];
-  __shared__ F128d we[ZV_TILE];
-  __shared__ F128d we4[ZV_TILE / 4][16];  // we4[q][v] = sum of we[4 q + k] over the bits k of v
-  uint32_t cc = blockIdx.x / n_split, sp = blockIdx.x % n_split;
-  uint64_t rows = 1ull << nu, per = rows / n_split;
-  uint64_t r0 = sp * per;
-  uint32_t t = threadIdx.x, limb = t >> 5, sh = t & 31;
-  F128d acc = f128_zero();
-  for (uint64_t base = r0; base < r0 + per; base += ZV_TILE) {
-    uint32_t n = (uint32_t)(ZV_TILE < r0 + per - base ? (uint64_t)ZV_TILE : r0 + per - base);
-    __syncthreads();
-    for (uint32_t i = t; i < n; i += blockDim.x) {
-      wz[i] = z[((uint64_t)cc << nu) + base + i];
-      we[i] = eq[base + i];
-    }
-    __syncthreads();
-    // four rows at a time: their bits t index the subset sums of their eq weights (rows
-    // past n are left out of every subset sum)
-    const uint32_t groups = (n + 3) / 4;
-    for (uint32_t i = t; i < groups * 16; i += blockDim.x) {
-      const uint32_t q = i >> 4, v = i & 15;
-      F128d s4 = f128_zero();
-#pragma unroll
-      for (uint32_t k = 0; k < 4; ++k)
-        if (((v >> k) & 1) && 4 * q + k < n) s4 += we[4 * q + k];
-      we4[q][v] = s4;
-    }
-    __syncthreads();
-    for (uint32_t q = 0; q < groups; ++q) {
-      const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&wz[4 * q]) + limb;  // 4 words per row
-      const uint32_t v = ((w0[0] >> sh) & 1) | (((w0[4] >> sh) & 1) << 1) | (((w0[8] >> sh) & 1) << 2) |
-                         (((w0[12] >> sh) & 1) << 3);
-      acc += we4[q][v];
-    }
-  }
-  part[(uint64_t)blockIdx.x * 128 + t] = acc;
-}
 __global__ void lc_zvec_reduce_kernel(const F128d* __restrict__ part, uint32_t n_split, uint32_t n_out,
                                       F128d* __restrict__ zv) {
   uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;  // o = 128 cc + t
@@ -1041,15 +1112,14 @@ __global__ void lc_zvec_reduce_kernel(const F128d* __restrict__ part, uint32_t n
   for (uint32_t sp = 0; sp < n_split; ++sp) acc += part[((uint64_t)cc * n_split + sp) * 128 + t];
   zv[o] = acc;
 }
-void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F128d* eq, F128d* part, F128d* zv,
-                    cudaStream_t s) {
-  uint32_t n_split = 1;
-  while ((uint64_t)used_chunks * n_split < (uint64_t)sm_count() * 8 && (n_split << 1) <= (1u << nu) / 64)
-    n_split <<= 1;
-  lc_zvec_kernel<<<used_chunks * n_split, 128, 0, s>>>(z, nu, n_split, eq, part);
-  LAUNCH_OK();
+// z_vec[128 cc + t] = sum_row eq(row) * bit_t(z[(cc << nu) + row]).
+void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F128d* eq_lo, uint32_t lo_bits,
+                    const F128d* eq_hi, F128d* part, uint64_t part_cap, F128d* zv, cudaStream_t s) {
+  const uint64_t rows = 1ull << nu;
+  const BitSumPlan p = bit_sum_plan(used_chunks, rows, part_cap / (used_chunks * 128ull));
+  bit_sums<BITS_RAW>(p, z, rows, 1, used_chunks, rows, eq_lo, lo_bits, eq_hi, nullptr, part, s);
   uint32_t n_out = used_chunks * 128;
-  lc_zvec_reduce_kernel<<<(n_out + 127) / 128, 128, 0, s>>>(part, n_split, n_out, zv);
+  lc_zvec_reduce_kernel<<<(n_out + 127) / 128, 128, 0, s>>>(part, p.splits, n_out, zv);
   LAUNCH_OK();
 }
 
@@ -1330,74 +1400,14 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
 // times: the whole Ligerito stage took 26.4 ms of a Keccak-f 2^18 proof (now 9.3), 4.8 ms of
 // SHA-256 2^16 (2.6), 0.94 ms of BLAKE3 2^12 (0.69; six kernels and round trips fewer).
 
-// Lane dots: part[split * lanes + l] = the split's share of h[l]. Chunk (2^13 rows) c of a
-// lane: h[l] = sum_a eq_lo[a] G[a], G[a] = sum_c eq_hi[c] q[l D + c 2^13 + a], thread t of the
-// 512 owning a = t + 512 k, so the products per word are by the chunk's constant eq_hi[c]:
-// three in four from its window table, one in four split (both pipes; 1.12e11 products/s in
-// isolation). One block per (lane, split), one block per SM beside the 169 KB table.
-constexpr uint32_t LANE_DOT_LO_BITS = 13;
-__global__ void __launch_bounds__(512, 1)
-lg_lane_dots_tbl_kernel(const F128d* __restrict__ q, uint32_t lanes, uint32_t log_d, uint32_t splits,
-                        const F128d* __restrict__ eq_lo, const F128d* __restrict__ eq_hi, F128d* __restrict__ part) {
-  extern __shared__ __align__(16) char wt[];  // WinTable<6>
-  __shared__ F128split hs;
-  __shared__ F128d sh[32];
-  const uint32_t l = blockIdx.x % lanes, sp = blockIdx.x / lanes, lane16 = win_lane();
-  const uint32_t n_ch = 1u << (log_d - LANE_DOT_LO_BITS), per = n_ch / splits;
-  F128d h[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) h[k] = f128_zero();
-  for (uint32_t ch = sp * per; ch < (sp + 1) * per; ++ch) {
-    __syncthreads();  // the previous chunk's table and split are no longer read
-    const F128d e = eq_hi[ch];
-    if (threadIdx.x == 0) hs = split_factor(e);
-    build_win_table<6>(e, wt);
-    __syncthreads();
-    const F128d* fc = q + ((uint64_t)l << log_d) + ((uint64_t)ch << LANE_DOT_LO_BITS) + threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const F128d x = fc[512 * k];
-      h[k] += (k & 3) == 3 ? mul_split(x, hs) : mul_win<6>(x, wt, lane16);
-    }
-  }
-  F128d g = f128_zero();
-#pragma unroll
-  for (int k = 0; k < 16; ++k) g += mul_call(h[k], eq_lo[threadIdx.x + 512 * k]);
-  g = block_xor(g, sh);
-  if (threadIdx.x == 0) part[(uint64_t)sp * lanes + l] = g;
+// Lane dots h[l] = sum_p q[l D + p] eq(p), as rows of `lanes` partials.
+uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, uint32_t lo_bits,
+                             const F128d* eq_hi, F128d* part, cudaStream_t s) {
+  const uint64_t rows = 1ull << log_d;
+  const BitSumPlan p = bit_sum_plan(lanes, rows, 1024);
+  bit_sums<BITS_DOT>(p, q, rows, 1, lanes, rows, eq_lo, lo_bits, eq_hi, nullptr, part, s);
+  return p.splits;
 }
-// The same for few rows: block (lane, chunk of 2^lo_bits rows), one product a word.
-__global__ void __launch_bounds__(256)
-lg_lane_dots_kernel(const F128d* __restrict__ q, uint32_t lanes, uint32_t log_d, const F128d* __restrict__ eq_lo,
-                    uint32_t lo_bits, const F128d* __restrict__ eq_hi, F128d* __restrict__ part) {
-  __shared__ F128d sh[32];
-  const uint32_t l = blockIdx.x % lanes, ch = blockIdx.x / lanes;
-  const F128d* fc = q + ((uint64_t)l << log_d) + ((uint64_t)ch << lo_bits);
-  F128d g = f128_zero();
-  for (uint32_t a = threadIdx.x; a < (1u << lo_bits); a += blockDim.x) g += mul_call(fc[a], eq_lo[a]);
-  g = block_xor(g, sh);
-  if (threadIdx.x == 0) part[(uint64_t)ch * lanes + l] = mul_call(eq_hi[ch], g);
-}
-// From 2^16 rows (eight chunks a lane) the table form: below, its blocks would hold a chunk or
-// two each and a 169 KB table build apiece.
-constexpr uint32_t LANE_DOT_TABLE_MIN_LOG = 16;
-uint32_t lane_dots_lo_bits(uint32_t log_d) { return log_d >= LANE_DOT_TABLE_MIN_LOG ? LANE_DOT_LO_BITS : std::min(log_d, 10u); }
-uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, const F128d* eq_hi,
-                             F128d* part, cudaStream_t s) {
-  const uint32_t lo = lane_dots_lo_bits(log_d);
-  if (lo == LANE_DOT_LO_BITS) {
-    uint32_t splits = 1;  // eight blocks per SM in all: the last wave then costs a few percent
-    while (splits < (1u << (log_d - lo)) && splits * lanes < (uint32_t)sm_count() * 8) splits <<= 1;
-    set_dynamic_smem((const void*)lg_lane_dots_tbl_kernel, WinTable<6>::BYTES);
-    lg_lane_dots_tbl_kernel<<<lanes * splits, 512, WinTable<6>::BYTES, s>>>(q, lanes, log_d, splits, eq_lo, eq_hi, part);
-    LAUNCH_OK();
-    return splits;
-  }
-  lg_lane_dots_kernel<<<lanes << (log_d - lo), 256, 0, s>>>(q, lanes, log_d, eq_lo, lo, eq_hi, part);
-  LAUNCH_OK();
-  return 1u << (log_d - lo);
-}
-
 // The fold of all lanes: part[g D + p] = sum over the lanes of group g of lambda_l q[l D + p].
 // A block holds LANE_FOLD_ROWS rows' F256 sums in registers and walks its lanes: per lane the
 // window tables of lambda's two halves (W = 5, 202 KB, one block per SM), the next lane's words
