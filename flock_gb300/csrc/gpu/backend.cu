@@ -789,8 +789,9 @@ void GpuBackend::lc_start(F128 alpha, const std::vector<SlotComb>& sc, F128& e1,
 }
 
 void GpuBackend::lc_round(F128 r, bool last, F128& e1, F128& ei) {
-  FusedPublish fp = last ? FusedPublish() : fused_publish();
-  { Mark mk(this, ST_LINCHECK); launch_lc_round(comb_, zv_, lc_len_, dev(r), !last, part_, st_, fp); }
+  // the last round's message is not used
+  FusedPublish fp = fused_publish();
+  { Mark mk(this, ST_LINCHECK); launch_lc_round(comb_, zv_, lc_len_, dev(r), part_, st_, fp); }
   lc_len_ /= 2;
   if (!last) {
     auto v = read_published(fp.seq, 2);

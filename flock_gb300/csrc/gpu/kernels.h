@@ -125,8 +125,7 @@ void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F12
                     const F128d* eq_hi, F128d* part, uint64_t part_cap, F128d* zv, cudaStream_t s);
 uint32_t launch_lc_start(const F128d* ca, const F128d* cb, F128d alpha, F128d beta, uint32_t pin, uint32_t K,
                          F128d* comb, const F128d* zv, F128d* part, cudaStream_t s);                   // width 2
-uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, bool msg, F128d* part, cudaStream_t s,
-                         FusedPublish pub = FusedPublish());
+uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, F128d* part, cudaStream_t s, FusedPublish pub);
 // Union lincheck: one slot's weighted comb (out = weight (alpha ca + cb), + beta at pin),
 // and the first message of a comb built that way.
 void launch_lc_slot_comb(const F128d* ca, const F128d* cb, F128d alpha, F128d weight, F128d beta, uint32_t pin,
@@ -176,8 +175,7 @@ uint32_t launch_lg_lane_switch(const F256d* fpart, uint32_t groups, const LaneTe
 uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64_t d, F128d* part, cudaStream_t s,
                               FusedPublish pub = FusedPublish());
 uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, uint64_t d_fold, uint64_t d_msg,
-                               F256d* fo, F256d* bo, F128d* part, cudaStream_t s,
-                               FusedPublish pub = FusedPublish());                                  // width 4
+                               F256d* fo, F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub);  // width 4
 void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, const F256d* r_dev, uint64_t d,
                        F256d* fo, F256d* bo, cudaStream_t s);
 void launch_lg_code_switch(const F256d* f, const F256d* b, uint64_t n, F256d* fo, F256d* bo, cudaStream_t s);

@@ -30,8 +30,21 @@ __device__ __forceinline__ F128d eq_at(const F128d* lo, uint32_t lo_bits, const 
 // Called by every block after thread 0 stored its `width` partials at part[block * width]:
 // the block takes a ticket; the block that takes the last one reduces all partials (the
 // other blocks' stores are visible to it after their fences and the atomic), writes the
-// message to mapped memory, then the sequence number, and resets the counter.
+// message to mapped memory, then the sequence number, and resets the counter. A block alone
+// writes its partials out directly.
 static __device__ void publish_if_last(const F128d* part, uint32_t width, const FusedPublish& pub, F128d* sh) {
+  if (gridDim.x == 1) {  // the block's own partials are the message
+    if (threadIdx.x == 0) {
+      volatile F128d* o = pub.out;
+      for (uint32_t j = 0; j < width; ++j) {
+        o[j].lo = part[j].lo;
+        o[j].hi = part[j].hi;
+      }
+      __threadfence_system();
+      *(volatile uint32_t*)pub.flag = pub.seq;
+    }
+    return;
+  }
   __shared__ uint32_t ticket;
   if (threadIdx.x == 0) {
     __threadfence();

@@ -831,9 +831,9 @@ void launch_factor_table(const F128d* f, uint32_t n, F128d* out, cudaStream_t s)
 // n_pairs = output length / 2 (>= 1). eq by mode:
 enum PairEq : int {
   EQ_NONE,   // eq = 1
-  EQ_FIXED,  // eq(j) = eq_lo[j mod 2^lo_bits] (the zerocheck's weighted form): the grid's thread
-             // count is a multiple of 2^lo_bits, so a thread multiplies its sum by eq_lo once
-  EQ_SPLIT,  // eq(j) = eq_lo[j mod 2^lo_bits] eq_hi[j >> lo_bits], one eq_hi per chunk
+  EQ_FIXED,  // eq(j) = eq_lo[j mod 2^lo_bits] (the zerocheck's weighted form); in the table form the
+             // grid's thread count is a multiple of 2^lo_bits, so a thread multiplies its sum once
+  EQ_SPLIT,  // eq(j) = eq_lo[j mod 2^lo_bits] eq_hi[j >> lo_bits]
 };
 // Folds of at least this many pairs take their products by r from the window table of r (six
 // bits, 169 KB, one block per SM): four table products (11 cycles of the shared-memory pipe)
@@ -879,65 +879,70 @@ pair_fold_tbl_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bi
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = g1; part[blockIdx.x * 2 + 1] = gi; }
   publish_if_last(part, 2, pub, sh);
 }
-// The same with r split once per block for mul_split (small, latency-bound rounds). unweight
-// (when not null): the folded a entry i is multiplied by unweight[i] before it is stored.
-template <int EQ>
-__global__ void __launch_bounds__(256, 2)
-pair_fold_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bin, uint64_t n_pairs, uint64_t live_pairs,
-                 F128d r, const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi,
-                 const F128d* __restrict__ unweight, F128d* __restrict__ aout, F128d* __restrict__ bout,
-                 F128d* __restrict__ part, FusedPublish pub) {
-  __shared__ F128d sh[32];
+// Small rounds are bound by the latency of a chain of products (a product is about 400
+// instructions, and a warp alone on its scheduler issues one every few cycles), so a block takes
+// 64 pairs with 256 threads and every thread forms one product at a time: four folds a pair,
+// then the two message products beside eq(j) where it is split, then the product by eq. Three
+// products deep instead of ten in one thread (14 -> 9 us a round under the profiler; zerocheck folds
+// of BLAKE3 2^12 0.35 -> 0.255 ms). Where the two vectors' entries of a pair lie:
+// PAIRS (4j .. 4j + 3 in, 2j and 2j + 1 out) or TOP (the top variable bound in place, for the
+// lincheck: i, i + h; i + q, i + q + h in, i and i + q out, h = 2q = half the length).
+// unweight (or null): factors of the folded a entries.
+constexpr uint32_t SMALL_PAIRS = 64, SMALL_THREADS = 4 * SMALL_PAIRS;
+enum PairMap : int { MAP_PAIRS, MAP_TOP };
+template <int EQ, int MAP>
+__global__ void __launch_bounds__(SMALL_THREADS)
+pair_fold_small_kernel(const F128d* ain, const F128d* bin, uint64_t n_pairs, uint64_t live_pairs, F128d r,
+                       const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi,
+                       const F128d* __restrict__ unweight, F128d* aout, F128d* bout, F128d* __restrict__ part,
+                       FusedPublish pub) {
   __shared__ F128split rs;  // the fold challenge, split once
+  __shared__ F128d v[4][SMALL_PAIRS];  // A0, A1, B0, B1
+  __shared__ F128d ev[SMALL_PAIRS];    // eq(j)
+  __shared__ F128d sh[SMALL_THREADS / 32];
   if (threadIdx.x == 0) rs = split_factor(r);
-  __syncthreads();
-  // pairs are walked in chunks of 2^lo_bits under EQ_SPLIT, with the grid's stride otherwise
-  const uint64_t chunk = EQ == EQ_SPLIT ? 1ull << lo_bits : n_pairs;
-  const uint64_t n_chunks = EQ == EQ_SPLIT ? (n_pairs + chunk - 1) / chunk : 1;
-  const uint64_t j0 = EQ == EQ_SPLIT ? threadIdx.x : (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t step = EQ == EQ_SPLIT ? blockDim.x : (uint64_t)gridDim.x * blockDim.x;
-  F128d G1 = f128_zero(), GI = f128_zero();
-  for (uint64_t ch = EQ == EQ_SPLIT ? blockIdx.x : 0; ch < n_chunks; ch += EQ == EQ_SPLIT ? gridDim.x : 1) {
-    F128d g1 = f128_zero(), gi = f128_zero();
-    const uint64_t end = min(n_pairs, (ch + 1) * chunk);
-    for (uint64_t j = ch * chunk + j0; j < end; j += step) {
-      if (j >= live_pairs) {  // zero inputs: zero outputs, nothing added to the message
-        aout[2 * j] = aout[2 * j + 1] = bout[2 * j] = bout[2 * j + 1] = f128_zero();
-        continue;
-      }
-      F128d x0 = ain[4 * j], x1 = ain[4 * j + 1], x2 = ain[4 * j + 2], x3 = ain[4 * j + 3];
-      F128d y0 = bin[4 * j], y1 = bin[4 * j + 1], y2 = bin[4 * j + 2], y3 = bin[4 * j + 3];
-      F128d A0 = x0 + mul_split_call(x1 + x0, &rs), A1 = x2 + mul_split_call(x3 + x2, &rs);
-      F128d B0 = y0 + mul_split_call(y1 + y0, &rs), B1 = y2 + mul_split_call(y3 + y2, &rs);
-      if (unweight) {
-        A0 = mul_call(A0, unweight[2 * j]);
-        A1 = mul_call(A1, unweight[2 * j + 1]);
-      }
-      aout[2 * j] = A0; aout[2 * j + 1] = A1;
-      bout[2 * j] = B0; bout[2 * j + 1] = B1;
-      F128d t1 = mul_call(A1, B1), ti = mul_call(A0 + A1, B0 + B1);
-      if (EQ == EQ_SPLIT) {
-        F128d e = eq_lo[j & (chunk - 1)];
-        t1 = mul_call(e, t1);
-        ti = mul_call(e, ti);
-      }
-      g1 += t1;
-      gi += ti;
+  const uint64_t base = (uint64_t)blockIdx.x * SMALL_PAIRS;
+  {
+    // vector a's pairs by the first half of the block, b's by the second; k = 0, 1: out entry
+    const uint32_t which = threadIdx.x / (2 * SMALL_PAIRS), i = threadIdx.x % (2 * SMALL_PAIRS);
+    const uint32_t p = MAP == MAP_PAIRS ? i >> 1 : i % SMALL_PAIRS, k = MAP == MAP_PAIRS ? i & 1 : i / SMALL_PAIRS;
+    const uint64_t j = base + p;
+    const F128d* in = which ? bin : ain;
+    F128d* out = which ? bout : aout;
+    F128d x0 = f128_zero(), d = f128_zero();
+    if (j < live_pairs) {
+      const uint64_t i0 = MAP == MAP_PAIRS ? 4 * j + 2 * k : j + k * n_pairs;
+      x0 = in[i0];
+      d = in[MAP == MAP_PAIRS ? i0 + 1 : i0 + 2 * n_pairs] + x0;
     }
-    if (EQ == EQ_FIXED) {
-      const F128d e = eq_lo[j0 & ((1ull << lo_bits) - 1)];
-      g1 = mul_call(e, g1);
-      gi = mul_call(e, gi);
-    }
-    g1 = block_xor(g1, sh);
-    gi = block_xor(gi, sh);
-    if (threadIdx.x == 0) {
-      const F128d h = EQ == EQ_SPLIT && eq_hi ? eq_hi[ch] : f128_one();
-      G1 += h * g1;
-      GI += h * gi;
-    }
+    __syncthreads();
+    F128d f = x0 + mul_split(d, rs);
+    const uint64_t o = MAP == MAP_PAIRS ? 2 * j + k : j + k * n_pairs;
+    if (unweight && !which && j < live_pairs) f = mul_call(f, unweight[o]);
+    if (j < n_pairs) out[o] = f;  // pairs past the live ones have zero inputs
+    v[2 * which + k][p] = f;
   }
-  if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+  __syncthreads();
+  const uint32_t p = threadIdx.x % SMALL_PAIRS, job = threadIdx.x / SMALL_PAIRS;  // whole warps share a job
+  F128d t = f128_zero();
+  if (job < 2) {
+    t = mul_call(job ? v[0][p] + v[1][p] : v[1][p], job ? v[2][p] + v[3][p] : v[3][p]);
+  } else if (EQ != EQ_NONE && job == 2) {
+    const uint64_t j = min(base + p, n_pairs - 1);
+    const F128d lo = eq_lo[j & ((1ull << lo_bits) - 1)];
+    ev[p] = EQ == EQ_SPLIT ? mul_call(lo, eq_hi[j >> lo_bits]) : lo;
+  }
+  if (EQ != EQ_NONE) {
+    __syncthreads();
+    if (job < 2) t = mul_call(t, ev[p]);
+  }
+  t = warp_xor(t);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {  // jobs 0 and 1 are two warps each
+    part[blockIdx.x * 2] = sh[0] + sh[1];
+    part[blockIdx.x * 2 + 1] = sh[2] + sh[3];
+  }
   publish_if_last(part, 2, pub, sh);
 }
 uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, uint64_t live_pairs, F128d r,
@@ -965,25 +970,11 @@ uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, 
     LAUNCH_OK();
     return blocks;
   }
-  if (eq_hi) {
-    const uint64_t n_chunks = (n_pairs + (1ull << lo_bits) - 1) >> lo_bits;
-    const uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
-    pair_fold_kernel<EQ_SPLIT><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo, lo_bits, eq_hi, unweight,
-                                                      aout, bout, part, pub);
-    LAUNCH_OK();
-    return blocks;
-  }
-  uint32_t blocks = (uint32_t)std::min<uint64_t>((n_pairs + 255) / 256, (uint64_t)sm_count() * 8);
-  if (fixed && (uint64_t)blocks * 256 < n_pairs && (1u << lo_bits) > 256) {
-    const uint32_t q = (1u << lo_bits) / 256;
-    blocks = std::max(q, blocks / q * q);
-  }
-  if (fixed)
-    pair_fold_kernel<EQ_FIXED><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo, lo_bits, nullptr, unweight,
-                                                      aout, bout, part, pub);
-  else
-    pair_fold_kernel<EQ_NONE><<<blocks, 256, 0, s>>>(ain, bin, n_pairs, live_pairs, r, nullptr, 0, nullptr, unweight, aout,
-                                                     bout, part, pub);
+  const uint32_t blocks = (uint32_t)((n_pairs + SMALL_PAIRS - 1) / SMALL_PAIRS);
+  auto* kernel = eq_hi ? pair_fold_small_kernel<EQ_SPLIT, MAP_PAIRS>
+                       : (fixed ? pair_fold_small_kernel<EQ_FIXED, MAP_PAIRS> : pair_fold_small_kernel<EQ_NONE, MAP_PAIRS>);
+  kernel<<<blocks, SMALL_THREADS, 0, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo, lo_bits, eq_hi, unweight, aout, bout,
+                                          part, pub);
   LAUNCH_OK();
   return blocks;
 }
@@ -1190,42 +1181,14 @@ uint32_t launch_lc_top_message(const F128d* comb, const F128d* zv, uint32_t K, F
 }
 
 // Bind the top variable of comb and zv (length len -> len/2) in place and emit the next
-// top-variable message over the bound vectors (pairs (i, i + len/4)).
-__global__ void lc_round_kernel(F128d* __restrict__ comb, F128d* __restrict__ zv, uint32_t len, F128d r, int msg,
-                                F128d* __restrict__ part, FusedPublish pub) {
-  __shared__ F128d sh[32];
-  uint32_t h = len / 2, q = h / 2;
-  F128d e1 = f128_zero(), ei = f128_zero();
-  if (q == 0) {
-    // len == 2: single bind, no message
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      comb[0] = comb[0] + r * (comb[1] + comb[0]);
-      zv[0] = zv[0] + r * (zv[1] + zv[0]);
-    }
-  } else {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < q; i += gridDim.x * blockDim.x) {
-      F128d c0 = comb[i] + r * (comb[i + h] + comb[i]);
-      F128d c1 = comb[i + q] + r * (comb[i + q + h] + comb[i + q]);
-      F128d z0 = zv[i] + r * (zv[i + h] + zv[i]);
-      F128d z1 = zv[i + q] + r * (zv[i + q + h] + zv[i + q]);
-      comb[i] = c0; comb[i + q] = c1;
-      zv[i] = z0; zv[i + q] = z1;
-      if (msg) {
-        e1 += c1 * z1;
-        ei += (c0 + c1) * (z0 + z1);
-      }
-    }
-  }
-  e1 = block_xor(e1, sh);
-  ei = block_xor(ei, sh);
-  if (threadIdx.x == 0) { part[blockIdx.x * 2] = e1; part[blockIdx.x * 2 + 1] = ei; }
-  if (pub.out) publish_if_last(part, 2, pub, sh);
-}
-uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, bool msg, F128d* part, cudaStream_t s,
-                         FusedPublish pub) {
-  uint32_t q = len / 4;
-  uint32_t blocks = std::max(1u, std::min((q + 255) / 256, 256u));
-  lc_round_kernel<<<blocks, 256, 0, s>>>(comb, zv, len, r, msg ? 1 : 0, part, pub);
+// top-variable message over the bound vectors (pairs (i, i + len/4)): e1 = sum c1 z1, einf =
+// sum (c0 + c1) (z0 + z1).
+uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, F128d* part, cudaStream_t s, FusedPublish pub) {
+  const uint64_t q = len / 4;
+  if (q == 0) throw std::runtime_error("lincheck round: fewer than four entries");
+  const uint32_t blocks = (uint32_t)((q + SMALL_PAIRS - 1) / SMALL_PAIRS);
+  pair_fold_small_kernel<EQ_NONE, MAP_TOP><<<blocks, SMALL_THREADS, 0, s>>>(comb, zv, q, q, r, nullptr, 0, nullptr, nullptr,
+                                                                            comb, zv, part, pub);
   LAUNCH_OK();
   return blocks;
 }
@@ -1521,49 +1484,32 @@ void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, 
   LAUNCH_OK();
 }
 // One round's fold (at r, pairs d_fold apart) fused with the next round's message over the
-// folded vectors (pairs d_msg apart): each thread folds the two outputs of one message pair,
-// stores them, and accumulates u0 = sum f0 b0, u2 = sum (f0 + f1)(b0 + b1) over them. Same
-// index maps as lg_fold256_kernel and lg_message256_kernel; one pass instead of two.
-__device__ __forceinline__ void lg_fold_at(const F256d* __restrict__ f, const F256d* __restrict__ b, F256d r,
-                                        uint32_t d_log, uint64_t i, F256d& fi, F256d& bi) {
-  const uint64_t lo = pair_lo(i, d_log), hi = lo + (1ull << d_log);
-  const F256d f0 = f[lo], b0 = b[lo];
-  fi = f0 + f256_mul_call(r, f[hi] + f0);
-  bi = b0 + f256_mul_call(r, b[hi] + b0);
-}
-// TBL: the products by r come from byte tables of r.c0 and r.c1 plus the split form of
+// folded vectors (pairs d_msg apart): u0 = sum f0 b0, u2 = sum (f0 + f1)(b0 + b1), same index
+// maps as lg_fold256_kernel and lg_message256_kernel.
+// Large rounds: the products by r come from byte tables of r.c0 and r.c1 plus the split form of
 // r.c0 + r.c1 (the Karatsuba terms of F256 product, see operator* in field.cuh): per pair
 // 8 table products on the load/store pipe beside 4 + 6 integer-multiply products. One
 // 512-thread block per SM holds the two tables (141 KB).
-template <bool TBL>
-__global__ void __launch_bounds__(TBL ? 512 : 256, TBL ? 1 : 2)
-lg_fold_msg256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, F256d r,
-                      uint32_t dlog_fold, uint32_t dlog_msg, F256d* __restrict__ fo, F256d* __restrict__ bo,
-                      F128d* __restrict__ part, FusedPublish pub) {
-  extern __shared__ __align__(16) F128d rtab[];  // TBL: tables of r.c0 and r.c1
+__global__ void __launch_bounds__(512, 1)
+lg_fold_msg256_tbl_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, F256d r,
+                          uint32_t dlog_fold, uint32_t dlog_msg, F256d* __restrict__ fo, F256d* __restrict__ bo,
+                          F128d* __restrict__ part, FusedPublish pub) {
+  extern __shared__ __align__(16) F128d rtab[];  // tables of r.c0 and r.c1
   __shared__ F128d sh[32];
   __shared__ F128split rsum;
-  if (TBL) {
-    if (threadIdx.x == 0) rsum = split_factor(r.c0 + r.c1);
-    build_byte_table(r.c0, rtab);
-    build_byte_table(r.c1, rtab + BYTE_TABLE_ENTRIES);  // its scratch follows the second table
-  }
-  // fold of entry i (see lg_fold_at)
+  if (threadIdx.x == 0) rsum = split_factor(r.c0 + r.c1);
+  build_byte_table(r.c0, rtab);
+  build_byte_table(r.c1, rtab + BYTE_TABLE_ENTRIES);  // its scratch follows the second table
+  auto fold = [&](F256d v0, F256d d) {
+    const F128d p0 = mul_table(d.c0, rtab), p1 = mul_table(d.c1, rtab + BYTE_TABLE_ENTRIES),
+                p2 = mul_split_call(d.c0 + d.c1, &rsum);
+    return v0 + f256(p0 + mul_by_x_inv(p1), p2 + p0);
+  };
   auto fold_at = [&](uint64_t i, F256d& fi, F256d& bi) {
-    if (TBL) {
-      const uint64_t lo = pair_lo(i, dlog_fold), hi = lo + (1ull << dlog_fold);
-      const F256d f0 = f[lo], b0 = b[lo], df = f[hi] + f0, db = b[hi] + b0;
-      const F128d* T0 = rtab;
-      const F128d* T1 = rtab + BYTE_TABLE_ENTRIES;
-      F128d p0 = mul_table(df.c0, T0), p1 = mul_table(df.c1, T1), p2 = mul_split_call(df.c0 + df.c1, &rsum);
-      fi = f0 + f256(p0 + mul_by_x_inv(p1), p2 + p0);
-      p0 = mul_table(db.c0, T0);
-      p1 = mul_table(db.c1, T1);
-      p2 = mul_split_call(db.c0 + db.c1, &rsum);
-      bi = b0 + f256(p0 + mul_by_x_inv(p1), p2 + p0);
-    } else {
-      lg_fold_at(f, b, r, dlog_fold, i, fi, bi);
-    }
+    const uint64_t lo = pair_lo(i, dlog_fold), hi = lo + (1ull << dlog_fold);
+    const F256d f0 = f[lo], b0 = b[lo];
+    fi = fold(f0, f[hi] + f0);
+    bi = fold(b0, b[hi] + b0);
   };
   F256d u0 = f256(f128_zero(), f128_zero()), u2 = u0;
   for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n_out / 2; p += (uint64_t)gridDim.x * blockDim.x) {
@@ -1583,7 +1529,65 @@ lg_fold_msg256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, 
     part[blockIdx.x * 4] = r0; part[blockIdx.x * 4 + 1] = r1;
     part[blockIdx.x * 4 + 2] = r2; part[blockIdx.x * 4 + 3] = r3;
   }
-  if (pub.out) publish_if_last(part, 4, pub, sh);
+  publish_if_last(part, 4, pub, sh);
+}
+// Small rounds (see pair_fold_small_kernel): a block takes 32 message pairs with 384 threads. A
+// warp forms one of the 12 products of the four folds (f and b, both entries, the three Karatsuba
+// products) for its 32 pairs, then one of the message's six; two products deep instead of
+// eighteen in one thread (28 us a round at any size before, 11 now, under the profiler).
+constexpr uint32_t LG_SMALL_THREADS = 12 * 32;
+__global__ void __launch_bounds__(LG_SMALL_THREADS)
+lg_fold_msg256_small_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, F256d r,
+                            uint32_t dlog_fold, uint32_t dlog_msg, F256d* __restrict__ fo, F256d* __restrict__ bo,
+                            F128d* __restrict__ part, FusedPublish pub) {
+  __shared__ F128split rs[3];     // r.c0, r.c1, r.c0 + r.c1
+  __shared__ F128d prod[12][32];
+  __shared__ F256d out[4][32];    // f low, b low, f high, b high entry of the pair
+  __shared__ F128d sh[32];
+  const uint32_t w = threadIdx.x >> 5, t = threadIdx.x & 31, vec = w / 3, comp = w % 3;
+  if (threadIdx.x < 3) rs[threadIdx.x] = split_factor(threadIdx.x == 0 ? r.c0 : threadIdx.x == 1 ? r.c1 : r.c0 + r.c1);
+  const uint64_t p = (uint64_t)blockIdx.x * 32 + t;
+  const bool have = p < n_out / 2;
+  auto part_of = [](F256d x, uint32_t c) { return c == 0 ? x.c0 : c == 1 ? x.c1 : x.c0 + x.c1; };
+  F256d v0 = f256(f128_zero(), f128_zero()), d = v0;
+  uint64_t o = 0;
+  if (have) {
+    const F256d* in = (vec & 1) ? b : f;
+    o = pair_lo(p, dlog_msg) + ((vec >> 1) ? 1ull << dlog_msg : 0);
+    const uint64_t lo = pair_lo(o, dlog_fold);
+    v0 = in[lo];
+    d = in[lo + (1ull << dlog_fold)] + v0;
+  }
+  __syncthreads();
+  const F128d mine = mul_split(part_of(d, comp), rs[comp]);
+  prod[w][t] = mine;
+  __syncthreads();
+  if (comp == 0) {
+    const F128d p1 = prod[w + 1][t], p2 = prod[w + 2][t];
+    const F256d v = v0 + f256(mine + mul_by_x_inv(p1), p2 + mine);
+    if (have) ((vec & 1) ? bo : fo)[o] = v;
+    out[vec][t] = v;
+  }
+  __syncthreads();
+  if (w < 6) {
+    const uint32_t sum = w / 3;  // u0, then u2
+    F256d x = out[0][t], y = out[1][t];
+    if (sum) {
+      x += out[2][t];
+      y += out[3][t];
+    }
+    const F128d q = warp_xor(mul(part_of(x, comp), part_of(y, comp)));
+    if (t == 0) prod[w][0] = q;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t k = 0; k < 2; ++k) {
+      const F128d q0 = prod[3 * k][0], q1 = prod[3 * k + 1][0], q2 = prod[3 * k + 2][0];
+      part[blockIdx.x * 4 + 2 * k] = q0 + mul_by_x_inv(q1);
+      part[blockIdx.x * 4 + 2 * k + 1] = q2 + q0;
+    }
+  }
+  publish_if_last(part, 4, pub, sh);
 }
 // Folds of at least this many output entries use the table form, with at least
 // LG_FOLD_TABLE_MIN_BLOCK_PAIRS message pairs per block for its two table builds.
@@ -1593,17 +1597,17 @@ uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, F
                                uint64_t d_msg, F256d* fo, F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub) {
   if (n_out >= LG_FOLD_TABLE_MIN_OUT) {
     const int smem = (int)((BYTE_TABLE_ENTRIES + BYTE_TABLE_SMEM_ENTRIES) * sizeof(F128d));
-    set_dynamic_smem((const void*)lg_fold_msg256_kernel<true>, smem);
+    set_dynamic_smem((const void*)lg_fold_msg256_tbl_kernel, smem);
     const uint32_t blocks = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>((uint64_t)sm_count(), n_out / 2 / LG_FOLD_TABLE_MIN_BLOCK_PAIRS));
-    lg_fold_msg256_kernel<true><<<blocks, 512, smem, s>>>(f, b, n_out, r, log2_distance(d_fold),
-                                                          log2_distance(d_msg), fo, bo, part, pub);
+    lg_fold_msg256_tbl_kernel<<<blocks, 512, smem, s>>>(f, b, n_out, r, log2_distance(d_fold), log2_distance(d_msg), fo,
+                                                        bo, part, pub);
     LAUNCH_OK();
     return blocks;
   }
-  uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n_out / 2 + 255) / 256, (uint64_t)sm_count() * 8));
-  lg_fold_msg256_kernel<false><<<blocks, 256, 0, s>>>(f, b, n_out, r, log2_distance(d_fold),
-                                                      log2_distance(d_msg), fo, bo, part, pub);
+  const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, (n_out / 2 + 31) / 32);
+  lg_fold_msg256_small_kernel<<<blocks, LG_SMALL_THREADS, 0, s>>>(f, b, n_out, r, log2_distance(d_fold),
+                                                                  log2_distance(d_msg), fo, bo, part, pub);
   LAUNCH_OK();
   return blocks;
 }
