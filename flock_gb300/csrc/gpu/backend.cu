@@ -123,7 +123,8 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   b += 6 * K * 16;                          // lincheck vectors
   for (const SlotInfo& t : S.slots) {
     b += 2 * (uint64_t(16) << t.k_log);
-    if (t.csc_a) b += 4 * (t.csc_a->col_ptr.size() + t.csc_a->rows_flat.size() + t.csc_b->col_ptr.size() + t.csc_b->rows_flat.size());
+    if (t.csc_a)
+      b += 4 * (t.csc_a->col_ptr.size() + t.csc_b->col_ptr.size()) + 2 * (t.csc_a->rows_flat.size() + t.csc_b->rows_flat.size());
   }
   b += (W + W + W / 2) * 16;                // merged weight and fold buffers
   const uint64_t D = uint64_t(1) << S.log_dim;
@@ -184,16 +185,14 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
     sd.ca = dmalloc<F128d>(sd.K, owned_, device_bytes_);
     sd.cb = dmalloc<F128d>(sd.K, owned_, device_bytes_);
     if (t.hash != HASH_KECCAK) {
-      const Csc& A = *t.csc_a;
-      const Csc& B = *t.csc_b;
-      sd.cola = dmalloc<uint32_t>(A.col_ptr.size(), owned_, device_bytes_);
-      sd.rowa = dmalloc<uint32_t>(A.rows_flat.size(), owned_, device_bytes_);
-      sd.colb = dmalloc<uint32_t>(B.col_ptr.size(), owned_, device_bytes_);
-      sd.rowb = dmalloc<uint32_t>(B.rows_flat.size(), owned_, device_bytes_);
-      CUDA_OK(cudaMemcpy(sd.cola, A.col_ptr.data(), A.col_ptr.size() * 4, cudaMemcpyHostToDevice));
-      CUDA_OK(cudaMemcpy(sd.rowa, A.rows_flat.data(), A.rows_flat.size() * 4, cudaMemcpyHostToDevice));
-      CUDA_OK(cudaMemcpy(sd.colb, B.col_ptr.data(), B.col_ptr.size() * 4, cudaMemcpyHostToDevice));
-      CUDA_OK(cudaMemcpy(sd.rowb, B.rows_flat.data(), B.rows_flat.size() * 4, cudaMemcpyHostToDevice));
+      for (auto [csc, d] : {std::make_pair(t.csc_a, &sd.a), std::make_pair(t.csc_b, &sd.b)}) {
+        uint32_t* ptr = dmalloc<uint32_t>(csc->col_ptr.size(), owned_, device_bytes_);
+        uint16_t* rows = dmalloc<uint16_t>(csc->rows_flat.size(), owned_, device_bytes_);
+        CUDA_OK(cudaMemcpy(ptr, csc->col_ptr.data(), csc->col_ptr.size() * 4, cudaMemcpyHostToDevice));
+        CUDA_OK(cudaMemcpy(rows, csc->rows_flat.data(), csc->rows_flat.size() * 2, cudaMemcpyHostToDevice));
+        d->col_ptr = ptr;
+        d->rows = rows;
+      }
     }
     slot_dev_.push_back(sd);
   }
@@ -623,7 +622,6 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
     d.p_off = t.off;
     d.n = t.n;
     d.out_off = total;
-    d.scale = dev(F128::one());
     zc_desc_.push_back(d);
     total += uint64_t(1) << t.n;
   }
@@ -633,7 +631,7 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   uint32_t nb;
   {
     Mark mk(this, ST_ZC_FOLD_SKIP);
-    launch_eq_tables(dp, ddesc, (uint32_t)zc_desc_.size(), total, zc_tabs_, st_);
+    launch_eq_tables(dp, ddesc, zc_desc_.data(), (uint32_t)zc_desc_.size(), zc_tabs_, st_);
     // words from zc_live_words_ on are zero and add nothing to the message
     const F128d* hi = zc_tabs_ + zc_desc_[1].out_off;
     nb = zc_w_ ? launch_zc_fold_skip_weighted(a_, b_, dw, zc_live_words_, zc_w_, zc_tabs_, hi, part_, st_)
@@ -752,8 +750,7 @@ void GpuBackend::lc_fold_slot(HashKind hash, const SlotDev& sd) {
     launch_keccak_lincheck_columns(eqi_, sd.ca, sd.cb, kc, st_);
     return;
   }
-  launch_csc_fold(sd.cola, sd.rowa, sd.K, eqi_, sd.ca, st_);
-  launch_csc_fold(sd.colb, sd.rowb, sd.K, eqi_, sd.cb, st_);
+  launch_csc_fold(sd.a, sd.b, sd.K, eqi_, sd.ca, sd.cb, st_);
 }
 
 void GpuBackend::lc_zvec(const std::vector<F128>& x_outer) {

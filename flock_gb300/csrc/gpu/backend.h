@@ -146,7 +146,7 @@ class GpuBackend : public ProverBackend {
   // per-slot lincheck state: the slot's column folds and its matrices (CSC) on the device
   struct SlotDev {
     F128d *ca = nullptr, *cb = nullptr;
-    uint32_t *cola = nullptr, *rowa = nullptr, *colb = nullptr, *rowb = nullptr;
+    CscDev a, b;
     uint32_t K = 0;
   };
   std::vector<SlotDev> slot_dev_;
@@ -169,7 +169,6 @@ class GpuBackend : public ProverBackend {
   F128d* zc_w64_ = nullptr;  // skip-point Lagrange weights (device)
 
   F128d *eqi_ = nullptr, *ca_ = nullptr, *cb_ = nullptr, *comb_ = nullptr, *zv_ = nullptr, *zvcap_ = nullptr;
-  uint32_t *cola_ = nullptr, *rowa_ = nullptr, *colb_ = nullptr, *rowb_ = nullptr;
   uint32_t lc_len_ = 0;
 
   F128d *mw_ = nullptr, *moAq_ = nullptr, *moAw_ = nullptr, *moBq_ = nullptr, *moBw_ = nullptr;

@@ -339,25 +339,35 @@ __global__ void merkle_level_kernel(uint32_t* __restrict__ tree, uint64_t in_off
 #pragma unroll
   for (int k = 0; k < 8; ++k) tree[o * 8 + k] = out[k];
 }
-// The top of the tree, from a level of n_in <= MERKLE_TOP_NODES nodes up to the level of
-// n_cap nodes (the cap), in one block: each level's nodes are hashed by the block's
-// threads, then a barrier.
-constexpr uint32_t MERKLE_TOP_NODES = 2048;
-__global__ void __launch_bounds__(1024) merkle_top_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint32_t n_in,
-                                                         uint32_t n_cap) {
-  uint64_t off = in_off;
-  for (uint32_t len = n_in; len > n_cap; len /= 2) {
-    const uint32_t nout = len / 2;
-    for (uint32_t i = threadIdx.x; i < nout; i += blockDim.x) {
-      const uint32_t* l = tree + (off + 2 * (uint64_t)i) * 8;
-      uint32_t out[8];
-      sha256_words([&](uint32_t k) { return l[k]; }, 16, out);
-      const uint64_t o = off + len + i;
+// Several small levels in one launch: a group of 2^(levels - 1) threads hashes 2^levels nodes up to
+// one, a digest passing to the thread that needs it through shared memory. A level of few nodes
+// is bound by the latency of its two compressions (about 5 us), whatever the launch; one block
+// for all of them, which this replaced, was bound by its one SM (2048 nodes to 256: 28 us).
+constexpr uint32_t MERKLE_SMALL_NODES = 1u << 15, MERKLE_SMALL_LEVELS = 3, MERKLE_SMALL_THREADS = 128;
+__global__ void __launch_bounds__(MERKLE_SMALL_THREADS)
+merkle_levels_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint64_t n_in, uint32_t levels) {
+  __shared__ uint32_t node[MERKLE_SMALL_THREADS][8];
+  uint64_t off = in_off, len = n_in;
+  const uint32_t t = threadIdx.x;
+  uint32_t out[8];
+  for (uint32_t k = 0; k < levels; ++k) {
+    // thread t of the block holds node first + t of this level's output, the first ones only
+    const uint32_t have = MERKLE_SMALL_THREADS >> k;
+    const uint64_t nout = len / 2, i = (uint64_t)blockIdx.x * have + t;
+    if (t < have && i < nout) {
+      const uint32_t* l = tree + (off + 2 * i) * 8;
+      sha256_words([&](uint32_t w) { return k ? node[2 * t + (w >> 3)][w & 7] : l[w]; }, 16, out);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) tree[o * 8 + k] = out[k];
+      for (int w = 0; w < 8; ++w) tree[(off + len + i) * 8 + w] = out[w];
+    }
+    __syncthreads();  // this level's inputs are read
+    if (t < have) {
+#pragma unroll
+      for (int w = 0; w < 8; ++w) node[t][w] = out[w];
     }
     __syncthreads();
     off += len;
+    len = nout;
   }
 }
 void launch_merkle(const F128d* rows, uint32_t lanes, uint64_t n_leaves, uint32_t cap_depth, uint8_t* tree,
@@ -368,16 +378,20 @@ void launch_merkle(const F128d* rows, uint32_t lanes, uint64_t n_leaves, uint32_
   merkle_leaves_kernel<<<(unsigned)((n_leaves + 127) / 128), 128, 0, s>>>(rows, lanes, n_leaves, (uint32_t*)tree);
   LAUNCH_OK();
   uint64_t off = 0, len = n_leaves;
-  while (len > MERKLE_TOP_NODES && len > n_cap) {
-    uint64_t nout = len / 2;
-    merkle_level_kernel<<<(unsigned)((nout + 127) / 128), 128, 0, s>>>((uint32_t*)tree, off, nout);
+  while (len > n_cap) {
+    uint32_t levels = 1;
+    if (len > MERKLE_SMALL_NODES) {
+      merkle_level_kernel<<<(unsigned)((len / 2 + 127) / 128), 128, 0, s>>>((uint32_t*)tree, off, len / 2);
+    } else {
+      while (levels < MERKLE_SMALL_LEVELS && (len >> levels) > n_cap) ++levels;
+      merkle_levels_kernel<<<(unsigned)((len / 2 + MERKLE_SMALL_THREADS - 1) / MERKLE_SMALL_THREADS), MERKLE_SMALL_THREADS, 0,
+                             s>>>((uint32_t*)tree, off, len, levels);
+    }
     LAUNCH_OK();
-    off += len;
-    len = nout;
-  }
-  if (len > n_cap) {
-    merkle_top_kernel<<<1, 1024, 0, s>>>((uint32_t*)tree, off, (uint32_t)len, (uint32_t)n_cap);
-    LAUNCH_OK();
+    for (; levels; --levels) {
+      off += len;
+      len /= 2;
+    }
   }
 }
 

@@ -109,7 +109,12 @@ uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, 
                           F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub);  // width 2
 
 void launch_lc_eq_inner(const F128d* w64, const F128d* er, uint32_t K, F128d* eqi, cudaStream_t s);
-void launch_csc_fold(const uint32_t* col_ptr, const uint32_t* rows, uint32_t K, const F128d* eqi, F128d* out,
+// A matrix by columns on the device (at most 2^16 rows).
+struct CscDev {
+  const uint32_t* col_ptr = nullptr;
+  const uint16_t* rows = nullptr;
+};
+void launch_csc_fold(const CscDev& A, const CscDev& B, uint32_t K, const F128d* eqi, F128d* outa, F128d* outb,
                      cudaStream_t s);
 // Keccak-f block R1CS: writes the nonzero entries of ca = eq^T A_0 and cb = eq^T B_0 (the
 // caller zeroes both K-word vectors first). rc = the 24 round constants, rho[a + 5 b] = the
@@ -199,10 +204,10 @@ void launch_reduce_publish(const F128d* part, uint32_t nb, uint32_t width, F128d
                            uint32_t seq, cudaStream_t s);
 struct EqDesc {
   uint32_t p_off, n;   // coordinates point[p_off .. p_off + n)
-  uint64_t out_off;    // first entry in the output (tables in increasing out_off)
-  F128d scale;
+  uint64_t out_off;    // first entry in the output
 };
-void launch_eq_tables(const F128d* point, const EqDesc* d_desc, uint32_t n_desc, uint64_t total, F128d* out,
+// d_desc: the n_desc descriptors on the device, desc: the same on the host.
+void launch_eq_tables(const F128d* point, const EqDesc* d_desc, const EqDesc* desc, uint32_t n_desc, F128d* out,
                       cudaStream_t s);
 
 }  // namespace gpu

@@ -26,6 +26,41 @@ __device__ __forceinline__ F128d eq_at(const F128d* lo, uint32_t lo_bits, const 
   return hi ? l * hi[i >> lo_bits] : l;
 }
 
+// ------------------------------------------------------------------ eq tables
+// eq over n coordinates as a product over groups of four: the 16 values of each group in shared
+// memory (a product tree of depth two), then an entry is a product tree over its groups. Four
+// products deep for twelve coordinates, where one factor after the other is twelve, and a
+// quarter of the products.
+constexpr uint32_t EQ_THREADS = 256;
+constexpr uint32_t EQ_MAX_GROUPS = 8;  // at most 32 coordinates
+// Every thread of the block calls this; a barrier before the tables are read.
+__device__ __forceinline__ void eq_sub_tables(const F128d* __restrict__ p, uint32_t n, F128d (*sub)[16]) {
+  for (uint32_t i = threadIdx.x; i < EQ_MAX_GROUPS * 16; i += blockDim.x) {
+    const uint32_t g = i >> 4, v = i & 15;
+    if (4 * g >= n) continue;
+    F128d f[4];
+#pragma unroll
+    for (uint32_t b = 0; b < 4; ++b) {
+      f[b] = f128_one();
+      if (4 * g + b < n) {
+        f[b] = p[4 * g + b];
+        if (!((v >> b) & 1)) f[b].lo ^= 1;
+      }
+    }
+    sub[g][v] = mul_call(mul_call(f[0], f[1]), mul_call(f[2], f[3]));
+  }
+}
+__device__ __forceinline__ F128d eq_from_sub(const F128d (*sub)[16], uint32_t n, uint64_t i) {
+  const uint32_t groups = (n + 3) / 4;
+  F128d v = f128_one();
+  for (uint32_t g = 0; g < groups; g += 2) {
+    F128d t = sub[g][(i >> (4 * g)) & 15];
+    if (g + 1 < groups) t = mul_call(t, sub[g + 1][(i >> (4 * g + 4)) & 15]);
+    v = g ? mul_call(v, t) : t;
+  }
+  return v;
+}
+
 // ------------------------------------------------------------------ fused publication
 // Called by every block after thread 0 stored its `width` partials at part[block * width]:
 // the block takes a ticket; the block that takes the last one reduces all partials (the

@@ -41,31 +41,32 @@ void launch_reduce_publish(const F128d* part, uint32_t nb, uint32_t width, F128d
   LAUNCH_OK();
 }
 
-// Several eq tables in one launch: table k = scale_k * eq(point[off_k .. off_k + n_k)) at out + out_k.
-__global__ void eq_tables_kernel(const F128d* __restrict__ point, const EqDesc* __restrict__ desc, uint32_t n_desc,
-                                 uint64_t total, F128d* __restrict__ out) {
-  __shared__ EqDesc sd[64];
-  for (uint32_t i = threadIdx.x; i < n_desc; i += blockDim.x) sd[i] = desc[i];
-  __syncthreads();
-  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t k = 0;
-    while (k + 1 < n_desc && sd[k + 1].out_off <= e) ++k;
-    const EqDesc& d = sd[k];
-    uint64_t i = e - d.out_off;
-    F128d v = d.scale;
-    for (uint32_t j = 0; j < d.n; ++j) {
-      F128d r = point[d.p_off + j];
-      if (!((i >> j) & 1)) r.lo ^= 1;
-      v = v * r;
-    }
-    out[e] = v;
+// Several eq tables in one launch: table k = eq(point[off_k .. off_k + n_k)) at out +
+// out_k. A block works on one table's entries [entry, entry + EQ_DESC_ENTRIES).
+constexpr uint32_t EQ_DESC_ENTRIES = 1024;
+__global__ void __launch_bounds__(EQ_THREADS)
+eq_tables_kernel(const F128d* __restrict__ point, const EqDesc* __restrict__ desc, uint32_t n_desc,
+                 F128d* __restrict__ out) {
+  __shared__ F128d sub[EQ_MAX_GROUPS][16];
+  uint32_t k = 0;
+  uint64_t block = blockIdx.x;
+  for (; k < n_desc; ++k) {  // the table of this block: tables take whole blocks, in order
+    const uint64_t blocks = ((1ull << desc[k].n) + EQ_DESC_ENTRIES - 1) / EQ_DESC_ENTRIES;
+    if (block < blocks) break;
+    block -= blocks;
   }
+  if (k == n_desc) return;
+  const EqDesc d = desc[k];
+  eq_sub_tables(point + d.p_off, d.n, sub);
+  __syncthreads();
+  const uint64_t end = min(uint64_t(1) << d.n, (block + 1) * EQ_DESC_ENTRIES);
+  for (uint64_t i = block * EQ_DESC_ENTRIES + threadIdx.x; i < end; i += EQ_THREADS) out[d.out_off + i] = eq_from_sub(sub, d.n, i);
 }
-void launch_eq_tables(const F128d* point, const EqDesc* d_desc, uint32_t n_desc, uint64_t total, F128d* out,
+void launch_eq_tables(const F128d* point, const EqDesc* d_desc, const EqDesc* desc, uint32_t n_desc, F128d* out,
                       cudaStream_t s) {
-  if (n_desc > 64) throw std::runtime_error("too many eq tables in one launch");
-  uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((total + 255) / 256, (uint64_t)sm_count() * 8));
-  eq_tables_kernel<<<blocks, 256, 0, s>>>(point, d_desc, n_desc, total, out);
+  uint64_t blocks = 0;
+  for (uint32_t k = 0; k < n_desc; ++k) blocks += ((1ull << desc[k].n) + EQ_DESC_ENTRIES - 1) / EQ_DESC_ENTRIES;
+  eq_tables_kernel<<<(unsigned)blocks, EQ_THREADS, 0, s>>>(point, d_desc, n_desc, out);
   LAUNCH_OK();
 }
 

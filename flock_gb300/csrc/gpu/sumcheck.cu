@@ -22,27 +22,29 @@ namespace gpu {
 // ------------------------------------------------------------------ generic pieces
 // Both tables of an eq split in one launch: lo = eq(p[0 .. lo_bits)) and
 // hi = scale * eq(p[lo_bits .. lo_bits + hi_bits)); entry e < 2^lo_bits is a lo entry.
-__global__ void eq_split_kernel(const F128d* __restrict__ p, uint32_t lo_bits, uint32_t hi_bits, F128d scale,
-                                F128d* __restrict__ lo, F128d* __restrict__ hi) {
-  const uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t n_lo = 1ull << lo_bits;
-  if (e >= n_lo + (1ull << hi_bits)) return;
-  const bool is_lo = e < n_lo;
-  const uint64_t i = is_lo ? e : e - n_lo;
-  const uint32_t n = is_lo ? lo_bits : hi_bits;
-  const F128d* q = is_lo ? p : p + lo_bits;
-  F128d v = is_lo ? f128_one() : scale;
-  for (uint32_t j = 0; j < n; ++j) {
-    F128d r = q[j];
-    if (!((i >> j) & 1)) r.lo ^= 1;
-    v = v * r;
+__global__ void __launch_bounds__(EQ_THREADS)
+eq_split_kernel(const F128d* __restrict__ p, uint32_t lo_bits, uint32_t hi_bits, F128d scale, F128d* __restrict__ lo,
+                F128d* __restrict__ hi) {
+  __shared__ F128d sub[2][EQ_MAX_GROUPS][16];
+  eq_sub_tables(p, lo_bits, sub[0]);
+  eq_sub_tables(p + lo_bits, hi_bits, sub[1]);
+  __syncthreads();
+  const uint64_t n_lo = 1ull << lo_bits, n = n_lo + (1ull << hi_bits);
+  const bool scaled = scale.lo != 1 || scale.hi != 0;
+  for (uint64_t e = (uint64_t)blockIdx.x * EQ_THREADS + threadIdx.x; e < n; e += (uint64_t)gridDim.x * EQ_THREADS) {
+    if (e < n_lo) {
+      lo[e] = eq_from_sub(sub[0], lo_bits, e);
+    } else {
+      const F128d v = eq_from_sub(sub[1], hi_bits, e - n_lo);
+      hi[e - n_lo] = scaled ? mul_call(scale, v) : v;
+    }
   }
-  (is_lo ? lo : hi)[i] = v;
 }
 void launch_eq_split(const F128d* d_point, uint32_t lo_bits, uint32_t hi_bits, F128d scale, F128d* lo, F128d* hi,
                      cudaStream_t s) {
   const uint64_t len = (1ull << lo_bits) + (1ull << hi_bits);
-  eq_split_kernel<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(d_point, lo_bits, hi_bits, scale, lo, hi);
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>((len + EQ_THREADS - 1) / EQ_THREADS, (uint64_t)sm_count() * 8);
+  eq_split_kernel<<<blocks, EQ_THREADS, 0, s>>>(d_point, lo_bits, hi_bits, scale, lo, hi);
   LAUNCH_OK();
 }
 
@@ -989,22 +991,38 @@ void launch_lc_eq_inner(const F128d* w64, const F128d* er, uint32_t K, F128d* eq
   lc_eq_inner_kernel<<<(K + 255) / 256, 256, 0, s>>>(w64, er, K, eqi);
   LAUNCH_OK();
 }
-// One warp per column: consecutive lanes read consecutive row indices.
-__global__ void csc_fold_kernel(const uint32_t* __restrict__ col_ptr, const uint32_t* __restrict__ rows,
-                                uint32_t K, const F128d* __restrict__ eqi, F128d* __restrict__ out) {
-  uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t c = warp; c < K; c += n_warps) {
-    F128d acc = f128_zero();
-    for (uint32_t p = col_ptr[c] + lane; p < col_ptr[c + 1]; p += 32) acc += eqi[__ldg(rows + p)];
-    acc = warp_xor(acc);
-    if (lane == 0) out[c] = acc;
+// Column folds of A_0 and B_0 (blockIdx.y) in one launch, one warp per column. The matrices are
+// dense for sparse ones (BLAKE3 27 M and 17 M entries, SHA-256 29 M and 19 M, columns of up to
+// 8943), so a launch is bound by the chain index -> weight of the longest columns and by the
+// index traffic: eight loads of each in flight a lane, indices of 16 bits (BLAKE3: two launches of
+// 46 us before, one of 74 now).
+__global__ void __launch_bounds__(256)
+csc_fold_kernel(CscDev A, CscDev B, uint32_t K, const F128d* __restrict__ eqi, F128d* __restrict__ outa,
+                F128d* __restrict__ outb) {
+  const CscDev& M = blockIdx.y ? B : A;
+  F128d* out = blockIdx.y ? outb : outa;
+  const uint32_t lane = threadIdx.x & 31, c = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (c >= K) return;
+  const uint32_t end = M.col_ptr[c + 1];
+  F128d acc = f128_zero();
+  uint32_t p = M.col_ptr[c] + lane;
+  for (; p + 7 * 32 < end; p += 8 * 32) {
+    uint32_t r[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r[k] = __ldg(M.rows + p + 32 * k);
+    F128d v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = eqi[r[k]];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc += v[k];
   }
+  for (; p < end; p += 32) acc += eqi[__ldg(M.rows + p)];
+  acc = warp_xor(acc);
+  if (lane == 0) out[c] = acc;
 }
-void launch_csc_fold(const uint32_t* col_ptr, const uint32_t* rows, uint32_t K, const F128d* eqi, F128d* out,
+void launch_csc_fold(const CscDev& A, const CscDev& B, uint32_t K, const F128d* eqi, F128d* outa, F128d* outb,
                      cudaStream_t s) {
-  uint32_t blocks = std::min<uint32_t>((K + 7) / 8, (uint32_t)sm_count() * 16);
-  csc_fold_kernel<<<blocks, 256, 0, s>>>(col_ptr, rows, K, eqi, out);
+  csc_fold_kernel<<<dim3((K + 7) / 8, 2), 256, 0, s>>>(A, B, K, eqi, outa, outb);
   LAUNCH_OK();
 }
 

@@ -6,6 +6,7 @@
 // :500-515 (xor_dedup).
 #pragma once
 #include <cstdint>
+#include <stdexcept>
 #include <vector>
 #include <algorithm>
 
@@ -42,9 +43,10 @@ inline std::vector<uint32_t> xor_dedup(std::vector<uint32_t> v) {
 struct Csc {
   uint32_t n_cols = 0;
   std::vector<uint32_t> col_ptr;
-  std::vector<uint32_t> rows_flat;
+  std::vector<uint16_t> rows_flat;  // at most 2^16 rows
 };
 inline Csc csc_from_rows(const SparseRows& m) {
+  if (m.rows.size() > (size_t(1) << 16)) throw std::runtime_error("a matrix by columns has at most 2^16 rows");
   Csc c;
   c.n_cols = m.num_cols;
   c.col_ptr.assign(m.num_cols + 1, 0);
@@ -54,7 +56,7 @@ inline Csc csc_from_rows(const SparseRows& m) {
   std::vector<uint32_t> next(c.col_ptr.begin(), c.col_ptr.end() - 1);
   c.rows_flat.resize(c.col_ptr.back());
   for (uint32_t r = 0; r < m.rows.size(); ++r)
-    for (uint32_t col : m.rows[r]) c.rows_flat[next[col]++] = r;
+    for (uint32_t col : m.rows[r]) c.rows_flat[next[col]++] = (uint16_t)r;
   return c;
 }
 

@@ -1,5 +1,6 @@
 """Small sumcheck rounds (one product per thread): rounds of one block with idle pairs, of several
-blocks, and with a zero tail that ends inside a block; byte identity with the oracle."""
+blocks, and with a zero tail that ends inside a block; the trees above these codewords take one to
+three fused levels. Byte identity with the oracle."""
 import pytest
 
 import flock_gb300
@@ -9,7 +10,7 @@ from flock_gb300 import BLAKE3, KECCAK, SHA256, inputs
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("kind,log_n", [(KECCAK, 6), (SHA256, 7), (BLAKE3, 9), (SHA256, 10)])
+@pytest.mark.parametrize("kind,log_n", [(KECCAK, 6), (SHA256, 7), (BLAKE3, 9), (SHA256, 10), (BLAKE3, 10)])
 def test_bundle_matches_oracle(kind, log_n):
     recs = inputs.batch(kind, 1 << log_n, 20 + log_n)
     with flock_gb300.SETUPS[kind](1 << log_n) as s:
