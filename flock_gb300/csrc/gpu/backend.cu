@@ -26,28 +26,25 @@ void upload_constants_once() {
   if (g_consts_done[dev]) return;
   [] {
     const SkipTables& st = skip_tables();
-    // eq factor of the three small zerocheck constants (bit j of K selects c_j or 1 + c_j)
-    const uint8_t c[3] = {0xF7, 0x53, 0xB5};
-    uint8_t mulk[8][256], e2[4];
-    for (int K = 0; K < 8; ++K) {
-      uint8_t e = 1;
-      for (int j = 0; j < 3; ++j) e = gf8_mul(e, ((K >> j) & 1) ? c[j] : (uint8_t)(c[j] ^ 1));
-      for (int v = 0; v < 256; ++v) mulk[K][v] = gf8_mul(e, (uint8_t)v);
-    }
+    const uint8_t c[3] = {0xF7, 0x53, 0xB5};  // the three small zerocheck constants
+    uint8_t e2[4];
     for (int K2 = 0; K2 < 4; ++K2) {
       uint8_t e = 1;
       for (int j = 0; j < 2; ++j) e = gf8_mul(e, ((K2 >> j) & 1) ? c[j + 1] : (uint8_t)(c[j + 1] ^ 1));
       e2[K2] = e;
     }
     // word 4M + K2 of an xo carries eq weight x^M * phi8(e2[K2]) (times D * eq_o(xo))
-    F128 wconst[64];
+    F128 wconst[64], pconst[128];
     for (int M = 0; M < 16; ++M) {
       F128 xm = F128::one();
       for (int i = 0; i < M; ++i) xm = mul_by_x(xm);
       for (int K2 = 0; K2 < 4; ++K2) wconst[4 * M + K2] = xm * phi8(e2[K2]);
+      for (int bit = 0; bit < 8; ++bit) pconst[8 * M + bit] = xm * phi8((uint8_t)(1u << bit));
     }
-    upload_zc_consts(st.ext.data(), reinterpret_cast<const F128d*>(phi8_table().data()), mulk,
-                     reinterpret_cast<const F128d*>(wconst));
+    std::vector<uint8_t> unit(64 * 64);
+    for (int s = 0; s < 64; ++s)
+      for (int i = 0; i < 64; ++i) unit[64 * s + i] = st.unit[s][i];
+    upload_zc_consts(unit.data(), reinterpret_cast<const F128d*>(wconst), reinterpret_cast<const F128d*>(pconst));
     upload_witness_constants();
   }();
   g_consts_done[dev] = true;
@@ -562,7 +559,7 @@ void GpuBackend::zc_round1(const std::vector<F128>& r, std::vector<F128>& ab, st
   F128d* part_svc = part_ + part_cap_ / 2;
   {
     Mark mk(this, ST_ZC_ROUND1);
-    launch_zc_round1(a_, b_, z_, m, zc_live_words_, e.lo, e.lo_bits, e.hi, part_, &nab, part_svc, &nsvc, st_);
+    launch_zc_round1(a_, b_, z_, m, zc_live_words_, e.lo, e.lo_bits, e.hi, zc2a_, part_, &nab, part_svc, &nsvc, st_);
   }
   if ((uint64_t)nab * 64 > part_cap_ / 2 || (uint64_t)nsvc * 128 > part_cap_ / 2)
     throw std::runtime_error("round-1 partials exceed the partials buffer");

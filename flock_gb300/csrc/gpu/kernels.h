@@ -63,13 +63,14 @@ void launch_eq_split(const F128d* d_point, uint32_t lo_bits, uint32_t hi_bits, F
                      cudaStream_t s);
 void launch_reduce_parts(const F128d* part, uint32_t n_blocks, uint32_t width, F128d* out, cudaStream_t s);
 
-void upload_zc_consts(const uint8_t* ext, const F128d* phi8, const uint8_t mulk[8][256], const F128d* wconst);
+// unit[64 s + i]: extension of row bit s at Lambda point i; wconst, pconst: see ZcConsts.
+void upload_zc_consts(const uint8_t* unit, const F128d* wconst, const F128d* pconst);
 // Round-1 partials: P_ab rows of width 64 into part_ab, s_hat_v_c rows of width 128 into part_svc.
 // Words of z, a and b from live_words on are zero (the zero tail of a single slot's chunk
-// columns) and are not read.
+// columns) and are not read. g: 2^(m - 7) words of scratch.
 void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m, uint64_t live_words,
-                      const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* part_ab, uint32_t* nrows_ab,
-                      F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s);
+                      const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* g, F128d* part_ab,
+                      uint32_t* nrows_ab, F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s);
 uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words, const F128d* eq_lo,
                              uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s);       // width 2
 // First multilinear fold (at rho) of the skip-folded a, b, computed from the bits; writes

@@ -15,6 +15,7 @@
 #include <mutex>
 #include <set>
 #include <tuple>
+#include <type_traits>
 
 namespace flock {
 namespace gpu {
@@ -111,6 +112,8 @@ enum BitSumOut : int {
   BITS_RAW,      // part[(col * splits + split) * 128 + t] = U
   BITS_COLUMNS,  // part[(split * groups + group) * 128 + t] = sum over the group's columns of weight[col] U
   BITS_DOT,      // part[split * n_cols + col] = sum_t x^t U
+  BITS_POINTS,   // the words of zc_round1_bits: part[(split * groups + group) * 64 + i] = the group's share of
+                 // sum_{M, bit} weight[8 M + bit] U at point i
 };
 constexpr uint32_t BITS_THREADS = 512, BITS_WARPS = BITS_THREADS / 32, BITS_EQ_ROWS = 512;
 constexpr uint32_t BITS_TABLE_BYTES = (2 * 128 + 3 * 64) * 128;
@@ -236,6 +239,29 @@ bit_sums_kernel(const F128d* __restrict__ z, uint64_t col_stride, uint64_t row_s
       v = warp_xor(v);
       if (t == 0 && col0 + c < n_cols) part[(uint64_t)blockIdx.y * n_cols + col0 + c] = v;
     }
+  } else if (OUT == BITS_POINTS) {
+    F128d* red = reinterpret_cast<F128d*>(bt);  // [column of the group][16 points]
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < CPW; ++c) {
+      F128d v = f128_zero();
+      const uint32_t w = col0 + c, m0 = 2 * (w >> 3), h = w & 1;  // w = 8 (M / 2) + 2 q + h
+#pragma unroll
+      for (int l = 0; l < 4; ++l) v += mul_call(weight[8 * ((m0 + (t >> 4)) & 15) + 4 * h + l], U[c][l]);
+      v.lo ^= __shfl_xor_sync(0xffffffffu, v.lo, 16);
+      v.hi ^= __shfl_xor_sync(0xffffffffu, v.hi, 16);
+      if (t < 16) red[(warp * CPW + c) * 16 + t] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 64) {
+      const uint32_t q = threadIdx.x >> 4;
+      F128d acc = f128_zero();
+      for (uint32_t c = 0; c < BITS_WARPS * CPW; ++c) {
+        const uint32_t w = blockIdx.x * BITS_WARPS * CPW + c;
+        if (w < n_cols && ((w >> 1) & 3) == q) acc += red[c * 16 + (threadIdx.x & 15)];
+      }
+      part[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * 64 + threadIdx.x] = acc;
+    }
   } else {
     F128d v[4];
 #pragma unroll
@@ -257,40 +283,32 @@ bit_sums_kernel(const F128d* __restrict__ z, uint64_t col_stride, uint64_t row_s
     }
   }
 }
-// Columns per warp and row splits. A block costs about 105 cycles a tile and column slot (used or
-// not) and 700 for the tile's tables; one block runs per SM, so the splits are the ones that fill
-// up to four whole waves best, within max_splits partial rows and at least a tile each.
+// Columns per warp and row splits: the pair of least time, for blocks that cost about 105 cycles a
+// tile and column slot (used or not), 700 for the tile's tables and 6000 + 4000 a column slot of
+// the warp for its start and end (the latter is what counts where there are few rows), one block
+// per SM at a time; at most max_splits partial rows and at least a tile each.
 struct BitSumPlan {
   uint32_t cpw, groups, splits;
   uint64_t rows_per_split;
 };
 static BitSumPlan bit_sum_plan(uint32_t n_cols, uint64_t n_rows, uint64_t max_splits) {
   BitSumPlan p{};
+  const uint64_t tiles = (n_rows + 31) / 32, sms = (uint64_t)sm_count();
+  max_splits = std::max<uint64_t>(1, std::min(max_splits, tiles));
   uint64_t best = ~0ull;
   for (uint32_t cpw = 1; cpw <= 4; ++cpw) {
     const uint32_t groups = (n_cols + BITS_WARPS * cpw - 1) / (BITS_WARPS * cpw);
-    const uint64_t cost = (uint64_t)groups * (105 * BITS_WARPS * cpw + 700);
-    if (cost < best) {
-      best = cost;
-      p.cpw = cpw;
-      p.groups = groups;
+    for (uint64_t waves = 1; waves <= 4; ++waves) {
+      const uint64_t want = std::min(max_splits, std::max<uint64_t>(1, waves * sms / groups));
+      const uint64_t per = (tiles + want - 1) / want, splits = (tiles + per - 1) / per;
+      const uint64_t used = (splits * groups + sms - 1) / sms;
+      const uint64_t cost = used * (per * (105 * BITS_WARPS * cpw + 700) + 4000 * cpw + 6000);
+      if (cost < best) {
+        best = cost;
+        p = {cpw, groups, (uint32_t)splits, per * 32};
+      }
     }
   }
-  const uint64_t tiles = (n_rows + 31) / 32, sms = (uint64_t)sm_count();
-  max_splits = std::max<uint64_t>(1, std::min(max_splits, tiles));
-  p.splits = 1;
-  double fill = 0;
-  for (uint64_t waves = 1; waves <= 4; ++waves) {
-    const uint64_t s = std::min(max_splits, std::max<uint64_t>(1, waves * sms / p.groups));
-    const uint64_t used = (s * p.groups + sms - 1) / sms;
-    const double f = (double)(s * p.groups) / (double)(used * sms);
-    if (f > fill + 0.02) {
-      fill = f;
-      p.splits = (uint32_t)s;
-    }
-  }
-  p.rows_per_split = (tiles + p.splits - 1) / p.splits * 32;
-  p.splits = (uint32_t)((n_rows + p.rows_per_split - 1) / p.rows_per_split);
   return p;
 }
 template <int CPW, int OUT>
@@ -327,134 +345,163 @@ static void bit_sums(const BitSumPlan& p, const F128d* z, uint64_t col_stride, u
 // per output. The same factorisation over words w = (K2: 2 bits, M, xo) with e2 over
 // r[7], r[8] gives s_hat_v_c[t] from bit t of z_w. P_c needs no pass of its own: it is
 // linear in the z bits and the host derives it from s_hat_v_c. D is applied by the host.
+// For P_ab the inner sums g_M(i) = sum_K e_K ext(a_x)(i) ext(b_x)(i) are formed as bits (below), and
+// since phi8 is additive the outer sums are bit sums:
+//   P_ab(i) = D * sum_{M, bit} x^M phi8(2^bit) * sum_xo eq_o(xo) * bit(g_M(i) of xo).
+constexpr uint32_t ZC_WINDOWS = 9;                           // of a 64-bit row: eight of 7 bits, one of 8
+constexpr uint32_t ZC_EXT_ENTRIES = 8 * 128 + 256;
+constexpr uint32_t ZC_EXT_BYTES = ZC_EXT_ENTRIES * 128;      // two 64-byte copies an entry
 struct ZcConsts {
-  uint8_t ext[8 * 256 * 64];   // ext[c][v][i]: extension of byte v at S[8c..8c+8)
-  F128d phi8[256];
-  uint8_t mulk[8][256];        // e_K * v
-  F128d wconst[64];            // word weights within an xo: x^M * phi8(e2[K2]) for word 4M + K2
-  uint8_t gmul[256 * 256];     // GF(2^8) products: gmul[256 a + b] = a * b
+  uint8_t ext[ZC_EXT_ENTRIES][64];  // extension of the window's bits, see upload_zc_consts
+  F128d wconst[64];                 // word weights within an xo: x^M * phi8(e2[K2]) for word 4M + K2
+  F128d pconst[128];                // x^M * phi8(2^bit) at 8 M + bit
 };
-constexpr size_t ZC_CONST_BYTES = (sizeof(ZcConsts) + 15) & ~size_t(15);
 
-// Byte b of a word, zero-extended: one byte-permute.
-__device__ __forceinline__ uint32_t byte_of(uint32_t v, int b) { return __byte_perm(v, 0, 0x4440 | b); }
-// Every byte of v set to 0xFF where its bit 7 is set (prmt with the sign-replicate bit
-// set in each selector nibble, which __byte_perm does not expose).
-__device__ __forceinline__ uint32_t msb_spread(uint32_t v) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, 0xBA98;" : "=r"(r) : "r"(v), "r"(0u));
-  return r;
-}
-// Four GF(2^8) products (AES polynomial) of packed bytes, shift-and-add in registers.
-__device__ __forceinline__ uint32_t gf8_mul4(uint32_t a, uint32_t b) {
+__host__ __device__ constexpr uint32_t gf8_const_mul(uint32_t a, uint32_t b) {
   uint32_t r = 0;
-#pragma unroll
   for (int k = 0; k < 8; ++k) {
-    r ^= a & msb_spread(b << (7 - k));  // bit k of each byte of b selects a * x^k
-    if (k < 7) a = ((a << 1) & 0xFEFEFEFEu) ^ (msb_spread(a) & 0x1B1B1B1Bu);
+    if ((b >> k) & 1) r ^= a;
+    a = (a << 1) ^ ((a & 0x80) ? 0x11Bu : 0u);
   }
-  return r;
+  return r & 0xFF;
+}
+// e_K over the three small constants of the zerocheck.
+__host__ __device__ constexpr uint32_t zc_e(int K) {
+  return gf8_const_mul(gf8_const_mul((K & 1) ? 0xF7u : 0xF6u, (K & 2) ? 0x53u : 0x52u), (K & 4) ? 0xB5u : 0xB4u);
+}
+// Where window k of a row starts.
+__host__ __device__ constexpr uint32_t zc_window_bit(uint32_t k) { return 7 * k; }
+
+// g += e_K * a * b for 32 pairs of GF(2^8) elements given as eight bit planes each: the fifteen
+// planes of the carry-less products, then the map c -> e_K c mod (x^8 + x^4 + x^3 + x + 1), whose
+// matrix is constant.
+template <int K>
+__device__ __forceinline__ void gf8_planes_mac(const uint32_t a[8], const uint32_t b[8], uint32_t g[8]) {
+  uint32_t c[15];
+#pragma unroll
+  for (int k = 0; k < 15; ++k) {
+    c[k] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k - i >= 0 && k - i < 8) c[k] ^= a[i] & b[k - i];
+  }
+#pragma unroll
+  for (int k = 14; k >= 8; --k) {
+    c[k - 4] ^= c[k];
+    c[k - 5] ^= c[k];
+    c[k - 7] ^= c[k];
+    c[k - 8] ^= c[k];
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t col = gf8_const_mul(zc_e(K), 1u << j);  // e_K x^j
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if ((col >> i) & 1) g[i] ^= c[j];
+  }
 }
 
-// P_ab: one team of 16 threads per xo, thread = four Lambda points; no block barriers
-// after the constants are staged. Per row x = 8M + K the team extends the a and b rows
-// (8 byte-table lookups each), multiplies pointwise in GF(2^8) (the 64 KB product table is
-// symmetric, so its index may put either factor high) and accumulates e_K * p into g_M;
-// then F = sum_M x^M phi8(g_M) (Horner) and acc += eq_o(xo) * F. Tables: about 199 KB of
-// shared memory, one block per SM.
-constexpr int ZC_TEAMS = 32;  // teams per block (512 threads)
-__global__ void __launch_bounds__(16 * ZC_TEAMS, 1)
-zc_round1_ab_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, uint64_t n_xo,
-                    const ZcConsts* __restrict__ gconst, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
-                    const F128d* __restrict__ eq_hi, F128d* __restrict__ part) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  ZcConsts& C = *reinterpret_cast<ZcConsts*>(smem);
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(gconst);
-    uint4* dst = reinterpret_cast<uint4*>(smem);
-    for (uint32_t i = threadIdx.x; i < ZC_CONST_BYTES / 16; i += blockDim.x) dst[i] = src[i];
+// g_M of every live xo as bits. A team of four lanes takes the row pairs (8M + K, 8(M+1) + K) of one
+// even M, lane q the points 16q .. 16q + 15: per row nine lookups of 16 bytes in the extension
+// tables, stored so that register r of an entry holds bit planes 2r (low half) and 2r + 1 of the
+// lane's 16 points; one byte permute per plane pair then sets the two rows side by side, and the
+// GF(2^8) products run on planes of 32 elements. A warp is one xo (eight teams, its 2 KB of a and
+// b read once); eight consecutive lanes are two teams, which read different copies of the 64-byte
+// entries, so no lookup conflicts. Per xo 1152 cycles of the shared-memory pipe (9 a row) and
+// about 1100 of the logic pipe. The form it replaced took 3160 (byte tables read with conflicts,
+// products from a 64 KB table and byte by byte, one F128 product an xo and point, a block per 32
+// xo): the whole round, with both bit sums, Keccak-f 2^18 15.4 -> 8.9 ms, SHA-256 2^16 2.41 -> 1.41,
+// BLAKE3 2^8 105 -> 42 us. Output word 8 (M / 2) + 2 q + h of the xo: limb l is plane 4 h + l, bits 0-15 the points
+// at M, bits 16-31 those at M + 1.
+constexpr uint32_t ZC_R1_THREADS = 512;
+__global__ void __launch_bounds__(ZC_R1_THREADS, 1)
+zc_round1_bits_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, uint64_t n_xo,
+                      const ZcConsts* __restrict__ gconst, uint4* __restrict__ g_out) {
+  extern __shared__ __align__(16) char ext[];  // ZC_EXT_BYTES
+  for (uint32_t i = threadIdx.x; i < ZC_EXT_ENTRIES * 4; i += ZC_R1_THREADS) {
+    const uint4 v = reinterpret_cast<const uint4*>(gconst->ext)[i];
+    uint4* o = reinterpret_cast<uint4*>(ext + (i >> 2) * 128) + (i & 3);
+    o[0] = v;
+    o[4] = v;
   }
   __syncthreads();
-  const uint32_t team = threadIdx.x >> 4, lane = threadIdx.x & 15;
-  // ext as bytes: table c, value v, this lane's four points at c * 16384 + v * 64 + 4 * lane
-  const uint8_t* extb = C.ext + 4 * lane;
-  F128d acc[4] = {f128_zero(), f128_zero(), f128_zero(), f128_zero()};
-  const uint64_t stride = (uint64_t)gridDim.x * ZC_TEAMS;
-  for (uint64_t xo = (uint64_t)blockIdx.x * ZC_TEAMS + team; xo < n_xo; xo += stride) {
-    const uint4* wa = reinterpret_cast<const uint4*>(a + xo * 64);
-    const uint4* wb = reinterpret_cast<const uint4*>(b + xo * 64);
-    uint32_t G[16];
-#pragma unroll 1
-    for (int M = 0; M < 16; ++M) {
-      uint32_t g = 0;
+  const uint32_t lane = threadIdx.x & 31, mp = lane >> 2;
+  const uint32_t off = (mp & 1) * 64 + (lane & 3) * 16;  // this team's copy, this lane's points
+  auto extend = [&](uint32_t lo, uint32_t hi) {
+    constexpr uint32_t M7 = 127u << 7;
+    const uint32_t o[ZC_WINDOWS] = {(lo << 7) & M7, lo & M7, (lo >> 7) & M7, (lo >> 14) & M7,
+                                    __funnelshift_r(lo, hi, 21) & M7, (hi << 4) & M7, (hi >> 3) & M7, (hi >> 10) & M7,
+                                    (hi >> 17) & (255u << 7)};
+    uint4 r = make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        uint4 A = wa[4 * M + kk], B = wb[4 * M + kk];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t a0 = h ? A.z : A.x, a1 = h ? A.w : A.y;  // the 64-bit row as two words
-          uint32_t b0 = h ? B.z : B.x, b1 = h ? B.w : B.y;
-          uint32_t ea = 0, eb = 0;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            ea ^= *reinterpret_cast<const uint32_t*>(extb + c * 16384 + (byte_of(a0, c) << 6)) ^
-                  *reinterpret_cast<const uint32_t*>(extb + (c + 4) * 16384 + (byte_of(a1, c) << 6));
-            eb ^= *reinterpret_cast<const uint32_t*>(extb + c * 16384 + (byte_of(b0, c) << 6)) ^
-                  *reinterpret_cast<const uint32_t*>(extb + (c + 4) * 16384 + (byte_of(b1, c) << 6));
-          }
-          // the four GF(2^8) products, then e_K times each (mulk table): half of the rows take
-          // the products from the 64 KB product table (shared-memory pipe), half compute them
-          // in registers (logic pipe), which balances the two pipes
-          const uint8_t* mk = C.mulk[2 * kk + h];
-          if (h == 0) {
-            const uint32_t i01 = __byte_perm(ea, eb, 0x5140), i23 = __byte_perm(ea, eb, 0x7362);
-            g ^= (uint32_t)mk[C.gmul[i01 & 0xFFFF]] | ((uint32_t)mk[C.gmul[i01 >> 16]] << 8) |
-                 ((uint32_t)mk[C.gmul[i23 & 0xFFFF]] << 16) | ((uint32_t)mk[C.gmul[i23 >> 16]] << 24);
-          } else {
-            const uint32_t p = gf8_mul4(ea, eb);
-            g ^= (uint32_t)mk[byte_of(p, 0)] | ((uint32_t)mk[byte_of(p, 1)] << 8) | ((uint32_t)mk[byte_of(p, 2)] << 16) |
-                 ((uint32_t)mk[byte_of(p, 3)] << 24);
-          }
-        }
-      }
-      G[M] = g;
+    for (uint32_t k = 0; k < ZC_WINDOWS; ++k) {
+      const uint4 t = *reinterpret_cast<const uint4*>(ext + k * 128 * 128 + (o[k] | off));
+      r.x ^= t.x;
+      r.y ^= t.y;
+      r.z ^= t.z;
+      r.w ^= t.w;
     }
-    F128d e = eq_at(eq_lo, lo_bits, eq_hi, xo);
+    return r;
+  };
+  auto planes = [](uint4 x, uint4 y, uint32_t o[8]) {  // rows of M and M + 1 side by side
+    o[0] = __byte_perm(x.x, y.x, 0x5410); o[1] = __byte_perm(x.x, y.x, 0x7632);
+    o[2] = __byte_perm(x.y, y.y, 0x5410); o[3] = __byte_perm(x.y, y.y, 0x7632);
+    o[4] = __byte_perm(x.z, y.z, 0x5410); o[5] = __byte_perm(x.z, y.z, 0x7632);
+    o[6] = __byte_perm(x.w, y.w, 0x5410); o[7] = __byte_perm(x.w, y.w, 0x7632);
+  };
+  for (uint64_t xo = (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; xo < n_xo;
+       xo += (uint64_t)gridDim.x * (ZC_R1_THREADS / 32)) {
+    const uint4* wa = reinterpret_cast<const uint4*>(a + xo * 64) + 8 * mp;  // words of M, then of M + 1
+    const uint4* wb = reinterpret_cast<const uint4*>(b + xo * 64) + 8 * mp;
+    uint32_t g[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      F128d F = f128_zero();
-#pragma unroll
-      for (int M = 15; M >= 0; --M) F = mul_by_x(F) + C.phi8[(G[M] >> (8 * k)) & 255];
-      acc[k] += mul_call(e, F);
-    }
+    for (int i = 0; i < 8; ++i) g[i] = 0;
+    auto rows = [&](auto kk) {  // the word's two rows K = 2 kk and 2 kk + 1
+      constexpr int k2 = decltype(kk)::value;
+      const uint4 A0 = wa[k2], A1 = wa[4 + k2], B0 = wb[k2], B1 = wb[4 + k2];
+      uint32_t pa[8], pb[8];
+      planes(extend(A0.x, A0.y), extend(A1.x, A1.y), pa);
+      planes(extend(B0.x, B0.y), extend(B1.x, B1.y), pb);
+      gf8_planes_mac<2 * k2>(pa, pb, g);
+      planes(extend(A0.z, A0.w), extend(A1.z, A1.w), pa);
+      planes(extend(B0.z, B0.w), extend(B1.z, B1.w), pb);
+      gf8_planes_mac<2 * k2 + 1>(pa, pb, g);
+    };
+    rows(std::integral_constant<int, 0>());
+    rows(std::integral_constant<int, 1>());
+    rows(std::integral_constant<int, 2>());
+    rows(std::integral_constant<int, 3>());
+    uint4* o = g_out + xo * 64 + 8 * mp + 2 * (lane & 3);
+    o[0] = make_uint4(g[0], g[1], g[2], g[3]);
+    o[1] = make_uint4(g[4], g[5], g[6], g[7]);
   }
-  uint64_t row = (uint64_t)blockIdx.x * ZC_TEAMS + team;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) part[row * 64 + 4 * lane + k] = acc[k];
 }
 
 static ZcConsts* g_zc_consts_dev[MAX_DEVICES] = {};  // written under the caller's lock, before any prover launches
 static ZcConsts* zc_consts() { return g_zc_consts_dev[current_device()]; }
-void upload_zc_consts(const uint8_t* ext, const F128d* phi8, const uint8_t mulk[8][256], const F128d* wconst) {
+// unit[64 s + i]: the extension of row bit s at Lambda point i.
+void upload_zc_consts(const uint8_t* unit, const F128d* wconst, const F128d* pconst) {
   const int dev = current_device();
   if (g_zc_consts_dev[dev]) return;
   ZcConsts* h = new ZcConsts();
-  memcpy(h->ext, ext, sizeof(h->ext));
-  memcpy(h->phi8, phi8, sizeof(h->phi8));
-  memcpy(h->mulk, mulk, sizeof(h->mulk));
-  memcpy(h->wconst, wconst, sizeof(h->wconst));
-  for (uint32_t a = 0; a < 256; ++a)
-    for (uint32_t b = 0; b < 256; ++b) {
-      uint32_t p = 0, x = a;  // shift-and-add modulo the AES polynomial x^8 + x^4 + x^3 + x + 1
-      for (int k = 0; k < 8; ++k) {
-        if ((b >> k) & 1) p ^= x;
-        x = (x << 1) ^ ((x & 0x80) ? 0x11B : 0);
-      }
-      h->gmul[256 * a + b] = (uint8_t)p;
+  for (uint32_t e = 0; e < ZC_EXT_ENTRIES; ++e) {
+    const uint32_t k = std::min(e >> 7, ZC_WINDOWS - 1), v = e - (k << 7);
+    for (uint32_t i = 0; i < 64; ++i) {
+      uint8_t x = 0;
+      for (uint32_t bit = 0; bit < 8; ++bit)
+        if ((v >> bit) & 1) x ^= unit[64 * (zc_window_bit(k) + bit) + i];
+      // plane p of points 16q .. 16q + 15: half p & 1 of 32-bit word 4 q + p / 2
+      for (uint32_t p = 0; p < 8; ++p)
+        if ((x >> p) & 1) {
+          const uint32_t pos = (i & 15) + 16 * (p & 1);
+          h->ext[e][16 * (i >> 4) + 4 * (p >> 1) + (pos >> 3)] |= (uint8_t)(1u << (pos & 7));
+        }
     }
+  }
+  memcpy(h->wconst, wconst, sizeof(h->wconst));
+  memcpy(h->pconst, pconst, sizeof(h->pconst));
   ZcConsts* d = nullptr;
-  CUDA_OK(cudaMalloc(&d, ZC_CONST_BYTES));
-  CUDA_OK(cudaMemset(d, 0, ZC_CONST_BYTES));
+  CUDA_OK(cudaMalloc(&d, sizeof(ZcConsts)));
   CUDA_OK(cudaMemcpy(d, h, sizeof(ZcConsts), cudaMemcpyHostToDevice));
   CUDA_OK(cudaDeviceSynchronize());  // complete before any kernel of a non-blocking stream reads it
   delete h;
@@ -462,24 +509,22 @@ void upload_zc_consts(const uint8_t* ext, const F128d* phi8, const uint8_t mulk[
 }
 
 void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m, uint64_t live_words,
-                      const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* part_ab, uint32_t* nrows_ab,
-                      F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s) {
-  ZcConsts* g_zc_consts = zc_consts();
-  if (!g_zc_consts) throw std::runtime_error("zerocheck constants not uploaded");
-  uint64_t n_xo = 1ull << (m - 13);
+                      const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* g, F128d* part_ab,
+                      uint32_t* nrows_ab, F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s) {
+  const ZcConsts* consts = zc_consts();
+  if (!consts) throw std::runtime_error("zerocheck constants not uploaded");
   // xo past the live words hold zero rows of z, a and b and add nothing to any sum
-  const uint64_t xo_live = std::min<uint64_t>(n_xo, (live_words + 63) / 64);
-  size_t smem = ZC_CONST_BYTES;
-  set_dynamic_smem((const void*)zc_round1_ab_kernel, (int)smem);
-  uint32_t blocks = (uint32_t)std::max<uint64_t>(
-      1, std::min<uint64_t>((xo_live + ZC_TEAMS - 1) / ZC_TEAMS, (uint64_t)sm_count()));
-  zc_round1_ab_kernel<<<blocks, 16 * ZC_TEAMS, smem, s>>>(a, b, xo_live, g_zc_consts, eq_lo, lo_bits, eq_hi, part_ab);
+  const uint64_t xo_live = std::min<uint64_t>(1ull << (m - 13), (live_words + 63) / 64);
+  set_dynamic_smem((const void*)zc_round1_bits_kernel, (int)ZC_EXT_BYTES);
+  // one block per SM; xo are dealt to the blocks first, then to their warps
+  const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(xo_live, (uint64_t)sm_count()));
+  zc_round1_bits_kernel<<<blocks, ZC_R1_THREADS, ZC_EXT_BYTES, s>>>(a, b, xo_live, consts, reinterpret_cast<uint4*>(g));
   LAUNCH_OK();
-  *nrows_ab = blocks * ZC_TEAMS;
-  // s_hat_v_c[t] = sum_xo eq_o(xo) sum_w wconst[w] bit_t(z[64 xo + w])
+  // both outer sums: 64 words an xo, rows = xo
   const BitSumPlan p = bit_sum_plan(64, xo_live, 1024);
-  bit_sums<BITS_COLUMNS>(p, z, 1, 64, 64, xo_live, eq_lo, lo_bits, eq_hi, g_zc_consts->wconst, part_svc, s);
-  *nrows_svc = p.groups * p.splits;
+  bit_sums<BITS_POINTS>(p, g, 1, 64, 64, xo_live, eq_lo, lo_bits, eq_hi, consts->pconst, part_ab, s);
+  bit_sums<BITS_COLUMNS>(p, z, 1, 64, 64, xo_live, eq_lo, lo_bits, eq_hi, consts->wconst, part_svc, s);
+  *nrows_ab = *nrows_svc = p.groups * p.splits;
 }
 
 // ------------------------------------------------------------------ zerocheck skip fold

@@ -7,8 +7,7 @@
 //    over the set bits j of `block`; stored flat as tw[(1 << layer) - 1 + block].
 //  * The univariate-skip extension S -> Lambda of a 64-point GF(2) row: the GF(2^8)
 //    additive NTT of crates/flock-core/src/ntt.rs:18-117 with cosets beta = 0 (S) and
-//    beta = 64 (Lambda), inverse on S then forward on Lambda, tabulated per input byte
-//    (ext[c][v][i] = sum over set bits b of v of unit(8c + b)[i]).
+//    beta = 64 (Lambda), inverse on S then forward on Lambda, of every unit vector.
 #pragma once
 #include "field.h"
 
@@ -89,10 +88,8 @@ struct Gf8Ntt64 {
   }
 };
 
-// ext[c * 256 * 64 + v * 64 + i]: extension on Lambda of the bits v placed at S[8c..8c+8).
 struct SkipTables {
-  std::vector<uint8_t> ext;   // 8 x 256 x 64
-  uint8_t unit[64][64];       // extension of each unit vector
+  uint8_t unit[64][64];       // extension on Lambda of each unit vector on S
 };
 inline const SkipTables& skip_tables() {
   static SkipTables t = [] {
@@ -105,12 +102,6 @@ inline const SkipTables& skip_tables() {
       on_l.forward(v, 64, 1);
       memcpy(s.unit[b], v, 64);
     }
-    s.ext.assign(8 * 256 * 64, 0);
-    for (int c = 0; c < 8; ++c)
-      for (int v = 0; v < 256; ++v)
-        for (int b = 0; b < 8; ++b)
-          if ((v >> b) & 1)
-            for (int i = 0; i < 64; ++i) s.ext[(c * 256 + v) * 64 + i] ^= s.unit[8 * c + b][i];
     return s;
   }();
   return t;
