@@ -209,7 +209,8 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
     lb_[k] = dmalloc<F256d>(2 * rows(), owned_, device_bytes_);
   }
   pend_ = dmalloc<F128d>(2 * rows(), owned_, device_bytes_);
-  CUDA_OK(cudaHostAlloc(&h_tail_, 2 * lanes_pow2() * sizeof(F128d), cudaHostAllocMapped));
+  static_assert(2 * TAIL >= 4 * LG_TAIL, "the tail buffer holds two F256 vectors of LG_TAIL entries");
+  CUDA_OK(cudaHostAlloc(&h_tail_, 2 * TAIL * sizeof(F128d), cudaHostAllocMapped));
   CUDA_OK(cudaHostGetDevicePointer(&d_tail_, h_tail_, 0));
   part_cap_ = 1u << 20;
   part_ = dmalloc<F128d>(part_cap_, owned_, device_bytes_);
@@ -545,6 +546,38 @@ std::vector<Hash> GpuBackend::read_cap(const uint8_t* tree, uint64_t n_leaves, u
   return cap;
 }
 
+// ------------------------------------------------------------------ tails on the host
+// Fold the low variable of both vectors at r; the message over the folded pairs, weighted by eq
+// (empty: 1): g1 = sum eq A1 B1, ginf = sum eq (A0 + A1) (B0 + B1).
+void GpuBackend::TailPair::fold(F128 r) {
+  const size_t half = a.size() / 2;
+  for (size_t i = 0; i < half; ++i) {
+    a[i] = a[2 * i] + r * (a[2 * i + 1] + a[2 * i]);
+    b[i] = b[2 * i] + r * (b[2 * i + 1] + b[2 * i]);
+  }
+  a.resize(half);
+  b.resize(half);
+}
+void GpuBackend::TailPair::message(const std::vector<F128>& eq, F128& g1, F128& gi) const {
+  g1 = gi = F128();
+  for (size_t j = 0; 2 * j + 1 < a.size(); ++j) {
+    const F128 t1 = a[2 * j + 1] * b[2 * j + 1], ti = (a[2 * j] + a[2 * j + 1]) * (b[2 * j] + b[2 * j + 1]);
+    g1 += eq.empty() ? t1 : eq[j] * t1;
+    gi += eq.empty() ? ti : eq[j] * ti;
+  }
+}
+// The two vectors of n entries that a published one-block fold left in mapped memory.
+GpuBackend::TailPair GpuBackend::read_tail(size_t n) {
+  TailPair t;
+  const volatile F128d* m = h_tail_;
+  for (size_t i = 0; i < n; ++i) {
+    t.a.push_back(F128(m[i].lo, m[i].hi));
+    t.b.push_back(F128(m[n + i].lo, m[n + i].hi));
+  }
+  d2h_ += 2 * n * sizeof(F128d);
+  return t;
+}
+
 // ------------------------------------------------------------------ zerocheck
 void GpuBackend::zc_round1(const std::vector<F128>& r, std::vector<F128>& ab, std::vector<F128>& c,
                            std::vector<F128>& svc) {
@@ -657,6 +690,7 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   auto v = reduce(nb, 2);
   g1 = v[0];
   gi = v[1];
+  zc_tail_ = TailPair();
   zc_cur_a_ = nullptr;  // the skip-folded vectors live only implicitly (a, b bits and the weights)
   zc_cur_b_ = nullptr;
   zc_len_ = 2 * W_;
@@ -671,6 +705,13 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
   if (k + 1 >= zc_desc_.size() ||
       zc_desc_[k].n + (zc_round_ < zc_w_ ? zc_desc_[1].n : zc_desc_[k + 1].n) != eq_point.size())
     throw std::runtime_error("zerocheck fold: round tables out of step");
+  if (!zc_tail_.a.empty()) {
+    zc_tail_.fold(rho);
+    zc_tail_.message(build_eq(eq_point), g1, gi);
+    zc_len_ /= 2;
+    zc_round_++;
+    return;
+  }
   const EqDesc& lo = zc_desc_[k];
   const EqDesc& hi = zc_desc_[k + 1];
   // pairs (4 entries in, 2 out) from live_pairs on read only the zero tail
@@ -678,6 +719,11 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
   // round 0 writes W words per vector into zc2; later rounds alternate zc1 <-> zc2
   F128d* oa = (zc_round_ == 0 || zc_cur_a_ == zc1a_) ? zc2a_ : zc1a_;
   F128d* ob = (zc_round_ == 0 || zc_cur_a_ == zc1a_) ? zc2b_ : zc1b_;
+  const bool tail = zc_round_ > 0 && 2 * n_pairs == TAIL;
+  if (tail) {
+    oa = d_tail_;
+    ob = d_tail_ + TAIL;
+  }
   uint32_t nb, pub_seq = 0;
   {
     Mark mk(this, ST_ZC_FOLDS);
@@ -702,6 +748,7 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
   auto v = pub_seq ? read_published(pub_seq, 2) : reduce(nb, 2);
   g1 = v[0];
   gi = v[1];
+  if (tail) zc_tail_ = read_tail(TAIL);
   zc_cur_a_ = oa;
   zc_cur_b_ = ob;
   zc_len_ /= 2;
@@ -710,11 +757,10 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
 }
 
 void GpuBackend::zc_final(F128 rho, F128& ae, F128& be) {
-  if (zc_len_ != 2) throw std::runtime_error("zerocheck final fold expects two values");
-  auto av = fetch(zc_cur_a_, 2);
-  auto bv = fetch(zc_cur_b_, 2);
-  ae = av[0] + rho * (av[1] + av[0]);
-  be = bv[0] + rho * (bv[1] + bv[0]);
+  if (zc_len_ != 2 || zc_tail_.a.size() != 2) throw std::runtime_error("zerocheck final fold expects two values");
+  zc_tail_.fold(rho);
+  ae = zc_tail_.a[0];
+  be = zc_tail_.b[0];
 }
 
 // ------------------------------------------------------------------ lincheck
@@ -762,6 +808,7 @@ void GpuBackend::lc_zvec(const std::vector<F128>& x_outer) {
   launch_lc_zvec(z_, nu, used, e.lo, e.lo_bits, e.hi, part_, part_cap_, zv_, st_);
   CUDA_OK(cudaMemcpyAsync(zvcap_, zv_, K_ * 16, cudaMemcpyDeviceToDevice, st_));
   lc_len_ = K_;
+  lc_tail_ = TailPair();
 }
 
 void GpuBackend::lc_start(F128 alpha, const std::vector<SlotComb>& sc, F128& e1, F128& ei) {
@@ -783,20 +830,38 @@ void GpuBackend::lc_start(F128 alpha, const std::vector<SlotComb>& sc, F128& e1,
 }
 
 void GpuBackend::lc_round(F128 r, bool last, F128& e1, F128& ei) {
-  // the last round's message is not used
-  FusedPublish fp = fused_publish();
-  { Mark mk(this, ST_LINCHECK); launch_lc_round(comb_, zv_, lc_len_, dev(r), part_, st_, fp); }
-  lc_len_ /= 2;
-  if (!last) {
-    auto v = read_published(fp.seq, 2);
-    e1 = v[0];
-    ei = v[1];
+  if (!lc_tail_.a.empty()) {  // the top variable of comb and zv, on the host
+    std::vector<F128>&c = lc_tail_.a, &z = lc_tail_.b;
+    const size_t h = c.size() / 2, q = h / 2;
+    for (size_t i = 0; i < h; ++i) {
+      c[i] = c[i] + r * (c[i + h] + c[i]);
+      z[i] = z[i] + r * (z[i + h] + z[i]);
+    }
+    c.resize(h);
+    z.resize(h);
+    lc_len_ /= 2;
+    e1 = ei = F128();
+    for (size_t i = 0; i < q && !last; ++i) {
+      e1 += c[i + q] * z[i + q];
+      ei += (c[i] + c[i + q]) * (z[i] + z[i + q]);
+    }
+    return;
   }
+  const bool tail = lc_len_ / 2 == TAIL;
+  F128d* co = tail ? d_tail_ : comb_;
+  F128d* zo = tail ? d_tail_ + TAIL : zv_;
+  FusedPublish fp = fused_publish();
+  { Mark mk(this, ST_LINCHECK); launch_lc_round(comb_, zv_, lc_len_, dev(r), co, zo, part_, st_, fp); }
+  lc_len_ /= 2;
+  auto v = read_published(fp.seq, 2);
+  e1 = v[0];
+  ei = v[1];
+  if (tail) lc_tail_ = read_tail(TAIL);
 }
 
 void GpuBackend::lc_partial(std::vector<F128>& zp) {
-  if (lc_len_ != 64) throw std::runtime_error("lincheck partial expects 64 values");
-  zp = fetch(zv_, 64);
+  if (lc_len_ != 64 || lc_tail_.b.size() != 64) throw std::runtime_error("lincheck partial expects 64 values");
+  zp = lc_tail_.b;
 }
 
 void GpuBackend::lc_matrix_evals(const std::vector<F128>& rest, const std::vector<F128>& zp,
@@ -862,38 +927,26 @@ void GpuBackend::mo_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uin
   mo_len_ = Q_;
   mo_live_ = std::min<uint64_t>(Q_, area);
   mo_chal_.clear();
-  mo_tail_q_.clear();
-  mo_tail_w_.clear();
+  mo_tail_ = TailPair();
   mo_lane_q_.clear();
 }
 
 void GpuBackend::mo_round(F128 r, bool last, F128& g1, F128& gi) {
   mo_chal_.push_back(r);
-  if (!mo_tail_q_.empty()) {  // the lane bits, on the host
-    std::vector<F128>&q = mo_tail_q_, &w = mo_tail_w_;
-    const size_t half = q.size() / 2;
-    for (size_t i = 0; i < half; ++i) {
-      q[i] = q[2 * i] + r * (q[2 * i + 1] + q[2 * i]);
-      w[i] = w[2 * i] + r * (w[2 * i + 1] + w[2 * i]);
-    }
-    q.resize(half);
-    w.resize(half);
-    g1 = gi = F128();
-    for (size_t i = 0; i + 1 < half && !last; i += 2) {
-      g1 += q[i + 1] * w[i + 1];
-      gi += (q[i] + q[i + 1]) * (w[i] + w[i + 1]);
-    }
+  if (!mo_tail_.a.empty()) {
+    mo_tail_.fold(r);
+    if (!last) mo_tail_.message({}, g1, gi);
+    if (mo_tail_.a.size() == lanes_pow2()) mo_lane_q_ = mo_tail_.a;
     return;
   }
   F128d* oq = (mo_q_ == moAq_) ? moBq_ : moAq_;
   F128d* ow = (mo_q_ == moAq_) ? moBw_ : moAw_;
   uint64_t n_pairs = mo_len_ / 4;
   const uint64_t live_pairs = std::min<uint64_t>(n_pairs, (mo_live_ + 3) / 4);
-  // one entry per lane left: written to mapped memory (one block, published with the message)
-  const bool tail = 2 * n_pairs == lanes_pow2();
+  const bool tail = 2 * n_pairs == TAIL;
   if (tail) {
     oq = d_tail_;
-    ow = d_tail_ + lanes_pow2();
+    ow = d_tail_ + TAIL;
   }
   FusedPublish fp = fused_publish();
   {
@@ -907,20 +960,12 @@ void GpuBackend::mo_round(F128 r, bool last, F128& g1, F128& gi) {
   auto v = read_published(fp.seq, 2);
   g1 = v[0];
   gi = v[1];
-  if (tail) {
-    const volatile F128d* t = h_tail_;
-    for (uint64_t i = 0; i < mo_len_; ++i) {
-      mo_tail_q_.push_back(F128(t[i].lo, t[i].hi));
-      mo_tail_w_.push_back(F128(t[mo_len_ + i].lo, t[mo_len_ + i].hi));
-    }
-    d2h_ += 2 * mo_len_ * sizeof(F128d);
-    mo_lane_q_ = mo_tail_q_;
-  }
+  if (tail) mo_tail_ = read_tail(TAIL);
 }
 
 F128 GpuBackend::mo_q_eval() {
-  if (mo_tail_q_.size() != 1) throw std::runtime_error("merged open: the claim is evaluated after its last round");
-  return mo_tail_q_[0];
+  if (mo_tail_.a.size() != 1) throw std::runtime_error("merged open: the claim is evaluated after its last round");
+  return mo_tail_.a[0];
 }
 
 // ------------------------------------------------------------------ Ligerito
@@ -952,6 +997,9 @@ void GpuBackend::add_lane_term(F128 coef, const std::vector<F128>& point) {
 void GpuBackend::lg_basis_eq(F128 gamma, const std::vector<F128>& rho) {
   if ((uint64_t(1) << rho.size()) != Q_) throw std::runtime_error("Ligerito basis size mismatch");
   lg_pend_fold_.active = lg_pend_switch_ = false;
+  lg_last_level_ = false;
+  lg_tail_f_.clear();
+  lg_tail_b_.clear();
   lane_ = LaneStage();
   lane_.active = true;
   lane_.w.assign(1, F256::one());
@@ -1039,12 +1087,26 @@ Msg256 GpuBackend::message256(const FusedPublish& fp) {
   return m;
 }
 
+// The message over neighbours of the last level's tail, u0 = sum f0 b0, u2 = sum (f0 + f1) (b0 + b1).
+Msg256 GpuBackend::lg_tail_message() const {
+  Msg256 m;
+  for (size_t i = 0; i + 1 < lg_tail_f_.size(); i += 2) {
+    m.u0 += lg_tail_f_[i] * lg_tail_b_[i];
+    m.u2 += (lg_tail_f_[i] + lg_tail_f_[i + 1]) * (lg_tail_b_[i] + lg_tail_b_[i + 1]);
+  }
+  return m;
+}
+
 Msg256 GpuBackend::lg_message(size_t d) {
   if (lane_.active) {
     if (lane_.folded && d == 1) return lane_switch();
     if (lane_.folded || lane_.bound == S.log_batch || d != rows())
       throw std::runtime_error("the lane stage's messages pair lanes, then the switched entries");
     return lane_message();
+  }
+  if (!lg_tail_f_.empty()) {
+    if (d != 1 && d != lg_n_) throw std::runtime_error("the last level's messages pair neighbours");
+    return lg_tail_message();
   }
   if (lg_pend_switch_ && (d == 1 || 2 * lg_n_ == d)) {
     // code switch and the message over its pairs (2i, 2i + 1) in one pass
@@ -1065,16 +1127,28 @@ Msg256 GpuBackend::lg_message(size_t d) {
     const uint64_t n_out = lg_n_ / 2;
     const size_t dm = (d == 1 || n_out == d) ? 1 : d;
     const int nx = lg_cur_ ^ 1;
+    // the last level's folds finish on the host once one block holds what is left
+    const bool tail = lg_last_level_ && n_out == LG_TAIL && lg_pend_fold_.d == 1 && dm == 1;
+    F256d* fo = tail ? reinterpret_cast<F256d*>(d_tail_) : lf_[nx];
+    F256d* bo = tail ? fo + LG_TAIL : lb_[nx];
     FusedPublish fp = fused_publish();
     {
       Mark mk(this, ST_LIGERITO);
-      launch_lg_fold_msg256(lf_[lg_cur_], lb_[lg_cur_], n_out, dev(lg_pend_fold_.r), lg_pend_fold_.d, dm, lf_[nx],
-                            lb_[nx], part_, st_, fp);
+      launch_lg_fold_msg256(lf_[lg_cur_], lb_[lg_cur_], n_out, dev(lg_pend_fold_.r), lg_pend_fold_.d, dm, fo, bo, part_,
+                            st_, fp);
     }
     lg_pend_fold_.active = false;
     lg_cur_ = nx;
     lg_n_ = n_out;
-    return message256(fp);
+    const Msg256 m = message256(fp);
+    if (tail) {
+      const TailPair t = read_tail(2 * LG_TAIL);  // f's halves, then b's
+      for (size_t i = 0; i < LG_TAIL; ++i) {
+        lg_tail_f_.push_back(F256(t.a[2 * i], t.a[2 * i + 1]));
+        lg_tail_b_.push_back(F256(t.b[2 * i], t.b[2 * i + 1]));
+      }
+    }
+    return m;
   }
   if (d == 1 || lg_n_ == d) d = 1;
   FusedPublish fp = fused_publish();
@@ -1113,6 +1187,15 @@ void GpuBackend::lg_fold(F256 r, size_t d) {
     lane_fold(r);
     return;
   }
+  if (!lg_tail_f_.empty()) {
+    if (d != 1) throw std::runtime_error("the last level folds neighbours");
+    for (std::vector<F256>* v : {&lg_tail_f_, &lg_tail_b_}) {
+      for (size_t i = 0; i < v->size() / 2; ++i) (*v)[i] = (*v)[2 * i] + r * ((*v)[2 * i + 1] + (*v)[2 * i]);
+      v->resize(v->size() / 2);
+    }
+    lg_n_ /= 2;
+    return;
+  }
   lg_flush_fold();
   // held back: the next message runs fused with it, any other call performs it first
   lg_pend_fold_.active = true;
@@ -1135,6 +1218,7 @@ void GpuBackend::lg_commit(uint32_t level, uint32_t log_cols, uint32_t log_lanes
                            uint32_t cap_depth, std::vector<Hash>& cap) {
   lg_flush_fold();
   if (lg_n_ != (uint64_t(1) << (log_cols + log_lanes))) throw std::runtime_error("Ligerito commit size mismatch");
+  lg_last_level_ = level == S.lig.r;
   if (levels_.size() < level + 1) levels_.resize(level + 1);
   Level& L = levels_[level];
   uint64_t block_len = uint64_t(1) << (log_cols + log_rate);
@@ -1244,6 +1328,7 @@ void GpuBackend::lg_open(uint32_t level, const std::vector<uint64_t>& pos, uint3
 }
 
 std::vector<F256> GpuBackend::lg_residual() {
+  if (!lg_tail_f_.empty()) return lg_tail_f_;
   lg_flush_fold();
   std::vector<F256> out(lg_n_);
   CUDA_OK(cudaMemcpyAsync(out.data(), lf_[lg_cur_], lg_n_ * sizeof(F256d), cudaMemcpyDeviceToHost, st_));

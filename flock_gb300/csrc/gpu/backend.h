@@ -177,10 +177,22 @@ class GpuBackend : public ProverBackend {
   uint64_t mo_len_ = 0;
   uint64_t mo_live_ = 0;  // entries of q and W that can be nonzero (both are zero from the area on)
 
-  // The tail of the merged open: the fold that leaves one entry per lane writes q and W to
-  // mapped memory, and the last rounds (over the lane bits) run on the host.
+  // The last rounds of the zerocheck, the lincheck, the merged open and Ligerito's last level: the
+  // fold that leaves TAIL entries (one block of the small-round kernel; LG_TAIL for F256) writes
+  // them to mapped memory beside its message, and the rest runs on the host. A round on so few
+  // entries costs the device about 15 us of launch, latency and publication, the host one to three.
+  static constexpr size_t TAIL = 128, LG_TAIL = 64;
+  struct TailPair {
+    std::vector<F128> a, b;
+    void fold(F128 r);
+    void message(const std::vector<F128>& eq, F128& g1, F128& gi) const;
+  };
+  TailPair read_tail(size_t n);
   F128d *h_tail_ = nullptr, *d_tail_ = nullptr;
-  std::vector<F128> mo_tail_q_, mo_tail_w_;  // current tail vectors (empty before the tail)
+  TailPair zc_tail_, lc_tail_, mo_tail_;     // empty before each tail
+  std::vector<F256> lg_tail_f_, lg_tail_b_;
+  bool lg_last_level_ = false;
+  Msg256 lg_tail_message() const;
   std::vector<F128> mo_chal_;                // the round challenges so far
   std::vector<F128> mo_lane_q_;              // q folded at the row challenges: the lane dots at that point
   uint64_t lanes_pow2() const { return uint64_t(1) << S.log_batch; }

@@ -131,7 +131,8 @@ void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F12
                     const F128d* eq_hi, F128d* part, uint64_t part_cap, F128d* zv, cudaStream_t s);
 uint32_t launch_lc_start(const F128d* ca, const F128d* cb, F128d alpha, F128d beta, uint32_t pin, uint32_t K,
                          F128d* comb, const F128d* zv, F128d* part, cudaStream_t s);                   // width 2
-uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, F128d* part, cudaStream_t s, FusedPublish pub);
+uint32_t launch_lc_round(const F128d* comb, const F128d* zv, uint32_t len, F128d r, F128d* comb_out, F128d* zv_out,
+                         F128d* part, cudaStream_t s, FusedPublish pub);
 // Union lincheck: one slot's weighted comb (out = weight (alpha ca + cb), + beta at pin),
 // and the first message of a comb built that way.
 void launch_lc_slot_comb(const F128d* ca, const F128d* cb, F128d alpha, F128d weight, F128d beta, uint32_t pin,

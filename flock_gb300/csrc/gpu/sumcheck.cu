@@ -1243,15 +1243,16 @@ uint32_t launch_lc_top_message(const F128d* comb, const F128d* zv, uint32_t K, F
   return blocks;
 }
 
-// Bind the top variable of comb and zv (length len -> len/2) in place and emit the next
+// Bind the top variable of comb and zv (length len -> len/2, in place or not) and emit the next
 // top-variable message over the bound vectors (pairs (i, i + len/4)): e1 = sum c1 z1, einf =
 // sum (c0 + c1) (z0 + z1).
-uint32_t launch_lc_round(F128d* comb, F128d* zv, uint32_t len, F128d r, F128d* part, cudaStream_t s, FusedPublish pub) {
+uint32_t launch_lc_round(const F128d* comb, const F128d* zv, uint32_t len, F128d r, F128d* comb_out, F128d* zv_out,
+                         F128d* part, cudaStream_t s, FusedPublish pub) {
   const uint64_t q = len / 4;
   if (q == 0) throw std::runtime_error("lincheck round: fewer than four entries");
   const uint32_t blocks = (uint32_t)((q + SMALL_PAIRS - 1) / SMALL_PAIRS);
   pair_fold_small_kernel<EQ_NONE, MAP_TOP><<<blocks, SMALL_THREADS, 0, s>>>(comb, zv, q, q, r, nullptr, 0, nullptr, nullptr,
-                                                                            comb, zv, part, pub);
+                                                                            comb_out, zv_out, part, pub);
   LAUNCH_OK();
   return blocks;
 }
