@@ -319,22 +319,43 @@ void launch_ntt(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t start_laye
 }
 
 // ---- Merkle
+template <bool MULADD>
 __global__ void merkle_leaves_kernel(const F128d* __restrict__ rows, uint32_t lanes, uint64_t n_leaves,
                                      uint32_t* __restrict__ tree) {
   uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_leaves) return;
-  const uint32_t* w = (const uint32_t*)(rows + p * lanes);
-  uint32_t out[8];
-  sha256_words([&](uint32_t i) { return __ldg(w + i); }, lanes * 4, out);
+  // blocks of four 16-byte words, then the rest with the padding (80, zeros, the bit length)
+  const uint4* w = reinterpret_cast<const uint4*>(rows + p * lanes);
+  uint32_t st[8], m[16];
+  sha256_init(st);
+  auto put = [&](int i, uint4 v) {
+    m[4 * i] = bswap32(v.x);
+    m[4 * i + 1] = bswap32(v.y);
+    m[4 * i + 2] = bswap32(v.z);
+    m[4 * i + 3] = bswap32(v.w);
+  };
+  uint32_t b = 0;
+  for (; b + 4 <= lanes; b += 4) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) tree[p * 8 + i] = out[i];
+    for (int i = 0; i < 4; ++i) put(i, __ldg(w + b + i));
+    sha256_compress<MULADD>(st, m);
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i)
+    put(i, b + i < lanes ? __ldg(w + b + i) : make_uint4(b + i == lanes ? 0x80u : 0u, 0, 0, 0));
+  m[14] = 0;
+  m[15] = lanes * 128;
+  sha256_compress<MULADD>(st, m);
+  uint4* o = reinterpret_cast<uint4*>(tree + p * 8);
+  o[0] = make_uint4(bswap32(st[0]), bswap32(st[1]), bswap32(st[2]), bswap32(st[3]));
+  o[1] = make_uint4(bswap32(st[4]), bswap32(st[5]), bswap32(st[6]), bswap32(st[7]));
 }
 __global__ void merkle_level_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint64_t n_out) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_out) return;
   const uint32_t* l = tree + (in_off + 2 * i) * 8;
   uint32_t out[8];
-  sha256_words([&](uint32_t k) { return l[k]; }, 16, out);
+  sha256_words<true>([&](uint32_t k) { return l[k]; }, 16, out);
   uint64_t o = in_off + 2 * n_out + i;
 #pragma unroll
   for (int k = 0; k < 8; ++k) tree[o * 8 + k] = out[k];
@@ -375,7 +396,10 @@ void launch_merkle(const F128d* rows, uint32_t lanes, uint64_t n_leaves, uint32_
   // levels above the cap are never read (the cap is the commitment, paths stop below it)
   const uint64_t n_cap = uint64_t(1) << cap_depth;
   if (n_cap > n_leaves) throw std::runtime_error("Merkle cap wider than the leaf level");
-  merkle_leaves_kernel<<<(unsigned)((n_leaves + 127) / 128), 128, 0, s>>>(rows, lanes, n_leaves, (uint32_t*)tree);
+  // from about a thousand leaves an SM on, the compressions are bound by the logic pipe, below
+  // by their latency
+  auto* leaves = n_leaves >= (uint64_t)sm_count() * 1024 ? merkle_leaves_kernel<true> : merkle_leaves_kernel<false>;
+  leaves<<<(unsigned)((n_leaves + 127) / 128), 128, 0, s>>>(rows, lanes, n_leaves, (uint32_t*)tree);
   LAUNCH_OK();
   uint64_t off = 0, len = n_leaves;
   while (len > n_cap) {
