@@ -1269,14 +1269,29 @@ Msg256 GpuBackend::lg_introduce_induced(uint32_t ln, uint32_t log_rate, const st
   for (uint64_t p : pos)
     if (p >> log_d) throw std::runtime_error("induced basis: position outside the codeword");
   uint32_t nq = (uint32_t)w.size();
-  const uint64_t* dpos = static_cast<const uint64_t*>(upload(pos.data(), pos.size() * 8));
-  const F128d* dw = upload(w);
+  // queries that share a block of the sparse layers together (the weights' order does not matter)
+  const uint32_t sparse = lg_sparse_layers(log_d, log_rate);
+  std::vector<uint32_t> order(nq), start;
+  for (uint32_t q = 0; q < nq; ++q) order[q] = q;
+  if (sparse) std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return pos[a] < pos[b]; });
+  std::vector<uint64_t> sp;
+  std::vector<F128> sw;
+  for (uint32_t q = 0; q < nq; ++q) {
+    if (!q || (pos[order[q]] >> sparse) != (sp.back() >> sparse)) start.push_back(q);
+    sp.push_back(pos[order[q]]);
+    sw.push_back(w[order[q]]);
+  }
+  const uint32_t n_groups = (uint32_t)start.size();
+  start.push_back(nq);
+  const uint64_t* dpos = static_cast<const uint64_t*>(upload(sp.data(), sp.size() * 8));
+  const F128d* dw = upload(sw);
+  const uint32_t* dstart = static_cast<const uint32_t*>(upload(start.data(), start.size() * 4));
   F128d* y = static_cast<F128d*>(scratch(size_t(16) << log_d));
   const F128d* tw = twiddles(log_d);
   FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_LIGERITO);
-    launch_lg_induced(dpos, dw, nq, ln, log_rate, tw, lf_[lg_cur_], y, pend_, part_, st_, fp);
+    launch_lg_induced(dpos, dw, nq, dstart, n_groups, ln, log_rate, tw, lf_[lg_cur_], y, pend_, part_, st_, fp);
   }
   auto v = read_published(fp.seq, 2);
   pend_induced_ = true;

@@ -194,9 +194,12 @@ void launch_lg_replicate(const F256d* f, uint64_t msg, uint64_t total, F128d* ma
 uint32_t launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n,
                             F128d* pend, F128d* part, cudaStream_t s,
                             FusedPublish pub = FusedPublish());  // width 3
-uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, uint32_t ln, uint32_t log_rate,
-                           const F128d* tw, const F256d* f, F128d* y, F128d* basis, F128d* part,
-                           cudaStream_t s, FusedPublish pub = FusedPublish());  // width 2
+// pos and w in order of pos >> lg_sparse_layers(...), start[g] the first query of group g (one
+// value of that; start[n_groups] = n_q); without sparse layers start is not read.
+uint32_t lg_sparse_layers(uint32_t log_d, uint32_t log_rate);
+uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, const uint32_t* start, uint32_t n_groups,
+                           uint32_t ln, uint32_t log_rate, const F128d* tw, const F256d* f, F128d* y, F128d* basis,
+                           F128d* part, cudaStream_t s, FusedPublish pub);  // width 2
 void launch_lg_glue(F256d* b, const F128d* p, F128d beta, uint64_t n, bool induced, cudaStream_t s);
 
 // rounds.cu

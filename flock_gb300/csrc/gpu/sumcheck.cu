@@ -1334,21 +1334,24 @@ mo_build_w_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er0, co
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = u0; part[blockIdx.x * 2 + 1] = u2; }
 }
 // The same weight under identity compaction with tall columns (col = d >> nu): in column c
-// the map x -> fold_slot(x ec_i[c], table_i) is GF(2)-linear, so the block builds its byte
-// tables once per (column, part) work item and W[d] = M0_c(er0[row]) + M1_c(er1[row]) is
-// 32 table lookups and no multiply; only the message's products stay integer multiplies.
-// Work item = 2^(nu - part_log) consecutive rows of one column.
-__global__ void __launch_bounds__(768, 1)
+// the map x -> fold_slot(x ec_i[c], table_i) is GF(2)-linear, so the block builds its window
+// tables (wintable.cuh, five bits, 2 x 101 KB) once per (column, part) work item and W[d] =
+// M0_c(er0[row]) + M1_c(er1[row]) is 52 conflict-free lookups and no multiply; only the message's
+// products stay integer multiplies. Work item = 2^(nu - part_log) consecutive rows of one column.
+// Byte tables (32 lookups, 58 % of their wavefronts conflicts) took 3.60 ms of Keccak-f 2^18, this
+// form 3.27; SHA-256 2^16 0.76 -> 0.63.
+__global__ void __launch_bounds__(512, 1)
 mo_build_w_cols_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er0, const F128d* __restrict__ ec0,
                        const F128d* __restrict__ er1, const F128d* __restrict__ ec1, const F128d* __restrict__ tables,
                        uint32_t nu, uint32_t part_log, uint64_t area, uint64_t n, F128d* __restrict__ w,
                        F128d* __restrict__ part) {
-  extern __shared__ __align__(16) F128d ct[];  // column tables M0, M1, then M1's scratch
+  extern __shared__ __align__(16) char wt[];  // the maps M0, then M1
+  __shared__ F128d img[2][128];
   __shared__ F128d sh[32];
-  F128d* T0 = ct;
-  F128d* T1 = ct + BYTE_TABLE_ENTRIES;
+  constexpr uint32_t TAB = WinMap<5, 128>::BYTES;
+  const uint32_t lane = win_lane(), half = threadIdx.x >> 8;  // two halves of the block build the two tables
   const uint64_t items = (n >> nu) << part_log, rows = 1ull << (nu - part_log);
-  F128d u0 = f128_zero(), u2 = f128_zero();
+  MulAcc u0, u2;
   for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
     const uint64_t col = it >> part_log, d0 = (col << nu) + ((it & ((1ull << part_log) - 1)) << (nu - part_log));
     const bool used = d0 < area;  // block-uniform
@@ -1357,31 +1360,27 @@ mo_build_w_cols_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er
       continue;
     }
     __syncthreads();  // the previous item's tables are no longer read
-    {
-      // M0's images (its scratch lies inside M1's table), then M1's
-      if (threadIdx.x < 128) byte_table_images(T0)[threadIdx.x] = fold_slot(mul_call(ec0[col], unit_power(threadIdx.x)), tables);
-      __syncthreads();
-      byte_table_from_images(T0);
-      if (threadIdx.x < 128)
-        byte_table_images(T1)[threadIdx.x] = fold_slot(mul_call(ec1[col], unit_power(threadIdx.x)), tables + 16 * 256);
-      __syncthreads();
-      byte_table_from_images(T1);
+    if (threadIdx.x < 256) {
+      const uint32_t k = threadIdx.x >> 7, t = threadIdx.x & 127;
+      img[k][t] = fold_slot(mul_by_power(k ? ec1[col] : ec0[col], t), tables + k * 16 * 256);
     }
+    __syncthreads();
+    build_win_map<5, 128>(img[half], wt + half * TAB, (threadIdx.x & 255) >> 3, 32);
+    __syncthreads();
     for (uint64_t j = threadIdx.x; j < rows / 2; j += blockDim.x) {
       const uint64_t d = d0 + 2 * j, row = d & ((1ull << nu) - 1);
       F128d W0 = f128_zero(), W1 = f128_zero();
-      if (d < area) W0 = mul_table(er0[row], T0) + mul_table(er1[row], T1);
-      if (d + 1 < area) W1 = mul_table(er0[row + 1], T0) + mul_table(er1[row + 1], T1);
+      if (d < area) W0 = mul_win<5>(er0[row], wt, lane) + mul_win<5>(er1[row], wt + TAB, lane);
+      if (d + 1 < area) W1 = mul_win<5>(er0[row + 1], wt, lane) + mul_win<5>(er1[row + 1], wt + TAB, lane);
       w[d] = W0;
       w[d + 1] = W1;
       const F128d q0 = q[d], q1 = q[d + 1];
-      u0 += mul_call(q0, W0);
-      u2 += mul_call(q0 + q1, W0 + W1);
+      u0.add(q0, W0);
+      u2.add(q0 + q1, W0 + W1);
     }
   }
-  u0 = block_xor(u0, sh);
-  u2 = block_xor(u2, sh);
-  if (threadIdx.x == 0) { part[blockIdx.x * 2] = u0; part[blockIdx.x * 2 + 1] = u2; }
+  const F128d r0 = block_xor(u0.value(), sh), r2 = block_xor(u2.value(), sh);
+  if (threadIdx.x == 0) { part[blockIdx.x * 2] = r0; part[blockIdx.x * 2 + 1] = r2; }
 }
 // Columns of at least 2^MO_COLS_MIN_NU rows take the column-table form.
 constexpr uint32_t MO_COLS_MIN_NU = 14;
@@ -1394,9 +1393,9 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
     while (nu - part_log > 13 && ((n >> nu) << part_log) < (uint64_t)sm_count() * 8) ++part_log;
     const uint64_t items = (n >> nu) << part_log;
     const uint32_t blocks = (uint32_t)std::min<uint64_t>(items, (uint64_t)sm_count());
-    const int smem = (int)((BYTE_TABLE_ENTRIES + BYTE_TABLE_SMEM_ENTRIES) * sizeof(F128d));
+    const int smem = 2 * WinMap<5, 128>::BYTES;
     set_dynamic_smem((const void*)mo_build_w_cols_kernel, smem);
-    mo_build_w_cols_kernel<<<blocks, 768, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, part_log, area, n, w, part);
+    mo_build_w_cols_kernel<<<blocks, 512, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, part_log, area, n, w, part);
     LAUNCH_OK();
     return blocks;
   }
@@ -1879,23 +1878,85 @@ ntt_t_fused_kernel(F128d* __restrict__ y, uint32_t log_d, uint32_t layer_hi, uin
   }
   if (have && t < P) y[base + ((uint64_t)t << sh_min)] = g[sub][t];
 }
-uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, uint32_t ln, uint32_t log_rate,
-                           const F128d* tw, const F256d* f, F128d* y, F128d* basis, F128d* part, cudaStream_t s,
-                           FusedPublish pub) {
-  uint32_t log_d = ln + log_rate;
+// The first transposed layers of a large level act on a vector that is zero but for the queried
+// positions: within the 2^L positions of a query's block they leave
+//   w prod_{k in bits(i)} (t_k + bit_k(pos)),  t_k the twiddle of layer k at pos >> (k + 1),
+// at position i, so those layers are formed directly (two products an entry and query, sixteen
+// values per four layers in shared memory) for the blocks that hold queries, instead of L passes
+// over the whole vector (Ligerito of Keccak-f 2^18 9.2 -> 8.4 ms, 35 launches fewer). Block (group of queries with one block, ENTRIES entries of it).
+constexpr uint32_t SPARSE_ENTRIES = 1024, SPARSE_MAX_LAYERS = 12;
+__global__ void __launch_bounds__(256)
+ntt_t_sparse_kernel(const uint64_t* __restrict__ pos, const F128d* __restrict__ w, const uint32_t* __restrict__ start,
+                    uint32_t log_d, uint32_t L, const F128d* __restrict__ tw, F128d* __restrict__ y) {
+  __shared__ F128d fac[SPARSE_MAX_LAYERS];
+  __shared__ F128d sub[SPARSE_MAX_LAYERS / 4][16];
+  const uint32_t q0 = start[blockIdx.x], q1 = start[blockIdx.x + 1], n = 1u << L;
+  F128d acc[SPARSE_ENTRIES / 256];
+#pragma unroll
+  for (uint32_t e = 0; e < SPARSE_ENTRIES / 256; ++e) acc[e] = f128_zero();
+  for (uint32_t q = q0; q < q1; ++q) {
+    const uint64_t p = pos[q];
+    __syncthreads();  // the previous query's tables are no longer read
+    if (threadIdx.x < SPARSE_MAX_LAYERS) {
+      const uint32_t k = threadIdx.x;
+      F128d f = f128_one();
+      if (k < L) {
+        f = tw[(1ull << (log_d - 1 - k)) - 1 + (p >> (k + 1))];
+        f.lo ^= (p >> k) & 1;
+      }
+      fac[k] = f;
+    }
+    __syncthreads();
+    if (threadIdx.x < SPARSE_MAX_LAYERS * 4) {
+      const uint32_t g = threadIdx.x >> 4, v = threadIdx.x & 15;
+      F128d f[4];
+#pragma unroll
+      for (uint32_t b = 0; b < 4; ++b) f[b] = (v >> b) & 1 ? fac[4 * g + b] : f128_one();
+      F128d s = mul_call(mul_call(f[0], f[1]), mul_call(f[2], f[3]));
+      if (g == 0) s = mul_call(s, w[q]);
+      sub[g][v] = s;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t e = 0; e < SPARSE_ENTRIES / 256; ++e) {
+      const uint32_t i = blockIdx.y * SPARSE_ENTRIES + e * 256 + threadIdx.x;
+      acc[e] += mul_call(mul_call(sub[0][i & 15], sub[1][(i >> 4) & 15]), sub[2][(i >> 8) & 15]);
+    }
+  }
+  const uint64_t base = (pos[q0] >> L) << L;
+#pragma unroll
+  for (uint32_t e = 0; e < SPARSE_ENTRIES / 256; ++e) {
+    const uint32_t i = blockIdx.y * SPARSE_ENTRIES + e * 256 + threadIdx.x;
+    if (i < n) y[base + i] = acc[e];
+  }
+}
+// Layers formed that way: blocks of 2^(log_d - 9) positions, so that few of a level's queries (at
+// most 279) share one; levels of at most 2^NTT_T_FUSED_MAX_LOG positions run fused instead.
+uint32_t lg_sparse_layers(uint32_t log_d, uint32_t log_rate) {
+  return log_d > NTT_T_FUSED_MAX_LOG ? std::min({SPARSE_MAX_LAYERS, log_d - 9, log_d - log_rate}) : 0;
+}
+uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, const uint32_t* start, uint32_t n_groups,
+                           uint32_t ln, uint32_t log_rate, const F128d* tw, const F256d* f, F128d* y, F128d* basis,
+                           F128d* part, cudaStream_t s, FusedPublish pub) {
+  const uint32_t log_d = ln + log_rate, sparse = lg_sparse_layers(log_d, log_rate);
   CUDA_OK(cudaMemsetAsync(y, 0, (sizeof(F128d)) << log_d, s));
-  lg_scatter_kernel<<<(n_q + 127) / 128, 128, 0, s>>>(pos, w, n_q, y);
+  if (sparse) {
+    const uint32_t chunks = std::max(1u, (1u << sparse) / SPARSE_ENTRIES);
+    ntt_t_sparse_kernel<<<dim3(n_groups, chunks), 256, 0, s>>>(pos, w, start, log_d, sparse, tw, y);
+  } else {
+    lg_scatter_kernel<<<(n_q + 127) / 128, 128, 0, s>>>(pos, w, n_q, y);
+  }
   LAUNCH_OK();
   uint64_t pairs = 1ull << (log_d - 1);
-  // transposed layers from log_d - 1 down to log_rate: for the small levels (launch-latency
-  // bound) up to NTT_T_FUSED per launch; the large ones one per launch (their fused groups
-  // would be strided and half the threads idle in every layer: slower, measured)
+  // transposed layers from log_d - 1 - sparse down to log_rate: for the small levels
+  // (launch-latency bound) up to NTT_T_FUSED per launch; the large ones one per launch (their
+  // fused groups would be strided and half the threads idle in every layer: slower, measured)
   const uint32_t per_launch = log_d <= NTT_T_FUSED_MAX_LOG ? NTT_T_FUSED : 1;
-  for (int layer = (int)log_d - 1; layer >= (int)log_rate;) {
+  for (int layer = (int)(log_d - 1 - sparse); layer >= (int)log_rate;) {
     const uint32_t nl = std::min<uint32_t>(per_launch, (uint32_t)(layer - (int)log_rate + 1));
     if (nl >= 2) {
-      const uint64_t n_groups = 1ull << (log_d - nl);
-      ntt_t_fused_kernel<<<(unsigned)((n_groups + 3) / 4), 256, 0, s>>>(y, log_d, (uint32_t)layer, nl, tw);
+      const uint64_t n_groups_t = 1ull << (log_d - nl);
+      ntt_t_fused_kernel<<<(unsigned)((n_groups_t + 3) / 4), 256, 0, s>>>(y, log_d, (uint32_t)layer, nl, tw);
     } else {
       ntt_t_layer_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(y, log_d, (uint32_t)layer, tw);
     }
