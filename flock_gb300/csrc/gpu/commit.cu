@@ -146,14 +146,13 @@ ntt_layer2_win_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, 
 }
 // Two layers run as a table pass while the first one's twiddle blocks hold at least this many
 // units (lanes 2^(sh-1)): from WIN units on with window tables, from TBL on with a byte table.
-// Against the fused pass (two of its layers): 42 lanes, 1344 units 2.59 against 4.24 ms; 50
-// lanes, 800 units 0.436 against 0.61, but then four layers are left for it instead of six,
-// which cost more each (1.38 for four, 1.84 for six): below TBL a pass is only taken while more
-// than six layers are left, down to MORE units (13 lanes, 416 units: 0.074 ms against about
-// 0.09). Each launch block gets at least NTT_TBL_MIN_BLOCK_BUTTERFLIES of a twiddle block's
+// Against fused passes down to the last layer: 42 lanes, 336 units 3.73 + 5.64 ms (three fused
+// layers left) against 8.68 (five); 50 lanes, 800 units 0.436 + 1.08 (four left) against 1.62
+// (six). Below TBL a pass is only taken while more than six layers are left, down to MORE units
+// (13 lanes, 416 units: 0.074 + 0.203 against 0.38 ms for fused passes of four and three). Each launch block gets at least NTT_TBL_MIN_BLOCK_BUTTERFLIES of a twiddle block's
 // butterflies, and the transform has to give every SM two such blocks.
 constexpr uint64_t NTT_WIN_MIN_UNITS = 8192;
-constexpr uint64_t NTT_TBL_MIN_UNITS = 1024;
+constexpr uint64_t NTT_TBL_MIN_UNITS = 768;
 constexpr uint64_t NTT_TBL_MORE_UNITS = 256;
 constexpr uint64_t NTT_TBL_MIN_BLOCK_BUTTERFLIES = uint64_t(1) << 12;
 
@@ -162,8 +161,15 @@ constexpr uint64_t NTT_TBL_MIN_BLOCK_BUTTERFLIES = uint64_t(1) << 12;
 // block of the first fused layer) for a slice of lanes; each fused layer pairs positions
 // within that set. Fused layer k meets 2^k twiddles; the block stages all 2^nl - 1 of them
 // once, already split for mul_split, after the positions' data.
+// BOTTOM >= 1 (the pass ends with the transform's last layer): with the basis x^i the twiddle of
+// layer log_d - 1 - i is the i-th Carlitz polynomial of a polynomial a of degree below log_d, an
+// integral one of degree (deg a - i) 2^i: below 32 for the last layer and below 64 for the one
+// before (any log_d to 32), and for the third from last where log_d <= 18 (BOTTOM = 2), so their
+// products take four and six of the nine partial ones. Five layers of 42 lanes and 2^22 positions:
+// 10.6 ms with nine for all, 8.7 so.
+constexpr uint32_t NTT_BOTTOM3_MAX_LOG = 18;
 constexpr uint32_t NTT_MAX_THREADS = 320;  // with 3 blocks per SM: at most 64 registers a thread
-template <int NL>
+template <int NL, int BOTTOM>
 __global__ void __launch_bounds__(NTT_MAX_THREADS, 3)
 ntt_fused_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, uint32_t layer, const F128d* __restrict__ tw,
                  uint32_t lane_tile) {
@@ -194,45 +200,51 @@ ntt_fused_kernel(F128d* __restrict__ data, uint32_t lanes, uint32_t log_d, uint3
       split_classes(y0 ^ y1, tws[t].w[3 * q + 2]);
     }
   }
-  for (uint32_t i = threadIdx.x; i < P * nl_here; i += blockDim.x) {
-    uint32_t pos = i / nl_here, l = i - pos * nl_here;
-    sm[pos * lane_tile + l] = data[(base + ((uint64_t)pos << stride_log)) * lanes + l0 + l];
-  }
-  __syncthreads();
-  // (pair, lane) of this thread's first butterfly and the step between its butterflies
+  // (pair, lane) of this thread's first element or butterfly and the step between them
   const uint32_t pr0 = threadIdx.x / nl_here, ln0 = threadIdx.x - pr0 * nl_here;
   const uint32_t dpr = blockDim.x / nl_here, dln = blockDim.x - dpr * nl_here;
+  auto step = [&](uint32_t& pr, uint32_t& l) {
+    pr += dpr;
+    l += dln;
+    if (l >= nl_here) {
+      l -= nl_here;
+      ++pr;
+    }
+  };
+  F128d* g = data + base * lanes + l0;
+  const uint64_t g_stride = (uint64_t)lanes << stride_log;
+  __syncthreads();
 #pragma unroll
-  for (int k = 0; k < NL; ++k) {
+  for (int k = 0; k < NL; ++k) {  // the first layer reads global memory, the last one writes it
     const uint32_t half = P >> (k + 1);  // pairing distance inside the group (in group positions)
     uint32_t pr = pr0, l = ln0;
     for (uint32_t i = threadIdx.x; i < (P / 2) * nl_here; i += blockDim.x) {
       uint32_t blk = pr / half, w = pr - blk * half;
       uint32_t i0 = blk * 2 * half + w, i1 = i0 + half;
-      F128d u = sm[i0 * lane_tile + l], v = sm[i1 * lane_tile + l];
+      F128d* pu = k == 0 ? g + i0 * g_stride + l : sm + i0 * lane_tile + l;
+      F128d* pv = k == 0 ? g + i1 * g_stride + l : sm + i1 * lane_tile + l;
+      F128d u = *pu, v = *pv;
       // the first block's twiddle is zero in every layer
-      F128d nu = (outer == 0 && blk == 0) ? u : u + mul_split(v, tws[(1u << k) - 1 + blk]);
-      sm[i0 * lane_tile + l] = nu;
-      sm[i1 * lane_tile + l] = v + nu;
-      pr += dpr;
-      l += dln;
-      if (l >= nl_here) {
-        l -= nl_here;
-        ++pr;
-      }
+      const F128split& t = tws[(1u << k) - 1 + blk];
+      F128d nu = u;
+      if (outer != 0 || blk != 0)
+        nu += BOTTOM >= 1 && k == NL - 1 ? mul_split_deg32(v, t)
+              : (BOTTOM >= 1 && k == NL - 2) || (BOTTOM >= 2 && k == NL - 3) ? mul_split_deg64(v, t)
+                                                                             : mul_split(v, t);
+      pu = k == NL - 1 ? g + i0 * g_stride + l : sm + i0 * lane_tile + l;
+      pv = k == NL - 1 ? g + i1 * g_stride + l : sm + i1 * lane_tile + l;
+      *pu = nu;
+      *pv = v + nu;
+      step(pr, l);
     }
-    __syncthreads();
-  }
-  for (uint32_t i = threadIdx.x; i < P * nl_here; i += blockDim.x) {
-    uint32_t pos = i / nl_here, l = i - pos * nl_here;
-    data[(base + ((uint64_t)pos << stride_log)) * lanes + l0 + l] = sm[pos * lane_tile + l];
+    if (k < NL - 1) __syncthreads();
   }
 }
 
 // Threads per fused-NTT block for a lane tile: among the multiples of 32 in [192, 320], the
 // one with the most busy resident warps per SM (resident warps, capped at 32, times the
 // fraction of threads with a butterfly in a layer's passes). Cached per device and tile.
-template <int NL>
+template <int NL, int BOTTOM>
 static uint32_t ntt_block_threads(uint32_t lane_tile, size_t smem) {
   static std::atomic<uint32_t> cache[MAX_DEVICES][65];
   int dev = 0;
@@ -244,7 +256,7 @@ static uint32_t ntt_block_threads(uint32_t lane_tile, size_t smem) {
   double best_score = -1.0;
   for (uint32_t t = 192; t <= NTT_MAX_THREADS; t += 32) {
     int blocks = 0;
-    CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ntt_fused_kernel<NL>, (int)t, smem));
+    CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, ntt_fused_kernel<NL, BOTTOM>, (int)t, smem));
     const uint32_t passes = (butterflies + t - 1) / t;
     const double score = std::min(blocks * t / 32.0, 32.0) * butterflies / (double)(passes * t);
     if (score > best_score + 1e-9) {
@@ -256,17 +268,25 @@ static uint32_t ntt_block_threads(uint32_t lane_tile, size_t smem) {
   return best;
 }
 
-template <int NL>
-static void launch_ntt_fused(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t layer, const F128d* tw,
+template <int NL, int BOTTOM>
+static void launch_ntt_fused_pass(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t layer, const F128d* tw,
                              cudaStream_t s) {
   const uint32_t lane_tile = lanes < 64 ? lanes : 64;
   const size_t tw_bytes = ((1u << NL) - 1) * sizeof(F128split);
   const uint64_t n_groups = 1ull << (log_d - NL), lane_tiles = (lanes + lane_tile - 1) / lane_tile;
   const size_t smem = (size_t)(1u << NL) * lane_tile * sizeof(F128d) + tw_bytes;
-  set_dynamic_smem((const void*)ntt_fused_kernel<NL>, (int)((1u << NL) * 64 * sizeof(F128d) + tw_bytes));
-  const uint32_t threads = ntt_block_threads<NL>(lane_tile, smem);
-  ntt_fused_kernel<NL><<<(unsigned)(n_groups * lane_tiles), threads, smem, s>>>(data, lanes, log_d, layer, tw, lane_tile);
+  set_dynamic_smem((const void*)ntt_fused_kernel<NL, BOTTOM>, (int)((1u << NL) * 64 * sizeof(F128d) + tw_bytes));
+  const uint32_t threads = ntt_block_threads<NL, BOTTOM>(lane_tile, smem);
+  ntt_fused_kernel<NL, BOTTOM><<<(unsigned)(n_groups * lane_tiles), threads, smem, s>>>(data, lanes, log_d, layer, tw, lane_tile);
   LAUNCH_OK();
+}
+
+template <int NL>
+static void launch_ntt_fused(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t layer, const F128d* tw,
+                             cudaStream_t s) {
+  if (layer + NL < log_d) launch_ntt_fused_pass<NL, 0>(data, lanes, log_d, layer, tw, s);
+  else if (log_d > NTT_BOTTOM3_MAX_LOG) launch_ntt_fused_pass<NL, 1>(data, lanes, log_d, layer, tw, s);
+  else launch_ntt_fused_pass<NL, 2>(data, lanes, log_d, layer, tw, s);
 }
 
 void launch_ntt(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t start_layer, const F128d* tw, cudaStream_t s) {

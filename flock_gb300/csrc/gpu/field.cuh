@@ -176,6 +176,22 @@ __device__ __forceinline__ F128d mul_split(F128d a, const F128split& b) {
   return ghash_reduce(l0, l1 ^ m0, h0 ^ m1, h1);
 }
 
+// a * b for b of degree below 32 and below 64: four and six 32 x 32 carry-less products instead of
+// nine, and a shorter reduction.
+__device__ __forceinline__ F128d mul_split_deg32(F128d a, const F128split& b) {
+  const uint64_t c0 = clmul32_split((uint32_t)a.lo, b.w[0]), c1 = clmul32_split((uint32_t)(a.lo >> 32), b.w[0]);
+  const uint64_t c2 = clmul32_split((uint32_t)a.hi, b.w[0]), c3 = clmul32_split((uint32_t)(a.hi >> 32), b.w[0]);
+  const uint64_t t = c3 >> 32;  // of x^128, below x^31
+  return f128(c0 ^ (c1 << 32) ^ t ^ (t << 1) ^ (t << 2) ^ (t << 7), (c1 >> 32) ^ c2 ^ (c3 << 32));
+}
+__device__ __forceinline__ F128d mul_split_deg64(F128d a, const F128split& b) {
+  uint64_t l0, l1, h0, h1;
+  clmul64_split(a.lo, b.w, l0, l1);
+  clmul64_split(a.hi, b.w, h0, h1);  // h1: of x^128, below x^63
+  const uint64_t ov = (h1 >> 62) ^ (h1 >> 57);  // h1 << 2 and h1 << 7 past x^64
+  return f128(l0 ^ h1 ^ (h1 << 1) ^ (h1 << 2) ^ (h1 << 7), l1 ^ h0 ^ ov);
+}
+
 // Out-of-line mul_split (see mul_call); b is typically staged once per block in shared
 // memory.
 __device__ __noinline__ static F128d mul_split_call(F128d a, const F128split* b) { return mul_split(a, *b); }
