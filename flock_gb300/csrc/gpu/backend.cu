@@ -127,7 +127,7 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   const uint64_t D = uint64_t(1) << S.log_dim;
   b += lane_fold_groups(S.lanes, D) * D * 32;  // Ligerito: lane fold partials,
   b += 4 * 2 * D * 32 + 2 * D * 16;            // f/b ping-pong, pending
-  b += (uint64_t(1) << 20) * 16 + 4096 * 16 + (size_t(96) << 20) + (size_t(8) << 20);  // partials, scratch, staging
+  b += (uint64_t(1) << 20) * 16 + (size_t(96) << 20) + (size_t(8) << 20);  // partials, scratch, staging
   b += n_pos * 16;                          // L0 twiddles
   // recursive levels: codeword 2^(log_cols + rate) x 2^k, tree, twiddles
   const LigeritoParams& P = S.lig;
@@ -170,7 +170,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   zc1b_ = dmalloc<F128d>(W / 2, owned_, device_bytes_);
   zc2a_ = dmalloc<F128d>(W, owned_, device_bytes_);
   zc2b_ = dmalloc<F128d>(W, owned_, device_bytes_);
-  zc_w64_ = dmalloc<F128d>(64, owned_, device_bytes_);
+  zc_w64_ = dmalloc<F128d>(64 + 64 + 2 * 64, owned_, device_bytes_);  // weights, point, table list
   comb_ = dmalloc<F128d>(K_, owned_, device_bytes_);
   zv_ = dmalloc<F128d>(K_, owned_, device_bytes_);
   zvcap_ = dmalloc<F128d>(K_, owned_, device_bytes_);
@@ -214,15 +214,19 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   CUDA_OK(cudaHostGetDevicePointer(&d_tail_, h_tail_, 0));
   part_cap_ = 1u << 20;
   part_ = dmalloc<F128d>(part_cap_, owned_, device_bytes_);
-  red_ = dmalloc<F128d>(4096, owned_, device_bytes_);
-  CUDA_OK(cudaMallocHost(&h_red_, 4096 * sizeof(F128d)));
   scr_cap_ = size_t(96) << 20;
   scr_ = dmalloc<uint8_t>(scr_cap_, owned_, device_bytes_);
   stage_cap_ = size_t(8) << 20;
   d_stage_ = dmalloc<uint8_t>(stage_cap_, owned_, device_bytes_);
   CUDA_OK(cudaMallocHost(&h_stage_, stage_cap_));
-  CUDA_OK(cudaHostAlloc(&h_pub_, 64 * sizeof(F128d), cudaHostAllocMapped));
+  CUDA_OK(cudaHostAlloc(&h_pub_, PUB_WORDS * sizeof(F128d), cudaHostAllocMapped));
   CUDA_OK(cudaHostGetDevicePointer(&d_pub_, h_pub_, 0));
+  size_t open_bytes = 0;  // the largest opening: rows and whole paths of a level's queries
+  for (uint32_t l = 0; l <= S.lig.r; ++l) {
+    const size_t row = l ? size_t(16) << S.lig.recursive_ks[l - 1] : size_t(16) * S.lanes;
+    open_bytes = std::max(open_bytes, S.lig.queries[l] * (row + 32 * 40));
+  }
+  d_open(open_bytes);
   CUDA_OK(cudaHostAlloc(&h_flag_, 64, cudaHostAllocMapped));
   CUDA_OK(cudaHostGetDevicePointer(&d_flag_, h_flag_, 0));
   *(volatile uint32_t*)h_flag_ = 0;
@@ -254,7 +258,7 @@ GpuBackend::~GpuBackend() {
   for (auto& L : levels_) { cudaFree(L.mat); cudaFree(L.tree); }
   for (cudaEvent_t e : ev_pool_) cudaEventDestroy(e);
   cudaFreeHost(h_in_);
-  cudaFreeHost(h_red_);
+  cudaFreeHost(h_open_);
   cudaFreeHost(h_stage_);
   cudaFreeHost(h_pow_);
   cudaFreeHost(h_pow_flag_);
@@ -376,6 +380,17 @@ const void* GpuBackend::upload(const void* src, size_t bytes) {
   stage_off_ = off + bytes;
   return d_stage_ + off;
 }
+void GpuBackend::upload_to(void* dst, const void* src, size_t bytes) {
+  size_t off = (stage_off_ + 255) & ~size_t(255);
+  if (off + bytes > stage_cap_) {
+    sync();
+    off = 0;
+  }
+  memcpy(h_stage_ + off, src, bytes);
+  CUDA_OK(cudaMemcpyAsync(dst, h_stage_ + off, bytes, cudaMemcpyHostToDevice, st_));
+  h2d_ += bytes;
+  stage_off_ = off + bytes;
+}
 const F128d* GpuBackend::upload(const std::vector<F128>& v) {
   return static_cast<const F128d*>(upload(v.data(), v.size() * sizeof(F128)));
 }
@@ -384,12 +399,8 @@ void GpuBackend::sync() {
   stage_off_ = 0;
 }
 std::vector<F128> GpuBackend::reduce(uint32_t n_blocks, uint32_t width) {
-  if ((uint64_t)n_blocks * width > part_cap_) throw std::runtime_error("partials buffer too small");
-  if (width > 64) {
-    launch_reduce_parts(part_, n_blocks, width, red_, st_);
-    return fetch(red_, width);
-  }
-  // round messages: one block reduces and publishes into mapped host memory
+  if ((uint64_t)n_blocks * width > part_cap_ || width > PUB_WORDS) throw std::runtime_error("partials buffer too small");
+  // one block reduces and publishes into mapped host memory
   uint32_t seq = ++seq_;
   launch_reduce_publish(part_, n_blocks, width, d_pub_, d_flag_, seq, st_);
   return read_published(seq, width);
@@ -424,18 +435,6 @@ void GpuBackend::wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stre
   }
   std::atomic_thread_fence(std::memory_order_acquire);
 }
-std::vector<F128> GpuBackend::fetch(const F128d* d, size_t n) {
-  std::vector<F128> out(n);
-  F128d* h = h_red_;
-  bool big = n > 4096;
-  if (big) h = reinterpret_cast<F128d*>(out.data());
-  CUDA_OK(cudaMemcpyAsync(h, d, n * sizeof(F128d), cudaMemcpyDeviceToHost, st_));
-  d2h_ += n * sizeof(F128d);
-  sync();
-  if (!big) memcpy(out.data(), h, n * sizeof(F128d));
-  return out;
-}
-
 // eq(point) split as lo (first lo_bits coordinates) x hi (rest, times scale).
 GpuBackend::EqSplit GpuBackend::eq_split(const std::vector<F128>& point, F128 scale, uint32_t max_lo) {
   EqSplit e;
@@ -443,18 +442,6 @@ GpuBackend::EqSplit GpuBackend::eq_split(const std::vector<F128>& point, F128 sc
   e.lo_bits = std::min(n, max_lo);
   uint32_t hi_bits = n - e.lo_bits;
   const F128d* dp = upload(point);
-  F128d* lo = static_cast<F128d*>(scratch((size_t(16)) << e.lo_bits));
-  F128d* hi = static_cast<F128d*>(scratch((size_t(16)) << hi_bits));
-  launch_eq_split(dp, e.lo_bits, hi_bits, dev(scale), lo, hi, st_);
-  e.lo = lo;
-  e.hi = hi;
-  return e;
-}
-
-GpuBackend::EqSplit GpuBackend::eq_split_dev(const F128d* dp, uint32_t n, F128 scale, uint32_t max_lo) {
-  EqSplit e;
-  e.lo_bits = std::min(n, max_lo);
-  uint32_t hi_bits = n - e.lo_bits;
   F128d* lo = static_cast<F128d*>(scratch((size_t(16)) << e.lo_bits));
   F128d* hi = static_cast<F128d*>(scratch((size_t(16)) << hi_bits));
   launch_eq_split(dp, e.lo_bits, hi_bits, dev(scale), lo, hi, st_);
@@ -533,17 +520,35 @@ void GpuBackend::commit_l0(uint32_t cap_depth, std::vector<Hash>& cap) {
   }
   { Mark mk(this, ST_L0_FILL); launch_fill_lane_major(q_, cw0_, S.lanes, S.log_dim, S.k_code, st_); }
   { Mark mk(this, ST_L0_NTT); launch_ntt(cw0_, S.lanes, S.k_code, 1, tw0_, st_); }
-  { Mark mk(this, ST_L0_MERKLE); launch_merkle(cw0_, S.lanes, n_pos0_, cap_depth, tree0_, st_); }
-  cap = read_cap(tree0_, n_pos0_, cap_depth);
+  const FusedPublish fp = fused_publish();
+  {
+    Mark mk(this, ST_L0_MERKLE);
+    launch_merkle(cw0_, S.lanes, n_pos0_, cap_depth, tree0_, st_, d_open(size_t(32) << cap_depth), fp);
+  }
+  cap = read_cap(cap_depth, fp);
 }
 
-std::vector<Hash> GpuBackend::read_cap(const uint8_t* tree, uint64_t n_leaves, uint32_t cap_depth) {
-  uint64_t l = uint64_t(1) << cap_depth;
-  std::vector<Hash> cap(l);
-  CUDA_OK(cudaMemcpyAsync(cap.data(), tree + (2 * n_leaves - 2 * l) * 32, l * 32, cudaMemcpyDeviceToHost, st_));
-  d2h_ += l * 32;
-  sync();
+std::vector<Hash> GpuBackend::read_cap(uint32_t cap_depth, const FusedPublish& fp) {
+  wait_published(fp.seq);
+  std::vector<Hash> cap(size_t(1) << cap_depth);
+  memcpy(cap.data(), h_open_, cap.size() * 32);
+  d2h_ += cap.size() * 32;
   return cap;
+}
+// Mapped memory of at least `bytes` for a cap or an opening.
+uint8_t* GpuBackend::d_open(size_t bytes) {
+  if (bytes > open_cap_) {
+    if (h_open_) {
+      sync();
+      cudaFreeHost(h_open_);
+      h_open_ = nullptr;
+      open_cap_ = 0;
+    }
+    CUDA_OK(cudaHostAlloc(&h_open_, bytes, cudaHostAllocMapped));
+    CUDA_OK(cudaHostGetDevicePointer(&d_open_, h_open_, 0));
+    open_cap_ = bytes;
+  }
+  return d_open_;
 }
 
 // ------------------------------------------------------------------ tails on the host
@@ -596,9 +601,9 @@ void GpuBackend::zc_round1(const std::vector<F128>& r, std::vector<F128>& ab, st
   }
   if ((uint64_t)nab * 64 > part_cap_ / 2 || (uint64_t)nsvc * 128 > part_cap_ / 2)
     throw std::runtime_error("round-1 partials exceed the partials buffer");
-  launch_reduce_parts(part_, nab, 64, red_, st_);
-  launch_reduce_parts(part_svc, nsvc, 128, red_ + 64, st_);
-  auto v = fetch(red_, 192);
+  const FusedPublish fp = fused_publish();
+  launch_reduce_pair(part_, nab, 64, part_svc, nsvc, 128, st_, fp);
+  auto v = read_published(fp.seq, 192);
   // D = prod (1 + g_i)^-1 over the medium constants' g_i = x^1, x^2, x^4, x^8
   static const F128 D = [] {
     F128 d = F128::one();
@@ -637,8 +642,6 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   scr_off_ = 0;
   const uint32_t L = (uint32_t)eq_point.size();  // m - 7
   if (L < 10) throw std::runtime_error("zerocheck skip fold needs m >= 17");
-  const F128d* dw = upload(w);
-  const F128d* dp = upload(eq_point);
   // the weighted form divides by the high coordinates' eq once: none may be 0 or 1
   zc_w_ = zc_weighted_lo_bits(zc_live_words_);
   for (uint32_t j = zc_w_; zc_w_ && j < L; ++j)
@@ -657,16 +660,23 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   }
   zc_inv_ = zc_tabs_ + total;
   if (total + (zc_w_ ? uint64_t(1) << (L - zc_w_) : 0) > zc_tabs_cap_) throw std::runtime_error("zerocheck eq tables: size mismatch");
-  const EqDesc* ddesc = static_cast<const EqDesc*>(upload(zc_desc_.data(), zc_desc_.size() * sizeof(EqDesc)));
-  uint32_t nb;
+  // the weights, the point and the table list in one copy, to a place of their own (the first
+  // fold reads the weights again)
+  std::vector<uint8_t> args(64 * sizeof(F128) + L * sizeof(F128) + zc_desc_.size() * sizeof(EqDesc));
+  memcpy(args.data(), w.data(), 64 * sizeof(F128));
+  memcpy(args.data() + 64 * sizeof(F128), eq_point.data(), L * sizeof(F128));
+  memcpy(args.data() + (64 + L) * sizeof(F128), zc_desc_.data(), zc_desc_.size() * sizeof(EqDesc));
+  upload_to(zc_w64_, args.data(), args.size());
+  const F128d *dw = zc_w64_, *dp = zc_w64_ + 64;
+  const EqDesc* ddesc = reinterpret_cast<const EqDesc*>(zc_w64_ + 64 + L);
+  const FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_ZC_FOLD_SKIP);
     launch_eq_tables(dp, ddesc, zc_desc_.data(), (uint32_t)zc_desc_.size(), zc_tabs_, st_);
     // words from zc_live_words_ on are zero and add nothing to the message
     const F128d* hi = zc_tabs_ + zc_desc_[1].out_off;
-    nb = zc_w_ ? launch_zc_fold_skip_weighted(a_, b_, dw, zc_live_words_, zc_w_, zc_tabs_, hi, part_, st_)
-               : launch_zc_fold_skip(a_, b_, dw, zc_live_words_, zc_tabs_, 10, hi, part_, st_);
-    CUDA_OK(cudaMemcpyAsync(zc_w64_, dw, 64 * sizeof(F128d), cudaMemcpyDeviceToDevice, st_));
+    if (zc_w_) launch_zc_fold_skip_weighted(a_, b_, dw, zc_live_words_, zc_w_, zc_tabs_, hi, part_, st_, fp);
+    else launch_zc_fold_skip(a_, b_, dw, zc_live_words_, zc_tabs_, 10, hi, part_, st_, fp);
   }
   if (zc_w_) {
     // reciprocals of 1 + r_j and r_j (one inversion of their product), then of the weights h;
@@ -687,7 +697,7 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
     }
     launch_factor_table(upload(f), L - zc_w_, zc_inv_, st_);
   }
-  auto v = reduce(nb, 2);
+  auto v = read_published(fp.seq, 2);
   g1 = v[0];
   gi = v[1];
   zc_tail_ = TailPair();
@@ -724,28 +734,25 @@ void GpuBackend::zc_fold(F128 rho, const std::vector<F128>& eq_point, F128& g1, 
     oa = d_tail_;
     ob = d_tail_ + TAIL;
   }
-  uint32_t nb, pub_seq = 0;
+  const FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_ZC_FOLDS);
     const F128d* elo = zc_tabs_ + lo.out_off;
     const bool weighted = zc_round_ < zc_w_;  // the low coordinates of the weighted form
     const F128d* ehi = weighted ? nullptr : zc_tabs_ + hi.out_off;
     if (zc_round_ == 0 && weighted) {
-      nb = launch_zc_fold2_weighted(a_, b_, zc_w64_, dev(rho), n_pairs, live_pairs, zc_w_, elo,
-                                    zc_tabs_ + zc_desc_[1].out_off, oa, ob, part_, st_);
+      launch_zc_fold2_weighted(a_, b_, zc_w64_, dev(rho), n_pairs, live_pairs, zc_w_, elo, zc_tabs_ + zc_desc_[1].out_off,
+                               oa, ob, part_, st_, fp);
     } else if (zc_round_ == 0) {
       F128d* tabs = static_cast<F128d*>(scratch(4096 * sizeof(F128d)));
-      nb = launch_zc_fold2(a_, b_, zc_w64_, dev(rho), tabs, n_pairs, live_pairs, elo, lo.n, ehi, oa, ob, part_, st_);
+      launch_zc_fold2(a_, b_, zc_w64_, dev(rho), tabs, n_pairs, live_pairs, elo, lo.n, ehi, oa, ob, part_, st_, fp);
     } else {
-      FusedPublish fp = fused_publish();
       // the first fold past the weighted rounds divides by h
       launch_pair_fold(zc_cur_a_, zc_cur_b_, n_pairs, live_pairs, dev(rho), elo, lo.n, ehi,
                        zc_w_ && zc_round_ == zc_w_ ? zc_inv_ : nullptr, oa, ob, part_, st_, fp);
-      nb = 0;
-      pub_seq = fp.seq;
     }
   }
-  auto v = pub_seq ? read_published(pub_seq, 2) : reduce(nb, 2);
+  auto v = read_published(fp.seq, 2);
   g1 = v[0];
   gi = v[1];
   if (tail) zc_tail_ = read_tail(TAIL);
@@ -766,14 +773,16 @@ void GpuBackend::zc_final(F128 rho, F128& ae, F128& be) {
 // ------------------------------------------------------------------ lincheck
 void GpuBackend::lc_comb(const std::vector<F128>& skip_w, const std::vector<F128>& xir) {
   scr_off_ = 0;
-  const F128d* dw = upload(skip_w);
   for (size_t t = 0; t < S.slots.size(); ++t) {
     // slot t folds its own matrices by skip_w (x) eq(xir[.. k_log_t - 6])
     const SlotInfo& T = S.slots[t];
     const SlotDev& sd = slot_dev_[t];
-    const F128d* der = upload(build_eq(std::vector<F128>(xir.begin(), xir.begin() + (T.k_log - 6))));
+    std::vector<F128> args(skip_w);  // 64 weights, then the eq table
+    const std::vector<F128> er = build_eq(std::vector<F128>(xir.begin(), xir.begin() + (T.k_log - 6)));
+    args.insert(args.end(), er.begin(), er.end());
+    const F128d* dw = upload(args);
     Mark mk(this, ST_LINCHECK);
-    launch_lc_eq_inner(dw, der, sd.K, eqi_, st_);
+    launch_lc_eq_inner(dw, dw + 64, sd.K, eqi_, st_);
     lc_fold_slot(T.hash, sd);
   }
 }
@@ -804,27 +813,25 @@ void GpuBackend::lc_zvec(const std::vector<F128>& x_outer) {
   // a single slot folds its used columns only; a union folds every union column (the
   // gaps and unused columns of z are zero)
   uint32_t used = S.slots.size() == 1 ? (uint32_t)S.slots[0].used_cols : K_ / 128;
-  if ((uint64_t)used * 128 < K_) CUDA_OK(cudaMemsetAsync(zv_ + used * 128, 0, (K_ - used * 128) * 16, st_));
-  launch_lc_zvec(z_, nu, used, e.lo, e.lo_bits, e.hi, part_, part_cap_, zv_, st_);
-  CUDA_OK(cudaMemcpyAsync(zvcap_, zv_, K_ * 16, cudaMemcpyDeviceToDevice, st_));
+  launch_lc_zvec(z_, nu, used, e.lo, e.lo_bits, e.hi, part_, part_cap_, K_, zv_, zvcap_, st_);
   lc_len_ = K_;
   lc_tail_ = TailPair();
 }
 
 void GpuBackend::lc_start(F128 alpha, const std::vector<SlotComb>& sc, F128& e1, F128& ei) {
-  uint32_t nb;
+  const FusedPublish fp = fused_publish();
   if (S.slots.size() == 1 && sc[0].offset == 0 && sc[0].weight == F128::one()) {
     Mark mk(this, ST_LINCHECK);
-    nb = launch_lc_start(ca_, cb_, dev(alpha), dev(sc[0].beta), sc[0].pin, K_, comb_, zv_, part_, st_);
+    launch_lc_start(ca_, cb_, dev(alpha), dev(sc[0].beta), sc[0].pin, K_, comb_, zv_, part_, st_, fp);
   } else {
     Mark mk(this, ST_LINCHECK);
     CUDA_OK(cudaMemsetAsync(comb_, 0, size_t(K_) * 16, st_));
     for (size_t t = 0; t < S.slots.size(); ++t)
       launch_lc_slot_comb(slot_dev_[t].ca, slot_dev_[t].cb, dev(alpha), dev(sc[t].weight), dev(sc[t].beta), sc[t].pin,
                           slot_dev_[t].K, comb_ + sc[t].offset, st_);
-    nb = launch_lc_top_message(comb_, zv_, K_, part_, st_);
+    launch_lc_top_message(comb_, zv_, K_, part_, st_, fp);
   }
-  auto v = reduce(nb, 2);
+  auto v = read_published(fp.seq, 2);
   e1 = v[0];
   ei = v[1];
 }
@@ -869,14 +876,17 @@ void GpuBackend::lc_matrix_evals(const std::vector<F128>& rest, const std::vecto
   for (size_t t = 0; t < S.slots.size(); ++t) {
     scr_off_ = 0;
     const SlotInfo& T = S.slots[t];
-    const F128d* der = upload(build_eq(std::vector<F128>(rest.begin(), rest.begin() + (T.k_log - 6))));
-    const F128d* dzp = upload(zp);
-    uint32_t nb;
+    std::vector<F128> args(zp);  // 64 partial values, then the eq table
+    const std::vector<F128> er = build_eq(std::vector<F128>(rest.begin(), rest.begin() + (T.k_log - 6)));
+    args.insert(args.end(), er.begin(), er.end());
+    const F128d* dzp = upload(args);
+    const F128d* der = dzp + 64;
+    const FusedPublish fp = fused_publish();
     {
       Mark mk(this, ST_LINCHECK);
-      nb = launch_lc_matrix_evals(slot_dev_[t].ca, slot_dev_[t].cb, der, dzp, slot_dev_[t].K, part_, st_);
+      launch_lc_matrix_evals(slot_dev_[t].ca, slot_dev_[t].cb, der, dzp, slot_dev_[t].K, part_, st_, fp);
     }
-    auto v = reduce(nb, 2);
+    auto v = read_published(fp.seq, 2);
     evals.push_back({v[0], v[1]});
   }
 }
@@ -884,42 +894,49 @@ void GpuBackend::lc_matrix_evals(const std::vector<F128>& rest, const std::vecto
 void GpuBackend::lc_s_hat_v(const std::vector<F128>& tail, std::vector<F128>& out) {
   auto et = build_eq(tail);
   const F128d* det = upload(et);
-  { Mark mk(this, ST_LINCHECK); launch_lc_s_hat_v(zvcap_, det, (uint32_t)et.size(), red_, st_); }
-  out = fetch(red_, 128);
+  const FusedPublish fp = fused_publish();
+  { Mark mk(this, ST_LINCHECK); launch_lc_s_hat_v(zvcap_, det, (uint32_t)et.size(), st_, fp); }
+  out = read_published(fp.seq, 128);
 }
 
 // ------------------------------------------------------------------ merged open
-uint32_t GpuBackend::launch_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area) {
+void GpuBackend::launch_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area, const FusedPublish& fp) {
   if (cl.size() != 2) throw std::runtime_error("merged open expects the AB and C claims");
+  // both claims' points (z_row | z_col) and byte tables in one copy; the row and column tables of
+  // a claim in one launch
+  std::vector<F128> args;
+  for (int i = 0; i < 2; ++i) args.insert(args.end(), cl[i].table.begin(), cl[i].table.end());
+  for (int i = 0; i < 2; ++i) {
+    args.insert(args.end(), cl[i].z_row.begin(), cl[i].z_row.end());
+    args.insert(args.end(), cl[i].z_col.begin(), cl[i].z_col.end());
+  }
+  const F128d* dt = upload(args);
+  const F128d* point = dt + cl[0].table.size() + cl[1].table.size();
   F128d* er[2];
   F128d* ec[2];
   for (int i = 0; i < 2; ++i) {
-    // the row and column tables of one claim in one launch, from the point (z_row | z_col)
-    std::vector<F128> rc(cl[i].z_row);
-    rc.insert(rc.end(), cl[i].z_col.begin(), cl[i].z_col.end());
-    const F128d* prc = upload(rc);
     er[i] = static_cast<F128d*>(scratch(size_t(16) << cl[i].z_row.size()));
     ec[i] = static_cast<F128d*>(scratch(size_t(16) << cl[i].z_col.size()));
-    launch_eq_split(prc, (uint32_t)cl[i].z_row.size(), (uint32_t)cl[i].z_col.size(), dev(F128::one()), er[i], ec[i],
+    launch_eq_split(point, (uint32_t)cl[i].z_row.size(), (uint32_t)cl[i].z_col.size(), dev(F128::one()), er[i], ec[i],
                     st_);
+    point += cl[i].z_row.size() + cl[i].z_col.size();
   }
-  std::vector<F128> tabs(cl[0].table);
-  tabs.insert(tabs.end(), cl[1].table.begin(), cl[1].table.end());
-  const F128d* dt = upload(tabs);
-  if (S.slots.size() == 1 && S.identity)
-    return launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_);
+  if (S.slots.size() == 1 && S.identity) {
+    launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_, fp);
+    return;
+  }
   const JaggedSegs g = jagged_segs(S);
-  return launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_, &g);
+  launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_, fp, &g);
 }
 
 void GpuBackend::mo_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area, F128& u0, F128& u2) {
   scr_off_ = 0;
-  uint32_t nb;
+  const FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_MO_BUILD_W);
-    nb = launch_build_w(cl, nu, area);
+    launch_build_w(cl, nu, area, fp);
   }
-  auto v = reduce(nb, 2);
+  auto v = read_published(fp.seq, 2);
   u0 = v[0];
   u2 = v[1];
   mo_q_ = q_;
@@ -1238,8 +1255,12 @@ void GpuBackend::lg_commit(uint32_t level, uint32_t log_cols, uint32_t log_lanes
   const F128d* tw = twiddles(log_cols + log_rate);
   { Mark mk(this, ST_LIGERITO); launch_lg_replicate(lf_[lg_cur_], lg_n_, block_len * lanes, L.mat, st_); }
   { Mark mk(this, ST_LG_NTT); launch_ntt(L.mat, lanes, log_cols + log_rate, log_rate, tw, st_); }
-  { Mark mk(this, ST_LG_MERKLE); launch_merkle(L.mat, lanes, block_len, cap_depth, L.tree, st_); }
-  cap = read_cap(L.tree, block_len, cap_depth);
+  const FusedPublish fp = fused_publish();
+  {
+    Mark mk(this, ST_LG_MERKLE);
+    launch_merkle(L.mat, lanes, block_len, cap_depth, L.tree, st_, d_open(size_t(32) << cap_depth), fp);
+  }
+  cap = read_cap(cap_depth, fp);
 }
 
 Msg256 GpuBackend::lg_introduce_eq(const std::vector<F128>& zp, F128& answer) {
@@ -1325,21 +1346,19 @@ void GpuBackend::lg_open(uint32_t level, const std::vector<uint64_t>& pos, uint3
   while ((uint64_t(1) << depth) < n_leaves) ++depth;
   uint32_t plen = depth - cap_depth;
   const uint64_t* dpos = static_cast<const uint64_t*>(upload(pos.data(), n * 8));
-  F128d* drows = static_cast<F128d*>(scratch((size_t)n * lanes * 16));
-  uint8_t* dpaths = static_cast<uint8_t*>(scratch((size_t)n * plen * 32 + 32));
+  const size_t row_bytes = (size_t)n * lanes * 16, path_bytes = (size_t)n * plen * 32;
+  uint8_t* d = d_open(row_bytes + path_bytes);
+  const FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_LIGERITO);
-    launch_gather_rows(mat, lanes, dpos, n, drows, st_);
-    launch_gather_paths(tree, n_leaves, dpos, n, cap_depth, dpaths, st_);
+    launch_gather_open(mat, lanes, tree, n_leaves, dpos, n, cap_depth, reinterpret_cast<F128d*>(d), d + row_bytes, st_, fp);
   }
-  std::vector<F128> hr((size_t)n * lanes);
-  std::vector<Hash> hp((size_t)n * plen);
-  CUDA_OK(cudaMemcpyAsync(hr.data(), drows, hr.size() * 16, cudaMemcpyDeviceToHost, st_));
-  if (plen) CUDA_OK(cudaMemcpyAsync(hp.data(), dpaths, hp.size() * 32, cudaMemcpyDeviceToHost, st_));
-  d2h_ += hr.size() * 16 + (plen ? hp.size() * 32 : 0);
-  sync();
-  for (uint32_t q = 0; q < n; ++q) rows.emplace_back(hr.begin() + (size_t)q * lanes, hr.begin() + (size_t)(q + 1) * lanes);
-  paths.insert(paths.end(), hp.begin(), hp.end());
+  wait_published(fp.seq);
+  d2h_ += row_bytes + path_bytes;
+  const F128* hr = reinterpret_cast<const F128*>(h_open_);
+  const Hash* hp = reinterpret_cast<const Hash*>(h_open_ + row_bytes);
+  for (uint32_t q = 0; q < n; ++q) rows.emplace_back(hr + (size_t)q * lanes, hr + (size_t)(q + 1) * lanes);
+  paths.insert(paths.end(), hp, hp + (size_t)n * plen);
 }
 
 std::vector<F256> GpuBackend::lg_residual() {

@@ -102,13 +102,13 @@ class GpuBackend : public ProverBackend {
   const F128d* upload(const std::vector<F128>& v);
   void sync();
   std::vector<F128> reduce(uint32_t n_blocks, uint32_t width);
-  std::vector<F128> fetch(const F128d* d, size_t n);
+  void upload_to(void* dst, const void* src, size_t bytes);
   EqSplit eq_split(const std::vector<F128>& point, F128 scale, uint32_t max_lo);
-  EqSplit eq_split_dev(const F128d* d_point, uint32_t n, F128 scale, uint32_t max_lo);
   // build the merged-open weight and launch its round-0 reduction (per-block partials)
-  uint32_t launch_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area);
+  void launch_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area, const FusedPublish& fp);
   const F128d* twiddles(uint32_t log_d);
-  std::vector<Hash> read_cap(const uint8_t* tree, uint64_t n_leaves, uint32_t cap_depth);
+  std::vector<Hash> read_cap(uint32_t cap_depth, const FusedPublish& fp);
+  uint8_t* d_open(size_t bytes);
 
   struct Mark {
     GpuBackend* b;
@@ -243,7 +243,11 @@ class GpuBackend : public ProverBackend {
   std::vector<Level> levels_;
   std::unique_ptr<JaggedAssist> jagged_;
 
+  // mapped memory that caps and openings are written to (grows to the largest opening)
+  uint8_t *h_open_ = nullptr, *d_open_ = nullptr;
+  size_t open_cap_ = 0;
   // mapped pinned memory the message reductions publish into
+  static constexpr uint32_t PUB_WORDS = 256;
   F128d* h_pub_ = nullptr;
   F128d* d_pub_ = nullptr;
   uint32_t* h_flag_ = nullptr;
@@ -275,8 +279,6 @@ class GpuBackend : public ProverBackend {
 
   F128d* part_ = nullptr;
   uint32_t part_cap_ = 0;
-  F128d* red_ = nullptr;
-  F128d* h_red_ = nullptr;
   uint8_t* scr_ = nullptr;
   size_t scr_cap_ = 0, scr_off_ = 0;
   uint8_t* d_stage_ = nullptr;

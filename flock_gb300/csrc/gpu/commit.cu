@@ -8,6 +8,7 @@
 // Layout: codewords are position-major SoA, data[pos * lanes + lane]; a Merkle leaf is
 // one position's `lanes` words. Trees are flat: leaves [0, N), then each level, root last.
 #include "kernels.h"
+#include "reduce.cuh"
 #include "sha256.cuh"
 #include "wintable.cuh"
 #include <atomic>
@@ -386,7 +387,8 @@ __global__ void merkle_level_kernel(uint32_t* __restrict__ tree, uint64_t in_off
 // for all of them, which this replaced, was bound by its one SM (2048 nodes to 256: 28 us).
 constexpr uint32_t MERKLE_SMALL_NODES = 1u << 15, MERKLE_SMALL_LEVELS = 3, MERKLE_SMALL_THREADS = 128;
 __global__ void __launch_bounds__(MERKLE_SMALL_THREADS)
-merkle_levels_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint64_t n_in, uint32_t levels) {
+merkle_levels_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint64_t n_in, uint32_t levels,
+                     uint32_t* __restrict__ cap, FusedPublish pub) {
   __shared__ uint32_t node[MERKLE_SMALL_THREADS][8];
   uint64_t off = in_off, len = n_in;
   const uint32_t t = threadIdx.x;
@@ -400,6 +402,10 @@ merkle_levels_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint64_t n_in
       sha256_words([&](uint32_t w) { return k ? node[2 * t + (w >> 3)][w & 7] : l[w]; }, 16, out);
 #pragma unroll
       for (int w = 0; w < 8; ++w) tree[(off + len + i) * 8 + w] = out[w];
+      if (cap && k == levels - 1) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) cap[i * 8 + w] = out[w];
+      }
     }
     __syncthreads();  // this level's inputs are read
     if (t < have) {
@@ -410,9 +416,16 @@ merkle_levels_kernel(uint32_t* __restrict__ tree, uint64_t in_off, uint64_t n_in
     off += len;
     len = nout;
   }
+  if (cap) publish_data(pub);
+}
+// The nodes [first, first + n) of the tree to mapped memory (a tree that is all cap).
+__global__ void publish_nodes_kernel(const uint32_t* __restrict__ tree, uint32_t n, uint32_t* __restrict__ cap,
+                                     FusedPublish pub) {
+  for (uint32_t i = threadIdx.x; i < n * 8; i += blockDim.x) cap[i] = tree[i];
+  publish_data(pub);
 }
 void launch_merkle(const F128d* rows, uint32_t lanes, uint64_t n_leaves, uint32_t cap_depth, uint8_t* tree,
-                   cudaStream_t s) {
+                   cudaStream_t s, uint8_t* cap, FusedPublish pub) {
   // levels above the cap are never read (the cap is the commitment, paths stop below it)
   const uint64_t n_cap = uint64_t(1) << cap_depth;
   if (n_cap > n_leaves) throw std::runtime_error("Merkle cap wider than the leaf level");
@@ -422,20 +435,27 @@ void launch_merkle(const F128d* rows, uint32_t lanes, uint64_t n_leaves, uint32_
   leaves<<<(unsigned)((n_leaves + 127) / 128), 128, 0, s>>>(rows, lanes, n_leaves, (uint32_t*)tree);
   LAUNCH_OK();
   uint64_t off = 0, len = n_leaves;
+  bool published = false;
   while (len > n_cap) {
     uint32_t levels = 1;
     if (len > MERKLE_SMALL_NODES) {
       merkle_level_kernel<<<(unsigned)((len / 2 + 127) / 128), 128, 0, s>>>((uint32_t*)tree, off, len / 2);
     } else {
       while (levels < MERKLE_SMALL_LEVELS && (len >> levels) > n_cap) ++levels;
+      const bool last = (len >> levels) == n_cap;
       merkle_levels_kernel<<<(unsigned)((len / 2 + MERKLE_SMALL_THREADS - 1) / MERKLE_SMALL_THREADS), MERKLE_SMALL_THREADS, 0,
-                             s>>>((uint32_t*)tree, off, len, levels);
+                             s>>>((uint32_t*)tree, off, len, levels, last ? (uint32_t*)cap : nullptr, pub);
+      published |= last;
     }
     LAUNCH_OK();
     for (; levels; --levels) {
       off += len;
       len /= 2;
     }
+  }
+  if (cap && !published) {
+    publish_nodes_kernel<<<1, 256, 0, s>>>((const uint32_t*)tree + off * 8, (uint32_t)n_cap, (uint32_t*)cap, pub);
+    LAUNCH_OK();
   }
 }
 
@@ -501,41 +521,33 @@ void launch_pow(const uint32_t digest_le[8], uint32_t bits, uint64_t start, uint
 }
 
 // ---- openings
-__global__ void gather_rows_kernel(const F128d* __restrict__ mat, uint32_t lanes, const uint64_t* __restrict__ pos,
-                                   uint32_t n, F128d* __restrict__ out) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * lanes) return;
-  uint32_t q = i / lanes, l = i - q * lanes;
-  out[i] = mat[pos[q] * lanes + l];
-}
-void launch_gather_rows(const F128d* mat, uint32_t lanes, const uint64_t* d_pos, uint32_t n, F128d* out,
-                        cudaStream_t s) {
-  uint32_t work = n * lanes;
-  gather_rows_kernel<<<(work + 255) / 256, 256, 0, s>>>(mat, lanes, d_pos, n, out);
-  LAUNCH_OK();
-}
-__global__ void gather_paths_kernel(const uint8_t* __restrict__ tree, uint64_t n_leaves,
-                                    const uint64_t* __restrict__ pos, uint32_t n, uint32_t cap_depth,
-                                    uint8_t* __restrict__ out) {
-  uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  uint32_t depth = 0;
-  while ((1ull << depth) < n_leaves) ++depth;
-  uint32_t plen = depth - cap_depth;
-  uint64_t start = 0, len = n_leaves, idx = pos[q];
-  for (uint32_t k = 0; k < plen; ++k) {  // 32-byte nodes: two 16-byte copies (tree and out are 16-byte aligned)
-    const uint4* src = reinterpret_cast<const uint4*>(tree + (start + (idx ^ 1)) * 32);
-    uint4* dst = reinterpret_cast<uint4*>(out + ((uint64_t)q * plen + k) * 32);
-    dst[0] = src[0];
-    dst[1] = src[1];
-    start += len;
-    len >>= 1;
-    idx >>= 1;
+// Rows and sibling paths of n positions straight to mapped memory, 16 bytes a thread: position q's
+// row is `lanes` pieces, its path two per level (the sibling of pos >> k in level k, which starts
+// at node 2 n_leaves - (2 n_leaves >> k)).
+__global__ void gather_open_kernel(const uint4* __restrict__ mat, uint32_t lanes, const uint4* __restrict__ tree,
+                                   uint64_t n_leaves, const uint64_t* __restrict__ pos, uint32_t n, uint32_t plen,
+                                   uint4* __restrict__ rows, uint4* __restrict__ paths, FusedPublish pub) {
+  const uint32_t per = lanes + 2 * plen, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n * per) {
+    const uint32_t q = i / per, r = i - q * per;
+    if (r < lanes) {
+      rows[q * lanes + r] = mat[pos[q] * lanes + r];
+    } else {
+      const uint32_t k = (r - lanes) >> 1, half = (r - lanes) & 1;
+      const uint64_t node = 2 * n_leaves - ((2 * n_leaves) >> k) + ((pos[q] >> k) ^ 1);
+      paths[(q * plen + k) * 2 + half] = tree[node * 2 + half];
+    }
   }
+  publish_data(pub);
 }
-void launch_gather_paths(const uint8_t* tree, uint64_t n_leaves, const uint64_t* d_pos, uint32_t n,
-                         uint32_t cap_depth, uint8_t* out, cudaStream_t s) {
-  gather_paths_kernel<<<(n + 127) / 128, 128, 0, s>>>(tree, n_leaves, d_pos, n, cap_depth, out);
+void launch_gather_open(const F128d* mat, uint32_t lanes, const uint8_t* tree, uint64_t n_leaves, const uint64_t* d_pos,
+                        uint32_t n, uint32_t cap_depth, F128d* rows, uint8_t* paths, cudaStream_t s, FusedPublish pub) {
+  uint32_t depth = 0;
+  while ((uint64_t(1) << depth) < n_leaves) ++depth;
+  const uint32_t plen = depth - cap_depth, work = n * (lanes + 2 * plen);
+  gather_open_kernel<<<std::max(1u, (work + 255) / 256), 256, 0, s>>>(
+      reinterpret_cast<const uint4*>(mat), lanes, reinterpret_cast<const uint4*>(tree), n_leaves, d_pos, n, plen,
+      reinterpret_cast<uint4*>(rows), reinterpret_cast<uint4*>(paths), pub);
   LAUNCH_OK();
 }
 

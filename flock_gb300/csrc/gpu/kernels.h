@@ -36,6 +36,17 @@ void set_dynamic_smem(const void* kernel, int bytes);
 
 int sm_count();
 
+// In-kernel publication of a round message: the last block to finish (a device-wide
+// ticket counter) XOR-reduces every block's partials, writes the message to mapped host
+// memory and then the sequence number, as launch_reduce_publish does in a launch of its
+// own. counter must be zero before the launch; the last block resets it.
+struct FusedPublish {
+  F128d* out = nullptr;        // mapped host memory (null: no publication)
+  uint32_t* flag = nullptr;    // mapped host memory
+  uint32_t* counter = nullptr; // device memory
+  uint32_t seq = 0;
+};
+
 // witness.cu — writes chunk columns [0, used_chunks) of z, a, b
 void upload_witness_constants();  // once per process (synchronous symbol copies)
 void launch_witness(int hash, const void* d_inputs, uint32_t n_inst, uint32_t nu, F128d* z, F128d* a, F128d* b,
@@ -47,21 +58,23 @@ void launch_fill_lane_major(const F128d* q, F128d* cw, uint32_t lanes, uint32_t 
 void launch_ntt(F128d* data, uint32_t lanes, uint32_t log_d, uint32_t start_layer, const F128d* tw, cudaStream_t s);
 // Leaves and the levels up to the cap level (2^cap_depth nodes); the levels above it are
 // not computed.
+// With `cap` (mapped memory, 32 2^cap_depth bytes) the cap is also written there and published.
 void launch_merkle(const F128d* rows, uint32_t lanes, uint64_t n_leaves, uint32_t cap_depth, uint8_t* tree,
-                   cudaStream_t s);
+                   cudaStream_t s, uint8_t* cap = nullptr, FusedPublish pub = FusedPublish());
 void launch_pow(const uint32_t digest_le[8], uint32_t bits, uint64_t start, uint64_t count, unsigned long long* d_min,
                 uint32_t* d_counter, unsigned long long* out, uint32_t* flag, uint32_t seq, cudaStream_t s);
-void launch_gather_rows(const F128d* mat, uint32_t lanes, const uint64_t* d_pos, uint32_t n, F128d* out,
-                        cudaStream_t s);
-void launch_gather_paths(const uint8_t* tree, uint64_t n_leaves, const uint64_t* d_pos, uint32_t n,
-                         uint32_t cap_depth, uint8_t* out, cudaStream_t s);
+// An opening of n positions into mapped memory, published: the rows (lanes words each) at rows, the
+// sibling paths (depth - cap_depth nodes each) at paths.
+void launch_gather_open(const F128d* mat, uint32_t lanes, const uint8_t* tree, uint64_t n_leaves, const uint64_t* d_pos,
+                        uint32_t n, uint32_t cap_depth, F128d* rows, uint8_t* paths, cudaStream_t s, FusedPublish pub);
 
 // sumcheck.cu. Kernels returning a block count wrote per-block partials of the stated
-// width into `part`; launch_reduce_parts XORs them.
+// width into `part` and, with a FusedPublish, publish their sum.
 // The lo and hi tables of an eq split (lo unscaled, hi times scale) in one launch.
 void launch_eq_split(const F128d* d_point, uint32_t lo_bits, uint32_t hi_bits, F128d scale, F128d* lo, F128d* hi,
                      cudaStream_t s);
-void launch_reduce_parts(const F128d* part, uint32_t n_blocks, uint32_t width, F128d* out, cudaStream_t s);
+void launch_reduce_pair(const F128d* pa, uint32_t na, uint32_t wa, const F128d* pb, uint32_t nb, uint32_t wb,
+                        cudaStream_t s, FusedPublish pub);
 
 // unit[64 s + i]: extension of row bit s at Lambda point i; wconst, pconst: see ZcConsts.
 void upload_zc_consts(const uint8_t* unit, const F128d* wconst, const F128d* pconst);
@@ -72,36 +85,26 @@ void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m
                       const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* g, F128d* part_ab,
                       uint32_t* nrows_ab, F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s);
 uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words, const F128d* eq_lo,
-                             uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s);       // width 2
+                             uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s, FusedPublish pub);       // width 2
 // First multilinear fold (at rho) of the skip-folded a, b, computed from the bits; writes
 // n_pairs * 2 words of each folded vector and the next message. tabs: 4096-word scratch.
 // Pairs from live_pairs on have zero inputs: their outputs are written as zeros and they
 // add nothing to the message.
 uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d rho, F128d* tabs, uint64_t n_pairs,
                          uint64_t live_pairs, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* aout,
-                         F128d* bout, F128d* part, cudaStream_t s);                                     // width 2
+                         F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub);                                     // width 2
 // The weighted form (see the kernels): low bits of its chunks for this many live words, 0 where
 // the plain form runs; the skip fold's message and the first fold with its message. eq_lo: eq
 // over the chunk's low coordinates (of words, then of pairs), h: eq over the high ones.
 uint32_t zc_weighted_lo_bits(uint64_t live_words);
 uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
                                       uint32_t lo_bits, const F128d* eq_lo, const F128d* h, F128d* part,
-                                      cudaStream_t s);                                                   // width 2
+                                      cudaStream_t s, FusedPublish pub);                                                   // width 2
 uint32_t launch_zc_fold2_weighted(const F128d* a, const F128d* b, const F128d* w64, F128d rho, uint64_t n_pairs,
                                   uint64_t live_pairs, uint32_t lo_bits, const F128d* eq_lo, const F128d* h,
-                                  F128d* aout, F128d* bout, F128d* part, cudaStream_t s);                // width 2
+                                  F128d* aout, F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub);                // width 2
 // out[c] = prod_j f[2j + bit j of c] over n factor pairs.
 void launch_factor_table(const F128d* f, uint32_t n, F128d* out, cudaStream_t s);
-// In-kernel publication of a round message: the last block to finish (a device-wide
-// ticket counter) XOR-reduces every block's partials, writes the message to mapped host
-// memory and then the sequence number, as launch_reduce_publish does in a launch of its
-// own. counter must be zero before the launch; the last block resets it.
-struct FusedPublish {
-  F128d* out = nullptr;        // mapped host memory (null: no publication)
-  uint32_t* flag = nullptr;    // mapped host memory
-  uint32_t* counter = nullptr; // device memory
-  uint32_t seq = 0;
-};
 // eq_lo == nullptr: eq = 1; eq_hi == nullptr: eq(j) = eq_lo[j mod 2^lo_bits]; else the split eq.
 // unweight (or null): factors of the folded a entries. Pairs from live_pairs on have zero
 // inputs (zeros written, nothing added to the message).
@@ -126,21 +129,23 @@ struct KeccakColumnConsts {
 };
 void launch_keccak_lincheck_columns(const F128d* eqi, F128d* ca, F128d* cb, const KeccakColumnConsts& kc,
                                     cudaStream_t s);
-// Row fold of the used chunk columns; part holds part_cap entries (at least 128 a column).
+// Row fold of the used chunk columns into zv and a copy of it (K entries, zero past the used
+// columns); part holds part_cap entries (at least 128 a column).
 void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F128d* eq_lo, uint32_t lo_bits,
-                    const F128d* eq_hi, F128d* part, uint64_t part_cap, F128d* zv, cudaStream_t s);
+                    const F128d* eq_hi, F128d* part, uint64_t part_cap, uint32_t K, F128d* zv, F128d* captured,
+                    cudaStream_t s);
 uint32_t launch_lc_start(const F128d* ca, const F128d* cb, F128d alpha, F128d beta, uint32_t pin, uint32_t K,
-                         F128d* comb, const F128d* zv, F128d* part, cudaStream_t s);                   // width 2
+                         F128d* comb, const F128d* zv, F128d* part, cudaStream_t s, FusedPublish pub);                   // width 2
 uint32_t launch_lc_round(const F128d* comb, const F128d* zv, uint32_t len, F128d r, F128d* comb_out, F128d* zv_out,
                          F128d* part, cudaStream_t s, FusedPublish pub);
 // Union lincheck: one slot's weighted comb (out = weight (alpha ca + cb), + beta at pin),
 // and the first message of a comb built that way.
 void launch_lc_slot_comb(const F128d* ca, const F128d* cb, F128d alpha, F128d weight, F128d beta, uint32_t pin,
                          uint32_t K, F128d* out, cudaStream_t s);
-uint32_t launch_lc_top_message(const F128d* comb, const F128d* zv, uint32_t K, F128d* part, cudaStream_t s);  // width 2
+uint32_t launch_lc_top_message(const F128d* comb, const F128d* zv, uint32_t K, F128d* part, cudaStream_t s, FusedPublish pub);  // width 2
 uint32_t launch_lc_matrix_evals(const F128d* ca, const F128d* cb, const F128d* er, const F128d* zp, uint32_t K,
-                                F128d* part, cudaStream_t s);                                          // width 2
-void launch_lc_s_hat_v(const F128d* zv, const F128d* et, uint32_t n_tail, F128d* out, cudaStream_t s);
+                                F128d* part, cudaStream_t s, FusedPublish pub);                                          // width 2
+void launch_lc_s_hat_v(const F128d* zv, const F128d* et, uint32_t n_tail, cudaStream_t s, FusedPublish pub);
 
 // The committed stack of a union with non-identity compaction, as at most four slot
 // segments (dense [base, base + rows * cols), column-major, first column col_off).
@@ -151,7 +156,7 @@ struct JaggedSegs {
 // segs == nullptr: the aligned layout (row = d mod 2^nu, col = d >> nu).
 uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, const F128d* er1, const F128d* ec1,
                            const F128d* tables, uint32_t nu, uint64_t area, uint64_t n, F128d* w, F128d* part,
-                           cudaStream_t s, const JaggedSegs* segs = nullptr);                          // width 2
+                           cudaStream_t s, FusedPublish pub, const JaggedSegs* segs = nullptr);                          // width 2
 
 // rounds.cu: the multipoint assist over a general jagged layout (union proofs). Dual values
 // out[i * n_points + j] of claim i (row points z_row[i * n ..), run weights w[i * n_runs ..)) at

@@ -108,6 +108,20 @@ static __device__ void publish_if_last(const F128d* part, uint32_t width, const 
   }
 }
 
+// Publication of data that the blocks wrote to mapped memory themselves: every thread of the
+// block calls this after its writes; the last block to arrive sets the sequence number.
+static __device__ void publish_data(const FusedPublish& pub) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    if (atomicAdd(pub.counter, 1u) == gridDim.x * gridDim.y - 1) {
+      *pub.counter = 0;
+      __threadfence_system();
+      *(volatile uint32_t*)pub.flag = pub.seq;
+    }
+  }
+}
+
 // ------------------------------------------------------------------ byte-table maps, jagged layout
 __device__ __forceinline__ F128d fold_slot(F128d x, const F128d* tab) {
   F128d acc = f128_zero();

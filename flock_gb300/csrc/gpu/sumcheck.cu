@@ -4,7 +4,8 @@
 // code switch, induced basis).
 //
 // Reductions: every message kernel writes per-block XOR partials to `part`
-// (part[block * width + j]); reduce_parts XORs them into `width` values.
+// (part[block * width + j]); the last block to arrive XORs them into `width` values
+// and publishes these to mapped memory.
 // Eq tables over many variables are never materialised: eq(i) = lo[i & (2^lo_bits - 1)]
 // * hi[i >> lo_bits], and kernels that sum eq-weighted terms walk chunks of 2^lo_bits
 // consecutive indices, summing lo-weighted terms and multiplying by hi once per chunk.
@@ -49,17 +50,24 @@ void launch_eq_split(const F128d* d_point, uint32_t lo_bits, uint32_t hi_bits, F
   LAUNCH_OK();
 }
 
-__global__ void reduce_parts_kernel(const F128d* __restrict__ part, uint32_t n_blocks, uint32_t width,
-                                    F128d* __restrict__ out) {
+// XOR of the rows of two partial arrays (na rows of width wa, nb of width wb), published side by
+// side; one block a value.
+__global__ void __launch_bounds__(128)
+reduce_pair_kernel(const F128d* __restrict__ pa, uint32_t na, uint32_t wa, const F128d* __restrict__ pb, uint32_t nb,
+                   uint32_t wb, FusedPublish pub) {
   __shared__ F128d sh[32];
-  uint32_t col = blockIdx.x;
+  const bool second = blockIdx.x >= wa;
+  const F128d* p = second ? pb + (blockIdx.x - wa) : pa + blockIdx.x;
+  const uint32_t n = second ? nb : na, w = second ? wb : wa;
   F128d acc = f128_zero();
-  for (uint32_t b = threadIdx.x; b < n_blocks; b += blockDim.x) acc += part[(uint64_t)b * width + col];
+  for (uint32_t b = threadIdx.x; b < n; b += blockDim.x) acc += p[(uint64_t)b * w];
   acc = block_xor(acc, sh);
-  if (threadIdx.x == 0) out[col] = acc;
+  if (threadIdx.x == 0) pub.out[blockIdx.x] = acc;
+  publish_data(pub);
 }
-void launch_reduce_parts(const F128d* part, uint32_t n_blocks, uint32_t width, F128d* out, cudaStream_t s) {
-  reduce_parts_kernel<<<width, 256, 0, s>>>(part, n_blocks, width, out);
+void launch_reduce_pair(const F128d* pa, uint32_t na, uint32_t wa, const F128d* pb, uint32_t nb, uint32_t wb,
+                        cudaStream_t s, FusedPublish pub) {
+  reduce_pair_kernel<<<wa + wb, 128, 0, s>>>(pa, na, wa, pb, nb, wb, pub);
   LAUNCH_OK();
 }
 
@@ -535,7 +543,7 @@ void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m
 __global__ void __launch_bounds__(256)
 zc_fold_skip_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ w64,
                     uint64_t n_words, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
-                    const F128d* __restrict__ eq_hi, F128d* __restrict__ part) {
+                    const F128d* __restrict__ eq_hi, F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d T[8][256];
   __shared__ F128d sh[32];
   for (uint32_t e = threadIdx.x; e < 2048; e += blockDim.x) {
@@ -575,6 +583,7 @@ zc_fold_skip_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, co
     }
   }
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+  publish_if_last(part, 2, pub, sh);
 }
 // ---- the weighted form of the zerocheck rounds
 // The eq factor of a message over words is eq_lo(low coordinates) * h(chunk), a chunk being
@@ -599,7 +608,7 @@ template <int LO>
 __global__ void __launch_bounds__(ZC_W_THREADS, 1)
 zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ w64,
                              uint64_t n_chunks, uint64_t n_words, const F128d* __restrict__ eq_lo,
-                             const F128d* __restrict__ h, F128d* __restrict__ part) {
+                             const F128d* __restrict__ h, F128d* __restrict__ part, FusedPublish pub) {
   constexpr uint32_t PER = (1u << LO) / ZC_W_THREADS;
   extern __shared__ __align__(16) char wt[];  // a's table, then b's
   __shared__ F128d img[64];
@@ -641,6 +650,7 @@ zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restric
   G1 = block_xor(G1, sh);
   GI = block_xor(GI, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+  publish_if_last(part, 2, pub, sh);
 }
 // A chunk's tables are rebuilt for it (about 2000 cycles beside 13 a word), so chunks are as
 // long as leaves every SM four, down to 2^10 words with one an SM; smaller vectors take the
@@ -653,27 +663,27 @@ uint32_t zc_weighted_lo_bits(uint64_t live_words) {
 }
 template <int LO>
 static uint32_t fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
-                                   const F128d* eq_lo, const F128d* h, F128d* part, cudaStream_t s) {
+                                   const F128d* eq_lo, const F128d* h, F128d* part, cudaStream_t s, FusedPublish pub) {
   const uint64_t n_chunks = (n_words + (1ull << LO) - 1) >> LO;
   const uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count());
   const int smem = 2 * WinMap<6, 64>::BYTES;
   set_dynamic_smem((const void*)zc_fold_skip_weighted_kernel<LO>, smem);
-  zc_fold_skip_weighted_kernel<LO><<<blocks, ZC_W_THREADS, smem, s>>>(a, b, w64, n_chunks, n_words, eq_lo, h, part);
+  zc_fold_skip_weighted_kernel<LO><<<blocks, ZC_W_THREADS, smem, s>>>(a, b, w64, n_chunks, n_words, eq_lo, h, part, pub);
   LAUNCH_OK();
   return blocks;
 }
 uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
                                       uint32_t lo_bits, const F128d* eq_lo, const F128d* h, F128d* part,
-                                      cudaStream_t s) {
-  if (lo_bits == 12) return fold_skip_weighted<12>(a, b, w64, n_words, eq_lo, h, part, s);
-  if (lo_bits == 11) return fold_skip_weighted<11>(a, b, w64, n_words, eq_lo, h, part, s);
-  return fold_skip_weighted<10>(a, b, w64, n_words, eq_lo, h, part, s);
+                                      cudaStream_t s, FusedPublish pub) {
+  if (lo_bits == 12) return fold_skip_weighted<12>(a, b, w64, n_words, eq_lo, h, part, s, pub);
+  if (lo_bits == 11) return fold_skip_weighted<11>(a, b, w64, n_words, eq_lo, h, part, s, pub);
+  return fold_skip_weighted<10>(a, b, w64, n_words, eq_lo, h, part, s, pub);
 }
 uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words, const F128d* eq_lo,
-                             uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s) {
+                             uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s, FusedPublish pub) {
   uint64_t n_chunks = (n_words + (1ull << lo_bits) - 1) >> lo_bits;
   uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
-  zc_fold_skip_kernel<<<blocks, 256, 0, s>>>(a, b, w64, n_words, eq_lo, lo_bits, eq_hi, part);
+  zc_fold_skip_kernel<<<blocks, 256, 0, s>>>(a, b, w64, n_words, eq_lo, lo_bits, eq_hi, part, pub);
   LAUNCH_OK();
   return blocks;
 }
@@ -703,7 +713,7 @@ __global__ void __launch_bounds__(256)
 zc_fold2_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ tabs,
                 uint64_t n_pairs, uint64_t live_pairs, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
                 const F128d* __restrict__ eq_hi, F128d* __restrict__ aout, F128d* __restrict__ bout,
-                F128d* __restrict__ part) {
+                F128d* __restrict__ part, FusedPublish pub) {
   extern __shared__ __align__(16) F128d T[];  // [2][8][256]: (1 + rho) w tables, then rho w tables
   __shared__ F128d sh[32];
   for (uint32_t e = threadIdx.x; e < 4096; e += blockDim.x) T[e] = tabs[e];
@@ -749,10 +759,11 @@ zc_fold2_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const 
     }
   }
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+  publish_if_last(part, 2, pub, sh);
 }
 uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d rho, F128d* tabs, uint64_t n_pairs,
                          uint64_t live_pairs, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* aout,
-                         F128d* bout, F128d* part, cudaStream_t s) {
+                         F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub) {
   live_pairs = std::min(live_pairs, n_pairs);
   zc_scaled_tables_kernel<<<16, 256, 0, s>>>(w64, rho, tabs);
   LAUNCH_OK();
@@ -760,7 +771,7 @@ uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d
   uint64_t n_chunks = (n_pairs + (1ull << lo_bits) - 1) >> lo_bits;
   uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 3);
   zc_fold2_kernel<<<blocks, 256, 4096 * 16, s>>>(a, b, tabs, n_pairs, live_pairs, eq_lo, lo_bits, eq_hi, aout, bout,
-                                                  part);
+                                                  part, pub);
   LAUNCH_OK();
   return blocks;
 }
@@ -773,7 +784,7 @@ __global__ void __launch_bounds__(ZC_W_THREADS, 1)
 zc_fold2_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, const F128d* __restrict__ w64,
                          F128d rho, uint64_t n_pairs, uint64_t live_pairs, const F128d* __restrict__ eq_lo,
                          const F128d* __restrict__ h, F128d* __restrict__ aout, F128d* __restrict__ bout,
-                         F128d* __restrict__ part) {
+                         F128d* __restrict__ part, FusedPublish pub) {
   constexpr uint32_t PAIRS = 1u << (LO - 1), PER = PAIRS / ZC_W_THREADS, TAB = WinMap<5, 64>::BYTES;
   extern __shared__ __align__(16) char wt[];  // a's tables for the low and high halves, then b's
   __shared__ F128d wr[2][64], img[2][64];
@@ -836,26 +847,27 @@ zc_fold2_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ 
   G1 = block_xor(G1, sh);
   GI = block_xor(GI, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
+  publish_if_last(part, 2, pub, sh);
 }
 template <int LO>
 static uint32_t fold2_weighted(const F128d* a, const F128d* b, const F128d* w64, F128d rho, uint64_t n_pairs,
                                uint64_t live_pairs, const F128d* eq_lo, const F128d* h, F128d* aout, F128d* bout,
-                               F128d* part, cudaStream_t s) {
+                               F128d* part, cudaStream_t s, FusedPublish pub) {
   const int smem = 4 * WinMap<5, 64>::BYTES;
   set_dynamic_smem((const void*)zc_fold2_weighted_kernel<LO>, smem);
   const uint32_t blocks = (uint32_t)std::min<uint64_t>((n_pairs + (1ull << (LO - 1)) - 1) >> (LO - 1), (uint64_t)sm_count());
   zc_fold2_weighted_kernel<LO><<<blocks, ZC_W_THREADS, smem, s>>>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout,
-                                                                  bout, part);
+                                                                  bout, part, pub);
   LAUNCH_OK();
   return blocks;
 }
 uint32_t launch_zc_fold2_weighted(const F128d* a, const F128d* b, const F128d* w64, F128d rho, uint64_t n_pairs,
                                   uint64_t live_pairs, uint32_t lo_bits, const F128d* eq_lo, const F128d* h,
-                                  F128d* aout, F128d* bout, F128d* part, cudaStream_t s) {
+                                  F128d* aout, F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub) {
   live_pairs = std::min(live_pairs, n_pairs);
-  if (lo_bits == 12) return fold2_weighted<12>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s);
-  if (lo_bits == 11) return fold2_weighted<11>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s);
-  return fold2_weighted<10>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s);
+  if (lo_bits == 12) return fold2_weighted<12>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s, pub);
+  if (lo_bits == 11) return fold2_weighted<11>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s, pub);
+  return fold2_weighted<10>(a, b, w64, rho, n_pairs, live_pairs, eq_lo, h, aout, bout, part, s, pub);
 }
 // out[c] = prod_j (bit j of c ? f[2j + 1] : f[2j]), j < n: the reciprocals of an eq table from
 // those of its factors.
@@ -1157,23 +1169,27 @@ void launch_keccak_lincheck_columns(const F128d* eqi, F128d* ca, F128d* cb, cons
   LAUNCH_OK();
 }
 
-__global__ void lc_zvec_reduce_kernel(const F128d* __restrict__ part, uint32_t n_split, uint32_t n_out,
-                                      F128d* __restrict__ zv) {
+// The splits' sums of the used columns into zv and its captured copy, zeros in the others.
+__global__ void lc_zvec_reduce_kernel(const F128d* __restrict__ part, uint32_t n_split, uint32_t n_out, uint32_t K,
+                                      F128d* __restrict__ zv, F128d* __restrict__ captured) {
   uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;  // o = 128 cc + t
-  if (o >= n_out) return;
-  uint32_t cc = o >> 7, t = o & 127;
+  if (o >= K) return;
   F128d acc = f128_zero();
-  for (uint32_t sp = 0; sp < n_split; ++sp) acc += part[((uint64_t)cc * n_split + sp) * 128 + t];
+  if (o < n_out) {
+    uint32_t cc = o >> 7, t = o & 127;
+    for (uint32_t sp = 0; sp < n_split; ++sp) acc += part[((uint64_t)cc * n_split + sp) * 128 + t];
+  }
   zv[o] = acc;
+  captured[o] = acc;
 }
 // z_vec[128 cc + t] = sum_row eq(row) * bit_t(z[(cc << nu) + row]).
 void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F128d* eq_lo, uint32_t lo_bits,
-                    const F128d* eq_hi, F128d* part, uint64_t part_cap, F128d* zv, cudaStream_t s) {
+                    const F128d* eq_hi, F128d* part, uint64_t part_cap, uint32_t K, F128d* zv, F128d* captured,
+                    cudaStream_t s) {
   const uint64_t rows = 1ull << nu;
   const BitSumPlan p = bit_sum_plan(used_chunks, rows, part_cap / (used_chunks * 128ull));
   bit_sums<BITS_RAW>(p, z, rows, 1, used_chunks, rows, eq_lo, lo_bits, eq_hi, nullptr, part, s);
-  uint32_t n_out = used_chunks * 128;
-  lc_zvec_reduce_kernel<<<(n_out + 127) / 128, 128, 0, s>>>(part, p.splits, n_out, zv);
+  lc_zvec_reduce_kernel<<<(K + 127) / 128, 128, 0, s>>>(part, p.splits, used_chunks * 128, K, zv, captured);
   LAUNCH_OK();
 }
 
@@ -1181,7 +1197,7 @@ void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F12
 //   e1 = sum_i comb[h+i] zv[h+i], einf = sum_i (comb[h+i] + comb[i]) (zv[h+i] + zv[i]).
 __global__ void lc_start_kernel(const F128d* __restrict__ ca, const F128d* __restrict__ cb, F128d alpha, F128d beta,
                                 uint32_t pin, uint32_t K, F128d* __restrict__ comb, const F128d* __restrict__ zv,
-                                F128d* __restrict__ part) {
+                                F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d sh[32];
   uint32_t h = K / 2;
   F128d e1 = f128_zero(), ei = f128_zero();
@@ -1197,11 +1213,12 @@ __global__ void lc_start_kernel(const F128d* __restrict__ ca, const F128d* __res
   e1 = block_xor(e1, sh);
   ei = block_xor(ei, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = e1; part[blockIdx.x * 2 + 1] = ei; }
+  publish_if_last(part, 2, pub, sh);
 }
 uint32_t launch_lc_start(const F128d* ca, const F128d* cb, F128d alpha, F128d beta, uint32_t pin, uint32_t K,
-                         F128d* comb, const F128d* zv, F128d* part, cudaStream_t s) {
+                         F128d* comb, const F128d* zv, F128d* part, cudaStream_t s, FusedPublish pub) {
   uint32_t blocks = std::max(1u, std::min((K / 2 + 255) / 256, 256u));
-  lc_start_kernel<<<blocks, 256, 0, s>>>(ca, cb, alpha, beta, pin, K, comb, zv, part);
+  lc_start_kernel<<<blocks, 256, 0, s>>>(ca, cb, alpha, beta, pin, K, comb, zv, part, pub);
   LAUNCH_OK();
   return blocks;
 }
@@ -1223,7 +1240,7 @@ void launch_lc_slot_comb(const F128d* ca, const F128d* cb, F128d alpha, F128d we
 }
 // First top-variable message of a built comb against zv (pairs (i, i + K/2)).
 __global__ void lc_top_message_kernel(const F128d* __restrict__ comb, const F128d* __restrict__ zv, uint32_t K,
-                                      F128d* __restrict__ part) {
+                                      F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d sh[32];
   uint32_t h = K / 2;
   F128d e1 = f128_zero(), ei = f128_zero();
@@ -1235,10 +1252,11 @@ __global__ void lc_top_message_kernel(const F128d* __restrict__ comb, const F128
   e1 = block_xor(e1, sh);
   ei = block_xor(ei, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = e1; part[blockIdx.x * 2 + 1] = ei; }
+  publish_if_last(part, 2, pub, sh);
 }
-uint32_t launch_lc_top_message(const F128d* comb, const F128d* zv, uint32_t K, F128d* part, cudaStream_t s) {
+uint32_t launch_lc_top_message(const F128d* comb, const F128d* zv, uint32_t K, F128d* part, cudaStream_t s, FusedPublish pub) {
   uint32_t blocks = std::max(1u, std::min((K / 2 + 255) / 256, 256u));
-  lc_top_message_kernel<<<blocks, 256, 0, s>>>(comb, zv, K, part);
+  lc_top_message_kernel<<<blocks, 256, 0, s>>>(comb, zv, K, part, pub);
   LAUNCH_OK();
   return blocks;
 }
@@ -1259,7 +1277,7 @@ uint32_t launch_lc_round(const F128d* comb, const F128d* zv, uint32_t len, F128d
 // (<w, comb_a>, <w, comb_b>), w[c] = er[c >> 6] * zp[c & 63].
 __global__ void lc_matrix_evals_kernel(const F128d* __restrict__ ca, const F128d* __restrict__ cb,
                                        const F128d* __restrict__ er, const F128d* __restrict__ zp, uint32_t K,
-                                       F128d* __restrict__ part) {
+                                       F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d sh[32];
   F128d ea = f128_zero(), eb = f128_zero();
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < K; c += gridDim.x * blockDim.x) {
@@ -1270,26 +1288,28 @@ __global__ void lc_matrix_evals_kernel(const F128d* __restrict__ ca, const F128d
   ea = block_xor(ea, sh);
   eb = block_xor(eb, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = ea; part[blockIdx.x * 2 + 1] = eb; }
+  publish_if_last(part, 2, pub, sh);
 }
 uint32_t launch_lc_matrix_evals(const F128d* ca, const F128d* cb, const F128d* er, const F128d* zp, uint32_t K,
-                                F128d* part, cudaStream_t s) {
+                                F128d* part, cudaStream_t s, FusedPublish pub) {
   uint32_t blocks = std::max(1u, std::min((K + 255) / 256, 256u));
-  lc_matrix_evals_kernel<<<blocks, 256, 0, s>>>(ca, cb, er, zp, K, part);
+  lc_matrix_evals_kernel<<<blocks, 256, 0, s>>>(ca, cb, er, zp, K, part, pub);
   LAUNCH_OK();
   return blocks;
 }
-// out[b] = sum_k et[k] * zv[b + 128 k]; one block per b.
+// pub.out[b] = sum_k et[k] * zv[b + 128 k]; one block per b.
 __global__ void lc_s_hat_v_kernel(const F128d* __restrict__ zv, const F128d* __restrict__ et, uint32_t n_tail,
-                                  F128d* __restrict__ out) {
+                                  FusedPublish pub) {
   __shared__ F128d sh[32];
   uint32_t bb = blockIdx.x;
   F128d acc = f128_zero();
   for (uint32_t k = threadIdx.x; k < n_tail; k += blockDim.x) acc += et[k] * zv[bb + 128 * k];
   acc = block_xor(acc, sh);
-  if (threadIdx.x == 0) out[bb] = acc;
+  if (threadIdx.x == 0) pub.out[bb] = acc;
+  publish_data(pub);
 }
-void launch_lc_s_hat_v(const F128d* zv, const F128d* et, uint32_t n_tail, F128d* out, cudaStream_t s) {
-  lc_s_hat_v_kernel<<<128, 128, 0, s>>>(zv, et, n_tail, out);
+void launch_lc_s_hat_v(const F128d* zv, const F128d* et, uint32_t n_tail, cudaStream_t s, FusedPublish pub) {
+  lc_s_hat_v_kernel<<<128, 128, 0, s>>>(zv, et, n_tail, pub);
   LAUNCH_OK();
 }
 
@@ -1302,7 +1322,7 @@ __global__ void __launch_bounds__(512, 1)
 mo_build_w_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er0, const F128d* __restrict__ ec0,
                   const F128d* __restrict__ er1, const F128d* __restrict__ ec1, const F128d* __restrict__ tables,
                   uint32_t nu, uint64_t area, uint64_t n, F128d* __restrict__ w, F128d* __restrict__ part,
-                  JaggedSegs segs) {
+                  JaggedSegs segs, FusedPublish pub) {
   extern __shared__ __align__(16) F128d tab[];  // 2 x 16 x 256
   __shared__ F128d sh[32];
   for (uint32_t i = threadIdx.x; i < 2 * 16 * 256; i += blockDim.x) tab[i] = tables[i];
@@ -1332,6 +1352,7 @@ mo_build_w_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er0, co
   u0 = block_xor(u0, sh);
   u2 = block_xor(u2, sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = u0; part[blockIdx.x * 2 + 1] = u2; }
+  publish_if_last(part, 2, pub, sh);
 }
 // The same weight under identity compaction with tall columns (col = d >> nu): in column c
 // the map x -> fold_slot(x ec_i[c], table_i) is GF(2)-linear, so the block builds its window
@@ -1344,7 +1365,7 @@ __global__ void __launch_bounds__(512, 1)
 mo_build_w_cols_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er0, const F128d* __restrict__ ec0,
                        const F128d* __restrict__ er1, const F128d* __restrict__ ec1, const F128d* __restrict__ tables,
                        uint32_t nu, uint32_t part_log, uint64_t area, uint64_t n, F128d* __restrict__ w,
-                       F128d* __restrict__ part) {
+                       F128d* __restrict__ part, FusedPublish pub) {
   extern __shared__ __align__(16) char wt[];  // the maps M0, then M1
   __shared__ F128d img[2][128];
   __shared__ F128d sh[32];
@@ -1381,12 +1402,13 @@ mo_build_w_cols_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er
   }
   const F128d r0 = block_xor(u0.value(), sh), r2 = block_xor(u2.value(), sh);
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = r0; part[blockIdx.x * 2 + 1] = r2; }
+  publish_if_last(part, 2, pub, sh);
 }
 // Columns of at least 2^MO_COLS_MIN_NU rows take the column-table form.
 constexpr uint32_t MO_COLS_MIN_NU = 14;
 uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, const F128d* er1, const F128d* ec1,
                            const F128d* tables, uint32_t nu, uint64_t area, uint64_t n, F128d* w, F128d* part,
-                           cudaStream_t s, const JaggedSegs* segs) {
+                           cudaStream_t s, FusedPublish pub, const JaggedSegs* segs) {
   if (!segs && nu >= MO_COLS_MIN_NU && (n >> nu) >= 1 && (n & ((1ull << nu) - 1)) == 0) {
     // work items of at least 2^13 rows, about eight per SM in all
     uint32_t part_log = 0;
@@ -1395,7 +1417,7 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
     const uint32_t blocks = (uint32_t)std::min<uint64_t>(items, (uint64_t)sm_count());
     const int smem = 2 * WinMap<5, 128>::BYTES;
     set_dynamic_smem((const void*)mo_build_w_cols_kernel, smem);
-    mo_build_w_cols_kernel<<<blocks, 512, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, part_log, area, n, w, part);
+    mo_build_w_cols_kernel<<<blocks, 512, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, part_log, area, n, w, part, pub);
     LAUNCH_OK();
     return blocks;
   }
@@ -1403,11 +1425,11 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
   uint32_t blocks = (uint32_t)std::min<uint64_t>((n / 2 + 511) / 512, (uint64_t)sm_count());
   if (segs) {
     set_dynamic_smem((const void*)mo_build_w_kernel<true>, (int)smem);
-    mo_build_w_kernel<true><<<blocks, 512, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, area, n, w, part, *segs);
+    mo_build_w_kernel<true><<<blocks, 512, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, area, n, w, part, *segs, pub);
   } else {
     set_dynamic_smem((const void*)mo_build_w_kernel<false>, (int)smem);
     mo_build_w_kernel<false><<<blocks, 512, smem, s>>>(q, er0, ec0, er1, ec1, tables, nu, area, n, w, part,
-                                                       JaggedSegs());
+                                                       JaggedSegs(), pub);
   }
   LAUNCH_OK();
   return blocks;
