@@ -101,13 +101,13 @@ static uint64_t live_words_of(const Statement& S) {
 }
 // Room for either form (a degenerate challenge takes the plain one), and for the reciprocal
 // weights beside the tables.
-static uint64_t zc_tables_room(const Statement& S) {
-  const uint32_t L = S.m - 7, w = zc_weighted_lo_bits(live_words_of(S));
+static uint64_t zc_tables_room(const Statement& S, uint64_t sms) {
+  const uint32_t L = S.m - 7, w = zc_weighted_lo_bits(live_words_of(S), sms);
   return std::max(zc_tables_entries(L, 0), w ? zc_tables_entries(L, w) + (uint64_t(1) << (L - w)) : 0);
 }
 
 // Device bytes a backend for this statement holds after its first prove (the buffers of
-// the constructor, the Ligerito level codewords and trees, the twiddle tables).
+// the constructor, the Ligerito level codewords and trees, the twiddle tables). Needs no device.
 uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   const uint64_t W = uint64_t(1) << (S.m - 7), K = uint64_t(1) << S.k_log, n_pos = uint64_t(1) << S.k_code;
   uint64_t b = 0;
@@ -116,7 +116,7 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   if (!S.identity) b += S.committed_words * 16;  // the compacted stack
   b += n_pos * S.lanes * 16 + 2 * n_pos * 32;  // L0 codeword and tree
   b += (W / 2 * 2 + W * 2 + 64) * 16;       // zerocheck folds
-  b += zc_tables_room(S) * 16;
+  b += zc_tables_room(S, GB300_SMS) * 16;
   b += 6 * K * 16;                          // lincheck vectors
   for (const SlotInfo& t : S.slots) {
     b += 2 * (uint64_t(16) << t.k_log);
@@ -125,7 +125,7 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   }
   b += (W + W + W / 2) * 16;                // merged weight and fold buffers
   const uint64_t D = uint64_t(1) << S.log_dim;
-  b += lane_fold_groups(S.lanes, D) * D * 32;  // Ligerito: lane fold partials,
+  b += lane_fold_groups(S.lanes, D, GB300_SMS) * D * 32;  // Ligerito: lane fold partials,
   b += 4 * 2 * D * 32 + 2 * D * 16;            // f/b ping-pong, pending
   b += (uint64_t(1) << 20) * 16 + (size_t(96) << 20) + (size_t(8) << 20);  // partials, scratch, staging
   b += n_pos * 16;                          // L0 twiddles
@@ -203,7 +203,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   moAw_ = dmalloc<F128d>(W / 2, owned_, device_bytes_);
   moBq_ = dmalloc<F128d>(W / 4, owned_, device_bytes_);
   moBw_ = dmalloc<F128d>(W / 4, owned_, device_bytes_);
-  lane_part_ = dmalloc<F256d>(lane_fold_groups(S.lanes, rows()) * rows(), owned_, device_bytes_);
+  lane_part_ = dmalloc<F256d>(lane_fold_groups(S.lanes, rows(), (uint64_t)sm_count()) * rows(), owned_, device_bytes_);
   for (int k = 0; k < 2; ++k) {
     lf_[k] = dmalloc<F256d>(2 * rows(), owned_, device_bytes_);
     lb_[k] = dmalloc<F256d>(2 * rows(), owned_, device_bytes_);
@@ -232,7 +232,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   *(volatile uint32_t*)h_flag_ = 0;
   pub_counter_ = dmalloc<uint32_t>(1, owned_, device_bytes_);
   CUDA_OK(cudaMemsetAsync(pub_counter_, 0, sizeof(uint32_t), st_));
-  zc_tabs_cap_ = zc_tables_room(S);
+  zc_tabs_cap_ = zc_tables_room(S, (uint64_t)sm_count());
   zc_tabs_ = dmalloc<F128d>(zc_tabs_cap_, owned_, device_bytes_);
   CUDA_OK(cudaStreamCreateWithFlags(&pow_st_, cudaStreamNonBlocking));
   d_pow_ = dmalloc<unsigned long long>(1, owned_, device_bytes_);
@@ -643,7 +643,7 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   const uint32_t L = (uint32_t)eq_point.size();  // m - 7
   if (L < 10) throw std::runtime_error("zerocheck skip fold needs m >= 17");
   // the weighted form divides by the high coordinates' eq once: none may be 0 or 1
-  zc_w_ = zc_weighted_lo_bits(zc_live_words_);
+  zc_w_ = zc_weighted_lo_bits(zc_live_words_, (uint64_t)sm_count());
   for (uint32_t j = zc_w_; zc_w_ && j < L; ++j)
     if (eq_point[j].is_zero() || eq_point[j] == F128::one()) zc_w_ = 0;
   // Every later fold round i uses eq over the suffix eq_point[1 + i ..]: build all the
@@ -1088,7 +1088,7 @@ Msg256 GpuBackend::lane_switch() {
   {
     Mark mk(this, ST_LIGERITO);
     launch_lg_lane_fold(q_, dw, S.lanes, rows(), lane_part_, st_);
-    launch_lg_lane_switch(lane_part_, lane_fold_groups(S.lanes, rows()), lt, rows(), lf_[0], lb_[0], part_, st_, fp);
+    launch_lg_lane_switch(lane_part_, lane_fold_groups(S.lanes, rows(), (uint64_t)sm_count()), lt, rows(), lf_[0], lb_[0], part_, st_, fp);
   }
   lane_ = LaneStage();
   lg_cur_ = 0;

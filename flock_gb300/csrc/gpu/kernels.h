@@ -35,6 +35,7 @@ void set_dynamic_smem(const void* kernel, int bytes);
   } while (0)
 
 int sm_count();
+constexpr uint64_t GB300_SMS = 152;  // for sizes computed without a device
 
 // In-kernel publication of a round message: the last block to finish (a device-wide
 // ticket counter) XOR-reduces every block's partials, writes the message to mapped host
@@ -96,7 +97,7 @@ uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d
 // The weighted form (see the kernels): low bits of its chunks for this many live words, 0 where
 // the plain form runs; the skip fold's message and the first fold with its message. eq_lo: eq
 // over the chunk's low coordinates (of words, then of pairs), h: eq over the high ones.
-uint32_t zc_weighted_lo_bits(uint64_t live_words);
+uint32_t zc_weighted_lo_bits(uint64_t live_words, uint64_t sms);
 uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
                                       uint32_t lo_bits, const F128d* eq_lo, const F128d* h, F128d* part,
                                       cudaStream_t s, FusedPublish pub);                                                   // width 2
@@ -173,7 +174,7 @@ void launch_as_build(const F128d* er0, const F128d* ec0, const F128d* er1, const
 // and the switched vectors with their message.
 uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, uint32_t lo_bits,
                              const F128d* eq_hi, F128d* part, cudaStream_t s);
-uint32_t lane_fold_groups(uint32_t lanes, uint64_t D);
+uint32_t lane_fold_groups(uint32_t lanes, uint64_t D, uint64_t sms);
 void launch_lg_lane_fold(const F128d* q, const F256d* lambda, uint32_t lanes, uint64_t D, F256d* part, cudaStream_t s);
 // b = sum of n terms coef eq(point), each point's eq as lo (lo_bits) x hi tables.
 struct LaneTerms {

@@ -655,8 +655,7 @@ zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restric
 // A chunk's tables are rebuilt for it (about 2000 cycles beside 13 a word), so chunks are as
 // long as leaves every SM four, down to 2^10 words with one an SM; smaller vectors take the
 // plain form, whose launches are bound by latency.
-uint32_t zc_weighted_lo_bits(uint64_t live_words) {
-  const uint64_t sms = (uint64_t)sm_count();
+uint32_t zc_weighted_lo_bits(uint64_t live_words, uint64_t sms) {
   if ((live_words >> 12) >= 4 * sms) return 12;
   if ((live_words >> 11) >= 4 * sms) return 11;
   return (live_words >> 10) >= sms ? 10 : 0;
@@ -1504,14 +1503,14 @@ lg_lane_fold_kernel(const F128d* __restrict__ q, const F256d* __restrict__ lambd
   }
 }
 // Lane groups: enough that the grid holds about eight blocks per SM (or a lane a group).
-uint32_t lane_fold_groups(uint32_t lanes, uint64_t D) {
-  const uint64_t rows = (D + LANE_FOLD_ROWS - 1) / LANE_FOLD_ROWS, want = (uint64_t)sm_count() * 8;
+uint32_t lane_fold_groups(uint32_t lanes, uint64_t D, uint64_t sms) {
+  const uint64_t rows = (D + LANE_FOLD_ROWS - 1) / LANE_FOLD_ROWS, want = sms * 8;
   return (uint32_t)std::min<uint64_t>(lanes, (want + rows - 1) / rows);
 }
 void launch_lg_lane_fold(const F128d* q, const F256d* lambda, uint32_t lanes, uint64_t D, F256d* part, cudaStream_t s) {
   const int smem = 2 * WinTable<5>::BYTES;
   set_dynamic_smem((const void*)lg_lane_fold_kernel, smem);
-  const dim3 grid((unsigned)((D + LANE_FOLD_ROWS - 1) / LANE_FOLD_ROWS), lane_fold_groups(lanes, D));
+  const dim3 grid((unsigned)((D + LANE_FOLD_ROWS - 1) / LANE_FOLD_ROWS), lane_fold_groups(lanes, D, (uint64_t)sm_count()));
   lg_lane_fold_kernel<<<grid, LANE_FOLD_THREADS, smem, s>>>(q, lambda, lanes, D, part);
   LAUNCH_OK();
 }
