@@ -400,10 +400,9 @@ void GpuBackend::sync() {
 }
 std::vector<F128> GpuBackend::reduce(uint32_t n_blocks, uint32_t width) {
   if ((uint64_t)n_blocks * width > part_cap_ || width > PUB_WORDS) throw std::runtime_error("partials buffer too small");
-  // one block reduces and publishes into mapped host memory
-  uint32_t seq = ++seq_;
-  launch_reduce_publish(part_, n_blocks, width, d_pub_, d_flag_, seq, st_);
-  return read_published(seq, width);
+  const FusedPublish fp = fused_publish();
+  launch_reduce_pair(part_, n_blocks, width, nullptr, 0, 0, st_, fp);
+  return read_published(fp.seq, width);
 }
 std::vector<F128> GpuBackend::read_published(uint32_t seq, uint32_t width) {
   wait_published(seq);

@@ -51,7 +51,7 @@ void launch_eq_split(const F128d* d_point, uint32_t lo_bits, uint32_t hi_bits, F
 }
 
 // XOR of the rows of two partial arrays (na rows of width wa, nb of width wb), published side by
-// side; one block a value.
+// side; one block a value (46 values of 360 rows by one block, which this replaced: 30 us).
 __global__ void __launch_bounds__(128)
 reduce_pair_kernel(const F128d* __restrict__ pa, uint32_t na, uint32_t wa, const F128d* __restrict__ pb, uint32_t nb,
                    uint32_t wb, FusedPublish pub) {
