@@ -181,6 +181,10 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
     k_max = std::max(k_max, sd.K);
     sd.ca = dmalloc<F128d>(sd.K, owned_, device_bytes_);
     sd.cb = dmalloc<F128d>(sd.K, owned_, device_bytes_);
+    if (t.hash == HASH_KECCAK) {  // the walker writes the constrained columns only
+      CUDA_OK(cudaMemsetAsync(sd.ca, 0, sd.K * 16, st_));
+      CUDA_OK(cudaMemsetAsync(sd.cb, 0, sd.K * 16, st_));
+    }
     if (t.hash != HASH_KECCAK) {
       for (auto [csc, d] : {std::make_pair(t.csc_a, &sd.a), std::make_pair(t.csc_b, &sd.b)}) {
         uint32_t* ptr = dmalloc<uint32_t>(csc->col_ptr.size(), owned_, device_bytes_);
@@ -796,8 +800,6 @@ void GpuBackend::lc_fold_slot(HashKind hash, const SlotDev& sd) {
         for (int b = 0; b < 5; ++b) c.rho[a + 5 * b] = (uint8_t)(kr1cs::RHO[a][b] % 64);
       return c;
     }();
-    CUDA_OK(cudaMemsetAsync(sd.ca, 0, sd.K * 16, st_));
-    CUDA_OK(cudaMemsetAsync(sd.cb, 0, sd.K * 16, st_));
     launch_keccak_lincheck_columns(eqi_, sd.ca, sd.cb, kc, st_);
     return;
   }

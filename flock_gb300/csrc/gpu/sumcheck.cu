@@ -554,13 +554,13 @@ zc_fold_skip_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, co
     T[c][v] = acc;
   }
   __syncthreads();
+  // a piece of a chunk at a time, one word a thread: the vectors that come here are short
   const uint64_t chunk = 1ull << lo_bits;
-  const uint64_t n_chunks = (n_words + chunk - 1) / chunk;
   F128d G1 = f128_zero(), GI = f128_zero();
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
+  for (uint64_t w0 = (uint64_t)blockIdx.x * blockDim.x; w0 < n_words; w0 += (uint64_t)gridDim.x * blockDim.x) {
     F128d g1 = f128_zero(), gi = f128_zero();
-    uint64_t end = min(n_words, (ch + 1) * chunk);
-    for (uint64_t wi = ch * chunk + threadIdx.x; wi < end; wi += blockDim.x) {
+    const uint64_t wi = w0 + threadIdx.x;
+    if (wi < n_words) {
       F128d av = a[wi], bv = b[wi];
       F128d a0 = f128_zero(), a1 = f128_zero(), b0 = f128_zero(), b1 = f128_zero();
 #pragma unroll
@@ -571,13 +571,13 @@ zc_fold_skip_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, co
         b1 += T[c][(bv.hi >> (8 * c)) & 255];
       }
       F128d e = eq_lo[wi & (chunk - 1)];
-      g1 += mul_call(e, mul_call(a1, b1));
-      gi += mul_call(e, mul_call(a0 + a1, b0 + b1));
+      g1 = mul_call(e, mul_call(a1, b1));
+      gi = mul_call(e, mul_call(a0 + a1, b0 + b1));
     }
     g1 = block_xor(g1, sh);
     gi = block_xor(gi, sh);
     if (threadIdx.x == 0) {
-      F128d h = eq_hi ? eq_hi[ch] : f128_one();
+      F128d h = eq_hi ? eq_hi[w0 >> lo_bits] : f128_one();
       G1 += h * g1;
       GI += h * gi;
     }
@@ -680,8 +680,7 @@ uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128
 }
 uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words, const F128d* eq_lo,
                              uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s, FusedPublish pub) {
-  uint64_t n_chunks = (n_words + (1ull << lo_bits) - 1) >> lo_bits;
-  uint32_t blocks = (uint32_t)std::min<uint64_t>(n_chunks, (uint64_t)sm_count() * 8);
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>((n_words + 255) / 256, (uint64_t)sm_count() * 8);
   zc_fold_skip_kernel<<<blocks, 256, 0, s>>>(a, b, w64, n_words, eq_lo, lo_bits, eq_hi, part, pub);
   LAUNCH_OK();
   return blocks;
@@ -1096,73 +1095,78 @@ void launch_csc_fold(const CscDev& A, const CscDev& B, uint32_t K, const F128d* 
 // phi^T = theta^T o (pi o rho)^T:
 //   (pi o rho)^T: out[a,b,c] = in[b, 2(a-b) mod 5, c + rho(a,b)]
 //   theta^T: out[x,y,z] = in[x,y,z] + sum_y' in[x+1,y',z] + sum_y' in[x-1,y',z+1].
-// One block per side; the 1600-word vectors live in shared memory.
-constexpr uint32_t KW_THREADS = 512;
-constexpr uint32_t KW_STATE = 1600;
+// One block per side, two state words a thread: a thread's lambda stays in its registers, mu goes
+// through shared memory (two buffers, so a round has two barriers), every index is formed once and
+// the next round's eq weights are on their way while this one is folded. Bound by those 24
+// dependent rounds; recomputed indices, four barriers and the loads' latency in each
+// made it 131 us a proof.
+constexpr uint32_t KW_THREADS = 800, KW_PER = 2;
+constexpr uint32_t KW_STATE = KW_THREADS * KW_PER;
 constexpr uint32_t KW_S24_WORD = 2048 / 64, KW_T_WORD = 4160 / 64, KW_Z = 4096;
 __device__ __forceinline__ uint32_t kw_pos(uint32_t base_word, uint32_t s) { return (base_word + s % 25) * 64 + s / 25; }
 
 __global__ void __launch_bounds__(KW_THREADS)
 keccak_lincheck_columns_kernel(const F128d* __restrict__ eqi, F128d* __restrict__ ca, F128d* __restrict__ cb,
                                KeccakColumnConsts kc) {
-  extern __shared__ F128d kw_sh[];
-  F128d* lam = kw_sh;                // lambda, then mu in place
-  F128d* P = lam + KW_STATE;         // (pi o rho)^T mu
-  F128d* C = P + KW_STATE;           // column sums of P: C[x + 5 z]
+  extern __shared__ F128d kw_sh[];     // mu of the even, then of the odd rounds
+  __shared__ F128d C[320];             // column sums of P = (pi o rho)^T mu: C[x + 5 z]
   __shared__ F128d red[KW_THREADS / 32];
   const bool bside = blockIdx.x == 1;
   F128d* out = bside ? cb : ca;
   const uint32_t shift = bside ? 2 : 1, tid = threadIdx.x;
   F128d zacc = f128_zero();  // this thread's share of column Z beyond eq[Z]
-  for (uint32_t s = tid; s < KW_STATE; s += KW_THREADS) {
-    const F128d e = eqi[kw_pos(KW_S24_WORD, s)];
-    if (bside) { lam[s] = f128_zero(); zacc += e; }
-    else lam[s] = e;
+  auto source = [&](uint32_t o) {  // P[o] = mu[source(o)]
+    const uint32_t a = o % 5, b = (o / 5) % 5, c = o / 25, y = (2 * (a + 5 - b)) % 5;
+    return b + 5 * y + 25 * ((c + kc.rho[a + 5 * b]) & 63);
+  };
+  F128d lam[KW_PER], e[KW_PER];
+  uint32_t own[KW_PER], eqo[KW_PER], src[KW_PER], c1[KW_PER], c2[KW_PER], col[5] = {};
+#pragma unroll
+  for (uint32_t k = 0; k < KW_PER; ++k) {
+    const uint32_t s = tid + k * KW_THREADS, x = s % 5, z = s / 25;
+    own[k] = kw_pos(KW_T_WORD, s);                              // columns of t_r: + 1600 r
+    eqo[k] = kw_pos(KW_T_WORD, s - x + (x + 5 - shift) % 5);
+    src[k] = source(s);
+    c1[k] = (x + 1) % 5 + 5 * z;
+    c2[k] = (x + 4) % 5 + 5 * ((z + 1) & 63);
+    const F128d v = eqi[kw_pos(KW_S24_WORD, s)];
+    lam[k] = bside ? f128_zero() : v;
+    if (bside) zacc += v;
+    e[k] = eqi[eqo[k] + 1600 * 23];
   }
-  __syncthreads();
+  if (tid < 320)
+#pragma unroll
+    for (uint32_t y = 0; y < 5; ++y) col[y] = source(tid % 5 + 5 * y + 25 * (tid / 5));
   for (int r = 23; r >= 0; --r) {
-    const uint32_t tb = KW_T_WORD + 25u * r;
-    for (uint32_t s = tid; s < KW_STATE; s += KW_THREADS) {
-      const F128d l = lam[s];
-      out[kw_pos(tb, s)] = l;
-      if (s % 25 == 0 && ((kc.rc[r] >> (s / 25)) & 1)) zacc += l;
-      const uint32_t x = s % 5;
-      const F128d e = eqi[kw_pos(tb, s - x + (x + 5 - shift) % 5)];
-      if (!bside) zacc += e;
-      lam[s] = l + e;
+    F128d* mu = kw_sh + (r & 1) * KW_STATE;
+#pragma unroll
+    for (uint32_t k = 0; k < KW_PER; ++k) {
+      const uint32_t s = tid + k * KW_THREADS;
+      out[own[k] + 1600 * r] = lam[k];
+      if (s % 25 == 0 && ((kc.rc[r] >> (s / 25)) & 1)) zacc += lam[k];
+      if (!bside) zacc += e[k];
+      mu[s] = lam[k] + e[k];
+      if (r) e[k] = eqi[eqo[k] + 1600 * (r - 1)];
     }
     __syncthreads();
-    for (uint32_t o = tid; o < KW_STATE; o += KW_THREADS) {
-      const uint32_t a = o % 5, b = (o / 5) % 5, c = o / 25;
-      const uint32_t y = (2 * (a + 5 - b)) % 5;
-      P[o] = lam[b + 5 * y + 25 * ((c + kc.rho[a + 5 * b]) & 63)];
-    }
+    if (tid < 320) C[tid] = mu[col[0]] + mu[col[1]] + mu[col[2]] + mu[col[3]] + mu[col[4]];
     __syncthreads();
-    for (uint32_t q = tid; q < 320; q += KW_THREADS) {
-      const uint32_t x = q % 5, z = q / 5;
-      F128d acc = f128_zero();
-      for (uint32_t y = 0; y < 5; ++y) acc += P[x + 5 * y + 25 * z];
-      C[q] = acc;
-    }
-    __syncthreads();
-    for (uint32_t s = tid; s < KW_STATE; s += KW_THREADS) {
-      const uint32_t x = s % 5, z = s / 25;
-      lam[s] = P[s] + C[(x + 1) % 5 + 5 * z] + C[(x + 4) % 5 + 5 * ((z + 1) & 63)];
-    }
-    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < KW_PER; ++k) lam[k] = mu[src[k]] + C[c1[k]] + C[c2[k]];
   }
-  for (uint32_t s = tid; s < KW_STATE; s += KW_THREADS) {
-    const uint32_t p = kw_pos(0, s);
-    const F128d e = eqi[p];
-    if (bside) { out[p] = lam[s]; zacc += e; }
-    else out[p] = lam[s] + e;
+#pragma unroll
+  for (uint32_t k = 0; k < KW_PER; ++k) {
+    const uint32_t p = kw_pos(0, tid + k * KW_THREADS);
+    const F128d v = eqi[p];
+    if (bside) zacc += v;
+    out[p] = bside ? lam[k] : lam[k] + v;
   }
   const F128d tot = block_xor(zacc, red);
   if (tid == 0) out[KW_Z] = eqi[KW_Z] + tot;
 }
 void launch_keccak_lincheck_columns(const F128d* eqi, F128d* ca, F128d* cb, const KeccakColumnConsts& kc,
                                     cudaStream_t s) {
-  const int smem = (int)((2 * KW_STATE + 320) * sizeof(F128d));
+  const int smem = (int)(2 * KW_STATE * sizeof(F128d));
   set_dynamic_smem((const void*)keccak_lincheck_columns_kernel, smem);
   keccak_lincheck_columns_kernel<<<2, KW_THREADS, smem, s>>>(eqi, ca, cb, kc);
   LAUNCH_OK();
@@ -1403,15 +1407,27 @@ mo_build_w_cols_kernel(const F128d* __restrict__ q, const F128d* __restrict__ er
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = r0; part[blockIdx.x * 2 + 1] = r2; }
   publish_if_last(part, 2, pub, sh);
 }
-// Columns of at least 2^MO_COLS_MIN_NU rows take the column-table form.
-constexpr uint32_t MO_COLS_MIN_NU = 14;
+// Columns of at least 2^MO_COLS_MIN_NU rows take the column-table form (stage times with and
+// without it, BLAKE3 2^11: 65 and 74 us, SHA-256 2^11: 83 and 85, 2^13: 141 and 183).
+constexpr uint32_t MO_COLS_MIN_NU = 11;
+// A work item's tables cost about as much as 2^10 rows: the split of the columns into 2^part_log
+// items each that gives the last block to finish the least to do (SHA-256 2^14 in items of 2^14,
+// 2^13 and 2^12 rows: 236, 209 and 230 us).
+static uint32_t mo_part_log(uint32_t nu, uint64_t area) {
+  uint32_t best = 0;
+  uint64_t least = ~0ull;
+  for (uint32_t p = 0; nu - p >= 11; ++p) {
+    const uint64_t rows = 1ull << (nu - p), items = (area + rows - 1) / rows, sms = (uint64_t)sm_count();
+    const uint64_t cost = (items + sms - 1) / sms * (rows + 1024);
+    if (cost < least) { least = cost; best = p; }
+  }
+  return best;
+}
 uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, const F128d* er1, const F128d* ec1,
                            const F128d* tables, uint32_t nu, uint64_t area, uint64_t n, F128d* w, F128d* part,
                            cudaStream_t s, FusedPublish pub, const JaggedSegs* segs) {
   if (!segs && nu >= MO_COLS_MIN_NU && (n >> nu) >= 1 && (n & ((1ull << nu) - 1)) == 0) {
-    // work items of at least 2^13 rows, about eight per SM in all
-    uint32_t part_log = 0;
-    while (nu - part_log > 13 && ((n >> nu) << part_log) < (uint64_t)sm_count() * 8) ++part_log;
+    const uint32_t part_log = mo_part_log(nu, area);
     const uint64_t items = (n >> nu) << part_log;
     const uint32_t blocks = (uint32_t)std::min<uint64_t>(items, (uint64_t)sm_count());
     const int smem = 2 * WinMap<5, 128>::BYTES;
@@ -1763,6 +1779,7 @@ __global__ void lg_lane_switch_kernel(const F256d* __restrict__ fpart, uint32_t 
   F128d u00 = f128_zero(), u01 = f128_zero(), u20 = f128_zero(), u21 = f128_zero();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (uint64_t)gridDim.x * blockDim.x) {
     F256d fv = fpart[i], bv = f256(f128_zero(), f128_zero());
+#pragma unroll 8
     for (uint32_t g = 1; g < groups; ++g) fv += fpart[g * D + i];
     for (uint32_t t = 0; t < terms.n; ++t) {
       const F128d e = mul_call(terms.lo[t][i & ((1ull << terms.lo_bits) - 1)], terms.hi[t][i >> terms.lo_bits]);
