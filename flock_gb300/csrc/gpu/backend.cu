@@ -453,6 +453,29 @@ GpuBackend::EqSplit GpuBackend::eq_split(const std::vector<F128>& point, F128 sc
   return e;
 }
 
+// The eq tables over the coordinates [first, second) of args, in one launch; args (with anything else
+// that the next kernel reads) travels in one copy, to the address returned.
+const F128d* GpuBackend::eq_tables(std::vector<F128> args, const std::vector<std::pair<size_t, size_t>>& of,
+                                   std::vector<F128d*>& out) {
+  std::vector<EqDesc> desc(of.size());
+  uint64_t total = 0;
+  for (size_t k = 0; k < of.size(); ++k) {
+    desc[k].p_off = (uint32_t)of[k].first;
+    desc[k].n = (uint32_t)(of[k].second - of[k].first);
+    desc[k].out_off = total;
+    total += uint64_t(1) << desc[k].n;
+  }
+  F128d* tabs = static_cast<F128d*>(scratch(total * sizeof(F128d)));
+  for (const EqDesc& d : desc) out.push_back(tabs + d.out_off);
+  static_assert(sizeof(EqDesc) == sizeof(F128), "a descriptor takes the place of a word");
+  const size_t words = args.size();
+  args.resize(words + desc.size());
+  memcpy(static_cast<void*>(args.data() + words), desc.data(), desc.size() * sizeof(EqDesc));
+  const F128d* d = upload(args);
+  launch_eq_tables(d, reinterpret_cast<const EqDesc*>(d + words), desc.data(), (uint32_t)desc.size(), tabs, st_);
+  return d;
+}
+
 // ------------------------------------------------------------------ witness + commit
 void GpuBackend::witness(const std::vector<const uint8_t*>& slot_inputs) {
   scr_off_ = 0;
@@ -903,25 +926,18 @@ void GpuBackend::lc_s_hat_v(const std::vector<F128>& tail, std::vector<F128>& ou
 // ------------------------------------------------------------------ merged open
 void GpuBackend::launch_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area, const FusedPublish& fp) {
   if (cl.size() != 2) throw std::runtime_error("merged open expects the AB and C claims");
-  // both claims' points (z_row | z_col) and byte tables in one copy; the row and column tables of
-  // a claim in one launch
+  // both claims' byte tables, then their points z_row and z_col
   std::vector<F128> args;
+  std::vector<std::pair<size_t, size_t>> of;
   for (int i = 0; i < 2; ++i) args.insert(args.end(), cl[i].table.begin(), cl[i].table.end());
-  for (int i = 0; i < 2; ++i) {
-    args.insert(args.end(), cl[i].z_row.begin(), cl[i].z_row.end());
-    args.insert(args.end(), cl[i].z_col.begin(), cl[i].z_col.end());
-  }
-  const F128d* dt = upload(args);
-  const F128d* point = dt + cl[0].table.size() + cl[1].table.size();
-  F128d* er[2];
-  F128d* ec[2];
-  for (int i = 0; i < 2; ++i) {
-    er[i] = static_cast<F128d*>(scratch(size_t(16) << cl[i].z_row.size()));
-    ec[i] = static_cast<F128d*>(scratch(size_t(16) << cl[i].z_col.size()));
-    launch_eq_split(point, (uint32_t)cl[i].z_row.size(), (uint32_t)cl[i].z_col.size(), dev(F128::one()), er[i], ec[i],
-                    st_);
-    point += cl[i].z_row.size() + cl[i].z_col.size();
-  }
+  for (int i = 0; i < 2; ++i)
+    for (const std::vector<F128>* p : {&cl[i].z_row, &cl[i].z_col}) {
+      of.emplace_back(args.size(), args.size() + p->size());
+      args.insert(args.end(), p->begin(), p->end());
+    }
+  std::vector<F128d*> eq;
+  const F128d* dt = eq_tables(std::move(args), of, eq);
+  F128d *er[2] = {eq[0], eq[2]}, *ec[2] = {eq[1], eq[3]};
   if (S.slots.size() == 1 && S.identity) {
     launch_mo_build_w(q_, er[0], ec[0], er[1], ec[1], dt, nu, area, Q_, mw_, part_, st_, fp);
     return;
@@ -1077,14 +1093,27 @@ Msg256 GpuBackend::lane_switch() {
   scr_off_ = 0;
   LaneTerms lt;
   lt.n = (uint32_t)lane_.terms.size();
+  lt.lo_bits = std::min(S.log_dim, 10u);
+  // lambda, then the terms' row points; both factors of every term's eq in one launch
+  std::vector<F128> args;
+  std::vector<std::pair<size_t, size_t>> of;
+  for (const F256& w : lane_.w) {
+    args.push_back(w.c0);
+    args.push_back(w.c1);
+  }
   for (uint32_t t = 0; t < lt.n; ++t) {
-    EqSplit e = eq_split(lane_.terms[t].row_point, F128::one(), 10);
-    lt.lo[t] = e.lo;
-    lt.hi[t] = e.hi;
-    lt.lo_bits = e.lo_bits;
+    const std::vector<F128>& p = lane_.terms[t].row_point;
+    of.emplace_back(args.size(), args.size() + lt.lo_bits);
+    of.emplace_back(args.size() + lt.lo_bits, args.size() + p.size());
+    args.insert(args.end(), p.begin(), p.end());
     lt.coef[t] = dev(lane_.terms[t].e[0] * lane_.terms[t].coef);
   }
-  const F256d* dw = static_cast<const F256d*>(upload(lane_.w.data(), lane_.w.size() * sizeof(F256)));
+  std::vector<F128d*> eq;
+  const F256d* dw = reinterpret_cast<const F256d*>(eq_tables(std::move(args), of, eq));
+  for (uint32_t t = 0; t < lt.n; ++t) {
+    lt.lo[t] = eq[2 * t];
+    lt.hi[t] = eq[2 * t + 1];
+  }
   FusedPublish fp = fused_publish();
   {
     Mark mk(this, ST_LIGERITO);
@@ -1268,16 +1297,28 @@ Msg256 GpuBackend::lg_introduce_eq(const std::vector<F128>& zp, F128& answer) {
   lg_flush_fold();
   scr_off_ = 0;
   if ((uint64_t(1) << zp.size()) != lg_n_) throw std::runtime_error("OOD point size mismatch");
-  EqSplit e = eq_split(zp, F128::one(), 10);
-  FusedPublish fp = fused_publish();
-  { Mark mk(this, ST_LIGERITO); launch_lg_intro_eq(lf_[lg_cur_], e.lo, e.lo_bits, e.hi, lg_n_, pend_, part_, st_, fp); }
-  auto v = read_published(fp.seq, 3);
-  answer = v[0];
+  if (zp.empty()) throw std::runtime_error("OOD point of no coordinates");
+  const std::vector<F128> rest(zp.begin() + 1, zp.end());
+  const uint64_t pairs = lg_n_ / 2;
+  const FusedPublish fp = fused_publish();
+  if (lg_intro_eq_direct(pairs)) {
+    const F128d* dp = upload(rest);
+    Mark mk(this, ST_LIGERITO);
+    launch_lg_intro_eq(lf_[lg_cur_], dp, (uint32_t)rest.size(), pairs, pend_, part_, st_, fp);
+  } else {
+    EqSplit e = eq_split(rest, F128::one(), 10);
+    Mark mk(this, ST_LIGERITO);
+    launch_lg_intro_eq(lf_[lg_cur_], e.lo, e.lo_bits, e.hi, pairs, pend_, part_, st_, fp);
+  }
+  auto v = read_published(fp.seq, 2);
   pend_induced_ = false;
-  pend_n_ = lg_n_;
+  pend_n_ = pairs;
+  pend_z_ = zp[0];
   Msg256 m;
-  m.u0 = F256(v[1]);
-  m.u2 = F256(v[2]);
+  const F128 even = (F128::one() + pend_z_) * v[0];
+  answer = even + pend_z_ * v[1];
+  m.u0 = F256(even);
+  m.u2 = F256(v[0] + v[1]);
   return m;
 }
 
@@ -1327,7 +1368,8 @@ Msg256 GpuBackend::lg_introduce_induced(uint32_t ln, uint32_t log_rate, const st
 void GpuBackend::lg_glue(F128 beta) {
   lg_flush_fold();
   Mark mk(this, ST_LIGERITO);
-  launch_lg_glue(lb_[lg_cur_], pend_, dev(beta), pend_n_, pend_induced_, st_);
+  const F128 odd = beta * pend_z_;
+  launch_lg_glue(lb_[lg_cur_], pend_, dev(pend_induced_ ? beta : beta + odd), dev(odd), pend_n_, pend_induced_, st_);
 }
 
 void GpuBackend::lg_open(uint32_t level, const std::vector<uint64_t>& pos, uint32_t cap_depth,

@@ -104,6 +104,8 @@ class GpuBackend : public ProverBackend {
   std::vector<F128> reduce(uint32_t n_blocks, uint32_t width);
   void upload_to(void* dst, const void* src, size_t bytes);
   EqSplit eq_split(const std::vector<F128>& point, F128 scale, uint32_t max_lo);
+  const F128d* eq_tables(std::vector<F128> args, const std::vector<std::pair<size_t, size_t>>& of,
+                         std::vector<F128d*>& out);
   // build the merged-open weight and launch its round-0 reduction (per-block partials)
   void launch_build_w(const std::vector<WeightClaim>& cl, uint32_t nu, uint64_t area, const FusedPublish& fp);
   const F128d* twiddles(uint32_t log_d);
@@ -239,6 +241,7 @@ class GpuBackend : public ProverBackend {
   uint64_t lg_n_ = 0;
   F128d* pend_ = nullptr;
   bool pend_induced_ = false;
+  F128 pend_z_;  // an eq basis is stored without its first coordinate
   uint64_t pend_n_ = 0;
   std::vector<Level> levels_;
   std::unique_ptr<JaggedAssist> jagged_;

@@ -197,16 +197,20 @@ void launch_lg_code_switch(const F256d* f, const F256d* b, uint64_t n, F256d* fo
 uint32_t launch_lg_switch_msg(const F256d* f, const F256d* b, uint64_t n, F256d* fo, F256d* bo, F128d* part, cudaStream_t s,
                               FusedPublish pub);
 void launch_lg_replicate(const F256d* f, uint64_t msg, uint64_t total, F128d* mat, cudaStream_t s);
-uint32_t launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n,
-                            F128d* pend, F128d* part, cudaStream_t s,
-                            FusedPublish pub = FusedPublish());  // width 3
+// The pending eq basis as t over z[1 ..] (n_vars coordinates at `point`, or its two tables), the sums
+// of f's even and odd entries with it published; the first form where lg_intro_eq_direct says so.
+bool lg_intro_eq_direct(uint64_t pairs);
+void launch_lg_intro_eq(const F256d* f, const F128d* point, uint32_t n_vars, uint64_t pairs, F128d* pend, F128d* part,
+                        cudaStream_t s, FusedPublish pub);
+void launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t pairs,
+                        F128d* pend, F128d* part, cudaStream_t s, FusedPublish pub);  // width 3
 // pos and w in order of pos >> lg_sparse_layers(...), start[g] the first query of group g (one
 // value of that; start[n_groups] = n_q); without sparse layers start is not read.
 uint32_t lg_sparse_layers(uint32_t log_d, uint32_t log_rate);
 uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, const uint32_t* start, uint32_t n_groups,
                            uint32_t ln, uint32_t log_rate, const F128d* tw, const F256d* f, F128d* y, F128d* basis,
                            F128d* part, cudaStream_t s, FusedPublish pub);  // width 2
-void launch_lg_glue(F256d* b, const F128d* p, F128d beta, uint64_t n, bool induced, cudaStream_t s);
+void launch_lg_glue(F256d* b, const F128d* p, F128d w0, F128d w1, uint64_t n, bool induced, cudaStream_t s);
 
 // rounds.cu
 // XOR-reduce width-wide partials with one block and publish the sums to mapped host

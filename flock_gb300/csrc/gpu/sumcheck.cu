@@ -1776,14 +1776,24 @@ __global__ void lg_lane_switch_kernel(const F256d* __restrict__ fpart, uint32_t 
                                       F256d* __restrict__ fo, F256d* __restrict__ bo, F128d* __restrict__ part,
                                       FusedPublish pub) {
   __shared__ F128d sh[32];
+  __shared__ F128d scale[2 * LaneTerms::MAX];  // coef_t hi_t of these 256 rows (one entry of hi covers them)
   F128d u00 = f128_zero(), u01 = f128_zero(), u20 = f128_zero(), u21 = f128_zero();
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (uint64_t)gridDim.x * blockDim.x) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < D; i0 += step) {
+    __syncthreads();  // the previous rows' factors are no longer read
+    if (threadIdx.x < 2 * terms.n) {
+      const uint32_t t = threadIdx.x >> 1;
+      scale[threadIdx.x] = mul_call(threadIdx.x & 1 ? terms.coef[t].c1 : terms.coef[t].c0, terms.hi[t][i0 >> terms.lo_bits]);
+    }
+    __syncthreads();
+    const uint64_t i = i0 + threadIdx.x;
+    if (i >= D) continue;
     F256d fv = fpart[i], bv = f256(f128_zero(), f128_zero());
 #pragma unroll 8
     for (uint32_t g = 1; g < groups; ++g) fv += fpart[g * D + i];
     for (uint32_t t = 0; t < terms.n; ++t) {
-      const F128d e = mul_call(terms.lo[t][i & ((1ull << terms.lo_bits) - 1)], terms.hi[t][i >> terms.lo_bits]);
-      bv += f256(mul_call(terms.coef[t].c0, e), mul_call(terms.coef[t].c1, e));
+      const F128d e = terms.lo[t][i & ((1ull << terms.lo_bits) - 1)];
+      bv += f256(mul_call(scale[2 * t], e), mul_call(scale[2 * t + 1], e));
     }
     switch_pair(fv, bv, i, fo, bo, u00, u01, u20, u21);
   }
@@ -1805,35 +1815,53 @@ void launch_lg_replicate(const F256d* f, uint64_t msg, uint64_t total, F128d* ma
   lg_replicate_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(f, msg, total, mat);
   LAUNCH_OK();
 }
-// Pending eq basis e = eq(z) over the (base-valued) f of length n: stores e, returns per
-// block (answer = sum f e, u0 = sum f[2j] e[2j], u2 = sum (f0 + f1)(e0 + e1)).
-__global__ void lg_intro_eq_kernel(const F256d* __restrict__ f, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
-                                   const F128d* __restrict__ eq_hi, uint64_t n, F128d* __restrict__ pend,
-                                   F128d* __restrict__ part, FusedPublish pub) {
+// Pending eq basis e = eq(z) over the (base-valued) f of length 2 pairs: with t(j) the eq over
+// z[1 ..], e[2j] = (1 + z_0) t(j) and e[2j + 1] = z_0 t(j), so the basis is stored as t and the
+// message comes from S0 = sum f[2j] t(j), S1 = sum f[2j + 1] t(j), published: three products a
+// pair (five with e itself). Up to a size (below) the block forms t's two factors itself, lo of
+// eight coordinates an entry a thread, hi for its 256 pairs, and no table launch precedes it.
+template <bool TABLES>
+__global__ void __launch_bounds__(EQ_THREADS)
+lg_intro_eq_kernel(const F256d* __restrict__ f, const F128d* __restrict__ point, uint32_t n_vars,
+                   const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi, uint64_t pairs,
+                   F128d* __restrict__ pend, F128d* __restrict__ part, FusedPublish pub) {
   __shared__ F128d sh[32];
-  F128d ans = f128_zero(), u0 = f128_zero(), u2 = f128_zero();
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n / 2; j += (uint64_t)gridDim.x * blockDim.x) {
-    F128d e0 = eq_at(eq_lo, lo_bits, eq_hi, 2 * j), e1 = eq_at(eq_lo, lo_bits, eq_hi, 2 * j + 1);
-    pend[2 * j] = e0;
-    pend[2 * j + 1] = e1;
-    F128d f0 = f[2 * j].c0, f1 = f[2 * j + 1].c0;
-    F128d p0 = f0 * e0;
-    ans += p0 + f1 * e1;
-    u0 += p0;
-    u2 += (f0 + f1) * (e0 + e1);
+  __shared__ F128d sub[TABLES ? 1 : 2][EQ_MAX_GROUPS][16];
+  F128d s0 = f128_zero(), s1 = f128_zero(), lo = f128_one();
+  const uint32_t lo_n = min(n_vars, 8u), hi_n = n_vars - lo_n;
+  if (!TABLES) {
+    eq_sub_tables(point, lo_n, sub[0]);
+    eq_sub_tables(point + lo_n, hi_n, sub[TABLES ? 0 : 1]);
+    __syncthreads();
+    lo = eq_from_sub(sub[0], lo_n, threadIdx.x & ((1u << lo_n) - 1));
   }
-  ans = block_xor(ans, sh);
-  u0 = block_xor(u0, sh);
-  u2 = block_xor(u2, sh);
-  if (threadIdx.x == 0) { part[blockIdx.x * 3] = ans; part[blockIdx.x * 3 + 1] = u0; part[blockIdx.x * 3 + 2] = u2; }
-  if (pub.out) publish_if_last(part, 3, pub, sh);
+  for (uint64_t j = (uint64_t)blockIdx.x * EQ_THREADS + threadIdx.x; j < pairs; j += (uint64_t)gridDim.x * EQ_THREADS) {
+    F128d t;
+    if (TABLES) t = eq_at(eq_lo, lo_bits, eq_hi, j);
+    else t = hi_n ? mul_call(lo, eq_from_sub(sub[TABLES ? 0 : 1], hi_n, j >> 8)) : lo;
+    pend[j] = t;
+    s0 += mul_call(f[2 * j].c0, t);
+    s1 += mul_call(f[2 * j + 1].c0, t);
+  }
+  s0 = block_xor(s0, sh);
+  s1 = block_xor(s1, sh);
+  if (threadIdx.x == 0) { part[blockIdx.x * 2] = s0; part[blockIdx.x * 2 + 1] = s1; }
+  publish_if_last(part, 2, pub, sh);
 }
-uint32_t launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t n,
-                            F128d* pend, F128d* part, cudaStream_t s, FusedPublish pub) {
-  uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n / 2 + 255) / 256, (uint64_t)sm_count() * 8));
-  lg_intro_eq_kernel<<<blocks, 256, 0, s>>>(f, eq_lo, lo_bits, eq_hi, n, pend, part, pub);
+// One pair a thread of at most four blocks of 256 on each SM.
+bool lg_intro_eq_direct(uint64_t pairs) { return pairs <= (uint64_t)sm_count() * 4 * EQ_THREADS; }
+void launch_lg_intro_eq(const F256d* f, const F128d* point, uint32_t n_vars, uint64_t pairs, F128d* pend, F128d* part,
+                        cudaStream_t s, FusedPublish pub) {
+  const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, (pairs + EQ_THREADS - 1) / EQ_THREADS);
+  lg_intro_eq_kernel<false><<<blocks, EQ_THREADS, 0, s>>>(f, point, n_vars, nullptr, 0, nullptr, pairs, pend, part, pub);
   LAUNCH_OK();
-  return blocks;
+}
+void launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t pairs,
+                        F128d* pend, F128d* part, cudaStream_t s, FusedPublish pub) {
+  const uint32_t blocks =
+      (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((pairs + EQ_THREADS - 1) / EQ_THREADS, (uint64_t)sm_count() * 8));
+  lg_intro_eq_kernel<true><<<blocks, EQ_THREADS, 0, s>>>(f, nullptr, 0, eq_lo, lo_bits, eq_hi, pairs, pend, part, pub);
+  LAUNCH_OK();
 }
 // Induced basis of the queried positions. The level's codeword is the NTT (layers
 // [log_rate, log_d)) of the message replicated 2^log_rate times, so for weights w_q at
@@ -2007,23 +2035,20 @@ uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, co
   LAUNCH_OK();
   return blocks;
 }
-// Glue a pending basis into b with weight beta.
-//   eq mode      : b[i].c0 += beta * p[i]
-//   induced mode : b[2i].c0 += beta * p[i], b[2i+1].c1 += beta * p[i]  (u * base = (0, base))
-__global__ void lg_glue_kernel(F256d* __restrict__ b, const F128d* __restrict__ p, F128d beta, uint64_t n,
+// Glue a pending basis of n values p into b:
+//   eq mode      : b[2i].c0 += w0 p[i], b[2i+1].c0 += w1 p[i]
+//   induced mode : b[2i].c0 += w0 p[i], b[2i+1].c1 += w0 p[i]  (u * base = (0, base))
+__global__ void lg_glue_kernel(F256d* __restrict__ b, const F128d* __restrict__ p, F128d w0, F128d w1, uint64_t n,
                                int induced) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  F128d v = beta * p[i];
-  if (induced) {
-    b[2 * i].c0 += v;
-    b[2 * i + 1].c1 += v;
-  } else {
-    b[i].c0 += v;
-  }
+  const F128d v = p[i], e = mul_call(w0, v);
+  b[2 * i].c0 += e;
+  if (induced) b[2 * i + 1].c1 += e;
+  else b[2 * i + 1].c0 += mul_call(w1, v);
 }
-void launch_lg_glue(F256d* b, const F128d* p, F128d beta, uint64_t n, bool induced, cudaStream_t s) {
-  lg_glue_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, p, beta, n, induced ? 1 : 0);
+void launch_lg_glue(F256d* b, const F128d* p, F128d w0, F128d w1, uint64_t n, bool induced, cudaStream_t s) {
+  lg_glue_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(b, p, w0, w1, n, induced ? 1 : 0);
   LAUNCH_OK();
 }
 
