@@ -408,8 +408,8 @@ std::vector<F128> GpuBackend::reduce(uint32_t n_blocks, uint32_t width) {
   launch_reduce_pair(part_, n_blocks, width, nullptr, 0, 0, st_, fp);
   return read_published(fp.seq, width);
 }
-std::vector<F128> GpuBackend::read_published(uint32_t seq, uint32_t width) {
-  wait_published(seq);
+std::vector<F128> GpuBackend::read_published(uint32_t seq, uint32_t width, bool stage) {
+  wait_published(seq, stage);
   std::vector<F128> out(width);
   const volatile F128d* p = h_pub_;
   for (uint32_t j = 0; j < width; ++j) out[j] = F128(p[j].lo, p[j].hi);
@@ -419,9 +419,10 @@ std::vector<F128> GpuBackend::read_published(uint32_t seq, uint32_t width) {
 // Wait for the published sequence number (the stream keeps running; no synchronisation):
 // a short hot spin for the common case of a message a few microseconds away, then a spin
 // that yields the core on every pass, so that concurrent provers' host work (assists,
-// transcripts) is not starved by waiting threads. A stalled stream is reported after 20 s.
-void GpuBackend::wait_published(uint32_t seq) { wait_flag(h_flag_, seq, st_); }
-void GpuBackend::wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream) {
+// transcripts) is not starved by waiting threads. A round's message is reported as stalled after
+// 20 s; results of whole stages (caps, openings, round 1) are waited for as long as the stream runs.
+void GpuBackend::wait_published(uint32_t seq, bool stage) { wait_flag(h_flag_, seq, st_, stage); }
+void GpuBackend::wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream, bool stage) {
   const volatile uint32_t* f = flag;
   uint64_t spins = 0;
   double t0 = 0;
@@ -429,11 +430,11 @@ void GpuBackend::wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stre
     ++spins;
     if (spins > 2048) std::this_thread::yield();
     if ((spins & 0x3FFF) == 0) {
-      double t = now_ms();
-      if (t0 == 0) t0 = t;
-      else if (t - t0 > 20000) throw std::runtime_error("device result not published within 20 s");
-      cudaError_t e = cudaStreamQuery(stream);
+      const cudaError_t e = cudaStreamQuery(stream);
       if (e != cudaSuccess && e != cudaErrorNotReady) CUDA_OK(e);
+      const double t = now_ms();
+      if (t0 == 0 || (stage && e == cudaErrorNotReady)) t0 = t;
+      else if (t - t0 > 20000) throw std::runtime_error("device result not published within 20 s");
     }
   }
   std::atomic_thread_fence(std::memory_order_acquire);
@@ -555,7 +556,7 @@ void GpuBackend::commit_l0(uint32_t cap_depth, std::vector<Hash>& cap) {
 }
 
 std::vector<Hash> GpuBackend::read_cap(uint32_t cap_depth, const FusedPublish& fp) {
-  wait_published(fp.seq);
+  wait_published(fp.seq, true);
   std::vector<Hash> cap(size_t(1) << cap_depth);
   memcpy(cap.data(), h_open_, cap.size() * 32);
   d2h_ += cap.size() * 32;
@@ -629,7 +630,7 @@ void GpuBackend::zc_round1(const std::vector<F128>& r, std::vector<F128>& ab, st
     throw std::runtime_error("round-1 partials exceed the partials buffer");
   const FusedPublish fp = fused_publish();
   launch_reduce_pair(part_, nab, 64, part_svc, nsvc, 128, st_, fp);
-  auto v = read_published(fp.seq, 192);
+  auto v = read_published(fp.seq, 192, true);
   // D = prod (1 + g_i)^-1 over the medium constants' g_i = x^1, x^2, x^4, x^8
   static const F128 D = [] {
     F128 d = F128::one();
@@ -920,7 +921,7 @@ void GpuBackend::lc_s_hat_v(const std::vector<F128>& tail, std::vector<F128>& ou
   const F128d* det = upload(et);
   const FusedPublish fp = fused_publish();
   { Mark mk(this, ST_LINCHECK); launch_lc_s_hat_v(zvcap_, det, (uint32_t)et.size(), st_, fp); }
-  out = read_published(fp.seq, 128);
+  out = read_published(fp.seq, 128, true);
 }
 
 // ------------------------------------------------------------------ merged open
@@ -1396,7 +1397,7 @@ void GpuBackend::lg_open(uint32_t level, const std::vector<uint64_t>& pos, uint3
     Mark mk(this, ST_LIGERITO);
     launch_gather_open(mat, lanes, tree, n_leaves, dpos, n, cap_depth, reinterpret_cast<F128d*>(d), d + row_bytes, st_, fp);
   }
-  wait_published(fp.seq);
+  wait_published(fp.seq, true);
   d2h_ += row_bytes + path_bytes;
   const F128* hr = reinterpret_cast<const F128*>(h_open_);
   const Hash* hp = reinterpret_cast<const Hash*>(h_open_ + row_bytes);

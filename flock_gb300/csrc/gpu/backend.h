@@ -58,7 +58,7 @@ class GpuBackend : public ProverBackend {
   JaggedAssistOps* jagged_assist() override { return jagged_.get(); }
   // Spin until the mapped flag holds seq (bounded: an error after 20 s, stream errors
   // reported as they occur).
-  static void wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream);
+  static void wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream, bool stage = false);
   // Device-time breakdown of a prove (CUDA events on the backend's stream).
   enum Stage {
     ST_WITNESS, ST_L0_FILL, ST_L0_NTT, ST_L0_MERKLE, ST_ZC_ROUND1, ST_ZC_FOLD_SKIP, ST_ZC_FOLDS, ST_LINCHECK,
@@ -256,8 +256,8 @@ class GpuBackend : public ProverBackend {
   uint32_t* h_flag_ = nullptr;
   uint32_t* d_flag_ = nullptr;
   uint32_t seq_ = 0;
-  void wait_published(uint32_t seq);
-  std::vector<F128> read_published(uint32_t seq, uint32_t width);
+  void wait_published(uint32_t seq, bool stage = false);
+  std::vector<F128> read_published(uint32_t seq, uint32_t width, bool stage = false);
   uint32_t* pub_counter_ = nullptr;  // ticket counter of in-kernel publication (device)
   FusedPublish fused_publish() { FusedPublish p; p.out = d_pub_; p.flag = d_flag_; p.counter = pub_counter_; p.seq = ++seq_; return p; }
   // eq tables of every zerocheck fold round, built once from the skip-fold point

@@ -272,7 +272,7 @@ FusedPublish JaggedAssist::publish() {
   return p;
 }
 void JaggedAssist::read(const FusedPublish& p, F128& g1, F128& gi) {
-  GpuBackend::wait_flag(h_flag_, p.seq, st_);
+  GpuBackend::wait_flag(h_flag_, p.seq, st_, true);
   const volatile F128d* o = h_pub_;
   g1 = F128(o[0].lo, o[0].hi);
   gi = F128(o[1].lo, o[1].hi);
