@@ -598,7 +598,10 @@ zc_fold_skip_kernel(const F128d* __restrict__ a, const F128d* __restrict__ b, co
 // every high coordinate to differ from 0 and 1; otherwise the plain form runs.
 // All lookups are from window tables (wintable.cuh). Keccak-f 2^18 (87 M live words): skip fold
 // 8.05 -> 5.59 ms, folds 12.4 -> 8.4; SHA-256 2^16: 1.25 -> 0.88, 2.25 -> 1.64; BLAKE3 2^12: 83 ->
-// 61 us, 0.39 -> 0.37 ms.
+// 61 us, 0.39 -> 0.37 ms. While a chunk is summed, its threads' next words are on their way and
+// the images that the next chunk's table is built from are formed (one barrier and a product's
+// latency less a chunk): skip fold 5.55 -> 5.31, folds 8.22 -> 7.88; SHA-256 2^16 0.877 -> 0.841,
+// 1.468 -> 1.409.
 //
 // Skip fold: tables of h w64 (for a) and w64 (for b), six-bit windows, 2 x 82 KB, one block per
 // SM; 44 lookups (5.5 cycles of the shared-memory pipe) and two products (13 of the multiply
@@ -611,7 +614,7 @@ zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restric
                              const F128d* __restrict__ h, F128d* __restrict__ part, FusedPublish pub) {
   constexpr uint32_t PER = (1u << LO) / ZC_W_THREADS;
   extern __shared__ __align__(16) char wt[];  // a's table, then b's
-  __shared__ F128d img[64];
+  __shared__ F128d img[2][64];  // the images of this chunk's table, and the next one's
   __shared__ F128d sh[32];
   const uint32_t lane = win_lane(), team = threadIdx.x >> 3, teams = ZC_W_THREADS / 8;
   char* TB = wt + WinMap<6, 64>::BYTES;
@@ -619,18 +622,29 @@ zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restric
   F128d S1[PER], SI[PER];
 #pragma unroll
   for (uint32_t k = 0; k < PER; ++k) S1[k] = SI[k] = f128_zero();
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
-    __syncthreads();  // the previous chunk's table is no longer read
-    if (threadIdx.x < 64) img[threadIdx.x] = mul_call(h[ch], w64[threadIdx.x]);
+  auto scale = [&](uint64_t ch, uint32_t buf) {
+    if (threadIdx.x < 64 && ch < n_chunks) img[buf][threadIdx.x] = mul_call(h[ch], w64[threadIdx.x]);
+  };
+  // a thread's words, the next pair of them on its way while this one is summed
+  F128d an = f128_zero(), bn = f128_zero();
+  auto load = [&](uint64_t wi) {
+    if (wi < n_words) { an = a[wi]; bn = b[wi]; }
+  };
+  scale(blockIdx.x, 0);
+  load(((uint64_t)blockIdx.x << LO) + threadIdx.x);
+  uint32_t buf = 0;
+  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x, buf ^= 1) {
+    __syncthreads();  // the previous chunk's table is no longer read, this one's images are there
+    build_win_map<6, 64>(img[buf], wt, team, teams);
     __syncthreads();
-    build_win_map<6, 64>(img, wt, team, teams);
-    __syncthreads();
+    scale(ch + gridDim.x, buf ^ 1);
     const uint64_t w0 = (ch << LO) + threadIdx.x;
 #pragma unroll
     for (uint32_t k = 0; k < PER; ++k) {
       const uint64_t wi = w0 + k * ZC_W_THREADS;
+      const F128d av = an, bv = bn;
+      load(k + 1 < PER ? wi + ZC_W_THREADS : ((ch + gridDim.x) << LO) + threadIdx.x);
       if (wi >= n_words) continue;  // a zero tail
-      const F128d av = a[wi], bv = b[wi];
       F128d a0 = f128_zero(), a1 = f128_zero(), b0 = f128_zero(), b1 = f128_zero();
       add_win_map64<6>(a1, av.hi, wt, lane);
       add_win_map64<6>(b1, bv.hi, TB, lane);
@@ -785,7 +799,7 @@ zc_fold2_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ 
                          F128d* __restrict__ part, FusedPublish pub) {
   constexpr uint32_t PAIRS = 1u << (LO - 1), PER = PAIRS / ZC_W_THREADS, TAB = WinMap<5, 64>::BYTES;
   extern __shared__ __align__(16) char wt[];  // a's tables for the low and high halves, then b's
-  __shared__ F128d wr[2][64], img[2][64];
+  __shared__ F128d wr[2][64], img[2][2][64];  // images of this chunk's tables, and the next one's
   __shared__ F128d sh[32];
   const uint32_t lane = win_lane();
   // two halves of the block build the two tables of a vector
@@ -802,14 +816,28 @@ zc_fold2_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ 
 #pragma unroll
   for (uint32_t k = 0; k < PER; ++k) S1[k] = SI[k] = f128_zero();
   const uint64_t n_chunks = (n_pairs + PAIRS - 1) / PAIRS;
-  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x) {
+  auto scale = [&](uint64_t ch, uint32_t buf) {
+    if (threadIdx.x < 128 && ch < n_chunks)
+      img[buf][threadIdx.x >> 6][threadIdx.x & 63] = mul_call(h[ch], wr[threadIdx.x >> 6][threadIdx.x & 63]);
+  };
+  // a pair's words, the next pair's on their way while this one is folded
+  F128d an[2], bn[2];
+  auto load = [&](uint64_t j) {
+    if (j >= live_pairs) return;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) { an[q] = a[2 * j + q]; bn[q] = b[2 * j + q]; }
+  };
+  an[0] = an[1] = bn[0] = bn[1] = f128_zero();
+  scale(blockIdx.x, 0);
+  load((uint64_t)blockIdx.x * PAIRS + threadIdx.x);
+  uint32_t buf = 0;
+  for (uint64_t ch = blockIdx.x; ch < n_chunks; ch += gridDim.x, buf ^= 1) {
     const bool live = ch * PAIRS < live_pairs;  // block-uniform
     if (live) {
-      __syncthreads();  // the previous chunk's tables are no longer read
-      if (threadIdx.x < 128) img[threadIdx.x >> 6][threadIdx.x & 63] = mul_call(h[ch], wr[threadIdx.x >> 6][threadIdx.x & 63]);
+      __syncthreads();  // the previous chunk's tables are no longer read, this one's images are there
+      build_win_map<5, 64>(img[buf][half], wt + half * TAB, team, teams);
       __syncthreads();
-      build_win_map<5, 64>(img[half], wt + half * TAB, team, teams);
-      __syncthreads();
+      scale(ch + gridDim.x, buf ^ 1);
     }
 #pragma unroll
     for (uint32_t k = 0; k < PER; ++k) {
@@ -819,10 +847,11 @@ zc_fold2_weighted_kernel(const F128d* __restrict__ a, const F128d* __restrict__ 
         aout[2 * j] = aout[2 * j + 1] = bout[2 * j] = bout[2 * j + 1] = f128_zero();
         continue;
       }
-      F128d A[2], B[2];
+      F128d A[2] = {an[0], an[1]}, B[2] = {bn[0], bn[1]};
+      load(k + 1 < PER ? j + ZC_W_THREADS : (ch + gridDim.x) * PAIRS + threadIdx.x);
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const F128d av = a[2 * j + q], bv = b[2 * j + q];
+        const F128d av = A[q], bv = B[q];
         A[q] = B[q] = f128_zero();
         add_win_map64<5>(A[q], av.lo, wt, lane);
         add_win_map64<5>(A[q], av.hi, wt + TAB, lane);
