@@ -925,7 +925,9 @@ enum PairEq : int {
 // bits, 169 KB, one block per SM): four table products (11 cycles of the shared-memory pipe)
 // beside the message's two products of variables (13 of the multiply pipe). The byte tables it
 // replaced (three 256-thread blocks per SM) took 4.8 ms for the merged open's rounds of Keccak-f
-// 2^18, this form 3.5. Below the threshold a block would fold less than two rounds of its threads.
+// 2^18, this form 3.36 (3.53 with a thread on a whole message pair, whose loads 64 bytes apart
+// took a quarter of the data pipe, and without the next entries' loads ahead; SHA-256 2^16 0.74 ->
+// 0.67). Below the threshold a block would fold less than two rounds of its threads.
 constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;
 constexpr uint32_t PAIR_FOLD_TABLE_THREADS = 512;
 template <int EQ>
@@ -938,21 +940,55 @@ pair_fold_tbl_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bi
   build_win_table<6>(r, wt);
   __syncthreads();
   const uint32_t lane = win_lane();
-  const uint64_t j0 = (uint64_t)blockIdx.x * PAIR_FOLD_TABLE_THREADS + threadIdx.x;
+  // A warp takes 32 message pairs, 64 folded entries: lane l folds entries l and 32 + l (two neighbours
+  // in memory each), then trades one of them with the lane beside it, so that an even lane has
+  // the pair l / 2 and an odd one the pair 16 + l / 2.
+  const uint32_t l = threadIdx.x & 31, odd = l & 1;
+  const uint64_t w0 = ((uint64_t)blockIdx.x * PAIR_FOLD_TABLE_THREADS + threadIdx.x) >> 5;
+  const uint64_t j0 = 32 * w0 + (l >> 1) + 16 * odd, n_warps = (uint64_t)gridDim.x * (PAIR_FOLD_TABLE_THREADS / 32);
   MulAcc m1, mi;
-  for (uint64_t j = j0; j < n_pairs; j += (uint64_t)gridDim.x * PAIR_FOLD_TABLE_THREADS) {
-    if (j >= live_pairs) {  // zero inputs: zero outputs, nothing added to the message
-      aout[2 * j] = aout[2 * j + 1] = bout[2 * j] = bout[2 * j + 1] = f128_zero();
-      continue;
+  auto trade = [&](F128d v) {
+    return f128(__shfl_xor_sync(0xffffffffu, v.lo, 1), __shfl_xor_sync(0xffffffffu, v.hi, 1));
+  };
+  F128d xn[4], yn[4];  // the next entries' words
+  auto load = [&](uint64_t w) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint64_t e = 64 * w + l + 32 * q;
+      xn[2 * q] = xn[2 * q + 1] = yn[2 * q] = yn[2 * q + 1] = f128_zero();
+      if (e < 2 * live_pairs) {
+        xn[2 * q] = ain[2 * e]; xn[2 * q + 1] = ain[2 * e + 1];
+        yn[2 * q] = bin[2 * e]; yn[2 * q + 1] = bin[2 * e + 1];
+      }
     }
-    const F128d x0 = ain[4 * j], x1 = ain[4 * j + 1], x2 = ain[4 * j + 2], x3 = ain[4 * j + 3];
-    const F128d y0 = bin[4 * j], y1 = bin[4 * j + 1], y2 = bin[4 * j + 2], y3 = bin[4 * j + 3];
-    const F128d A0 = x0 + mul_win<6>(x1 + x0, wt, lane), A1 = x2 + mul_win<6>(x3 + x2, wt, lane);
-    const F128d B0 = y0 + mul_win<6>(y1 + y0, wt, lane), B1 = y2 + mul_win<6>(y3 + y2, wt, lane);
-    aout[2 * j] = A0; aout[2 * j + 1] = A1;
-    bout[2 * j] = B0; bout[2 * j + 1] = B1;
-    m1.add(A1, B1);
-    mi.add(A0 + A1, B0 + B1);
+  };
+  load(w0);
+  for (uint64_t w = w0; 32 * w < n_pairs; w += n_warps) {
+    const uint64_t e0 = 64 * w + l;
+    F128d A[2], B[2];
+    if (32 * w < live_pairs) {  // warp-uniform
+      F128d x[4], y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { x[q] = xn[q]; y[q] = yn[q]; }
+      load(w + n_warps);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        A[q] = x[2 * q] + mul_win<6>(x[2 * q + 1] + x[2 * q], wt, lane);
+        B[q] = y[2 * q] + mul_win<6>(y[2 * q + 1] + y[2 * q], wt, lane);
+        if (e0 + 32 * q < 2 * n_pairs) {
+          aout[e0 + 32 * q] = A[q];
+          bout[e0 + 32 * q] = B[q];
+        }
+      }
+      const F128d ta = trade(odd ? A[0] : A[1]), tb = trade(odd ? B[0] : B[1]);
+      const F128d A0 = odd ? ta : A[0], A1 = odd ? A[1] : ta, B0 = odd ? tb : B[0], B1 = odd ? B[1] : tb;
+      m1.add(A1, B1);
+      mi.add(A0 + A1, B0 + B1);
+    } else {  // zero inputs: zero outputs, nothing added to the message
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (e0 + 32 * q < 2 * n_pairs) aout[e0 + 32 * q] = bout[e0 + 32 * q] = f128_zero();
+    }
   }
   F128d g1 = m1.value(), gi = mi.value();
   if (EQ == EQ_FIXED) {
