@@ -9,6 +9,7 @@
 #include <stdexcept>
 #include <string>
 #include "field.cuh"
+#include "plan.h"
 
 #define CUDA_OK(x)                                                                          \
   do {                                                                                      \

@@ -1,0 +1,52 @@
+// Launch shapes and buffer sizes that follow from a size and the SM count. No CUDA in here, so
+// that a host test can walk every SM count (a partition of the part reports fewer than 152).
+#pragma once
+#include <algorithm>
+#include <cstdint>
+
+namespace flock {
+namespace gpu {
+
+// ------------------------------------------------------------------ pair folds
+// Folds of at least this many pairs take the table form (see the kernels in sumcheck.cu).
+constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;
+constexpr uint32_t PAIR_FOLD_TABLE_THREADS = 512;
+constexpr uint32_t SMALL_PAIRS = 64;  // of a block of the small form
+enum PairEq : int {
+  EQ_NONE,   // eq = 1
+  EQ_FIXED,  // eq(j) = eq_lo[j mod 2^lo_bits] (the zerocheck's weighted form); in the table form the
+             // grid's thread count is a multiple of 2^lo_bits, so a thread multiplies its sum once
+  EQ_SPLIT,  // eq(j) = eq_lo[j mod 2^lo_bits] eq_hi[j >> lo_bits]
+};
+struct PairFoldPlan {
+  bool table;
+  uint32_t blocks;  // each writes two partials
+};
+inline PairFoldPlan pair_fold_plan(uint64_t n_pairs, PairEq eq, uint32_t lo_bits, bool unweight, uint64_t sms) {
+  if (n_pairs < PAIR_FOLD_TABLE_MIN_PAIRS || eq == EQ_SPLIT || unweight)
+    return {false, (uint32_t)((n_pairs + SMALL_PAIRS - 1) / SMALL_PAIRS)};
+  // one block per SM; under EQ_FIXED a multiple of 2^lo_bits threads in all
+  uint32_t blocks = (uint32_t)sms;
+  if (eq == EQ_FIXED && (1u << lo_bits) > PAIR_FOLD_TABLE_THREADS) {
+    const uint32_t q = (1u << lo_bits) / PAIR_FOLD_TABLE_THREADS;
+    blocks = std::max(q, blocks / q * q);
+  }
+  return {true, blocks};
+}
+
+// ------------------------------------------------------------------ the jagged assist
+constexpr uint32_t AS_BUILD_THREADS = 512;
+inline uint32_t as_build_blocks(uint64_t n, uint64_t sms) {
+  return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n / 2 + AS_BUILD_THREADS - 1) / AS_BUILD_THREADS, sms));
+}
+// Partials that the assist over n dense words needs room for: two a block of its widest launch
+// (the first small fold has 1024 blocks, whatever the SM count).
+inline uint64_t assist_partials(uint64_t n, uint64_t sms) {
+  uint64_t blocks = as_build_blocks(n, sms);
+  for (uint64_t pairs = n / 4; pairs; pairs /= 2)
+    blocks = std::max<uint64_t>(blocks, pair_fold_plan(pairs, EQ_NONE, 0, false, sms).blocks);
+  return 2 * blocks;
+}
+
+}  // namespace gpu
+}  // namespace flock

@@ -142,7 +142,7 @@ void launch_as_dual(const F128d* z_row, uint32_t n, const F128d* points, uint32_
 // g[2i + 1]). g is not zero past the area and enters later messages through pairs with one
 // live entry, so the whole vectors are built and folded. One block of 512 threads per SM beside
 // the 64 KB of tables; per entry three products and 16 lookups.
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(AS_BUILD_THREADS, 1)
 as_build_kernel(const F128d* __restrict__ er0, const F128d* __restrict__ ec0, const F128d* __restrict__ er1,
                 const F128d* __restrict__ ec1, const F128d* __restrict__ eq_lo, uint32_t lo_bits,
                 const F128d* __restrict__ eq_hi, const F128d* __restrict__ table, uint64_t area, uint64_t n, JaggedSegs segs,
@@ -177,8 +177,8 @@ void launch_as_build(const F128d* er0, const F128d* ec0, const F128d* er1, const
                      const JaggedSegs& segs, F128d* abar, F128d* g, F128d* part, cudaStream_t s, FusedPublish pub) {
   const int smem = 16 * 256 * (int)sizeof(F128d);
   set_dynamic_smem((const void*)as_build_kernel, smem);
-  const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((n / 2 + 511) / 512, (uint64_t)sm_count()));
-  as_build_kernel<<<blocks, 512, smem, s>>>(er0, ec0, er1, ec1, eq_lo, lo_bits, eq_hi, table, area, n, segs, abar, g,
+  const uint32_t blocks = as_build_blocks(n, (uint64_t)sm_count());
+  as_build_kernel<<<blocks, AS_BUILD_THREADS, smem, s>>>(er0, ec0, er1, ec1, eq_lo, lo_bits, eq_hi, table, area, n, segs, abar, g,
                                             part, pub);
   LAUNCH_OK();
 }
@@ -227,7 +227,7 @@ JaggedAssist::JaggedAssist(const Statement& s, int device) : S(s), device_(devic
   }
   eq_lo_ = alloc<F128d>(size_t(1) << lo);
   eq_hi_ = alloc<F128d>(size_t(1) << (m - lo));
-  part_ = alloc<F128d>((size_t)sm_count() * 16);
+  part_ = alloc<F128d>(assist_partials(n_, (uint64_t)sm_count()));
   out_ = alloc<F128d>(256);
   counter_ = alloc<uint32_t>(1);
   CUDA_OK(cudaMemsetAsync(counter_, 0, sizeof(uint32_t), st_));

@@ -914,22 +914,14 @@ void launch_factor_table(const F128d* f, uint32_t n, F128d* out, cudaStream_t s)
 // Fold the low variable of two vectors at r (out[i] = in[2i] + r (in[2i+1] + in[2i])) and emit
 // the pair message over the folded vectors:
 //   g1 = sum_j eq(j) A1 B1, ginf = sum_j eq(j) (A0 + A1)(B0 + B1), (A0, A1) = out[2j..2j+2).
-// n_pairs = output length / 2 (>= 1). eq by mode:
-enum PairEq : int {
-  EQ_NONE,   // eq = 1
-  EQ_FIXED,  // eq(j) = eq_lo[j mod 2^lo_bits] (the zerocheck's weighted form); in the table form the
-             // grid's thread count is a multiple of 2^lo_bits, so a thread multiplies its sum once
-  EQ_SPLIT,  // eq(j) = eq_lo[j mod 2^lo_bits] eq_hi[j >> lo_bits]
-};
-// Folds of at least this many pairs take their products by r from the window table of r (six
+// n_pairs = output length / 2 (>= 1); eq by mode (PairEq, plan.h).
+// Folds of at least PAIR_FOLD_TABLE_MIN_PAIRS pairs take their products by r from the window table of r (six
 // bits, 169 KB, one block per SM): four table products (11 cycles of the shared-memory pipe)
 // beside the message's two products of variables (13 of the multiply pipe). The byte tables it
 // replaced (three 256-thread blocks per SM) took 4.8 ms for the merged open's rounds of Keccak-f
 // 2^18, this form 3.36 (3.53 with a thread on a whole message pair, whose loads 64 bytes apart
 // took a quarter of the data pipe, and without the next entries' loads ahead; SHA-256 2^16 0.74 ->
 // 0.67). Below the threshold a block would fold less than two rounds of its threads.
-constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;
-constexpr uint32_t PAIR_FOLD_TABLE_THREADS = 512;
 template <int EQ>
 __global__ void __launch_bounds__(PAIR_FOLD_TABLE_THREADS, 1)
 pair_fold_tbl_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bin, uint64_t n_pairs, uint64_t live_pairs,
@@ -1010,7 +1002,7 @@ pair_fold_tbl_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bi
 // PAIRS (4j .. 4j + 3 in, 2j and 2j + 1 out) or TOP (the top variable bound in place, for the
 // lincheck: i, i + h; i + q, i + q + h in, i and i + q out, h = 2q = half the length).
 // unweight (or null): factors of the folded a entries.
-constexpr uint32_t SMALL_PAIRS = 64, SMALL_THREADS = 4 * SMALL_PAIRS;
+constexpr uint32_t SMALL_THREADS = 4 * SMALL_PAIRS;
 enum PairMap : int { MAP_PAIRS, MAP_TOP };
 template <int EQ, int MAP>
 __global__ void __launch_bounds__(SMALL_THREADS)
@@ -1072,14 +1064,11 @@ uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, 
                           F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub) {
   live_pairs = std::min(live_pairs, n_pairs);
   const bool fixed = eq_lo && !eq_hi;
-  if (n_pairs >= PAIR_FOLD_TABLE_MIN_PAIRS && !eq_hi && !unweight) {
-    // one block per SM; under EQ_FIXED a multiple of 2^lo_bits threads in all
+  const PairFoldPlan plan =
+      pair_fold_plan(n_pairs, eq_hi ? EQ_SPLIT : fixed ? EQ_FIXED : EQ_NONE, lo_bits, unweight != nullptr, (uint64_t)sm_count());
+  const uint32_t blocks = plan.blocks;
+  if (plan.table) {
     const int smem = WinTable<6>::BYTES;
-    uint32_t blocks = (uint32_t)sm_count();
-    if (fixed && (1u << lo_bits) > PAIR_FOLD_TABLE_THREADS) {
-      const uint32_t q = (1u << lo_bits) / PAIR_FOLD_TABLE_THREADS;
-      blocks = std::max(q, blocks / q * q);
-    }
     if (fixed) {
       set_dynamic_smem((const void*)pair_fold_tbl_kernel<EQ_FIXED>, smem);
       pair_fold_tbl_kernel<EQ_FIXED><<<blocks, PAIR_FOLD_TABLE_THREADS, smem, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo,
@@ -1092,7 +1081,6 @@ uint32_t launch_pair_fold(const F128d* ain, const F128d* bin, uint64_t n_pairs, 
     LAUNCH_OK();
     return blocks;
   }
-  const uint32_t blocks = (uint32_t)((n_pairs + SMALL_PAIRS - 1) / SMALL_PAIRS);
   auto* kernel = eq_hi ? pair_fold_small_kernel<EQ_SPLIT, MAP_PAIRS>
                        : (fixed ? pair_fold_small_kernel<EQ_FIXED, MAP_PAIRS> : pair_fold_small_kernel<EQ_NONE, MAP_PAIRS>);
   kernel<<<blocks, SMALL_THREADS, 0, s>>>(ain, bin, n_pairs, live_pairs, r, eq_lo, lo_bits, eq_hi, unweight, aout, bout,
