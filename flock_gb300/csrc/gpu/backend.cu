@@ -127,7 +127,7 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
   const uint64_t D = uint64_t(1) << S.log_dim;
   b += lane_fold_groups(S.lanes, D, GB300_SMS) * D * 32;  // Ligerito: lane fold partials,
   b += 4 * 2 * D * 32 + 2 * D * 16;            // f/b ping-pong, pending
-  b += (uint64_t(1) << 20) * 16 + (size_t(96) << 20) + (size_t(8) << 20);  // partials, scratch, staging
+  b += uint64_t(PART_ENTRIES) * 16 + (size_t(96) << 20) + (size_t(8) << 20);  // partials, scratch, staging
   b += n_pos * 16;                          // L0 twiddles
   // recursive levels: codeword 2^(log_cols + rate) x 2^k, tree, twiddles
   const LigeritoParams& P = S.lig;
@@ -216,7 +216,7 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   static_assert(2 * TAIL >= 4 * LG_TAIL, "the tail buffer holds two F256 vectors of LG_TAIL entries");
   CUDA_OK(cudaHostAlloc(&h_tail_, 2 * TAIL * sizeof(F128d), cudaHostAllocMapped));
   CUDA_OK(cudaHostGetDevicePointer(&d_tail_, h_tail_, 0));
-  part_cap_ = 1u << 20;
+  part_cap_ = PART_ENTRIES;
   part_ = dmalloc<F128d>(part_cap_, owned_, device_bytes_);
   scr_cap_ = size_t(96) << 20;
   scr_ = dmalloc<uint8_t>(scr_cap_, owned_, device_bytes_);

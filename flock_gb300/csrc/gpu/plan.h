@@ -7,6 +7,8 @@
 namespace flock {
 namespace gpu {
 
+constexpr uint32_t PART_ENTRIES = 1u << 20;  // a backend's buffer of per-block partials
+
 // ------------------------------------------------------------------ pair folds
 // Folds of at least this many pairs take the table form (see the kernels in sumcheck.cu).
 constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;
@@ -22,9 +24,13 @@ struct PairFoldPlan {
   bool table;
   uint32_t blocks;  // each writes two partials
 };
+// The small form's widest grid: what its folds below the table form take. Larger ones (the
+// zerocheck's plain form on a large vector, after a challenge the weighted form cannot divide by)
+// walk their pairs with it, so that their partials have room at any size.
+constexpr uint32_t PAIR_FOLD_SMALL_BLOCKS = PAIR_FOLD_TABLE_MIN_PAIRS / SMALL_PAIRS;
 inline PairFoldPlan pair_fold_plan(uint64_t n_pairs, PairEq eq, uint32_t lo_bits, bool unweight, uint64_t sms) {
   if (n_pairs < PAIR_FOLD_TABLE_MIN_PAIRS || eq == EQ_SPLIT || unweight)
-    return {false, (uint32_t)((n_pairs + SMALL_PAIRS - 1) / SMALL_PAIRS)};
+    return {false, (uint32_t)std::min<uint64_t>((n_pairs + SMALL_PAIRS - 1) / SMALL_PAIRS, PAIR_FOLD_SMALL_BLOCKS)};
   // one block per SM; under EQ_FIXED a multiple of 2^lo_bits threads in all
   uint32_t blocks = (uint32_t)sms;
   if (eq == EQ_FIXED && (1u << lo_bits) > PAIR_FOLD_TABLE_THREADS) {

@@ -1001,11 +1001,12 @@ pair_fold_tbl_kernel(const F128d* __restrict__ ain, const F128d* __restrict__ bi
 // of BLAKE3 2^12 0.35 -> 0.255 ms). Where the two vectors' entries of a pair lie:
 // PAIRS (4j .. 4j + 3 in, 2j and 2j + 1 out) or TOP (the top variable bound in place, for the
 // lincheck: i, i + h; i + q, i + q + h in, i and i + q out, h = 2q = half the length).
-// unweight (or null): factors of the folded a entries.
+// unweight (or null): factors of the folded a entries. Four blocks a SM: without the bound the walk
+// over a grid's pairs takes 70 registers and leaves three.
 constexpr uint32_t SMALL_THREADS = 4 * SMALL_PAIRS;
 enum PairMap : int { MAP_PAIRS, MAP_TOP };
 template <int EQ, int MAP>
-__global__ void __launch_bounds__(SMALL_THREADS)
+__global__ void __launch_bounds__(SMALL_THREADS, 4)
 pair_fold_small_kernel(const F128d* ain, const F128d* bin, uint64_t n_pairs, uint64_t live_pairs, F128d r,
                        const F128d* __restrict__ eq_lo, uint32_t lo_bits, const F128d* __restrict__ eq_hi,
                        const F128d* __restrict__ unweight, F128d* aout, F128d* bout, F128d* __restrict__ part,
@@ -1015,43 +1016,46 @@ pair_fold_small_kernel(const F128d* ain, const F128d* bin, uint64_t n_pairs, uin
   __shared__ F128d ev[SMALL_PAIRS];    // eq(j)
   __shared__ F128d sh[SMALL_THREADS / 32];
   if (threadIdx.x == 0) rs = split_factor(r);
-  const uint64_t base = (uint64_t)blockIdx.x * SMALL_PAIRS;
-  {
-    // vector a's pairs by the first half of the block, b's by the second; k = 0, 1: out entry
-    const uint32_t which = threadIdx.x / (2 * SMALL_PAIRS), i = threadIdx.x % (2 * SMALL_PAIRS);
-    const uint32_t p = MAP == MAP_PAIRS ? i >> 1 : i % SMALL_PAIRS, k = MAP == MAP_PAIRS ? i & 1 : i / SMALL_PAIRS;
-    const uint64_t j = base + p;
-    const F128d* in = which ? bin : ain;
-    F128d* out = which ? bout : aout;
-    F128d x0 = f128_zero(), d = f128_zero();
-    if (j < live_pairs) {
-      const uint64_t i0 = MAP == MAP_PAIRS ? 4 * j + 2 * k : j + k * n_pairs;
-      x0 = in[i0];
-      d = in[MAP == MAP_PAIRS ? i0 + 1 : i0 + 2 * n_pairs] + x0;
+  const uint32_t p = threadIdx.x % SMALL_PAIRS, job = threadIdx.x / SMALL_PAIRS;  // whole warps share a job
+  F128d acc = f128_zero();
+  for (uint64_t base = (uint64_t)blockIdx.x * SMALL_PAIRS; base < n_pairs; base += (uint64_t)gridDim.x * SMALL_PAIRS) {
+    {
+      // vector a's pairs by the first half of the block, b's by the second; k = 0, 1: out entry
+      const uint32_t which = threadIdx.x / (2 * SMALL_PAIRS), i = threadIdx.x % (2 * SMALL_PAIRS);
+      const uint32_t q = MAP == MAP_PAIRS ? i >> 1 : i % SMALL_PAIRS, k = MAP == MAP_PAIRS ? i & 1 : i / SMALL_PAIRS;
+      const uint64_t j = base + q;
+      const F128d* in = which ? bin : ain;
+      F128d* out = which ? bout : aout;
+      F128d x0 = f128_zero(), d = f128_zero();
+      if (j < live_pairs) {
+        const uint64_t i0 = MAP == MAP_PAIRS ? 4 * j + 2 * k : j + k * n_pairs;
+        x0 = in[i0];
+        d = in[MAP == MAP_PAIRS ? i0 + 1 : i0 + 2 * n_pairs] + x0;
+      }
+      __syncthreads();  // rs is there, the previous pairs' values are no longer read
+      F128d f = x0 + mul_split(d, rs);
+      const uint64_t o = MAP == MAP_PAIRS ? 2 * j + k : j + k * n_pairs;
+      if (unweight && !which && j < live_pairs) f = mul_call(f, unweight[o]);
+      if (j < n_pairs) out[o] = f;  // pairs past the live ones have zero inputs
+      v[2 * which + k][q] = f;
     }
     __syncthreads();
-    F128d f = x0 + mul_split(d, rs);
-    const uint64_t o = MAP == MAP_PAIRS ? 2 * j + k : j + k * n_pairs;
-    if (unweight && !which && j < live_pairs) f = mul_call(f, unweight[o]);
-    if (j < n_pairs) out[o] = f;  // pairs past the live ones have zero inputs
-    v[2 * which + k][p] = f;
+    F128d t = f128_zero();
+    if (job < 2) {
+      t = mul_call(job ? v[0][p] + v[1][p] : v[1][p], job ? v[2][p] + v[3][p] : v[3][p]);
+    } else if (EQ != EQ_NONE && job == 2) {
+      const uint64_t j = min(base + p, n_pairs - 1);
+      const F128d lo = eq_lo[j & ((1ull << lo_bits) - 1)];
+      ev[p] = EQ == EQ_SPLIT ? mul_call(lo, eq_hi[j >> lo_bits]) : lo;
+    }
+    if (EQ != EQ_NONE) {
+      __syncthreads();
+      if (job < 2) t = mul_call(t, ev[p]);
+    }
+    acc += t;
   }
-  __syncthreads();
-  const uint32_t p = threadIdx.x % SMALL_PAIRS, job = threadIdx.x / SMALL_PAIRS;  // whole warps share a job
-  F128d t = f128_zero();
-  if (job < 2) {
-    t = mul_call(job ? v[0][p] + v[1][p] : v[1][p], job ? v[2][p] + v[3][p] : v[3][p]);
-  } else if (EQ != EQ_NONE && job == 2) {
-    const uint64_t j = min(base + p, n_pairs - 1);
-    const F128d lo = eq_lo[j & ((1ull << lo_bits) - 1)];
-    ev[p] = EQ == EQ_SPLIT ? mul_call(lo, eq_hi[j >> lo_bits]) : lo;
-  }
-  if (EQ != EQ_NONE) {
-    __syncthreads();
-    if (job < 2) t = mul_call(t, ev[p]);
-  }
-  t = warp_xor(t);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+  acc = warp_xor(acc);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
   __syncthreads();
   if (threadIdx.x == 0) {  // jobs 0 and 1 are two warps each
     part[blockIdx.x * 2] = sh[0] + sh[1];

@@ -22,8 +22,21 @@ static void assist_partials_fit() {
     }
 }
 
+// Every fold's partials, the plain form's on large vectors among them.
+static void fold_partials_fit() {
+  for (uint64_t sms = 1; sms <= 200; ++sms)
+    for (uint64_t pairs = 1; pairs <= uint64_t(1) << 30; pairs *= 2)
+      for (PairEq eq : {EQ_NONE, EQ_FIXED, EQ_SPLIT})
+        for (uint32_t lo = 0; lo <= 11; ++lo)
+          for (bool unweight : {false, true}) {
+            const PairFoldPlan p = pair_fold_plan(pairs, eq, lo, unweight, sms);
+            expect(p.blocks >= 1 && 2 * uint64_t(p.blocks) <= PART_ENTRIES, "fold partials: SMs, pairs", sms, pairs);
+          }
+}
+
 int main() {
   assist_partials_fit();
+  fold_partials_fit();
   printf("failures %d\n", failures);
   return failures != 0;
 }
