@@ -102,7 +102,7 @@ static uint64_t live_words_of(const Statement& S) {
 // Room for either form (a degenerate challenge takes the plain one), and for the reciprocal
 // weights beside the tables.
 static uint64_t zc_tables_room(const Statement& S, uint64_t sms) {
-  const uint32_t L = S.m - 7, w = zc_weighted_lo_bits(live_words_of(S), sms);
+  const uint32_t L = S.m - 7, w = zc_weighted_lo_bits(live_words_of(S), L, sms);
   return std::max(zc_tables_entries(L, 0), w ? zc_tables_entries(L, w) + (uint64_t(1) << (L - w)) : 0);
 }
 
@@ -670,7 +670,7 @@ void GpuBackend::zc_fold_skip(const std::vector<F128>& w, const std::vector<F128
   const uint32_t L = (uint32_t)eq_point.size();  // m - 7
   if (L < 10) throw std::runtime_error("zerocheck skip fold needs m >= 17");
   // the weighted form divides by the high coordinates' eq once: none may be 0 or 1
-  zc_w_ = zc_weighted_lo_bits(zc_live_words_, (uint64_t)sm_count());
+  zc_w_ = zc_weighted_lo_bits(zc_live_words_, L, (uint64_t)sm_count());
   for (uint32_t j = zc_w_; zc_w_ && j < L; ++j)
     if (eq_point[j].is_zero() || eq_point[j] == F128::one()) zc_w_ = 0;
   // Every later fold round i uses eq over the suffix eq_point[1 + i ..]: build all the

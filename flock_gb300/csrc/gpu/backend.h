@@ -183,7 +183,7 @@ class GpuBackend : public ProverBackend {
   // fold that leaves TAIL entries (one block of the small-round kernel; LG_TAIL for F256) writes
   // them to mapped memory beside its message, and the rest runs on the host. A round on so few
   // entries costs the device about 15 us of launch, latency and publication, the host one to three.
-  static constexpr size_t TAIL = 128, LG_TAIL = 64;
+  static constexpr size_t TAIL = size_t(1) << TAIL_LOG, LG_TAIL = 64;
   struct TailPair {
     std::vector<F128> a, b;
     void fold(F128 r);

@@ -95,10 +95,9 @@ uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, u
 uint32_t launch_zc_fold2(const F128d* a, const F128d* b, const F128d* w64, F128d rho, F128d* tabs, uint64_t n_pairs,
                          uint64_t live_pairs, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* aout,
                          F128d* bout, F128d* part, cudaStream_t s, FusedPublish pub);                                     // width 2
-// The weighted form (see the kernels): low bits of its chunks for this many live words, 0 where
-// the plain form runs; the skip fold's message and the first fold with its message. eq_lo: eq
+// The weighted form (see the kernels; its chunks: zc_weighted_lo_bits in plan.h): the skip fold's
+// message and the first fold with its message. eq_lo: eq
 // over the chunk's low coordinates (of words, then of pairs), h: eq over the high ones.
-uint32_t zc_weighted_lo_bits(uint64_t live_words, uint64_t sms);
 uint32_t launch_zc_fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
                                       uint32_t lo_bits, const F128d* eq_lo, const F128d* h, F128d* part,
                                       cudaStream_t s, FusedPublish pub);                                                   // width 2

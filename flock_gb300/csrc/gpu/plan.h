@@ -40,6 +40,20 @@ inline PairFoldPlan pair_fold_plan(uint64_t n_pairs, PairEq eq, uint32_t lo_bits
   return {true, blocks};
 }
 
+// ------------------------------------------------------------------ zerocheck, weighted form
+// Entries that a sumcheck's last device fold leaves for the host (GpuBackend::TailPair).
+constexpr uint32_t TAIL_LOG = 7;
+// Low bits of the chunks of the weighted form over 2^L words, `live_words` of them live; 0 where
+// the plain form runs. A chunk's tables are rebuilt for it (about 2000 cycles beside 13 a word), so
+// chunks are as long as leaves every SM four, down to 2^10 words with one an SM; smaller vectors
+// take the plain form, whose launches are bound by latency. Round w of 2^w-word chunks divides by
+// the chunks' weights, and has to be a device round: round L - TAIL_LOG is the last one.
+inline uint32_t zc_weighted_lo_bits(uint64_t live_words, uint32_t L, uint64_t sms) {
+  if ((live_words >> 12) >= 4 * sms && 12 + TAIL_LOG <= L) return 12;
+  if ((live_words >> 11) >= 4 * sms && 11 + TAIL_LOG <= L) return 11;
+  return (live_words >> 10) >= sms && 10 + TAIL_LOG <= L ? 10 : 0;
+}
+
 // ------------------------------------------------------------------ the jagged assist
 constexpr uint32_t AS_BUILD_THREADS = 512;
 inline uint32_t as_build_blocks(uint64_t n, uint64_t sms) {

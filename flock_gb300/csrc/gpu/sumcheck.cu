@@ -666,14 +666,6 @@ zc_fold_skip_weighted_kernel(const F128d* __restrict__ a, const F128d* __restric
   if (threadIdx.x == 0) { part[blockIdx.x * 2] = G1; part[blockIdx.x * 2 + 1] = GI; }
   publish_if_last(part, 2, pub, sh);
 }
-// A chunk's tables are rebuilt for it (about 2000 cycles beside 13 a word), so chunks are as
-// long as leaves every SM four, down to 2^10 words with one an SM; smaller vectors take the
-// plain form, whose launches are bound by latency.
-uint32_t zc_weighted_lo_bits(uint64_t live_words, uint64_t sms) {
-  if ((live_words >> 12) >= 4 * sms) return 12;
-  if ((live_words >> 11) >= 4 * sms) return 11;
-  return (live_words >> 10) >= sms ? 10 : 0;
-}
 template <int LO>
 static uint32_t fold_skip_weighted(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words,
                                    const F128d* eq_lo, const F128d* h, F128d* part, cudaStream_t s, FusedPublish pub) {

@@ -34,7 +34,25 @@ static void fold_partials_fit() {
           }
 }
 
+// The weighted zerocheck's division (round w) is a device round: the fold that leaves the host's
+// tail of 2^TAIL_LOG entries, round L - TAIL_LOG, or one before it.
+static void division_before_the_tail() {
+  for (uint64_t sms = 1; sms <= 200; ++sms)
+    for (uint32_t L = 10; L <= 28; ++L)
+      for (uint64_t live = uint64_t(1) << (L - 1); live <= uint64_t(1) << L; live += uint64_t(1) << (L - 5)) {
+        const uint32_t w = zc_weighted_lo_bits(live, L, sms);
+        expect(w == 0 || (w >= 10 && w <= 12 && w + TAIL_LOG <= L), "weighted rounds: SMs, L", sms, L);
+      }
+  // the whole part's choices: BLAKE3 2^10 and 2^11, Keccak-f 2^9, SHA-256 2^13, Keccak-f 2^13
+  expect(zc_weighted_lo_bits(92 << 10, 17, 152) == 0, "plain", 17, 152);
+  expect(zc_weighted_lo_bits(92 << 11, 18, 152) == 10, "chunks of 2^10", 18, 152);
+  expect(zc_weighted_lo_bits(333 << 9, 18, 152) == 10, "chunks of 2^10", 18, 152);
+  expect(zc_weighted_lo_bits(199 << 13, 21, 152) == 11, "chunks of 2^11", 21, 152);
+  expect(zc_weighted_lo_bits(333 << 13, 22, 152) == 12, "chunks of 2^12", 22, 152);
+}
+
 int main() {
+  division_before_the_tail();
   assist_partials_fit();
   fold_partials_fit();
   printf("failures %d\n", failures);
