@@ -620,16 +620,15 @@ void GpuBackend::zc_round1(const std::vector<F128>& r, std::vector<F128>& ab, st
     if (r[6 + i] != fixed[i]) throw std::runtime_error("zerocheck round 1 expects the fixed challenges at r[6..13)");
   std::vector<F128> outer(r.begin() + 13, r.end());
   EqSplit e = eq_split(outer, F128::one(), 10);
-  uint32_t nab = 0, nsvc = 0;
+  uint32_t nrows = 0;
   F128d* part_svc = part_ + part_cap_ / 2;
   {
     Mark mk(this, ST_ZC_ROUND1);
-    launch_zc_round1(a_, b_, z_, m, zc_live_words_, e.lo, e.lo_bits, e.hi, zc2a_, part_, &nab, part_svc, &nsvc, st_);
+    launch_zc_round1(a_, b_, z_, m, zc_live_words_, e.lo, e.lo_bits, e.hi, zc2a_, part_, part_svc, part_cap_ / 2,
+                     &nrows, st_);
   }
-  if ((uint64_t)nab * 64 > part_cap_ / 2 || (uint64_t)nsvc * 128 > part_cap_ / 2)
-    throw std::runtime_error("round-1 partials exceed the partials buffer");
   const FusedPublish fp = fused_publish();
-  launch_reduce_pair(part_, nab, 64, part_svc, nsvc, 128, st_, fp);
+  launch_reduce_pair(part_, nrows, 64, part_svc, nrows, 128, st_, fp);
   auto v = read_published(fp.seq, 192, true);
   // D = prod (1 + g_i)^-1 over the medium constants' g_i = x^1, x^2, x^4, x^8
   static const F128 D = [] {
@@ -1013,7 +1012,7 @@ std::vector<F128> GpuBackend::lane_dots(const std::vector<F128>& point) {
   scr_off_ = 0;
   EqSplit e = eq_split(std::vector<F128>(point.begin(), point.begin() + S.log_dim), F128::one(), 10);
   uint32_t nb;
-  { Mark mk(this, ST_LIGERITO); nb = launch_lg_lane_dots(q_, S.lanes, S.log_dim, e.lo, e.lo_bits, e.hi, part_, st_); }
+  { Mark mk(this, ST_LIGERITO); nb = launch_lg_lane_dots(q_, S.lanes, S.log_dim, e.lo, e.lo_bits, e.hi, part_, part_cap_, st_); }
   std::vector<F128> h = reduce(nb, S.lanes);
   h.resize(lanes_pow2());  // the lanes past the committed ones are zero
   return h;

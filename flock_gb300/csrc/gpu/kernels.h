@@ -80,12 +80,13 @@ void launch_reduce_pair(const F128d* pa, uint32_t na, uint32_t wa, const F128d* 
 
 // unit[64 s + i]: extension of row bit s at Lambda point i; wconst, pconst: see ZcConsts.
 void upload_zc_consts(const uint8_t* unit, const F128d* wconst, const F128d* pconst);
-// Round-1 partials: P_ab rows of width 64 into part_ab, s_hat_v_c rows of width 128 into part_svc.
+// Round-1 partials: *nrows rows of P_ab of width 64 into part_ab, as many of s_hat_v_c of width 128
+// into part_svc, each array with room for part_room entries (checked before the launches).
 // Words of z, a and b from live_words on are zero (the zero tail of a single slot's chunk
 // columns) and are not read. g: 2^(m - 7) words of scratch.
 void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m, uint64_t live_words,
                       const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* g, F128d* part_ab,
-                      uint32_t* nrows_ab, F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s);
+                      F128d* part_svc, uint64_t part_room, uint32_t* nrows, cudaStream_t s);
 uint32_t launch_zc_fold_skip(const F128d* a, const F128d* b, const F128d* w64, uint64_t n_words, const F128d* eq_lo,
                              uint32_t lo_bits, const F128d* eq_hi, F128d* part, cudaStream_t s, FusedPublish pub);       // width 2
 // First multilinear fold (at rho) of the skip-folded a, b, computed from the bits; writes
@@ -173,7 +174,7 @@ void launch_as_build(const F128d* er0, const F128d* ec0, const F128d* er1, const
 // partial rows of width `lanes` (returned), the fold of every lane by lambda into lane_fold_groups(lanes, D) partial rows of D entries,
 // and the switched vectors with their message.
 uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, uint32_t lo_bits,
-                             const F128d* eq_hi, F128d* part, cudaStream_t s);
+                             const F128d* eq_hi, F128d* part, uint64_t part_room, cudaStream_t s);
 uint32_t lane_fold_groups(uint32_t lanes, uint64_t D, uint64_t sms);
 void launch_lg_lane_fold(const F128d* q, const F256d* lambda, uint32_t lanes, uint64_t D, F256d* part, cudaStream_t s);
 // b = sum of n terms coef eq(point), each point's eq as lo (lo_bits) x hi tables.

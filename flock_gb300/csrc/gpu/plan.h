@@ -9,6 +9,38 @@ namespace gpu {
 
 constexpr uint32_t PART_ENTRIES = 1u << 20;  // a backend's buffer of per-block partials
 
+// ------------------------------------------------------------------ bit sums
+constexpr uint32_t BITS_THREADS = 512, BITS_WARPS = BITS_THREADS / 32;
+constexpr uint32_t BITS_MAX_SPLITS = 1024;  // partial rows of round 1 and of the lane dots
+// Columns per warp and row splits: the pair of least time, for blocks that cost about 105 cycles a
+// tile and column slot (used or not), 700 for the tile's tables and 6000 + 4000 a column slot of
+// the warp for its start and end (the latter is what counts where there are few rows), one block
+// per SM at a time; at most max_splits partial rows and at least a tile each.
+struct BitSumPlan {
+  uint32_t cpw, groups, splits;
+  uint64_t rows_per_split;
+};
+inline BitSumPlan bit_sum_plan(uint32_t n_cols, uint64_t n_rows, uint64_t max_splits, uint64_t sms) {
+  BitSumPlan p{};
+  const uint64_t tiles = (n_rows + 31) / 32;
+  max_splits = std::max<uint64_t>(1, std::min(max_splits, tiles));
+  uint64_t best = ~0ull;
+  for (uint32_t cpw = 1; cpw <= 4; ++cpw) {
+    const uint32_t groups = (n_cols + BITS_WARPS * cpw - 1) / (BITS_WARPS * cpw);
+    for (uint64_t waves = 1; waves <= 4; ++waves) {
+      const uint64_t want = std::min(max_splits, std::max<uint64_t>(1, waves * sms / groups));
+      const uint64_t per = (tiles + want - 1) / want, splits = (tiles + per - 1) / per;
+      const uint64_t used = (splits * groups + sms - 1) / sms;
+      const uint64_t cost = used * (per * (105 * BITS_WARPS * cpw + 700) + 4000 * cpw + 6000);
+      if (cost < best) {
+        best = cost;
+        p = {cpw, groups, (uint32_t)splits, per * 32};
+      }
+    }
+  }
+  return p;
+}
+
 // ------------------------------------------------------------------ pair folds
 // Folds of at least this many pairs take the table form (see the kernels in sumcheck.cu).
 constexpr uint64_t PAIR_FOLD_TABLE_MIN_PAIRS = uint64_t(1) << 17;

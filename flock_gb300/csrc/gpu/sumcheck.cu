@@ -123,7 +123,7 @@ enum BitSumOut : int {
   BITS_POINTS,   // the words of zc_round1_bits: part[(split * groups + group) * 64 + i] = the group's share of
                  // sum_{M, bit} weight[8 M + bit] U at point i
 };
-constexpr uint32_t BITS_THREADS = 512, BITS_WARPS = BITS_THREADS / 32, BITS_EQ_ROWS = 512;
+constexpr uint32_t BITS_EQ_ROWS = 512;
 constexpr uint32_t BITS_TABLE_BYTES = (2 * 128 + 3 * 64) * 128;
 // Warp-wide 32 x 32 bit transpose: lane r holds word x_r; afterwards lane c holds the word
 // whose bit r is bit c of x_r (five exchange stages of halving block size).
@@ -290,34 +290,6 @@ bit_sums_kernel(const F128d* __restrict__ z, uint64_t col_stride, uint64_t row_s
       part[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * 128 + threadIdx.x] = a;
     }
   }
-}
-// Columns per warp and row splits: the pair of least time, for blocks that cost about 105 cycles a
-// tile and column slot (used or not), 700 for the tile's tables and 6000 + 4000 a column slot of
-// the warp for its start and end (the latter is what counts where there are few rows), one block
-// per SM at a time; at most max_splits partial rows and at least a tile each.
-struct BitSumPlan {
-  uint32_t cpw, groups, splits;
-  uint64_t rows_per_split;
-};
-static BitSumPlan bit_sum_plan(uint32_t n_cols, uint64_t n_rows, uint64_t max_splits) {
-  BitSumPlan p{};
-  const uint64_t tiles = (n_rows + 31) / 32, sms = (uint64_t)sm_count();
-  max_splits = std::max<uint64_t>(1, std::min(max_splits, tiles));
-  uint64_t best = ~0ull;
-  for (uint32_t cpw = 1; cpw <= 4; ++cpw) {
-    const uint32_t groups = (n_cols + BITS_WARPS * cpw - 1) / (BITS_WARPS * cpw);
-    for (uint64_t waves = 1; waves <= 4; ++waves) {
-      const uint64_t want = std::min(max_splits, std::max<uint64_t>(1, waves * sms / groups));
-      const uint64_t per = (tiles + want - 1) / want, splits = (tiles + per - 1) / per;
-      const uint64_t used = (splits * groups + sms - 1) / sms;
-      const uint64_t cost = used * (per * (105 * BITS_WARPS * cpw + 700) + 4000 * cpw + 6000);
-      if (cost < best) {
-        best = cost;
-        p = {cpw, groups, (uint32_t)splits, per * 32};
-      }
-    }
-  }
-  return p;
 }
 template <int CPW, int OUT>
 static void bit_sums_cpw(const BitSumPlan& p, const F128d* z, uint64_t col_stride, uint64_t row_stride, uint32_t n_cols,
@@ -518,21 +490,22 @@ void upload_zc_consts(const uint8_t* unit, const F128d* wconst, const F128d* pco
 
 void launch_zc_round1(const F128d* a, const F128d* b, const F128d* z, uint32_t m, uint64_t live_words,
                       const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, F128d* g, F128d* part_ab,
-                      uint32_t* nrows_ab, F128d* part_svc, uint32_t* nrows_svc, cudaStream_t s) {
+                      F128d* part_svc, uint64_t part_room, uint32_t* nrows, cudaStream_t s) {
   const ZcConsts* consts = zc_consts();
   if (!consts) throw std::runtime_error("zerocheck constants not uploaded");
   // xo past the live words hold zero rows of z, a and b and add nothing to any sum
   const uint64_t xo_live = std::min<uint64_t>(1ull << (m - 13), (live_words + 63) / 64);
+  const BitSumPlan p = bit_sum_plan(64, xo_live, BITS_MAX_SPLITS, (uint64_t)sm_count());
+  if (uint64_t(p.groups) * p.splits * 128 > part_room) throw std::runtime_error("round-1 partials exceed the partials buffer");
   set_dynamic_smem((const void*)zc_round1_bits_kernel, (int)ZC_EXT_BYTES);
   // one block per SM; xo are dealt to the blocks first, then to their warps
   const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(xo_live, (uint64_t)sm_count()));
   zc_round1_bits_kernel<<<blocks, ZC_R1_THREADS, ZC_EXT_BYTES, s>>>(a, b, xo_live, consts, reinterpret_cast<uint4*>(g));
   LAUNCH_OK();
   // both outer sums: 64 words an xo, rows = xo
-  const BitSumPlan p = bit_sum_plan(64, xo_live, 1024);
   bit_sums<BITS_POINTS>(p, g, 1, 64, 64, xo_live, eq_lo, lo_bits, eq_hi, consts->pconst, part_ab, s);
   bit_sums<BITS_COLUMNS>(p, z, 1, 64, 64, xo_live, eq_lo, lo_bits, eq_hi, consts->wconst, part_svc, s);
-  *nrows_ab = *nrows_svc = p.groups * p.splits;
+  *nrows = p.groups * p.splits;
 }
 
 // ------------------------------------------------------------------ zerocheck skip fold
@@ -1239,7 +1212,7 @@ void launch_lc_zvec(const F128d* z, uint32_t nu, uint32_t used_chunks, const F12
                     const F128d* eq_hi, F128d* part, uint64_t part_cap, uint32_t K, F128d* zv, F128d* captured,
                     cudaStream_t s) {
   const uint64_t rows = 1ull << nu;
-  const BitSumPlan p = bit_sum_plan(used_chunks, rows, part_cap / (used_chunks * 128ull));
+  const BitSumPlan p = bit_sum_plan(used_chunks, rows, part_cap / (used_chunks * 128ull), (uint64_t)sm_count());
   bit_sums<BITS_RAW>(p, z, rows, 1, used_chunks, rows, eq_lo, lo_bits, eq_hi, nullptr, part, s);
   lc_zvec_reduce_kernel<<<(K + 127) / 128, 128, 0, s>>>(part, p.splits, used_chunks * 128, K, zv, captured);
   LAUNCH_OK();
@@ -1514,9 +1487,10 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
 
 // Lane dots h[l] = sum_p q[l D + p] eq(p), as rows of `lanes` partials.
 uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, uint32_t lo_bits,
-                             const F128d* eq_hi, F128d* part, cudaStream_t s) {
+                             const F128d* eq_hi, F128d* part, uint64_t part_room, cudaStream_t s) {
   const uint64_t rows = 1ull << log_d;
-  const BitSumPlan p = bit_sum_plan(lanes, rows, 1024);
+  const BitSumPlan p = bit_sum_plan(lanes, rows, BITS_MAX_SPLITS, (uint64_t)sm_count());
+  if (uint64_t(p.splits) * lanes > part_room) throw std::runtime_error("lane dots exceed the partials buffer");
   bit_sums<BITS_DOT>(p, q, rows, 1, lanes, rows, eq_lo, lo_bits, eq_hi, nullptr, part, s);
   return p.splits;
 }

@@ -51,7 +51,25 @@ static void division_before_the_tail() {
   expect(zc_weighted_lo_bits(333 << 13, 22, 152) == 12, "chunks of 2^12", 22, 152);
 }
 
+// The bit sums' partials: round 1 (64 columns, half of the buffer for 128 a row), the lane dots (up to
+// 64 lanes), the lincheck's row fold (as many splits as the buffer has room for).
+static void bit_sums_fit() {
+  for (uint64_t sms = 1; sms <= 200; ++sms)
+    for (uint32_t k = 0; k <= 26; ++k)
+      for (uint64_t rows : {uint64_t(1) << k, (uint64_t(1) << k) + (uint64_t(1) << k / 2) + 1}) {
+        const BitSumPlan r1 = bit_sum_plan(64, rows, BITS_MAX_SPLITS, sms);
+        expect(uint64_t(r1.groups) * r1.splits * 128 <= PART_ENTRIES / 2, "round 1: SMs, rows", sms, rows);
+        for (uint32_t cols : {1u, 13u, 42u, 64u, 333u, 1024u}) {
+          const bool wide = cols > 64;
+          const BitSumPlan p = bit_sum_plan(cols, rows, wide ? PART_ENTRIES / (cols * 128ull) : BITS_MAX_SPLITS, sms);
+          expect(uint64_t(p.splits) * cols * (wide ? 128 : 1) <= PART_ENTRIES, "bit sums: SMs, rows", sms, rows);
+          expect(p.splits * p.rows_per_split >= rows && uint64_t(p.groups) * p.cpw * BITS_WARPS >= cols, "cover: SMs, rows", sms, rows);
+        }
+      }
+}
+
 int main() {
+  bit_sums_fit();
   division_before_the_tail();
   assist_partials_fit();
   fold_partials_fit();
