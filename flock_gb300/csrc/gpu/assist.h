@@ -23,7 +23,7 @@ class JaggedAssist : public JaggedAssistOps {
   template <class T> T* alloc(size_t n);
   const void* upload(const void* src, size_t bytes);
   FusedPublish publish();
-  void read(const FusedPublish& p, F128& g1, F128& gi);
+  void read(const FusedPublish& p, bool stage, F128& g1, F128& gi);
 
   const Statement& S;
   int device_;

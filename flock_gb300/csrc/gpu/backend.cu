@@ -5,6 +5,7 @@
 // O(m)-sized arithmetic between rounds; every round message comes back as a handful of
 // field elements.
 #include "backend.h"
+#include "wait.h"
 #include "../host/tables.h"
 #include <atomic>
 #include <thread>
@@ -416,28 +417,14 @@ std::vector<F128> GpuBackend::read_published(uint32_t seq, uint32_t width, bool 
   d2h_ += width * sizeof(F128d) + sizeof(uint32_t);
   return out;
 }
-// Wait for the published sequence number (the stream keeps running; no synchronisation):
-// a short hot spin for the common case of a message a few microseconds away, then a spin
-// that yields the core on every pass, so that concurrent provers' host work (assists,
-// transcripts) is not starved by waiting threads. A round's message is reported as stalled after
-// 20 s; results of whole stages (caps, openings, round 1) are waited for as long as the stream runs.
+// Wait for the published sequence number (the stream keeps running; no synchronisation).
 void GpuBackend::wait_published(uint32_t seq, bool stage) { wait_flag(h_flag_, seq, st_, stage); }
 void GpuBackend::wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream, bool stage) {
-  const volatile uint32_t* f = flag;
-  uint64_t spins = 0;
-  double t0 = 0;
-  while (*f != seq) {
-    ++spins;
-    if (spins > 2048) std::this_thread::yield();
-    if ((spins & 0x3FFF) == 0) {
-      const cudaError_t e = cudaStreamQuery(stream);
-      if (e != cudaSuccess && e != cudaErrorNotReady) CUDA_OK(e);
-      const double t = now_ms();
-      if (t0 == 0 || (stage && e == cudaErrorNotReady)) t0 = t;
-      else if (t - t0 > 20000) throw std::runtime_error("device result not published within 20 s");
-    }
-  }
-  std::atomic_thread_fence(std::memory_order_acquire);
+  wait_published_flag(flag, seq, stage, ROUND_WAIT_MS, [&] {
+    const cudaError_t e = cudaStreamQuery(stream);
+    if (e != cudaSuccess && e != cudaErrorNotReady) CUDA_OK(e);
+    return e == cudaErrorNotReady;
+  });
 }
 // eq(point) split as lo (first lo_bits coordinates) x hi (rest, times scale).
 GpuBackend::EqSplit GpuBackend::eq_split(const std::vector<F128>& point, F128 scale, uint32_t max_lo) {

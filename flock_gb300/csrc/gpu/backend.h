@@ -56,8 +56,8 @@ class GpuBackend : public ProverBackend {
   PowSearchFn pow_search() override;
   // A statement that is not one full-height slot takes the general jagged assist.
   JaggedAssistOps* jagged_assist() override { return jagged_.get(); }
-  // Spin until the mapped flag holds seq (bounded: an error after 20 s, stream errors
-  // reported as they occur).
+  // Spin until the mapped flag holds seq; stream errors are reported as they occur. A round's
+  // message is an error after 20 s, a stage's result is waited for as long as the stream runs.
   static void wait_flag(const uint32_t* flag, uint32_t seq, cudaStream_t stream, bool stage = false);
   // Device-time breakdown of a prove (CUDA events on the backend's stream).
   enum Stage {

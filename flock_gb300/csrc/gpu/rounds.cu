@@ -271,8 +271,8 @@ FusedPublish JaggedAssist::publish() {
   p.seq = ++seq_;
   return p;
 }
-void JaggedAssist::read(const FusedPublish& p, F128& g1, F128& gi) {
-  GpuBackend::wait_flag(h_flag_, p.seq, st_, true);
+void JaggedAssist::read(const FusedPublish& p, bool stage, F128& g1, F128& gi) {
+  GpuBackend::wait_flag(h_flag_, p.seq, st_, stage);
   const volatile F128d* o = h_pub_;
   g1 = F128(o[0].lo, o[0].hi);
   gi = F128(o[1].lo, o[1].hi);
@@ -325,7 +325,7 @@ void JaggedAssist::build(const std::vector<RsClaimPoint>& claims, const std::vec
                   part_, st_, fp);
   cur_ = 0;
   len_ = n_;
-  read(fp, g1, gi);
+  read(fp, true, g1, gi);
 }
 
 void JaggedAssist::fold(F128 r, F128& g1, F128& gi) {
@@ -337,7 +337,7 @@ void JaggedAssist::fold(F128 r, F128& g1, F128& gi) {
                    fp);
   cur_ = nx;
   len_ /= 2;
-  read(fp, g1, gi);
+  read(fp, false, g1, gi);
 }
 
 }  // namespace gpu
