@@ -18,6 +18,9 @@ class JaggedAssist : public JaggedAssistOps {
   void build(const std::vector<RsClaimPoint>& claims, const std::vector<F128>& scale, const std::vector<F128>& rho,
              const std::vector<F128>& table, F128& g1, F128& gi) override;
   void fold(F128 r, F128& g1, F128& gi) override;
+  // Device bytes held, and the same without a device.
+  uint64_t device_bytes() const { return device_bytes_; }
+  static uint64_t estimate_device_bytes(const Statement& s, uint64_t sms);
 
  private:
   template <class T> T* alloc(size_t n);
@@ -29,6 +32,7 @@ class JaggedAssist : public JaggedAssistOps {
   int device_;
   cudaStream_t st_ = nullptr;
   std::vector<void*> owned_;
+  uint64_t device_bytes_ = 0;
   uint64_t n_ = 0;                               // dense words 2^m
   F128d *a_[3] = {}, *g_[3] = {};                // n, n/2 and n/4 entries: fold 0 -> 1 -> 2 -> 1 ...
   int cur_ = 0;
@@ -40,6 +44,8 @@ class JaggedAssist : public JaggedAssistOps {
   uint32_t *h_flag_ = nullptr, *d_flag_ = nullptr, *counter_ = nullptr, seq_ = 0;
 };
 
+// A statement that is not one full-height slot takes the assist.
+inline bool takes_jagged_assist(const Statement& s) { return s.slots.size() != 1 || !s.identity; }
 // The committed stack of a union as slot segments (at most four non-empty slots).
 JaggedSegs jagged_segs(const Statement& S);
 

@@ -140,6 +140,7 @@ uint64_t GpuBackend::estimate_device_bytes(const Statement& S) {
     b += bl * (uint64_t(1) << k) * 16 + 2 * bl * 32 + bl * 16;
     split_dim = (split_dim - k) + 1;
   }
+  if (takes_jagged_assist(S)) b += JaggedAssist::estimate_device_bytes(S, GB300_SMS);
   return b;
 }
 
@@ -252,7 +253,10 @@ GpuBackend::GpuBackend(const Statement& s) : S(s) {
   // twiddles of the L0 transform; host tables used by every prove
   tw0_ = twiddles(S.k_code);
   (void)moore_inverse();
-  if (S.slots.size() != 1 || !S.identity) jagged_ = std::make_unique<JaggedAssist>(S, device_);
+  if (takes_jagged_assist(S)) {
+    jagged_ = std::make_unique<JaggedAssist>(S, device_);
+    device_bytes_ += jagged_->device_bytes();
+  }
   CUDA_OK(cudaDeviceSynchronize());
 }
 

@@ -209,8 +209,23 @@ template <class T>
 T* JaggedAssist::alloc(size_t n) {
   void* p = nullptr;
   CUDA_OK(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)));
+  device_bytes_ += std::max<size_t>(n, 1) * sizeof(T);
   owned_.push_back(p);
   return static_cast<T*>(p);
+}
+
+// The largest call stages the points of 128 twists, every run and its weights.
+static size_t assist_stage_bytes(const Statement& s) { return (size_t(1) << 18) + (size_t(48) << s.geo.col_log); }
+constexpr uint32_t ASSIST_OUT = 256;  // dual values: two claims at 128 points
+
+uint64_t JaggedAssist::estimate_device_bytes(const Statement& s, uint64_t sms) {
+  const uint64_t n = s.committed_words;
+  const uint32_t m = s.geo.dense_m - 7, lo = std::min(m, EQ_LO);
+  uint64_t words = 0;
+  for (int k = 0; k < 3; ++k) words += 2 * (n >> k);
+  words += 2 * ((uint64_t(1) << s.nu) + (uint64_t(1) << s.geo.col_log)) + (uint64_t(1) << lo) + (uint64_t(1) << (m - lo));
+  words += assist_partials(n, sms) + ASSIST_OUT;
+  return words * sizeof(F128d) + sizeof(uint32_t) + assist_stage_bytes(s);
 }
 
 JaggedAssist::JaggedAssist(const Statement& s, int device) : S(s), device_(device) {
@@ -228,14 +243,13 @@ JaggedAssist::JaggedAssist(const Statement& s, int device) : S(s), device_(devic
   eq_lo_ = alloc<F128d>(size_t(1) << lo);
   eq_hi_ = alloc<F128d>(size_t(1) << (m - lo));
   part_ = alloc<F128d>(assist_partials(n_, (uint64_t)sm_count()));
-  out_ = alloc<F128d>(256);
+  out_ = alloc<F128d>(ASSIST_OUT);
   counter_ = alloc<uint32_t>(1);
   CUDA_OK(cudaMemsetAsync(counter_, 0, sizeof(uint32_t), st_));
-  // the largest call stages the points of 128 twists, every run and its weights
-  stage_cap_ = (size_t(1) << 18) + (size_t(48) << S.geo.col_log);
+  stage_cap_ = assist_stage_bytes(S);
   d_stage_ = alloc<uint8_t>(stage_cap_);
   CUDA_OK(cudaMallocHost(&h_stage_, stage_cap_));
-  CUDA_OK(cudaMallocHost(&h_out_, 256 * sizeof(F128d)));
+  CUDA_OK(cudaMallocHost(&h_out_, ASSIST_OUT * sizeof(F128d)));
   CUDA_OK(cudaHostAlloc(&h_pub_, 2 * sizeof(F128d), cudaHostAllocMapped));
   CUDA_OK(cudaHostGetDevicePointer(&d_pub_, h_pub_, 0));
   CUDA_OK(cudaHostAlloc(&h_flag_, 64, cudaHostAllocMapped));
@@ -283,7 +297,7 @@ void JaggedAssist::dual_values(const std::vector<AssistStatement>& unit, const s
   CUDA_OK(cudaSetDevice(device_));  // the assist's thread
   stage_off_ = 0;
   const size_t nc = unit.size(), np = points.size(), nr = unit[0].w.size(), n = unit[0].z_row.size();
-  if (nc * np > 256) throw std::runtime_error("assist: too many dual values");
+  if (nc * np > ASSIST_OUT) throw std::runtime_error("assist: too many dual values");
   std::vector<F128> zr, pt, w;
   for (const AssistStatement& u : unit) {
     if (u.t != unit[0].t) throw std::runtime_error("assist: the claims' boundary runs differ");
