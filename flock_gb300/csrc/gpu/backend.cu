@@ -53,7 +53,6 @@ void upload_constants_once() {
 
 inline F128d dev(F128 v) { F128d r; r.lo = v.lo; r.hi = v.hi; return r; }
 inline F256d dev(F256 v) { F256d r; r.c0 = dev(v.c0); r.c1 = dev(v.c1); return r; }
-inline F128 host(F128d v) { return F128(v.lo, v.hi); }
 
 }  // namespace
 
@@ -1212,7 +1211,7 @@ void GpuBackend::lg_flush_fold() {
   const int nx = lg_cur_ ^ 1;
   {
     Mark mk(this, ST_LIGERITO);
-    launch_lg_fold256(lf_[lg_cur_], lb_[lg_cur_], n_out, dev(lg_pend_fold_.r), nullptr, lg_pend_fold_.d, lf_[nx], lb_[nx],
+    launch_lg_fold256(lf_[lg_cur_], lb_[lg_cur_], n_out, dev(lg_pend_fold_.r), lg_pend_fold_.d, lf_[nx], lb_[nx],
                       st_);
   }
   lg_cur_ = nx;

@@ -40,8 +40,8 @@ constexpr uint64_t GB300_SMS = 152;  // for sizes computed without a device
 
 // In-kernel publication of a round message: the last block to finish (a device-wide
 // ticket counter) XOR-reduces every block's partials, writes the message to mapped host
-// memory and then the sequence number, as launch_reduce_publish does in a launch of its
-// own. counter must be zero before the launch; the last block resets it.
+// memory and then the sequence number, on which the host waits instead of on a copy and a stream
+// synchronisation. counter must be zero before the launch; the last block resets it.
 struct FusedPublish {
   F128d* out = nullptr;        // mapped host memory (null: no publication)
   uint32_t* flag = nullptr;    // mapped host memory
@@ -190,7 +190,7 @@ uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64
                               FusedPublish pub = FusedPublish());
 uint32_t launch_lg_fold_msg256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, uint64_t d_fold, uint64_t d_msg,
                                F256d* fo, F256d* bo, F128d* part, cudaStream_t s, FusedPublish pub);  // width 4
-void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, const F256d* r_dev, uint64_t d,
+void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, uint64_t d,
                        F256d* fo, F256d* bo, cudaStream_t s);
 void launch_lg_code_switch(const F256d* f, const F256d* b, uint64_t n, F256d* fo, F256d* bo, cudaStream_t s);
 // The code switch and the round message over the switched vectors with pairs one apart,
@@ -214,10 +214,6 @@ uint32_t launch_lg_induced(const uint64_t* pos, const F128d* w, uint32_t n_q, co
 void launch_lg_glue(F256d* b, const F128d* p, F128d w0, F128d w1, uint64_t n, bool induced, cudaStream_t s);
 
 // rounds.cu
-// XOR-reduce width-wide partials with one block and publish the sums to mapped host
-// memory, then set *flag = seq (after a system-scope fence).
-void launch_reduce_publish(const F128d* part, uint32_t nb, uint32_t width, F128d* out_mapped, uint32_t* flag_mapped,
-                           uint32_t seq, cudaStream_t s);
 struct EqDesc {
   uint32_t p_off, n;   // coordinates point[p_off .. p_off + n)
   uint64_t out_off;    // first entry in the output

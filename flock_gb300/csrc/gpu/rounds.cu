@@ -1,45 +1,12 @@
-// Round messages published straight into mapped host memory (the host waits on a sequence
-// flag instead of a stream synchronisation and a device-to-host copy), the eq tables of many
-// rounds, and the multipoint assist over a general jagged layout (union proofs): the dual
-// values by the branching-program DP, and the two materialised vectors of its sumcheck with the
-// first message; the rounds after it are pair_fold launches.
+// The eq tables of many rounds in one launch, and the multipoint assist over a general jagged layout
+// (union proofs): the dual values by the branching-program DP, and the two materialised vectors of
+// its sumcheck with the first message; the rounds after it are pair_fold launches.
 #include "assist.h"
 #include "backend.h"
 #include "reduce.cuh"
 
 namespace flock {
 namespace gpu {
-
-__global__ void reduce_publish_kernel(const F128d* __restrict__ part, uint32_t nb, uint32_t width,
-                                      volatile F128d* out, volatile uint32_t* flag, uint32_t seq) {
-  __shared__ F128d sh[32];
-  for (uint32_t j = 0; j < width; ++j) {
-    F128d acc = f128_zero();
-    for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) acc += part[(uint64_t)b * width + j];
-    acc = warp_xor(acc);
-    const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncthreads();
-    if (l == 0) sh[w] = acc;
-    __syncthreads();
-    if (w == 0) {
-      F128d r = l < nw ? sh[l] : f128_zero();
-      r = warp_xor(r);
-      if (l == 0) {
-        out[j].lo = r.lo;
-        out[j].hi = r.hi;
-      }
-    }
-  }
-  if (threadIdx.x == 0) {
-    __threadfence_system();
-    *flag = seq;
-  }
-}
-void launch_reduce_publish(const F128d* part, uint32_t nb, uint32_t width, F128d* out_mapped, uint32_t* flag_mapped,
-                           uint32_t seq, cudaStream_t s) {
-  reduce_publish_kernel<<<1, 256, 0, s>>>(part, nb, width, out_mapped, flag_mapped, seq);
-  LAUNCH_OK();
-}
 
 // Several eq tables in one launch: table k = eq(point[off_k .. off_k + n_k)) at out +
 // out_k. A block works on one table's entries [entry, entry + EQ_DESC_ENTRIES).

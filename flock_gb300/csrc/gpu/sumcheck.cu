@@ -1591,19 +1591,17 @@ uint32_t launch_lg_message256(const F256d* f, const F256d* b, uint64_t n, uint64
   return blocks;
 }
 __global__ void lg_fold256_kernel(const F256d* __restrict__ f, const F256d* __restrict__ b, uint64_t n_out, F256d r,
-                                  const F256d* __restrict__ r_dev, uint32_t d_log, F256d* __restrict__ fo,
-                                  F256d* __restrict__ bo) {
+                                  uint32_t d_log, F256d* __restrict__ fo, F256d* __restrict__ bo) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_out) return;
   const uint64_t lo = pair_lo(i, d_log), hi = lo + (1ull << d_log);
   F256d f0 = f[lo], b0 = b[lo];
-  const F256d rv = r_dev ? *r_dev : r;
-  fo[i] = f0 + f256_mul_call(rv, f[hi] + f0);
-  bo[i] = b0 + f256_mul_call(rv, b[hi] + b0);
+  fo[i] = f0 + f256_mul_call(r, f[hi] + f0);
+  bo[i] = b0 + f256_mul_call(r, b[hi] + b0);
 }
-void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, const F256d* r_dev, uint64_t d,
+void launch_lg_fold256(const F256d* f, const F256d* b, uint64_t n_out, F256d r, uint64_t d,
                        F256d* fo, F256d* bo, cudaStream_t s) {
-  lg_fold256_kernel<<<(unsigned)((n_out + 255) / 256), 256, 0, s>>>(f, b, n_out, r, r_dev, log2_distance(d), fo, bo);
+  lg_fold256_kernel<<<(unsigned)((n_out + 255) / 256), 256, 0, s>>>(f, b, n_out, r, log2_distance(d), fo, bo);
   LAUNCH_OK();
 }
 // One round's fold (at r, pairs d_fold apart) fused with the next round's message over the
