@@ -421,7 +421,7 @@ def measure(wl, args, world, rank, local):
             roof["mul_pipe"] = {"achieved": rate, "peak": mix_peak, "unit": "F128 mul/s", "frac": rate / mix_peak,
                                 "algorithmic_muls": muls,
                                 "peak_source": "measured live: flock_gb300_f128_table_mix_rate (products by a block "
-                                               "constant, half from shared-memory byte tables, half integer-multiply)",
+                                               "constant, three in four from a shared-memory window table, one integer-multiply)",
                                 "peak_multiply_only": mul_peak,
                                 "frac_of_multiply_only": rate / mul_peak}
     if rank != 0:
