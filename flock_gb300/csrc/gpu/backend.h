@@ -51,7 +51,7 @@ class GpuBackend : public ProverBackend {
   void lg_open(uint32_t level, const std::vector<uint64_t>& positions, uint32_t cap_depth,
                std::vector<std::vector<F128>>& rows, std::vector<Hash>& paths) override;
   std::vector<F256> lg_residual() override;
-  // Proof-of-work searches of 6 or more bits run on the device (own stream, thread-safe:
+  // Proof-of-work searches of 9 or more bits run on the device (own stream, thread-safe:
   // the forked multipoint transcript grinds concurrently with the main one).
   PowSearchFn pow_search() override;
   // A statement that is not one full-height slot takes the general jagged assist.

@@ -204,7 +204,7 @@ bool lg_intro_eq_direct(uint64_t pairs);
 void launch_lg_intro_eq(const F256d* f, const F128d* point, uint32_t n_vars, uint64_t pairs, F128d* pend, F128d* part,
                         cudaStream_t s, FusedPublish pub);
 void launch_lg_intro_eq(const F256d* f, const F128d* eq_lo, uint32_t lo_bits, const F128d* eq_hi, uint64_t pairs,
-                        F128d* pend, F128d* part, cudaStream_t s, FusedPublish pub);  // width 3
+                        F128d* pend, F128d* part, cudaStream_t s, FusedPublish pub);  // width 2
 // pos and w in order of pos >> lg_sparse_layers(...), start[g] the first query of group g (one
 // value of that; start[n_groups] = n_q); without sparse layers start is not read.
 uint32_t lg_sparse_layers(uint32_t log_d, uint32_t log_rate);

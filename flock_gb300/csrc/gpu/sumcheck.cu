@@ -1482,8 +1482,9 @@ uint32_t launch_mo_build_w(const F128d* q, const F128d* er0, const F128d* ec0, c
 //   f[p] = sum_l lambda_l q[l D + p],  lambda = eq(challenges) in F256,
 // and the basis is sum_t e_t eq_t(p). This reads q once for the dots and once for the fold.
 // Forming the basis and folding both vectors challenge by challenge read and wrote them six
-// times: the whole Ligerito stage took 26.4 ms of a Keccak-f 2^18 proof (now 9.3), 4.8 ms of
-// SHA-256 2^16 (2.6), 0.94 ms of BLAKE3 2^12 (0.69; six kernels and round trips fewer).
+// times: the whole Ligerito stage took 26.4 ms of a Keccak-f 2^18 proof (9.3 with this stage, 8.0 with
+// the later changes to the levels), 4.8 ms of SHA-256 2^16 (2.6, 2.0), 0.94 ms of BLAKE3 2^12 (0.69,
+// 0.57; six kernels and round trips fewer).
 
 // Lane dots h[l] = sum_p q[l D + p] eq(p), as rows of `lanes` partials.
 uint32_t launch_lg_lane_dots(const F128d* q, uint32_t lanes, uint32_t log_d, const F128d* eq_lo, uint32_t lo_bits,
