@@ -10,7 +10,7 @@
 //
 // Admission is first fit over the queue in arrival order, with aging: a request that later
 // requests have overtaken MAX_BYPASS times becomes a barrier, and nothing behind it is
-// admitted until it is, so a large request (a Keccak-f 2^18 proof needs about 22 GB) is not
+// admitted until it is, so a large request (a Keccak-f 2^18 proof needs about 21 GiB) is not
 // starved by a stream of small ones. Statements (and their device-byte estimates) are
 // built by the submitting thread, and evicted backends are released by the worker that
 // evicted them after it leaves the engine lock, so neither a statement build nor a
